@@ -239,8 +239,12 @@ private:
         int64_t* rowptr = nullptr;
         int32_t* ci = nullptr;
         double* cv = nullptr;
-        double* rowabs = nullptr;
-        int64_t nnz = 0;
+        int64_t* fill = nullptr;      // the build's cursors, counts and unsorted entries
+        int* cnt = nullptr;
+        int32_t* ci2 = nullptr;
+        double* cv2 = nullptr;
+        int64_t cap = 0;              // entries the four entry arrays hold
+        int64_t nnz = -1;             // -1: no matrix yet
         double norm_inf = 0.0;
     } csr_;
     double* rbuf_ = nullptr;
