@@ -70,6 +70,8 @@ def load(int_kind=8):
         lib.spr_b200_autotune_tiles.restype = C.c_int
         lib.spr_b200_set_small_tile.argtypes = [vp, C.c_int]
         lib.spr_b200_set_small_tile.restype = C.c_int
+        lib.spr_b200_set_int_min.argtypes = [vp, C.c_double]
+        lib.spr_b200_set_int_min.restype = C.c_int
         lib.spr_b200_tc_stats.argtypes = [vp, vp]
         lib.spr_b200_tc_stats.restype = C.c_int
         lib.spr_b200_phase_ms.argtypes = [vp, vp]
@@ -378,6 +380,12 @@ class DeviceSolver:
 
     def set_small_tile(self, tile):
         self.lib.spr_b200_set_small_tile(self.h, int(tile))
+
+    def set_int_min(self, flops):
+        """FP64 mode: Schur-update launches of at least this many flops run on
+        the integer tensor cores (0 = all of them, inf = none)."""
+        if self.lib.spr_b200_set_int_min(self.h, float(flops)) != 0:
+            raise ValueError('bad flops %r' % (flops,))
 
     def tc_stats(self):
         """Mixed mode: (tensor-core update flops, their time in the last profiled factor, ms)."""

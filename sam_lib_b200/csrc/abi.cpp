@@ -1102,6 +1102,15 @@ int SPR_API(spr_b200_set_small_tile)(void* handle, int tile) {
     return 0;
 }
 
+// FP64 mode: the Schur updates of launches of at least this many flops run on
+// the integer tensor cores (0: all of the trailing and K = S updates;
+// infinity: none).
+int SPR_API(spr_b200_set_int_min)(void* handle, double flops) {
+    if (!handle || !(flops >= 0.0)) return -2;
+    static_cast<Engine*>(handle)->set_int_min(flops);
+    return 0;
+}
+
 // Mixed mode: out[0] = algorithmic flops of the updates that ran on tensor
 // cores in the last profiled factorisation (far trailing columns, the next
 // super-panels' columns and K = S updates above the tensor-core

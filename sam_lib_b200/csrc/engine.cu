@@ -135,6 +135,9 @@ struct PV {
     // node mask of a run split across GPUs: supernodes with skip[js] != 0 are
     // left alone (null: none)
     const uint8_t* skip;
+    // per equation (sign(d) sqrt|d|, its rounding error) of the large fronts'
+    // pivots, for the integer-digit updates (null: not wanted)
+    double* sqd;
 };
 
 struct Engine::Dev {
@@ -190,6 +193,11 @@ struct Engine::Dev {
     alignas(64) CUtensorMap slab_map;
     float* slab_far = nullptr;                   // slabs of the side-stream launches
     alignas(64) CUtensorMap slab_map_far;
+    // integer-digit updates: digit slabs, row scales, the TMA maps over the slabs
+    uint8_t* i8_slab = nullptr;
+    double* i8_scales = nullptr;
+    alignas(64) CUtensorMap i8_map_a, i8_map_b;
+    double* sqd = nullptr;                       // (sqrt|d| with d's sign, its rounding error) per equation
     cudaStream_t side = nullptr;                 // side stream: trailing updates beyond the next super-panel
     cudaStream_t ahead = nullptr;                // look-ahead stream: in-super-panel columns after the next panel
     cudaStream_t wbs = nullptr;                  // early writes of final super-panels to LNZ (streamed copies)
@@ -940,7 +948,15 @@ __global__ void __launch_bounds__(256) k_diag(const Job* jobs, PV P) {
             const int i = tx + 16 * a, j = ty + 16 * b;
             if (i >= j && i < nb && j < nb) front[(int64_t)(k0 + i) + (int64_t)(k0 + j) * ld] = A[i][j];
         }
-    if (tid < nb) P.dvec[fst + k0 + tid] = A[tid][tid];
+    if (tid < nb) {
+        const double d = A[tid][tid];
+        P.dvec[fst + k0 + tid] = d;
+        if (P.sqd) {
+            const double s = sqrt(fabs(d)), e = s > 0.0 ? fma(-s, s, fabs(d)) / (2.0 * s) : 0.0;
+            P.sqd[2 * (int64_t)(fst + k0 + tid)] = copysign(s, d);
+            P.sqd[2 * (int64_t)(fst + k0 + tid) + 1] = copysign(1.0, d) * e;
+        }
+    }
 }
 
 namespace gemm {
@@ -1271,6 +1287,7 @@ __device__ __forceinline__ void mma(float* c, const uint32_t* a, uint32_t b0, ui
 }  // namespace x3
 
 #include "tc_gemm.cuh"
+#include "i8_gemm.cuh"
 
 __global__ void __launch_bounds__(128) k_gemm_x3(const Job* jobs, int64_t njobs, const int32_t* tmap, PV P) {
     using namespace gemm;
@@ -2768,6 +2785,9 @@ Engine::~Engine() {
     if (d_->mbox) cudaFreeHost(d_->mbox);
     if (d_->slab) cudaFree(d_->slab);
     if (d_->slab_far) cudaFree(d_->slab_far);
+    if (d_->i8_slab) cudaFree(d_->i8_slab);
+    if (d_->i8_scales) cudaFree(d_->i8_scales);
+    if (d_->sqd) cudaFree(d_->sqd);
     for (void* p : {(void*)csr_.rowptr, (void*)csr_.fill, (void*)csr_.cnt, (void*)csr_.ci, (void*)csr_.cv,
                     (void*)csr_.ci2, (void*)csr_.cv2})
         cudaFree(p);
@@ -2897,7 +2917,19 @@ int Engine::open(const int64_t* mspar, const int64_t* mtrees, const int64_t* msi
     CK(cudaFuncSetAttribute(K_GEMM_TINY, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GemmTiny::smem));
     CK(cudaFuncSetAttribute(k_gemm_x3, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GemmSmall::smem));
     CK(cudaFuncSetAttribute(k_gemm_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc::kSmem));
+    CK(cudaFuncSetAttribute(k_gemm_i8, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)i8::kSmemI8));
+    set_int_min(i8_min_flops_);
     return 0;
+}
+
+void Engine::set_int_min(double flops) {
+    i8_min_flops_ = flops;
+    any_i8_ = false;
+    for (const LevelPlan& lp : P_.levels) {
+        for (size_t st = 0; st < lp.trail_i8.size(); ++st)
+            any_i8_ |= lp.trail_i8[st].gemm.ntasks > 0 && lp.next_flops[st] + lp.far_flops[st] >= flops;
+        any_i8_ |= !lp.outer_i8.empty() && lp.outer_flops >= flops;
+    }
 }
 
 // Operand slabs of the tensor-core updates and the 2-D TMA map over them:
@@ -2940,6 +2972,44 @@ int Engine::ensure_slabs() {
     return 0;
 }
 
+
+// Digit slabs of the integer updates: [i8_rows][128] bytes, one map with boxes of
+// 128 rows (row tiles) and one with 64 (column tiles), 128-byte swizzle.
+// Returns nonzero when they cannot be had.
+int Engine::ensure_i8() {
+    Dev& D = *d_;
+    if (D.i8_slab) return 0;
+    const int64_t rows = std::max<int64_t>(P_.i8_rows, i8::kM);
+    if (rows >= (int64_t(1) << 31)) return -3;                 // TMA row coordinates are 32-bit
+    void* fn = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q) != cudaSuccess || !fn)
+        return -4;
+    uint8_t* slab = nullptr;
+    if ((!D.sqd && cudaMalloc((void**)&D.sqd, P_.neq * 2 * sizeof(double)) != cudaSuccess) ||
+        (!D.i8_scales &&
+         cudaMalloc((void**)&D.i8_scales, std::max<int64_t>(P_.i8_scales, 1) * sizeof(double)) != cudaSuccess) ||
+        cudaMalloc((void**)&slab, rows * i8::kK) != cudaSuccess) {
+        cudaGetLastError();
+        return -4;
+    }
+    const cuuint64_t dims[2] = {(cuuint64_t)i8::kK, (cuuint64_t)rows};
+    const cuuint64_t strides[1] = {(cuuint64_t)i8::kK};
+    const cuuint32_t es[2] = {1, 1};
+    for (int m = 0; m < 2; ++m) {
+        const cuuint32_t box[2] = {(cuuint32_t)i8::kK, (cuuint32_t)(m == 0 ? i8::kM : i8::kN)};
+        const CUresult r = ((EncodeTiledFn)fn)(m == 0 ? &D.i8_map_a : &D.i8_map_b, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2,
+                                               slab, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                                               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                                               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        if (r != CUDA_SUCCESS) {
+            cudaFree(slab);
+            return -4;
+        }
+    }
+    D.i8_slab = slab;
+    return 0;
+}
 
 static cudaEvent_t record_event(cudaStream_t s) {
     cudaEvent_t e = nullptr;
@@ -2993,6 +3063,7 @@ static PV make_view(Engine::Dev& D, const Plan& P, double* d_sm, double tol1) {
     v.tc_drop = 0;
     v.adiag_in = nullptr;
     v.skip = D.skip_on ? D.skip : nullptr;
+    v.sqd = D.sqd;
     return v;
 }
 
@@ -3042,6 +3113,29 @@ void Engine::launch_tc(const TcLaunch& t, cudaStream_t s, const PV& pv, std::vec
                                                     t.gemm.ntasks, pv, far ? D.slab_map_far : D.slab_map);
     if (profile_) gev.push_back(record_event(s));
     timing.launches += 2;
+    ++timing.gemm_launches;
+}
+
+// The integer-digit form of an update: the panel's digits, then the products.
+void Engine::launch_i8_split(const I8Launch& t, cudaStream_t s, const PV& pv, std::vector<cudaEvent_t>& gev) {
+    if (profile_) gev.push_back(record_event(s));
+    k_split_i8<<<(int)t.split.ntasks, 256, 0, s>>>(d_->jobs + t.split.job_begin, t.split.job_count, TMAP(t.split), pv,
+                                                   d_->i8_slab, d_->i8_scales);
+    if (profile_) gev.push_back(record_event(s));
+    ++timing.launches;
+}
+
+void Engine::launch_i8_gemm(const Launch& l, cudaStream_t s, const PV& pv, std::vector<cudaEvent_t>& gev, bool far) {
+    if (l.ntasks <= 0) return;
+    Dev& D = *d_;
+    if (profile_) gev.push_back(record_event(s));
+    // a side-stream launch leaves SMs to the panel chain (one CTA holds an SM's shared memory)
+    const int cap = (far && !profile_) ? std::max(1, sm_count_ * i8_far_q_ / 8) : sm_count_;
+    const int grid = (int)std::min<int64_t>(l.ntasks, cap);
+    k_gemm_i8<<<grid, i8::kThreadsI8, i8::kSmemI8, s>>>(D.jobs + l.job_begin, l.job_count, TMAP(l), l.ntasks, pv,
+                                                        D.i8_scales, D.i8_map_a, D.i8_map_b);
+    if (profile_) gev.push_back(record_event(s));
+    ++timing.launches;
     ++timing.gemm_launches;
 }
 
@@ -3212,7 +3306,9 @@ void Engine::enqueue_factor(const PV& pv, cudaStream_t s, std::vector<cudaEvent_
             }
             const bool has_far = !lp.far[st].empty() || !lp.far_tc[st].empty();
             const bool far_tc = mixed_ == 1 && lp.far_flops[st] >= tc_min_flops_;
-            if (has_far && u != s) {
+            const bool trail_i8 = use_i8_ && lp.trail_i8[st].gemm.ntasks > 0 &&
+                                  lp.next_flops[st] + lp.far_flops[st] >= i8_min_flops_;
+            if (has_far && u != s && !trail_i8) {
                 // the super-panel is final: fork the far columns of its trailing update
                 cudaEvent_t e = D.evpool[evi++];
                 cudaEventRecord(e, s);
@@ -3250,7 +3346,17 @@ void Engine::enqueue_factor(const PV& pv, cudaStream_t s, std::vector<cudaEvent_
             // stay FP64 in both modes; in mixed mode the K = kSuperPanel one takes the
             // tensor cores when large enough.  They are issued first, the
             // look-ahead columns after them.
-            if (mixed_ == 1 && !lp.next_tc[st].empty() && lp.next_flops[st] >= tc_min_flops_) {
+            if (trail_i8) {
+                // one split serves both column ranges; the slabs are free again
+                // because the previous far update was joined above
+                launch_i8_split(lp.trail_i8[st], s, pv, gev);
+                if (has_far && u != s) {
+                    cudaEvent_t e = D.evpool[evi++];
+                    cudaEventRecord(e, s);
+                    cudaStreamWaitEvent(u, e, 0);
+                }
+                launch_i8_gemm(lp.trail_i8[st].gemm, s, pv, gev, false);
+            } else if (mixed_ == 1 && !lp.next_tc[st].empty() && lp.next_flops[st] >= tc_min_flops_) {
                 for (const TcLaunch& t : lp.next_tc[st]) launch_tc(t, s, pv, gev);
                 timing.tc_flops += lp.next_flops[st];
             } else {
@@ -3265,7 +3371,9 @@ void Engine::enqueue_factor(const PV& pv, cudaStream_t s, std::vector<cudaEvent_
                 }
             }
             if (has_far) {
-                if (far_tc) {
+                if (trail_i8) {
+                    launch_i8_gemm(lp.trail_i8[st].far, u, pv, gev, true);
+                } else if (far_tc) {
                     for (const TcLaunch& t : lp.far_tc[st]) launch_tc(t, u, pv, gev, true);
                     timing.tc_flops += lp.far_flops[st];
                 }
@@ -3284,6 +3392,11 @@ void Engine::enqueue_factor(const PV& pv, cudaStream_t s, std::vector<cudaEvent_
         if (mixed_ == 1 && lp.outer_flops >= tc_min_flops_) {
             for (const TcLaunch& t : lp.outer_tc) launch_tc(t, s, pv, gev);
             timing.tc_flops += lp.outer_flops;
+        } else if (use_i8_ && lp.outer_flops >= i8_min_flops_) {
+            for (const I8Launch& t : lp.outer_i8) {
+                launch_i8_split(t, s, pv, gev);
+                launch_i8_gemm(t.gemm, s, pv, gev, false);
+            }
         } else
             for (const Launch& ol : lp.outer) launch_gemm(ol, s, pv, gev);
         if (wrote_early) {
@@ -3313,6 +3426,8 @@ int Engine::factor(double* d_sm, double tol1, FactorResult& res, const Singular*
     NvtxRange range("spr_b200 factor");
     Dev& D = *d_;
     cudaStream_t s = stream_;
+    // without room for the slabs the updates stay on the FP64 kernel
+    use_i8_ = mixed_ == 0 && any_i8_ && ensure_i8() == 0;
     PV pv = make_view(D, P_, d_sm, tol1);
     if (fc3) {
         if (!fc3->d_dcor) return -2;
@@ -3377,8 +3492,8 @@ int Engine::factor(double* d_sm, double tol1, FactorResult& res, const Singular*
     const bool graph = use_graphs_ && !profile_ && s != nullptr && !tc_drop_ && wait_ns_ == 2000000000ull && !hooks_;
     if (graph) {
         const GraphKey key{(const void*)d_sm, nullptr, tol1, far_cap_q_,
-                           mixed_ | (chol_ ? 16 : 0) | (small_tile_ == kTileTiny ? 32 : 0),
-                           (int64_t)std::min(tc_min_flops_, 9.0e18), (const void*)pv.dcor, pv.tol4,
+                           mixed_ | (chol_ ? 16 : 0) | (small_tile_ == kTileTiny ? 32 : 0) | (use_i8_ ? 64 : 0),
+                           (int64_t)std::min(use_i8_ ? i8_min_flops_ : tc_min_flops_, 9.0e18), (const void*)pv.dcor, pv.tol4,
                            pv.near_tol};
         cudaGraphExec_t exec = find_graph(key);
         if (!exec) {

@@ -68,6 +68,8 @@ public:
     int open(const int64_t* mspar, const int64_t* mtrees, const int64_t* msifa);
     const Plan& plan() const { return P_; }
     void set_stream(cudaStream_t s) { stream_ = s; }
+    // least flops of a launch whose FP64 update runs on the integer tensor cores
+    void set_int_min(double flops);
     cudaStream_t stream() const { return stream_; }
     // Device-resident factorisation of sm = [D(NEQ) | LNZ(NZEROL)] (device pointer).
     int factor(double* d_sm, double tol1, FactorResult& res) { return factor(d_sm, tol1, res, nullptr); }
@@ -235,6 +237,19 @@ private:
     int ensure_slabs();
     void launch_tc(const TcLaunch& t, cudaStream_t s, const struct PV& pv, std::vector<cudaEvent_t>& gev,
                    bool far = false);
+    // Trailing and K = S updates of at least this many flops a launch run on
+    // the integer tensor cores.  Factor ms at 16^3 / 20^3 / 24^3 / 32^3 with the
+    // line at 1e8: 6.81 11.89 19.00 44.4, 1e9: 6.80 11.47 18.47 44.0, 3e9:
+    // 6.79 11.47 18.38 43.4, 1e10: 6.79 11.71 18.80 44.5, none: 6.79 11.71
+    // 19.69 55.7; below it the split and the 7.5 us tiles cost more than the
+    // FP64 kernel's small ones.
+    double i8_min_flops_ = 3e9;
+    int i8_far_q_ = 6;            // side-stream launches: eighths of the SMs (48^3: 4 320, 6 303, 8 307 ms)
+    bool any_i8_ = false;         // the plan has such an update
+    bool use_i8_ = false;         // and this factorisation runs them so
+    int ensure_i8();
+    void launch_i8_split(const I8Launch& t, cudaStream_t s, const struct PV& pv, std::vector<cudaEvent_t>& gev);
+    void launch_i8_gemm(const Launch& l, cudaStream_t s, const struct PV& pv, std::vector<cudaEvent_t>& gev, bool far);
     struct Csr {
         int64_t* rowptr = nullptr;
         int32_t* ci = nullptr;

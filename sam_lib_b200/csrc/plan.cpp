@@ -280,6 +280,7 @@ int build_plan(const int64_t* mspar, const int64_t* mtrees, const int64_t* msifa
     P.tc_flops = 0.0;
     P.slab_rows = 0;
     P.slab_rows_far = 0;
+    P.i8_rows = P.i8_scales = 0;
     P.small_flops = 0.0;
     for (int64_t js = 0; js < ns; ++js)
         if (P.F[js] <= kSmallMaxF) {
@@ -373,6 +374,51 @@ int build_plan(const int64_t* mspar, const int64_t* mtrees, const int64_t* msifa
             slab_max = std::max(slab_max, rows);
             out.push_back(t);
         };
+        // an integer-digit update: jobs jl (and the far part of the same panels,
+        // jfar, whose first column lies a multiple of kI8TileM after its job's)
+        auto emit_i8 = [&](const std::vector<Job>& jl, const std::vector<Job>& jfar, I8Launch& out) {
+            int64_t rows = 0, sc = 0;
+            std::vector<Job> base(jl);
+            for (Job& j : base) {
+                const int64_t nkb = (j.k_hi - j.k_lo + kI8BK - 1) / kI8BK;
+                j.np = (int32_t)((j.r_end - j.c0 + kI8TileM - 1) / kI8TileM * kI8TileM);
+                j.slab = rows;
+                j.aux_job = sc;
+                j.aux = sc + 8;
+                rows += 2 * nkb * kI8Digits * j.np;
+                sc += 8 + j.np;
+            }
+            P.i8_rows = std::max(P.i8_rows, rows);
+            P.i8_scales = std::max(P.i8_scales, sc);
+            auto tiles = [](const Job& j) -> int64_t {
+                const int64_t nct = (j.c_end - j.c0 + kI8TileN - 1) / kI8TileN;
+                const int64_t nr = (j.r_end - j.c0 + kI8TileM - 1) / kI8TileM;
+                int64_t n = 0;
+                for (int64_t it = 0; it < nr; ++it) n += std::min(nct, 2 * it + 2);
+                return n;
+            };
+            open_launch(out.split);
+            for (const Job& j : base) add_job(out.split, j, j.np / 32);
+            close_launch(out.split);
+            open_launch(out.gemm);
+            for (const Job& j : base) add_job(out.gemm, j, tiles(j));
+            close_launch(out.gemm);
+            open_launch(out.far);
+            for (const Job& f : jfar)
+                for (const Job& b : base)
+                    if (b.node == f.node) {
+                        Job j = f;
+                        j.np = b.np;
+                        j.slab = b.slab + (f.c0 - b.c0);
+                        j.aux_job = b.aux_job;
+                        j.aux = b.aux + (f.c0 - b.c0);
+                        add_job(out.far, j, tiles(j));
+                    }
+            close_launch(out.far);
+            out.gemm.tile = out.far.tile = kI8TileM;
+        };
+        lp.trail_i8.assign(nsteps, I8Launch());
+        lp.outer_i8.clear();
         lp.far.assign(nsteps, std::vector<Launch>());
         lp.ahead.assign(nsteps, std::vector<Launch>());
         lp.next_tc.assign(nsteps, std::vector<TcLaunch>());
@@ -422,7 +468,10 @@ int build_plan(const int64_t* mspar, const int64_t* mtrees, const int64_t* msifa
                 }
             }
             emit_updates(jl, lp.update[st]);
-            if (lp.next_flops[st] > 0.0) emit_tc(jl, lp.next_tc[st], P.slab_rows);
+            if (lp.next_flops[st] > 0.0) {
+                emit_tc(jl, lp.next_tc[st], P.slab_rows);
+                emit_i8(jl, jfar, lp.trail_i8[st]);
+            }
             emit_updates(jahead, lp.ahead[st]);
             emit_updates(jfar, lp.far[st]);
             emit_tc(jfar, lp.far_tc[st], P.slab_rows_far);
@@ -513,6 +562,18 @@ int build_plan(const int64_t* mspar, const int64_t* mtrees, const int64_t* msifa
             emit_updates(jl, lp.outer);
             lp.outer_tc.clear();
             emit_tc(jl, lp.outer_tc, P.slab_rows);
+            for (int32_t k0 = 0;; k0 += kI8MaxK) {
+                std::vector<Job> jk;
+                for (Job j : jl)
+                    if (j.k_hi > k0) {
+                        j.k_lo = k0;
+                        j.k_hi = std::min(j.k_hi, k0 + kI8MaxK);
+                        jk.push_back(j);
+                    }
+                if (jk.empty()) break;
+                lp.outer_i8.emplace_back();
+                emit_i8(jk, {}, lp.outer_i8.back());
+            }
         }
         open_launch(lp.writeback);
         for (int32_t js : lp.large_nodes)
@@ -572,6 +633,12 @@ int build_plan(const int64_t* mspar, const int64_t* mtrees, const int64_t* msifa
             build_map(t.split);
             build_map(t.gemm);
         }
+        for (std::vector<I8Launch>* v : {&lp.trail_i8, &lp.outer_i8})
+            for (I8Launch& t : *v) {
+                build_map(t.split);
+                build_map(t.gemm);
+                build_map(t.far);
+            }
         for (Launch& l : lp.fs_upd) build_map(l);
         for (Launch& l : lp.bs_upd) build_map(l);
         for (Launch& l : lp.blk_mv) build_map(l);
@@ -677,7 +744,7 @@ void check_plan(const Plan& P, int64_t& oob, int64_t& overlaps) {
 void check_coverage(const Plan& P, int64_t& fp64, int64_t& tc) {
     fp64 = tc = 0;
     const int64_t ns = P.nsuper;
-    for (int which = 0; which < 2; ++which) {
+    for (int which = 0; which < 3; ++which) {          // 2: the FP64 lists with the integer-digit updates
         // per front: per column, the K intervals it receives
         std::vector<std::vector<std::vector<std::pair<int32_t, int32_t>>>> cov(ns);
         auto add = [&](const Launch& l) {
@@ -689,14 +756,22 @@ void check_coverage(const Plan& P, int64_t& fp64, int64_t& tc) {
             }
         };
         for (const LevelPlan& lp : P.levels) {
-            for (const auto& v : lp.update)
-                for (const Launch& l : v) add(l);
+            for (size_t st = 0; st < lp.update.size(); ++st) {
+                if (which == 2 && lp.trail_i8[st].gemm.ntasks > 0) {
+                    add(lp.trail_i8[st].gemm);
+                    continue;
+                }
+                for (const Launch& l : lp.update[st]) add(l);
+            }
             for (const auto& v : lp.ahead)
                 for (const Launch& l : v) add(l);
             if (which == 0) {
                 for (const auto& v : lp.far)
                     for (const Launch& l : v) add(l);
                 for (const Launch& l : lp.outer) add(l);
+            } else if (which == 2) {
+                for (const I8Launch& t : lp.trail_i8) add(t.far);
+                for (const I8Launch& t : lp.outer_i8) add(t.gemm);
             } else {
                 for (const auto& v : lp.far_tc)
                     for (const TcLaunch& t : v) add(t.gemm);
@@ -726,7 +801,7 @@ void check_coverage(const Plan& P, int64_t& fp64, int64_t& tc) {
                 if (!ok || at != want) ++bad;
             }
         }
-        (which == 0 ? fp64 : tc) = bad;
+        (which == 1 ? tc : fp64) += bad;
     }
 }
 

@@ -49,6 +49,10 @@ struct Job {
     int32_t k_lo, k_hi;
     int64_t task0;                   // first task of this job within its launch
     int64_t slab = 0;                // tensor-core updates: first row of the job's operand slabs
+    // integer-digit updates: where the job's row scales and the job's flag
+    // (negative pivots) are, and the slabs' padded rows
+    int64_t aux = 0, aux_job = 0;
+    int32_t np = 0;
 };
 
 struct Launch {                      // a contiguous range of Plan::jobs
@@ -65,6 +69,19 @@ constexpr int kTcBK = 32;
 struct TcLaunch {
     Launch split;                    // one task per 32 rows x 32 columns of each job's panel
     Launch gemm;                     // one task per lower 128x128 tile of each job's block
+};
+
+// An FP64 Schur-update launch on the integer tensor cores: the split of the
+// panel into digit slabs, then the update of 128x64 lower tiles; for the
+// trailing updates the same slabs serve the next super-panel's columns (gemm)
+// and the ones beyond it (far).  The digit sums are exact in 32 bits for
+// K <= kI8MaxK (7 products of at most 2^14 in the last level).
+constexpr int kI8TileM = 128, kI8TileN = 64;
+constexpr int kI8BK = 128;
+constexpr int kI8Digits = 7;
+constexpr int kI8MaxK = 16384;
+struct I8Launch {
+    Launch split, gemm, far;
 };
 
 struct LevelPlan {
@@ -113,6 +130,9 @@ struct LevelPlan {
     std::vector<std::vector<TcLaunch>> far_tc;
     std::vector<double> far_flops;            // algorithmic flops of each step's far launches
     double outer_flops = 0.0;                 // and of the K = S update
+    // FP64 on the integer tensor cores: per panel step that ends a super-panel
+    // the trailing update, and the K = S update (one entry per kI8MaxK columns)
+    std::vector<I8Launch> trail_i8, outer_i8;
     std::vector<TcLaunch> outer_tc;                 // mixed precision: the K = S update
 };
 
@@ -183,6 +203,7 @@ struct Plan {
     double tc_flops = 0.0;                   // of those, the updates the mixed mode runs on tensor cores
     int64_t slab_rows = 0;                   // largest operand-slab need of one tensor-core launch (128-byte rows)
     int64_t slab_rows_far = 0;               // the same for the side-stream launches
+    int64_t i8_rows = 0, i8_scales = 0;      // largest digit slab (128-byte rows) and scale array of an integer launch
     double small_flops = 0.0;                // factor flops done by the fused small-front kernel
 };
 

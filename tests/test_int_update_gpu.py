@@ -1,0 +1,110 @@
+"""FP64 Schur updates as 8-bit digit products on the integer tensor cores.
+
+Dense fronts whose update sizes fall on and beside the edges of the 128 x 64
+tiles, of the 128-column K blocks and of the 512-column super-panels (odd
+first columns among them), with pivots of both signs and rows scaled over
+six decades.  The matrices are diagonally dominant (up to the scaling), so
+elimination does not grow their entries, and with A = S B S, |B_ii| = 1,
+
+    |A - L D L'|_ij <= c F 2^-53 S_i S_j
+
+for any order of the sums, F the front's order.  The digit form drops less
+than 2^-60 S_i S_j per term, far below; c = 8 covers the panel's product with
+the explicit inverse of its diagonal block and the comparison's own product."""
+import math
+
+import numpy as np
+import pytest
+
+from dense_structure import dense_chain, pack_dense
+
+pytestmark = pytest.mark.gpu
+
+
+def _matrix(neq, seed, negative):
+    rng = np.random.default_rng(seed)
+    b = rng.uniform(-1.0, 1.0, size=(neq, neq)) / neq
+    b = (b + b.T) / 2
+    sign = np.where(rng.random(neq) < 0.3, -1.0, 1.0) if negative else np.ones(neq)
+    np.fill_diagonal(b, sign)
+    s = 10.0 ** rng.uniform(-3.0, 3.0, size=neq)
+    return b * s[:, None] * s[None, :], s, int((sign < 0).sum())
+
+
+def _factor(ds, sm, least):
+    import torch
+    ds.set_int_min(least)
+    d = torch.from_numpy(sm).cuda()
+    r = ds.factor(d)
+    return r, d.cpu().numpy()
+
+
+def _unpack(sm, neq, mspar, mtrees, msifa):
+    m = int(mspar[10])
+    xsuper, xlnz = mtrees[:m + 1], msifa[mspar[47] - 1: mspar[47] + m]
+    low = np.zeros((neq, neq))
+    for j in range(m):
+        p = xlnz[j] - 1 + neq
+        for c in range(xsuper[j] - 1, xsuper[j + 1] - 1):
+            low[c:, c] = sm[p: p + neq - c]
+            p += neq - c
+    return low
+
+
+@pytest.mark.parametrize('negative', [False, True])
+@pytest.mark.parametrize('widths', [[64, 128], [65, 127], [200, 64], [129, 193], [513, 1], [640, 65], [576, 700],
+                                    [1025, 130, 400], [1600, 3]])
+def test_digit_updates_reproduce_the_matrix(widths, negative):
+    import sam_lib_b200 as spr
+    structure = dense_chain(widths)
+    neq = sum(widths)
+    a, s, nneg = _matrix(neq, neq, negative)
+    sm = pack_dense(a, *structure)
+    ds = spr.DeviceSolver(*structure)
+    r, f = _factor(ds, sm, 0.0)
+    launches = ds.info()['launches']
+    rg, fg = _factor(ds, sm, math.inf)                   # the general path
+    assert r['lierr'] == rg['lierr'] == 0 and r['numneg'] == rg['numneg'] == nneg
+    assert launches > ds.info()['launches']              # a split and a product for each update
+    low = _unpack(f, neq, *structure)
+    d = low.diagonal().copy()
+    np.fill_diagonal(low, 1.0)
+    err = np.abs(a - (low * d) @ low.T) / (s[:, None] * s[None, :])
+    assert err.max() <= 8 * neq * 2.0 ** -53
+    # the two paths' factors: both within the bound of A, and L is as well conditioned as B
+    scale = np.sqrt(np.abs(d))[None, :] / s[:, None]
+    lg = _unpack(fg, neq, *structure)
+    np.fill_diagonal(lg, 1.0)
+    assert (np.abs(low - lg) * scale).max() <= 32 * neq * 2.0 ** -53
+    ds.close()
+
+
+def test_nan_fails_at_the_same_equation():
+    import sam_lib_b200 as spr
+    structure = dense_chain([640, 200])
+    a, _, _ = _matrix(840, 3, False)
+    a[700, 5] = a[5, 700] = math.nan
+    sm = pack_dense(a, *structure)
+    ds = spr.DeviceSolver(*structure)
+    r, _ = _factor(ds, sm, 0.0)
+    rg, _ = _factor(ds, sm, math.inf)
+    assert r['lierr'] == rg['lierr'] == -30 and r['supeqt'] == rg['supeqt'] == 701
+    ds.close()
+
+
+def test_a_wait_that_runs_out_is_reported():
+    import sam_lib_b200 as spr
+    import torch
+    structure = dense_chain([640, 200])
+    a, _, _ = _matrix(840, 4, False)
+    sm = pack_dense(a, *structure)
+    ds = spr.DeviceSolver(*structure)
+    ds.set_int_min(0.0)
+    ds.set_watchdog(0.05, drop=True)                     # one CTA never loads its first operands
+    with pytest.raises(RuntimeError, match='-4'):
+        ds.factor(torch.from_numpy(sm).cuda())
+    ds.set_watchdog(2.0, drop=False)
+    r, f = _factor(ds, sm, 0.0)
+    rg, fg = _factor(ds, sm, math.inf)
+    assert r['lierr'] == rg['lierr'] == 0 and np.abs(f - fg).max() <= 1e-12 * np.abs(fg).max()
+    ds.close()
