@@ -23,10 +23,10 @@
 //               a second slab with the signs of D where a pivot is negative;
 //   k_gemm_i8   CTAs over the lower 128x64 tiles: a TMA warp streams, per block
 //               of 128 columns, the seven 64x128 digit tiles of the columns (double
-//               buffered) and the seven 128x128 digit tiles of the rows (a ring
-//               of six), one thread issues tcgen05.mma kind::i8 - digit p of the rows
+//               buffered) and the seven 128x128 digit tiles of the rows (one buffer per
+//               digit), one thread issues tcgen05.mma kind::i8 - digit p of the rows
 //               against the digits 0 .. 7-p of the columns (N up to 256 an
-//               instruction), which land in the levels p .. 7 - and eight epilogue
+//               instruction), which land in the levels p .. 7 - and sixteen epilogue
 //               warps put the levels of an entry together in 64-bit integers,
 //               scale them and subtract from the FP64 front.
 // Every mbarrier wait is bounded like those of k_gemm_tc.
@@ -38,16 +38,16 @@ using namespace tc;                           // mbarrier, TMA, TMEM helpers
 constexpr int kM = kI8TileM, kN = kI8TileN, kK = kI8BK;      // 128 x 64 tile, 128-byte K blocks
 constexpr int kDig = kI8Digits;               // digits of an entry
 constexpr int kLev = 8;                       // levels p + q = 0 .. 7: 8 x 64 TMEM columns
-constexpr int kSlots = 6;                     // ring of row digit tiles
 constexpr int kABytes = kM * kK;              // 16 KB
 constexpr int kBBytes = kN * kK;              // 8 KB, seven of them contiguous
-constexpr size_t kSmemI8 = 1024 + 2 * (size_t)kDig * kBBytes + (size_t)kSlots * kABytes;
-constexpr int kEpiWarps = 8;
+constexpr size_t kSmemI8 = 1024 + (size_t)kDig * (2 * kBBytes + kABytes);
+constexpr int kEpiWarps = 16;                 // four per TMEM quadrant, 16 columns each
+constexpr int kEpiCols = kN / (kEpiWarps / 4);
 constexpr int kThreadsI8 = 32 * (2 + kEpiWarps);
 // D s32, A and B signed 8-bit, both K-major, M = 128; N is added per instruction
 constexpr uint32_t kIdescI8 = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kM >> 4) << 24);
 // N = n column digits
-__device__ __forceinline__ uint32_t idesc(int n) { return kIdescI8 | ((uint32_t)(n * kN >> 3) << 17); }
+__device__ __forceinline__ constexpr uint32_t idesc(int n) { return kIdescI8 | ((uint32_t)(n * kN >> 3) << 17); }
 
 __device__ __forceinline__ void mma_i8(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
@@ -58,10 +58,10 @@ __device__ __forceinline__ void mma_i8(uint32_t d, uint64_t a, uint64_t b, uint3
         : "memory");
 }
 
-// 32 lanes x 8 consecutive 32-bit columns, without the wait
-__device__ __forceinline__ void tmem_ld8(uint32_t taddr, int (&r)[8]) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+// 32 lanes x 4 consecutive 32-bit columns, without the wait
+__device__ __forceinline__ void tmem_ld4(uint32_t taddr, int (&r)[4]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
                  : "r"(taddr));
 }
 
@@ -207,18 +207,19 @@ __global__ void __launch_bounds__(i8::kThreadsI8, 1)
               const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b) {
     using namespace i8;
     extern __shared__ uint8_t i8_raw[];
-    __shared__ uint64_t bars[2 * kSlots + 4 + 3];
+    __shared__ uint64_t bars[2 * kDig + 4 + 3];
+    __shared__ double scol[2][kN];                     // column scales of a tile and the next
     __shared__ uint32_t tmem_slot;
     __shared__ int failed;
     if (P.st->any_fail) return;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t base = (smem_u32(i8_raw) + 1023u) & ~1023u;
     const uint32_t sb = base, sa = base + 2u * kDig * kBBytes;
-    const uint32_t afull = smem_u32(&bars[0]), aempty = smem_u32(&bars[kSlots]);
-    const uint32_t bfull = smem_u32(&bars[2 * kSlots]), bempty = bfull + 16;
+    const uint32_t afull = smem_u32(&bars[0]), aempty = smem_u32(&bars[kDig]);
+    const uint32_t bfull = smem_u32(&bars[2 * kDig]), bempty = bfull + 16;
     const uint32_t accf = bfull + 32, acce = accf + 8, drain = accf + 16;
     if (threadIdx.x == 0) {
-        for (int s = 0; s < kSlots; ++s) {
+        for (int s = 0; s < kDig; ++s) {
             mbar_init(afull + 8 * s, 1);
             mbar_init(aempty + 8 * s, 1);
         }
@@ -245,92 +246,103 @@ __global__ void __launch_bounds__(i8::kThreadsI8, 1)
 
     if (warp == 0 && lane == 0) {
         // ---- TMA producer
-        int64_t ga = 0, gb = 0;
+        uint32_t issued = 0;                              // 8 K block + digit, of the last row load, + 1
+        uint32_t g = 0;                                   // K blocks so far
         bool stop = false;
         for (int64_t task = blockIdx.x; task < ntasks && !stop && !*(volatile int*)&failed; task += gridDim.x) {
             const Job& jb = job_of(jobs, njobs, tmap, task);
             if (P.sn_bad[jb.node] || node_off(P, jb.node)) continue;
             int it, jt;
             tile_of_i8(task - jb.task0, (jb.c_end - jb.c0 + kN - 1) / kN, (jb.r_end - jb.c0 + kM - 1) / kM, it, jt);
-            const int nkb = k_blocks_i8(jb);
-            const int64_t np = jb.np;
-            const int64_t wofs = scales[jb.aux_job] != 0.0 ? (int64_t)nkb * kDig * np : 0;   // signed row slab
-            const int64_t ya = jb.slab + wofs + (int64_t)it * kM, yb = jb.slab + (int64_t)jt * kN;
-            for (int kb = 0; kb < nkb && !stop; ++kb) {
-                const int b = (int)(gb & 1);
-                if (gb >= 2 && !mbar_wait(bempty + 8 * b, (uint32_t)((gb >> 1) - 1) & 1u, P.wait_ns)) {
+            const int nkb = k_blocks_i8(jb), np = jb.np;
+            const int wofs = scales[jb.aux_job] != 0.0 ? nkb * kDig * np : 0;   // signed row slab
+            int ya = (int)jb.slab + wofs + it * kM, yb = (int)jb.slab + jt * kN;
+            for (int kb = 0; kb < nkb && !stop; ++kb, ++g) {
+                const uint32_t b = g & 1u, bf = bfull + 8 * b;
+                if (g >= 2 && !mbar_wait(bempty + 8 * b, ((g >> 1) - 1) & 1u, P.wait_ns)) {
                     stop = true;
                     break;
                 }
-                if (!(P.tc_drop && blockIdx.x == 0 && gb == 0)) {         // watchdog test: never loaded
-                    mbar_expect_tx(bfull + 8 * b, kDig * kBBytes);
-                    for (int d = 0; d < kDig; ++d)
-                        tma_load_2d(sb + (uint32_t)(b * kDig + d) * kBBytes, &map_b, bfull + 8 * b, 0,
-                                    (int)(yb + ((int64_t)kb * kDig + d) * np));
+                if (!(P.tc_drop && blockIdx.x == 0 && g == 0)) {          // watchdog test: never loaded
+                    mbar_expect_tx(bf, kDig * kBBytes);
+                    const uint32_t dst = sb + b * (uint32_t)(kDig * kBBytes);
+#pragma unroll
+                    for (int d = 0; d < kDig; ++d, yb += np) tma_load_2d(dst + d * kBBytes, &map_b, bf, 0, yb);
+                } else {
+                    yb += kDig * np;
                 }
-                ++gb;
-                for (int d = 0; d < kDig; ++d, ++ga) {
-                    const int s = (int)(ga % kSlots);
-                    if (ga >= kSlots && !mbar_wait(aempty + 8 * s, (uint32_t)(ga / kSlots - 1) & 1u, P.wait_ns)) {
-                        stop = true;
-                        break;
+#pragma unroll
+                for (int d = 0; d < kDig; ++d, ya += np) {
+                    if (g >= 1 && !stop && !mbar_wait(aempty + 8 * d, (g - 1) & 1u, P.wait_ns)) stop = true;
+                    if (!stop) {
+                        mbar_expect_tx(afull + 8 * d, kABytes);
+                        tma_load_2d(sa + d * kABytes, &map_a, afull + 8 * d, 0, ya);
+                        issued = 8 * g + d + 1;
                     }
-                    mbar_expect_tx(afull + 8 * s, kABytes);
-                    tma_load_2d(sa + (uint32_t)s * kABytes, &map_a, afull + 8 * s, 0,
-                                (int)(ya + ((int64_t)kb * kDig + d) * np));
                 }
             }
         }
         if (stop) failed = 1;
-        // drain: what was issued must have landed before exit
-        for (int64_t q = (ga > kSlots ? ga - kSlots : 0); q < ga; ++q)
-            mbar_wait(afull + 8 * (int)(q % kSlots), (uint32_t)(q / kSlots) & 1u, P.wait_ns);
-        for (int64_t q = (gb > 2 ? gb - 2 : 0); q < gb; ++q)
-            mbar_wait(bfull + 8 * (int)(q & 1), (uint32_t)(q >> 1) & 1u, P.wait_ns);
+        // drain: what was issued must have landed before exit (the last use of
+        // each buffer; an earlier one has been consumed)
+        for (int d = 0; d < kDig; ++d)
+            if (issued > (uint32_t)d) {
+                const uint32_t last = (issued - 1 - d) >> 3;            // last K block whose digit d was issued
+                mbar_wait(afull + 8 * d, last & 1u, P.wait_ns);
+            }
+        if (issued) {
+            const uint32_t last = (issued - 1) >> 3;
+            mbar_wait(bfull + 8 * (last & 1u), (last >> 1) & 1u, P.wait_ns);
+            if (last) mbar_wait(bfull + 8 * ((last - 1) & 1u), ((last - 1) >> 1) & 1u, P.wait_ns);
+        }
     } else if (warp == 1 && lane == 0) {
         // ---- MMA issuer
-        int64_t ga = 0, gb = 0, tile = 0;
+        uint32_t g = 0, tile = 0;
         bool stop = false;
+        const uint64_t ad0 = sw128_desc(sa), bd0 = sw128_desc(sb);
         for (int64_t task = blockIdx.x; task < ntasks && !stop; task += gridDim.x) {
             const Job& jb = job_of(jobs, njobs, tmap, task);
             if (P.sn_bad[jb.node] || node_off(P, jb.node)) continue;
             const int nkb = k_blocks_i8(jb);
-            if (tile >= 1 && !mbar_wait(acce, (uint32_t)(tile - 1) & 1u, P.wait_ns)) {
+            if (tile >= 1 && !mbar_wait(acce, (tile - 1) & 1u, P.wait_ns)) {
                 stop = true;
                 break;
             }
             fence_after_sync();
-            for (int kb = 0; kb < nkb && !stop; ++kb, ++gb) {
-                const int b = (int)(gb & 1);
-                if (!mbar_wait(bfull + 8 * b, (uint32_t)(gb >> 1) & 1u, P.wait_ns) || *(volatile int*)&failed) {
+            for (int kb = 0; kb < nkb && !stop; ++kb, ++g) {
+                const uint32_t b = g & 1u;
+                if (!mbar_wait(bfull + 8 * b, (g >> 1) & 1u, P.wait_ns) || *(volatile int*)&failed) {
                     stop = true;
                     break;
                 }
-                for (int p = 0; p < kDig; ++p, ++ga) {
-                    const int s = (int)(ga % kSlots);
-                    if (!mbar_wait(afull + 8 * s, (uint32_t)(ga / kSlots) & 1u, P.wait_ns)) {
-                        stop = true;
-                        break;
-                    }
-                    fence_after_sync();
-                    const uint64_t ad = sw128_desc(sa + (uint32_t)s * kABytes);
-                    const uint64_t bd = sw128_desc(sb + (uint32_t)(b * kDig) * kBBytes);
-                    // digits q = 0 .. min(6, 7 - p) of the columns, levels p + q: four
-                    // digits in the first instruction, the rest in the second
-                    const int cnt = min(kDig, kLev - p), n0 = min(cnt, 4), n1 = cnt - n0;
+                const uint64_t bd = bd0 + (uint64_t)(b * (kDig * kBBytes >> 4));
+                const uint32_t first = kb ? 1u : 0u;
+                // straight-line code: every descriptor is a constant away from the
+                // base ones, so that one thread issues faster than the MMAs run
 #pragma unroll
-                    for (int kk = 0; kk < kK / 32; ++kk) {
-                        const uint64_t adv = (uint64_t)(kk * 32) >> 4, bq = (uint64_t)(kBBytes >> 4);
-                        const uint32_t add = (kb | p | kk) ? 1u : 0u;     // digit 0 opens the levels 0 .. 6
-                        mma_i8(tmem + (uint32_t)(kN * p), ad + adv, bd + adv, idesc(n0), add);
-                        if (p == 1 && kb == 0 && kk == 0) {               // and digit 1 the last level
-                            mma_i8(tmem + (uint32_t)(kN * 5), ad + adv, bd + adv + 4 * bq, idesc(2), 1u);
-                            mma_i8(tmem + (uint32_t)(kN * 7), ad + adv, bd + adv + 6 * bq, idesc(1), 0u);
-                        } else if (n1 > 0) {
-                            mma_i8(tmem + (uint32_t)(kN * (p + 4)), ad + adv, bd + adv + 4 * bq, idesc(n1), add);
+                for (int p = 0; p < kDig; ++p) {
+                    if (!stop && !mbar_wait(afull + 8 * p, g & 1u, P.wait_ns)) stop = true;
+                    if (!stop) {
+                        fence_after_sync();
+                        // digits q = 0 .. min(6, 7 - p) of the columns, levels p + q: four
+                        // digits in the first instruction, the rest in the second
+                        const int cnt = kDig < kLev - p ? kDig : kLev - p, n0 = cnt < 4 ? cnt : 4, n1 = cnt - n0;
+                        const uint64_t ad = ad0 + (uint64_t)(p * kABytes >> 4);
+                        constexpr uint64_t bq = (uint64_t)(kBBytes >> 4);
+#pragma unroll
+                        for (int kk = 0; kk < kK / 32; ++kk) {
+                            const uint64_t adv = (uint64_t)(kk * 32) >> 4;
+                            const uint32_t add = (p | kk) ? 1u : first;       // digit 0 opens the levels 0 .. 6
+                            mma_i8(tmem + (uint32_t)(kN * p), ad + adv, bd + adv, idesc(n0), add);
+                            if (p == 1 && kk == 0) {                          // and digit 1 the last level
+                                mma_i8(tmem + (uint32_t)(kN * 5), ad + adv, bd + adv + 4 * bq, idesc(2), 1u);
+                                mma_i8(tmem + (uint32_t)(kN * 7), ad + adv, bd + adv + 6 * bq, idesc(1), first);
+                            } else if (n1 > 0) {
+                                mma_i8(tmem + (uint32_t)(kN * (p + 4)), ad + adv, bd + adv + 4 * bq, idesc(n1), add);
+                            }
                         }
+                        mma_commit(aempty + 8 * p);
                     }
-                    mma_commit(aempty + 8 * s);
                 }
                 mma_commit(bempty + 8 * b);
             }
@@ -342,69 +354,69 @@ __global__ void __launch_bounds__(i8::kThreadsI8, 1)
         mma_commit(drain);
         if (!mbar_wait(drain, 0u, P.wait_ns)) failed = 1;
     } else if (warp >= 2) {
-        // ---- epilogue: TMEM lanes 32 (warp % 4) .. + 31, half of the 64 columns each
+        // ---- epilogue: TMEM lanes 32 (warp % 4) .. + 31, kEpiCols of the 64 columns each.
+        // The front's entries and the column scales are loaded before the wait for
+        // the products, so that a tile's TMEM is free again after the reads and
+        // the arithmetic alone (8192-row block, split included: K = 512 0.61 -> 0.46 ms,
+        // K = 2048 1.60 -> 1.53 ms).
         const int q = warp & 3, h = (warp - 2) >> 2;
-        const uint32_t lane_base = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(32 * h);
-        int64_t tile = 0;
+        const uint32_t lane_base = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(kEpiCols * h);
+        uint32_t tile = 0;
         for (int64_t task = blockIdx.x; task < ntasks; task += gridDim.x) {
             const Job& jb = job_of(jobs, njobs, tmap, task);
             const int js = jb.node;
             if (P.sn_bad[js] || node_off(P, js)) continue;
             int it, jt;
             tile_of_i8(task - jb.task0, (jb.c_end - jb.c0 + kN - 1) / kN, (jb.r_end - jb.c0 + kM - 1) / kM, it, jt);
-            const int row = it * kM + 32 * q + lane, col0 = jt * kN + 32 * h;
-            const int r = jb.c0 + row;
+            const int row = it * kM + 32 * q + lane, col0 = jt * kN + kEpiCols * h;
+            const int r = jb.c0 + row, c0 = jb.c0 + col0;
+            // columns of this thread's row that belong to the lower triangle of the block
+            const int ncol = r < jb.r_end ? min(kEpiCols, min(jb.c_end - c0, r - c0 + 1)) : 0;
             const int64_t ld = P.buf_ld[js];
             const double* sc = scales + jb.aux;
+            double* dst = P.arena + P.buf_off[js] + r + (int64_t)c0 * ld;
+            double cv[kEpiCols];
+#pragma unroll
+            for (int t = 0; t < kEpiCols; ++t) cv[t] = t < ncol ? __ldcg(dst + (int64_t)t * ld) : 0.0;
             const double si = sc[row];
-            double* dst = P.arena + P.buf_off[js] + r + (int64_t)(jb.c0 + col0) * ld;
-            if (!mbar_wait(accf, (uint32_t)tile & 1u, P.wait_ns) || *(volatile int*)&failed) {
+            // (the four quadrants' warps write the same values; a warp is never
+            // two tiles ahead of another)
+            double* sj = &scol[tile & 1u][kEpiCols * h];
+            if (lane < kEpiCols) sj[lane] = 16.0 * sc[col0 + lane];
+            __syncwarp();
+            if (!mbar_wait(accf, tile & 1u, P.wait_ns) || *(volatile int*)&failed) {
                 failed = 1;
                 break;
             }
             ++tile;
             fence_after_sync();
-            double v[32];
 #pragma unroll
-            for (int c8 = 0; c8 < 4; ++c8) {
-                int lv[kLev][8];
+            for (int c4 = 0; c4 < kEpiCols; c4 += 4) {
+                int lv[kLev][4];
 #pragma unroll
-                for (int s = 0; s < kLev; ++s) tmem_ld8(lane_base + (uint32_t)(kN * s + 8 * c8), lv[s]);
+                for (int s = 0; s < kLev; ++s) tmem_ld4(lane_base + (uint32_t)(kN * s + c4), lv[s]);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-                for (int t = 0; t < 8; ++t) {
+                for (int t = 0; t < 4; ++t) {
                     // sum of level s times 256^(6-s): the leading three levels (47 bits) and, with
                     // levels 6 and 7 rounded to 16, the others (51 bits) as exact doubles
                     const long long magic = 0x4338000000000000ll;        // 1.5 2^52
                     const long long hi = (long long)lv[0][t] * 65536 + ((long long)lv[1][t] * 256 + (magic + lv[2][t]));
                     const long long lo = (long long)lv[3][t] * (1 << 20) +
                                          ((long long)lv[4][t] * (1 << 12) +
-                                          ((long long)lv[5][t] * (1 << 4) + (magic + ((lv[6][t] + ((lv[7][t] + 128) >> 8) + 8) >> 4))));
-                    v[8 * c8 + t] = fma(__longlong_as_double(hi) - 6755399441055744.0, 268435456.0,
-                                        __longlong_as_double(lo) - 6755399441055744.0);
+                                          ((long long)lv[5][t] * (1 << 4) +
+                                           (magic + ((lv[6][t] + ((lv[7][t] + 128) >> 8) + 8) >> 4))));
+                    const double v = fma(__longlong_as_double(hi) - 6755399441055744.0, 268435456.0,
+                                         __longlong_as_double(lo) - 6755399441055744.0);
+                    cv[c4 + t] -= (v * si) * sj[c4 + t];
                 }
             }
             fence_before_sync();
             __syncwarp();
             if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(acce) : "memory");
-            if (r < jb.r_end) {
 #pragma unroll
-                for (int c8 = 0; c8 < 4; ++c8) {
-                    double cv[8];
-#pragma unroll
-                    for (int t = 0; t < 8; ++t) {
-                        const int c = jb.c0 + col0 + 8 * c8 + t;
-                        cv[t] = (c < jb.c_end && r >= c) ? __ldcg(dst + (int64_t)(8 * c8 + t) * ld) : 0.0;
-                    }
-#pragma unroll
-                    for (int t = 0; t < 8; ++t) {
-                        const int c = jb.c0 + col0 + 8 * c8 + t;
-                        if (c < jb.c_end && r >= c)
-                            dst[(int64_t)(8 * c8 + t) * ld] =
-                                cv[t] - (v[8 * c8 + t] * si) * (16.0 * __ldg(sc + col0 + 8 * c8 + t));
-                    }
-                }
-            }
+            for (int t = 0; t < kEpiCols; ++t)
+                if (t < ncol) dst[(int64_t)t * ld] = cv[t];
         }
     }
     __syncthreads();
