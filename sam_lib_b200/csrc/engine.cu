@@ -746,25 +746,115 @@ __global__ void __launch_bounds__(256) k_assemble(const Job* jobs, int64_t njobs
     }
 }
 
+namespace gemm {
+__device__ __forceinline__ void dmma(double& c0, double& c1, double a, double b) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+                 : "+d"(c0), "+d"(c1)
+                 : "d"(a), "d"(b));
+}
+}  // namespace gemm
+
 // LDL' of one nb x nb diagonal block, pivot test / inertia / TOL(2) as
-// SPRF17 (sprfc1.f:1272-1294).  256 threads on a 16x16 grid, each owning
-// rows i = tx + 16a and columns j = ty + 16b of the block; right-looking with
-// the unscaled column (a_ij -= a_ik * a_jk / d_k), scaled to L at the end.
-// Also forms X = L11^-1 (unit lower) for the panel TRSM and the solves.
+// SPRF17 (sprfc1.f:1272-1294), and X = L11^-1 (unit lower) for the panel TRSM
+// and the solves.  One CTA per block, so a chain of kNB dependent pivots
+// bounds it: reciprocal, scaling, update, next pivot.  The block goes in four
+// groups of 16 columns.  A group's columns are eliminated by up to three
+// warps without a CTA barrier: a lane holds one row's 16 entries in registers,
+// lanes 0-15 the group's own rows (every warp repeats them) and lanes 16-31 a
+// set of 16 rows below; the pivot goes round by a shuffle, the unscaled column
+// (a_ij -= a_ik * a_jk / d_k) through the warp's own shared memory.  The
+// columns after the group are updated with DMMA tiles (K = 16) by all warps.
+// The inverse of each group's 16x16 triangle is formed beside the next group's
+// elimination, and the 32- and 64-wide inverses by doubling (X21 = -X22 (L21 X11))
+// with DMMA.  32^3, one block: 39 us with 256 threads in lockstep, one barrier
+// per column.
+constexpr int kDG = 16;                              // columns of a group
+constexpr int kDPanLd = kDG + 4;                     // bank-conflict-free DMMA fragments
+
+// one group's elimination by one warp: rows below in set w (rows
+// c0 + 16 + 16 w ..), kmax columns; returns the failing column for the rule that
+// stops at once (kPivotChol4), or -1
+template <int PR>
+__device__ __forceinline__ int diag_group(const PV& P, int js, int k0, int c0, int kmax, int w, int lane, int nb,
+                                          double (*A)[kNB + 1], double (*Wp)[kDPanLd], double* colbuf,
+                                          double* dd, double* rdv, const double* adv) {
+    const int fst = P.fst[js];
+    const bool own = lane < kDG;
+    const int row = own ? c0 + lane : c0 + kDG * w + lane;       // 16 + 16 w + (lane - 16)
+    double a[kDG];
+#pragma unroll
+    for (int j = 0; j < kDG; ++j) a[j] = (row < nb && row >= c0 + j) ? A[row][c0 + j] : 0.0;
+#pragma unroll
+    for (int k = 0; k < kDG; ++k) {
+        if (k >= kmax) break;
+        double* cb = colbuf + (k & 1) * kDG;
+        double d = __shfl_sync(0xffffffffu, a[k], k);
+        const int col = c0 + k;
+        if (PR == kPivotReplace) {
+            const double d0 = d;
+            d = fc3_pivot(P, d0, adv[col]);
+            if (w == 0 && lane == 0) fc3_record(P, fst + k0 + col, d0, d);
+        }
+        if (PR == kPivotChol4) {
+            // records replacements while it goes, so it stops at a failing pivot
+            if (pivot_fails(PR, d, adv[col], P.tol1)) {
+                if (w == 0 && lane == 0) {
+                    record_fail(P, js, k0 + col, d, adv[col]);
+                    chol4_fail_record(P, fst + k0 + col, d);
+                }
+                return col;
+            }
+            d = chol4_pivot(P, fst + k0 + col, d, adv[col], w == 0 && lane == 0);
+        }
+        if (own && lane > k) cb[lane] = a[k];                    // the unscaled column
+        const double rd = recip_nr(d);
+        if (w == 0 && lane == k) {
+            dd[col] = d;
+            rdv[col] = rd;
+        }
+        const double l = a[k] * rd;
+        __syncwarp();
+#pragma unroll
+        for (int j = k + 1; j < kDG; ++j) a[j] -= l * cb[j];
+        if (own) {
+            if (w == 0 && lane > k && row < nb) A[row][col] = l;
+        } else if (row < nb) {
+            A[row][col] = l;
+            Wp[row][k] = a[k];
+        }
+    }
+    return -1;
+}
+
+// inverse of the unit-lower kDG x kDG block at c0 by one warp: lane j < 16 forms
+// column j; X[i][j] goes to A[c0 + j][c0 + i] (the free upper triangle)
+__device__ __forceinline__ void diag_group_inverse(double (*A)[kNB + 1], int c0, int nb, int lane) {
+    double x[kDG];
+#pragma unroll
+    for (int i = 0; i < kDG; ++i) {
+        double s0 = 0.0, s1 = 0.0;
+#pragma unroll
+        for (int m = 0; m < i; ++m) {
+            const double l = (c0 + i < nb) ? A[c0 + i][c0 + m] : 0.0;
+            if (m & 1) s1 += l * x[m];
+            else s0 += l * x[m];
+        }
+        x[i] = i == lane ? 1.0 : i < lane ? 0.0 : -(s0 + s1);
+    }
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < kDG; ++i)
+        if (lane < i && lane < kDG) A[c0 + lane][c0 + i] = x[i];
+}
+
 template <int PR>
 __global__ void __launch_bounds__(256) k_diag(const Job* jobs, PV P) {
-    // Register-resident: thread (tx, ty) keeps entries (tx + 16a, ty + 16b) of
-    // the block in v[a][b] through the elimination and of X = L^-1 in x[a][b]
-    // through the inverse; each step publishes one column of the block (or one
-    // row of X) through shared memory, one barrier per step.  Entries outside
-    // the lower triangle are carried along as don't-care values (never
-    // published nor stored), which keeps the step free of per-entry tests.
-    __shared__ double A[kNB][kNB + 1];      // L (lower, d on the diagonal)
-    __shared__ double vec[2][kNB];          // the published column / row (double buffered)
+    __shared__ double A[kNB][kNB + 1];      // L (lower, d on the diagonal), X transposed above
+    __shared__ double pan[kNB / 2 * (kNB / 2 + 4)];   // W of a group's rows below (16 .. 63); later T
+    __shared__ double colbuf[3][2 * kDG];
     __shared__ double rdv[kNB];
     __shared__ double dd[kNB];
     __shared__ double adv[kNB];
-    __shared__ double Tb[kNB * kNB / 4];    // T = L21 X11 of the inverse's doubling passes
     __shared__ int s_fail;
     if (P.st->any_fail) return;
     const Job& jb = jobs[blockIdx.x];
@@ -772,77 +862,59 @@ __global__ void __launch_bounds__(256) k_diag(const Job* jobs, PV P) {
     if (P.sn_bad[js] || node_off(P, js)) return;
     const int ld = P.buf_ld[js], fst = P.fst[js];
     double* front = P.arena + P.buf_off[js];
-    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-    constexpr int R = kNB / 16;
-    double v[R][R];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    // W's rows are 16 .. 63: a group's own rows are not among them
+    double(*Wp)[kDPanLd] = reinterpret_cast<double(*)[kDPanLd]>(pan) - kDG;
+    {
+        double v[kNB * kNB / 256];
 #pragma unroll
-    for (int b = 0; b < R; ++b)
-#pragma unroll
-        for (int a = 0; a < R; ++a) {
-            const int i = tx + 16 * a, j = ty + 16 * b;
-            v[a][b] = (i >= j && i < nb && j < nb) ? __ldcg(front + (int64_t)(k0 + i) + (int64_t)(k0 + j) * ld) : 0.0;
+        for (int q = 0; q < kNB * kNB / 256; ++q) {
+            const int i = tid & (kNB - 1), j = (tid >> 6) + 4 * q;
+            v[q] = (i >= j && i < nb) ? __ldcg(front + (int64_t)(k0 + i) + (int64_t)(k0 + j) * ld) : 0.0;
         }
-    if (tid < nb) adv[tid] = __ldcg(P.adiag + fst + k0 + tid);
-    for (int k = tid; k < 2 * kNB; k += blockDim.x) vec[k / kNB][k % kNB] = 0.0;
+        if (tid < nb) adv[tid] = __ldcg(P.adiag + fst + k0 + tid);
+        if (tid == 0) s_fail = kNB;
+#pragma unroll
+        for (int q = 0; q < kNB * kNB / 256; ++q) A[tid & (kNB - 1)][(tid >> 6) + 4 * q] = v[q];
+    }
     __syncthreads();
     int failed = -1;
-    // columns in groups of 16 (kb static inside a group, so the publishing
-    // threads read their register v[a][kb] directly)
-#pragma unroll
-    for (int kb = 0; kb < R; ++kb) {
-      if (16 * kb >= nb || failed >= 0) break;
-      for (int kk = 0; kk < 16; ++kk) {
-        const int k = 16 * kb + kk;
-        if (k >= nb) break;
-        const int buf = k & 1;
-        if (ty == kk) {
-#pragma unroll
-            for (int a = 0; a < R; ++a) {
-                const int i = tx + 16 * a;
-                double c = v[a][kb];
-                if (PR == kPivotReplace && i == k) {
-                    const double c0 = c;
-                    c = fc3_pivot(P, c0, adv[k]);
-                    fc3_record(P, fst + k0 + k, c0, c);
-                }
-                if (PR == kPivotChol4 && i == k && !pivot_fails(PR, c, adv[k], P.tol1))
-                    c = chol4_pivot(P, fst + k0 + k, c, adv[k], true);
-                if (i >= k && i < nb) vec[buf][i] = c;
-                if (i == k) {
-                    dd[k] = c;
-                    rdv[k] = recip_nr(c);
-                }
-            }
+    for (int c0 = 0; c0 < nb; c0 += kDG) {
+        const int kmax = min(kDG, nb - c0), rest = nb - c0 - kDG;         // rest: rows below the group
+        const int sets = rest > 0 ? (rest + kDG - 1) / kDG : 1;
+        if (warp < sets) {
+            const int f = diag_group<PR>(P, js, k0, c0, kmax, warp, lane, nb, A, Wp, colbuf[warp], dd, rdv, adv);
+            if (PR == kPivotChol4 && f >= 0 && lane == 0) s_fail = f;     // every warp finds the same column
+        } else if (warp == 4 && c0 > 0) {
+            diag_group_inverse(A, c0 - kDG, nb, lane);
         }
         __syncthreads();
-        const double d = vec[buf][k];
-        // SPRFC4's rule records replacements while it goes, so it stops at a
-        // failing pivot here; the other rules are tested after the loop (the
-        // steps after a failure only compute values that are thrown away)
-        if (PR == kPivotChol4 && pivot_fails(PR, d, adv[k], P.tol1)) {
-            failed = k;
-            if (tid == 0) {
-                record_fail(P, js, k0 + k, d, adv[k]);
-                chol4_fail_record(P, fst + k0 + k, d);
-            }
+        if (PR == kPivotChol4 && s_fail < kNB) {
+            failed = s_fail;
             break;
         }
-        const double rd = rdv[k];
-        double vj[R];
+        if (rest <= 0) continue;
+        // A[i][j] -= sum_k L[i][k] W[j][k] on the lower 8x8 tiles of what follows
+        const int nt = (rest + 7) >> 3, r0 = c0 + kDG;
+        for (int t = warp; t < nt * (nt + 1) / 2; t += 8) {
+            int ti = 0, u = t;
+            while (u > ti) u -= ++ti;
+            const int i = r0 + 8 * ti + (lane >> 2), j = r0 + 8 * u + (lane >> 2);
+            const int jc = r0 + 8 * u + 2 * (lane & 3);
+            double c[2] = {0.0, 0.0};
 #pragma unroll
-        for (int b = 0; b < R; ++b) vj[b] = vec[buf][ty + 16 * b];
-#pragma unroll
-        for (int a = 0; a < R; ++a) {
-            const double aik = vec[buf][tx + 16 * a] * rd;
-#pragma unroll
-            for (int b = 0; b < R; ++b)
-                if (ty + 16 * b > k) v[a][b] -= aik * vj[b];
+            for (int kk = 0; kk < kDG; kk += 4)
+                gemm::dmma(c[0], c[1], i < nb ? A[i][c0 + kk + (lane & 3)] : 0.0, j < nb ? Wp[j][kk + (lane & 3)] : 0.0);
+            if (i < nb) {
+                if (i >= jc) A[i][jc] -= c[0];
+                if (i >= jc + 1) A[i][jc + 1] -= c[1];
+            }
         }
-      }
-    }
-    // the first failing pivot (sprfc1.f:1274-1279), for the rules tested here
-    if (PR == kPivotLDL || PR == kPivotChol) {
         __syncthreads();
+    }
+    // the first failing pivot (sprfc1.f:1274-1279), for the rules tested here (the
+    // steps after a failure only computed values that are thrown away)
+    if (PR == kPivotLDL || PR == kPivotChol) {
         if (tid < 32) {
             int f = nb;
             for (int k = tid; k < nb; k += 32)
@@ -879,77 +951,14 @@ __global__ void __launch_bounds__(256) k_diag(const Job* jobs, PV P) {
         }
     }
     if (failed >= 0) return;
-    // L below the diagonal (scaled), d on it
-#pragma unroll
-    for (int a = 0; a < R; ++a)
-#pragma unroll
-        for (int b = 0; b < R; ++b) {
-            const int i = tx + 16 * a, j = ty + 16 * b;
-            if (i >= j && i < nb && j < nb)
-                A[i][j] = (i > j) ? v[a][b] * rdv[j] : ((PR == kPivotReplace || PR == kPivotChol4) ? dd[j] : v[a][b]);
-        }
-    __syncthreads();
-    // X = L^-1 by recursive doubling: after the pass of order b, each aligned
-    // diagonal block of X of order 2b is final, its lower-left quarter being
-    // X21 = -X22 (L21 X11) (X11, X22 from the pass before; unit diagonals).
-    // X is kept transposed in the free upper triangle of A (X[i][j] at A[j][i]),
-    // T = L21 X11 in Tb; 12 barriers instead of one per column.
-    // Each thread takes up to kInvQ elements of a pass and runs their sums side
-    // by side (independent chains), each in the same order as one at a time.
-    constexpr int kInvQ = kNB * kNB / 4 / 256;
-    for (int b = 1; b < kNB; b <<= 1) {
-        const int bb = b * b, tot = (kNB / (2 * b)) * bb;
-        int e_[kInvQ], gi_[kInvQ], gj_[kInvQ], bs_[kInvQ], i_[kInvQ], j_[kInvQ];
-        bool on[kInvQ];
-        double t[kInvQ];
-#pragma unroll
-        for (int q = 0; q < kInvQ; ++q) {
-            const int e = tid + q * (int)blockDim.x;
-            const int kq = e / bb, r = e - kq * bb;
-            e_[q] = e;
-            i_[q] = r / b;
-            j_[q] = r - i_[q] * b;
-            bs_[q] = 2 * kq * b;
-            gi_[q] = bs_[q] + b + i_[q];
-            gj_[q] = bs_[q] + j_[q];
-            on[q] = e < tot && gi_[q] < nb;
-            t[q] = on[q] ? A[gi_[q]][gj_[q]] : 0.0;                // X11[j][j] = 1
-        }
-        for (int m = 1; m < b; ++m)
-#pragma unroll
-            for (int q = 0; q < kInvQ; ++q)                            // L21[i][m] X11[m][j], m > j
-                if (on[q] && m > j_[q]) t[q] += A[gi_[q]][bs_[q] + m] * A[gj_[q]][bs_[q] + m];
-#pragma unroll
-        for (int q = 0; q < kInvQ; ++q)
-            if (e_[q] < tot) Tb[e_[q]] = t[q];
-        __syncthreads();
-        double x[kInvQ];
-#pragma unroll
-        for (int q = 0; q < kInvQ; ++q) x[q] = e_[q] < tot ? Tb[e_[q]] : 0.0;   // X22[i][i] = 1
-        for (int m = 0; m + 1 < b; ++m)
-#pragma unroll
-            for (int q = 0; q < kInvQ; ++q)                            // X22[i][m] T[m][j], m < i
-                if (e_[q] < tot && m < i_[q])
-                    x[q] += A[bs_[q] + b + m][gi_[q]] * Tb[(e_[q] / bb) * bb + m * b + j_[q]];
-#pragma unroll
-        for (int q = 0; q < kInvQ; ++q)
-            if (e_[q] < tot) A[bs_[q] + j_[q]][gi_[q]] = -x[q];
-        __syncthreads();
-    }
-    double* lv = P.linv + P.linv_off[js] + (int64_t)(k0 / kNB) * kNB * kNB;
-    for (int e = tid; e < kNB * kNB; e += blockDim.x) {
-        const int i = e % kNB, j = e / kNB;
-        lv[e] = (i < nb && j < nb) ? (i > j ? A[j][i] : (i == j ? 1.0 : 0.0)) : 0.0;
-    }
-#pragma unroll
-    for (int a = 0; a < R; ++a)
-#pragma unroll
-        for (int b = 0; b < R; ++b) {
-            const int i = tx + 16 * a, j = ty + 16 * b;
-            if (i >= j && i < nb && j < nb) front[(int64_t)(k0 + i) + (int64_t)(k0 + j) * ld] = A[i][j];
+    // L and D back to the front (final since the last group)
+    if (warp >= 1)
+        for (int e = tid - 32; e < kNB * kNB; e += 224) {
+            const int i = e & (kNB - 1), j = e >> 6;
+            if (i >= j && i < nb) front[(int64_t)(k0 + i) + (int64_t)(k0 + j) * ld] = i == j ? dd[i] : A[i][j];
         }
     if (tid < nb) {
-        const double d = A[tid][tid];
+        const double d = dd[tid];
         P.dvec[fst + k0 + tid] = d;
         if (P.sqd) {
             const double s = sqrt(fabs(d)), e = s > 0.0 ? fma(-s, s, fabs(d)) / (2.0 * s) : 0.0;
@@ -957,15 +966,48 @@ __global__ void __launch_bounds__(256) k_diag(const Job* jobs, PV P) {
             P.sqd[2 * (int64_t)(fst + k0 + tid) + 1] = copysign(1.0, d) * e;
         }
     }
+    if (warp == 4) diag_group_inverse(A, (nb - 1) / kDG * kDG, nb, lane);
+    __syncthreads();
+    // inverses of the aligned diagonal blocks of order 2b from those of order b
+    double* T = pan;                                          // T = L21 X11, (b x b) per pair
+    for (int b = kDG; b < kNB && b < nb; b <<= 1) {
+        const int tb = b >> 3, ldt = b + 4, npair = kNB / (2 * b);
+        for (int t = warp; t < npair * tb * tb; t += 8) {
+            const int bs = t / (tb * tb) * 2 * b, i0 = t / tb % tb * 8, j0 = t % tb * 8;
+            const int gi = bs + b + i0 + (lane >> 2), j = j0 + (lane >> 2);
+            double c[2] = {0.0, 0.0};
+            for (int m0 = j0; m0 < b; m0 += 4) {               // X11[m][j] = 0 for m < j
+                const int m = m0 + (lane & 3);
+                const double x = m > j ? A[bs + j][bs + m] : m == j ? 1.0 : 0.0;
+                gemm::dmma(c[0], c[1], gi < nb ? A[gi][bs + m] : 0.0, x);
+            }
+            double* to = T + (bs / (2 * b)) * b * ldt + (i0 + (lane >> 2)) * ldt + j0 + 2 * (lane & 3);
+            to[0] = c[0];
+            to[1] = c[1];
+        }
+        __syncthreads();
+        for (int t = warp; t < npair * tb * tb; t += 8) {
+            const int bs = t / (tb * tb) * 2 * b, i0 = t / tb % tb * 8, j0 = t % tb * 8;
+            const int i = i0 + (lane >> 2), gb = bs + b;
+            const double* tp = T + (bs / (2 * b)) * b * ldt;
+            double c[2] = {0.0, 0.0};
+            for (int m0 = 0; m0 < i0 + 8; m0 += 4) {           // X22[i][m] = 0 for m > i
+                const int m = m0 + (lane & 3);
+                const double x = m < i ? A[gb + m][gb + i] : m == i ? 1.0 : 0.0;
+                gemm::dmma(c[0], c[1], x, tp[m * ldt + j0 + (lane >> 2)]);
+            }
+            const int jc = bs + j0 + 2 * (lane & 3);
+            A[jc][gb + i] = -c[0];
+            A[jc + 1][gb + i] = -c[1];
+        }
+        __syncthreads();
+    }
+    double* lv = P.linv + P.linv_off[js] + (int64_t)(k0 / kNB) * kNB * kNB;
+    for (int e = tid; e < kNB * kNB; e += blockDim.x) {
+        const int i = e % kNB, j = e / kNB;
+        lv[e] = (i < nb && j < nb) ? (i > j ? A[j][i] : (i == j ? 1.0 : 0.0)) : 0.0;
+    }
 }
-
-namespace gemm {
-__device__ __forceinline__ void dmma(double& c0, double& c1, double a, double b) {
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-                 : "+d"(c0), "+d"(c1)
-                 : "d"(a), "d"(b));
-}
-}  // namespace gemm
 
 // Panel TRSM as a product with the stored inverse: for a 64-row block of the
 // rows below the diagonal block, W = A21 X' (X = L11^-1), L21 = W D^-1.
