@@ -204,9 +204,10 @@ int spr_b200_recip_check(const double* x, int64_t n, double* out);
 int spr_b200_autotune_tiles(void* handle, const double* d_sm_assembled, double* out);
 /* Sets that tile explicitly (64 or 32). */
 int spr_b200_set_small_tile(void* handle, int tile);
-/* FP64 mode: Schur-update launches of at least this many flops run on the
- * integer tensor cores as sums of 8-bit digit products (3e9 by default; 0: all
- * trailing and K = S updates, infinity: none). */
+/* FP64 mode: Schur-update launches of at least this many flops (in fronts with
+ * at least 1024 rows to update and 128 columns) run on the integer tensor cores as
+ * sums of 8-bit digit products (1e9 by default; 0: all such trailing and K = S
+ * updates, infinity: none). */
 int spr_b200_set_int_min(void* handle, double flops);
 /* Mixed mode: out[0] = algorithmic flops of the Schur updates that run on the
  * tensor cores (trailing columns beyond the next super-panel, K = S updates),

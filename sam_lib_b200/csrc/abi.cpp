@@ -1103,8 +1103,8 @@ int SPR_API(spr_b200_set_small_tile)(void* handle, int tile) {
 }
 
 // FP64 mode: the Schur updates of launches of at least this many flops run on
-// the integer tensor cores (0: all of the trailing and K = S updates;
-// infinity: none).
+// the integer tensor cores (0: all of the trailing and K = S updates that have
+// the rows and columns for it; infinity: none).
 int SPR_API(spr_b200_set_int_min)(void* handle, double flops) {
     if (!handle || !(flops >= 0.0)) return -2;
     static_cast<Engine*>(handle)->set_int_min(flops);

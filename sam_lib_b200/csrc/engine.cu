@@ -766,7 +766,8 @@ __device__ __forceinline__ void dmma(double& c0, double& c1, double a, double b)
 // columns after the group are updated with DMMA tiles (K = 16) by all warps.
 // The inverse of each group's 16x16 triangle is formed beside the next group's
 // elimination, and the 32- and 64-wide inverses by doubling (X21 = -X22 (L21 X11))
-// with DMMA.  32^3, one block: 39 us with 256 threads in lockstep, one barrier
+// with DMMA.  Every entry takes its multiply-adds in ascending k (DMMA chains
+// them in that order), so the factors do not depend on the grouping.  32^3, one block: 39 us with 256 threads in lockstep, one barrier
 // per column.
 constexpr int kDG = 16;                              // columns of a group
 constexpr int kDPanLd = kDG + 4;                     // bank-conflict-free DMMA fragments
@@ -826,25 +827,35 @@ __device__ __forceinline__ int diag_group(const PV& P, int js, int k0, int c0, i
     return -1;
 }
 
-// inverse of the unit-lower kDG x kDG block at c0 by one warp: lane j < 16 forms
-// column j; X[i][j] goes to A[c0 + j][c0 + i] (the free upper triangle)
-__device__ __forceinline__ void diag_group_inverse(double (*A)[kNB + 1], int c0, int nb, int lane) {
-    double x[kDG];
+// inverse of the unit-lower kDG x kDG block at c0 by one warp: doubling from
+// order b = 1 (X21 = -X22 (L21 X11)); X[i][j] goes to A[c0 + j][c0 + i] (the free
+// upper triangle), T = L21 X11 through t
+__device__ __forceinline__ void diag_group_inverse(double (*A)[kNB + 1], double* t, int c0, int nb, int lane) {
 #pragma unroll
-    for (int i = 0; i < kDG; ++i) {
-        double s0 = 0.0, s1 = 0.0;
+    for (int b = 1; b < kDG; b <<= 1) {
+        const int bb = b * b, tot = kDG / 2 * b;
+        for (int e = lane; e < tot; e += 32) {
+            const int bs = c0 + e / bb * 2 * b, i = e % bb / b, j = e % b;
+            double v = 0.0;
+            if (bs + b + i < nb) {
+                v = A[bs + b + i][bs + j];                                 // X11[j][j] = 1
 #pragma unroll
-        for (int m = 0; m < i; ++m) {
-            const double l = (c0 + i < nb) ? A[c0 + i][c0 + m] : 0.0;
-            if (m & 1) s1 += l * x[m];
-            else s0 += l * x[m];
+                for (int m = 1; m < b; ++m)
+                    if (m > j) v = fma(A[bs + b + i][bs + m], A[bs + j][bs + m], v);
+            }
+            t[e] = v;
         }
-        x[i] = i == lane ? 1.0 : i < lane ? 0.0 : -(s0 + s1);
-    }
-    __syncwarp();
+        __syncwarp();
+        for (int e = lane; e < tot; e += 32) {
+            const int bs = c0 + e / bb * 2 * b, i = e % bb / b, j = e % b;
+            double v = t[e];                                               // X22[i][i] = 1
 #pragma unroll
-    for (int i = 0; i < kDG; ++i)
-        if (lane < i && lane < kDG) A[c0 + lane][c0 + i] = x[i];
+            for (int m = 0; m + 1 < b; ++m)
+                if (m < i) v = fma(A[bs + b + m][bs + b + i], t[e / bb * bb + m * b + j], v);
+            A[bs + j][bs + b + i] = -v;
+        }
+        __syncwarp();
+    }
 }
 
 template <int PR>
@@ -852,6 +863,7 @@ __global__ void __launch_bounds__(256) k_diag(const Job* jobs, PV P) {
     __shared__ double A[kNB][kNB + 1];      // L (lower, d on the diagonal), X transposed above
     __shared__ double pan[kNB / 2 * (kNB / 2 + 4)];   // W of a group's rows below (16 .. 63); later T
     __shared__ double colbuf[3][2 * kDG];
+    __shared__ double tinv[kDG * kDG / 4];
     __shared__ double rdv[kNB];
     __shared__ double dd[kNB];
     __shared__ double adv[kNB];
@@ -886,7 +898,7 @@ __global__ void __launch_bounds__(256) k_diag(const Job* jobs, PV P) {
             const int f = diag_group<PR>(P, js, k0, c0, kmax, warp, lane, nb, A, Wp, colbuf[warp], dd, rdv, adv);
             if (PR == kPivotChol4 && f >= 0 && lane == 0) s_fail = f;     // every warp finds the same column
         } else if (warp == 4 && c0 > 0) {
-            diag_group_inverse(A, c0 - kDG, nb, lane);
+            diag_group_inverse(A, tinv, c0 - kDG, nb, lane);
         }
         __syncthreads();
         if (PR == kPivotChol4 && s_fail < kNB) {
@@ -901,13 +913,13 @@ __global__ void __launch_bounds__(256) k_diag(const Job* jobs, PV P) {
             while (u > ti) u -= ++ti;
             const int i = r0 + 8 * ti + (lane >> 2), j = r0 + 8 * u + (lane >> 2);
             const int jc = r0 + 8 * u + 2 * (lane & 3);
-            double c[2] = {0.0, 0.0};
+            double c[2] = {i < nb && i >= jc ? A[i][jc] : 0.0, i < nb && i > jc ? A[i][jc + 1] : 0.0};
 #pragma unroll
             for (int kk = 0; kk < kDG; kk += 4)
-                gemm::dmma(c[0], c[1], i < nb ? A[i][c0 + kk + (lane & 3)] : 0.0, j < nb ? Wp[j][kk + (lane & 3)] : 0.0);
+                gemm::dmma(c[0], c[1], i < nb ? -A[i][c0 + kk + (lane & 3)] : 0.0, j < nb ? Wp[j][kk + (lane & 3)] : 0.0);
             if (i < nb) {
-                if (i >= jc) A[i][jc] -= c[0];
-                if (i >= jc + 1) A[i][jc + 1] -= c[1];
+                if (i >= jc) A[i][jc] = c[0];
+                if (i > jc) A[i][jc + 1] = c[1];
             }
         }
         __syncthreads();
@@ -966,7 +978,7 @@ __global__ void __launch_bounds__(256) k_diag(const Job* jobs, PV P) {
             P.sqd[2 * (int64_t)(fst + k0 + tid) + 1] = copysign(1.0, d) * e;
         }
     }
-    if (warp == 4) diag_group_inverse(A, (nb - 1) / kDG * kDG, nb, lane);
+    if (warp == 4) diag_group_inverse(A, tinv, (nb - 1) / kDG * kDG, nb, lane);
     __syncthreads();
     // inverses of the aligned diagonal blocks of order 2b from those of order b
     double* T = pan;                                          // T = L21 X11, (b x b) per pair
@@ -990,11 +1002,10 @@ __global__ void __launch_bounds__(256) k_diag(const Job* jobs, PV P) {
             const int bs = t / (tb * tb) * 2 * b, i0 = t / tb % tb * 8, j0 = t % tb * 8;
             const int i = i0 + (lane >> 2), gb = bs + b;
             const double* tp = T + (bs / (2 * b)) * b * ldt;
-            double c[2] = {0.0, 0.0};
+            double c[2] = {tp[i * ldt + j0 + 2 * (lane & 3)], tp[i * ldt + j0 + 2 * (lane & 3) + 1]};   // X22[i][i] = 1
             for (int m0 = 0; m0 < i0 + 8; m0 += 4) {           // X22[i][m] = 0 for m > i
                 const int m = m0 + (lane & 3);
-                const double x = m < i ? A[gb + m][gb + i] : m == i ? 1.0 : 0.0;
-                gemm::dmma(c[0], c[1], x, tp[m * ldt + j0 + (lane >> 2)]);
+                gemm::dmma(c[0], c[1], m < i ? A[gb + m][gb + i] : 0.0, tp[m * ldt + j0 + (lane >> 2)]);
             }
             const int jc = bs + j0 + 2 * (lane & 3);
             A[jc][gb + i] = -c[0];
@@ -2968,9 +2979,8 @@ void Engine::set_int_min(double flops) {
     i8_min_flops_ = flops;
     any_i8_ = false;
     for (const LevelPlan& lp : P_.levels) {
-        for (size_t st = 0; st < lp.trail_i8.size(); ++st)
-            any_i8_ |= lp.trail_i8[st].gemm.ntasks > 0 && lp.next_flops[st] + lp.far_flops[st] >= flops;
-        any_i8_ |= !lp.outer_i8.empty() && lp.outer_flops >= flops;
+        for (const I8Launch& t : lp.trail_i8) any_i8_ |= t.gemm.ntasks > 0 && t.flops >= flops;
+        any_i8_ |= !lp.outer_i8.empty() && lp.outer_i8[0].flops >= flops;
     }
 }
 
@@ -3348,8 +3358,7 @@ void Engine::enqueue_factor(const PV& pv, cudaStream_t s, std::vector<cudaEvent_
             }
             const bool has_far = !lp.far[st].empty() || !lp.far_tc[st].empty();
             const bool far_tc = mixed_ == 1 && lp.far_flops[st] >= tc_min_flops_;
-            const bool trail_i8 = use_i8_ && lp.trail_i8[st].gemm.ntasks > 0 &&
-                                  lp.next_flops[st] + lp.far_flops[st] >= i8_min_flops_;
+            const bool trail_i8 = use_i8_ && lp.trail_i8[st].gemm.ntasks > 0 && lp.trail_i8[st].flops >= i8_min_flops_;
             if (has_far && u != s && !trail_i8) {
                 // the super-panel is final: fork the far columns of its trailing update
                 cudaEvent_t e = D.evpool[evi++];
@@ -3398,6 +3407,7 @@ void Engine::enqueue_factor(const PV& pv, cudaStream_t s, std::vector<cudaEvent_
                     cudaStreamWaitEvent(u, e, 0);
                 }
                 launch_i8_gemm(lp.trail_i8[st].gemm, s, pv, gev, false);
+                for (const Launch& ul : lp.trail_i8[st].rest) launch_gemm(ul, s, pv, gev);
             } else if (mixed_ == 1 && !lp.next_tc[st].empty() && lp.next_flops[st] >= tc_min_flops_) {
                 for (const TcLaunch& t : lp.next_tc[st]) launch_tc(t, s, pv, gev);
                 timing.tc_flops += lp.next_flops[st];
@@ -3415,6 +3425,8 @@ void Engine::enqueue_factor(const PV& pv, cudaStream_t s, std::vector<cudaEvent_
             if (has_far) {
                 if (trail_i8) {
                     launch_i8_gemm(lp.trail_i8[st].far, u, pv, gev, true);
+                    for (const Launch& fl : lp.trail_i8[st].far_rest) launch_gemm(fl, u, pv, gev);
+                    for (const Launch& fl : lp.trail_i8[st].far_rest) launch_gemm(fl, u, pv, gev);
                 } else if (far_tc) {
                     for (const TcLaunch& t : lp.far_tc[st]) launch_tc(t, u, pv, gev, true);
                     timing.tc_flops += lp.far_flops[st];
@@ -3434,10 +3446,13 @@ void Engine::enqueue_factor(const PV& pv, cudaStream_t s, std::vector<cudaEvent_
         if (mixed_ == 1 && lp.outer_flops >= tc_min_flops_) {
             for (const TcLaunch& t : lp.outer_tc) launch_tc(t, s, pv, gev);
             timing.tc_flops += lp.outer_flops;
-        } else if (use_i8_ && lp.outer_flops >= i8_min_flops_) {
+        } else if (use_i8_ && !lp.outer_i8.empty() && lp.outer_i8[0].flops >= i8_min_flops_) {
             for (const I8Launch& t : lp.outer_i8) {
-                launch_i8_split(t, s, pv, gev);
-                launch_i8_gemm(t.gemm, s, pv, gev, false);
+                if (t.gemm.ntasks > 0) {
+                    launch_i8_split(t, s, pv, gev);
+                    launch_i8_gemm(t.gemm, s, pv, gev, false);
+                }
+                for (const Launch& ol : t.rest) launch_gemm(ol, s, pv, gev);
             }
         } else
             for (const Launch& ol : lp.outer) launch_gemm(ol, s, pv, gev);

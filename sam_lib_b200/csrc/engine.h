@@ -239,11 +239,10 @@ private:
                    bool far = false);
     // Trailing and K = S updates of at least this many flops a launch run on
     // the integer tensor cores.  Factor ms at 16^3 / 20^3 / 24^3 / 32^3 with the
-    // line at 1e8: 6.81 11.89 19.00 44.4, 1e9: 6.80 11.47 18.47 44.0, 3e9:
-    // 6.79 11.47 18.38 43.4, 1e10: 6.79 11.71 18.80 44.5, none: 6.79 11.71
-    // 19.69 55.7; below it the split and the 7.5 us tiles cost more than the
-    // FP64 kernel's small ones.
-    double i8_min_flops_ = 3e9;
+    // line at 3e8: 5.55 9.32 14.86 34.9, 1e9: 5.55 9.32 14.82 34.9, 3e9: 5.58
+    // 9.39 14.94 34.9, 1e10: 5.57 9.82 15.69 36.6, none: 5.61 9.83 16.90 50.9;
+    // below it the split and the 7 us tiles cost what the products save.
+    double i8_min_flops_ = 1e9;
     int i8_far_q_ = 6;            // side-stream launches: eighths of the SMs (48^3: 4 320, 6 303, 8 307 ms)
     bool any_i8_ = false;         // the plan has such an update
     bool use_i8_ = false;         // and this factorisation runs them so

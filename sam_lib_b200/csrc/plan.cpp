@@ -378,7 +378,16 @@ int build_plan(const int64_t* mspar, const int64_t* mtrees, const int64_t* msifa
         // jfar, whose first column lies a multiple of kI8TileM after its job's)
         auto emit_i8 = [&](const std::vector<Job>& jl, const std::vector<Job>& jfar, I8Launch& out) {
             int64_t rows = 0, sc = 0;
-            std::vector<Job> base(jl);
+            std::vector<Job> base, small, small_far;
+            for (const Job& j : jl)
+                (j.r_end - j.c0 >= kI8MinRows && j.k_hi - j.k_lo >= kI8MinK ? base : small).push_back(j);
+            for (const Job& j : jfar)
+                for (const Job& k : small)
+                    if (k.node == j.node) small_far.push_back(j);
+            emit_updates(small, out.rest);
+            emit_updates(small_far, out.far_rest);
+            if (base.empty()) return;
+            for (const Job& j : base) out.flops += update_flops(j.c0, j.c_end, j.r_end, j.k_hi - j.k_lo);
             for (Job& j : base) {
                 const int64_t nkb = (j.k_hi - j.k_lo + kI8BK - 1) / kI8BK;
                 j.np = (int32_t)((j.r_end - j.c0 + kI8TileM - 1) / kI8TileM * kI8TileM);
@@ -412,6 +421,8 @@ int build_plan(const int64_t* mspar, const int64_t* mtrees, const int64_t* msifa
                         j.slab = b.slab + (f.c0 - b.c0);
                         j.aux_job = b.aux_job;
                         j.aux = b.aux + (f.c0 - b.c0);
+                        out.flops += update_flops(j.c0, j.c_end, j.r_end, j.k_hi - j.k_lo);
+                        out.flops += update_flops(j.c0, j.c_end, j.r_end, j.k_hi - j.k_lo);
                         add_job(out.far, j, tiles(j));
                     }
             close_launch(out.far);
@@ -571,8 +582,10 @@ int build_plan(const int64_t* mspar, const int64_t* mtrees, const int64_t* msifa
                         jk.push_back(j);
                     }
                 if (jk.empty()) break;
-                lp.outer_i8.emplace_back();
-                emit_i8(jk, {}, lp.outer_i8.back());
+                I8Launch t;
+                emit_i8(jk, {}, t);
+                if (k0 == 0 && t.gemm.ntasks <= 0) break;     // later parts have fewer jobs and columns
+                lp.outer_i8.push_back(t);
             }
         }
         open_launch(lp.writeback);
@@ -638,6 +651,8 @@ int build_plan(const int64_t* mspar, const int64_t* mtrees, const int64_t* msifa
                 build_map(t.split);
                 build_map(t.gemm);
                 build_map(t.far);
+                for (Launch& l : t.rest) build_map(l);
+                for (Launch& l : t.far_rest) build_map(l);
             }
         for (Launch& l : lp.fs_upd) build_map(l);
         for (Launch& l : lp.bs_upd) build_map(l);
@@ -759,6 +774,9 @@ void check_coverage(const Plan& P, int64_t& fp64, int64_t& tc) {
             for (size_t st = 0; st < lp.update.size(); ++st) {
                 if (which == 2 && lp.trail_i8[st].gemm.ntasks > 0) {
                     add(lp.trail_i8[st].gemm);
+                    add(lp.trail_i8[st].far);
+                    for (const Launch& l : lp.trail_i8[st].rest) add(l);
+                    for (const Launch& l : lp.trail_i8[st].far_rest) add(l);
                     continue;
                 }
                 for (const Launch& l : lp.update[st]) add(l);
@@ -770,8 +788,15 @@ void check_coverage(const Plan& P, int64_t& fp64, int64_t& tc) {
                     for (const Launch& l : v) add(l);
                 for (const Launch& l : lp.outer) add(l);
             } else if (which == 2) {
-                for (const I8Launch& t : lp.trail_i8) add(t.far);
-                for (const I8Launch& t : lp.outer_i8) add(t.gemm);
+                for (size_t st = 0; st < lp.far.size(); ++st)
+                    if (lp.trail_i8[st].gemm.ntasks <= 0)
+                        for (const Launch& l : lp.far[st]) add(l);
+                if (lp.outer_i8.empty())
+                    for (const Launch& l : lp.outer) add(l);
+                for (const I8Launch& t : lp.outer_i8) {
+                    add(t.gemm);
+                    for (const Launch& l : t.rest) add(l);
+                }
             } else {
                 for (const auto& v : lp.far_tc)
                     for (const TcLaunch& t : v) add(t.gemm);

@@ -80,8 +80,18 @@ constexpr int kI8TileM = 128, kI8TileN = 64;
 constexpr int kI8BK = 128;
 constexpr int kI8Digits = 7;
 constexpr int kI8MaxK = 16384;
+constexpr int kI8MinRows = 1024;
+constexpr int kI8MinK = 128;
+// Fronts whose update is too small for that (fewer than kI8MinRows rows or
+// kI8MinK columns) stay on the FP64 kernel: rest and far_rest.  A small front
+// has few 128-row tiles, half of them on the diagonal.  Factor ms with the line at
+// 256/128, 512/256, 1024/128, 1024/384 and with none: 512 boxes of 3^3 to 12^3
+// 30.5, 30.2, 30.4, 30.4, 31.8 (no integer update at all: 30.6); 24^3 14.93, 14.92,
+// 14.82, 14.98, 15.07; 32^3 35.2, 35.3, 34.9, 35.8, 35.0.
 struct I8Launch {
     Launch split, gemm, far;
+    std::vector<Launch> rest, far_rest;
+    double flops = 0.0;              // algorithmic flops of gemm and far
 };
 
 struct LevelPlan {

@@ -1,8 +1,9 @@
 """FP64 Schur updates as 8-bit digit products on the integer tensor cores.
 
-Dense fronts whose update sizes fall on and beside the edges of the 128 x 64
-tiles, of the 128-column K blocks and of the 512-column super-panels (odd
-first columns among them), with pivots of both signs and rows scaled over
+Dense fronts whose update sizes fall on and beside the smallest that the digit
+form takes (1024 rows, 128 columns), the edges of the 128 x 64 tiles, of the
+128-column K blocks and of the 512-column super-panels (odd first columns among
+them), with pivots of both signs and rows scaled over
 six decades.  The matrices are diagonally dominant (up to the scaling), so
 elimination does not grow their entries, and with A = S B S, |B_ii| = 1,
 
@@ -52,8 +53,8 @@ def _unpack(sm, neq, mspar, mtrees, msifa):
 
 
 @pytest.mark.parametrize('negative', [False, True])
-@pytest.mark.parametrize('widths', [[64, 128], [65, 127], [200, 64], [129, 193], [513, 1], [640, 65], [576, 700],
-                                    [1025, 130, 400], [1600, 3]])
+@pytest.mark.parametrize('widths', [[128, 1024], [129, 1025], [200, 1087], [255, 1088], [513, 1024], [640, 1089],
+                                    [576, 1200], [1025, 130, 1100], [1600, 1027]])
 def test_digit_updates_reproduce_the_matrix(widths, negative):
     import sam_lib_b200 as spr
     structure = dense_chain(widths)
@@ -79,10 +80,26 @@ def test_digit_updates_reproduce_the_matrix(widths, negative):
     ds.close()
 
 
+def test_levels_with_large_and_small_fronts():
+    """16^3: levels whose fronts go partly to the digit form and partly to the
+    FP64 kernel; the factor within the parity tests' 1e-10 of the general path's."""
+    import sam_lib_b200 as spr
+    from sam_lib_b200.system import HexSystem
+    hs = HexSystem(16)
+    sm = hs.assemble()
+    ds = spr.DeviceSolver(hs.mspar, hs.mtrees, hs.msifa)
+    r, f = _factor(ds, sm, 0.0)
+    launches = ds.info()['launches']
+    rg, fg = _factor(ds, sm, math.inf)
+    assert r['lierr'] == rg['lierr'] == 0 and launches > ds.info()['launches']
+    assert np.abs(f - fg).max() <= 1e-10 * np.abs(fg).max()
+    ds.close()
+
+
 def test_nan_fails_at_the_same_equation():
     import sam_lib_b200 as spr
-    structure = dense_chain([640, 200])
-    a, _, _ = _matrix(840, 3, False)
+    structure = dense_chain([640, 1024])
+    a, _, _ = _matrix(1664, 3, False)
     a[700, 5] = a[5, 700] = math.nan
     sm = pack_dense(a, *structure)
     ds = spr.DeviceSolver(*structure)
@@ -95,8 +112,8 @@ def test_nan_fails_at_the_same_equation():
 def test_a_wait_that_runs_out_is_reported():
     import sam_lib_b200 as spr
     import torch
-    structure = dense_chain([640, 200])
-    a, _, _ = _matrix(840, 4, False)
+    structure = dense_chain([640, 1024])
+    a, _, _ = _matrix(1664, 4, False)
     sm = pack_dense(a, *structure)
     ds = spr.DeviceSolver(*structure)
     ds.set_int_min(0.0)
