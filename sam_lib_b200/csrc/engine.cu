@@ -66,7 +66,8 @@ void trace_point(const char* what) {
         }                                                                        \
     } while (0)
 
-constexpr int kMaxRHS = 16;          // right-hand sides per solve pass
+constexpr int kMaxRHS = 16;          // right-hand sides per CTA of the small fronts and per residual pass
+constexpr int kPassRHS = 48;         // right-hand sides per pass over the factor
 
 // NVTX range for the host timeline of a profiler (no-op without one).
 struct NvtxRange {
@@ -107,11 +108,8 @@ struct PV {
     Stats* st;
     const int64_t* linv_off;
     double* linv;            // inverses of the unit-lower diagonal blocks
-    const int64_t* xinv_off;
-    double* xinv;            // inverses of the kSolveBlock-wide diagonal blocks
     const int64_t* rect_off;
     const int64_t* fwd_off;
-    const int64_t* tri_off;  // first block-ready flag of each large front (solves)
     double tol1;
     // SPRFC3 semantics (sprfc3.f:549-572, 1083-1099): a zero diagonal becomes
     // 1 and a pivot at or below TOL(1)|a_jj| is replaced instead of stopping;
@@ -149,13 +147,10 @@ struct Engine::Dev {
     Job* jobs = nullptr;
     int64_t* linv_off = nullptr;
     double* linv = nullptr;
-    int64_t* xinv_off = nullptr;
-    double* xinv = nullptr;
     int32_t* task_map = nullptr;
     int64_t* rect_off = nullptr;
     int64_t* fwd_off = nullptr;
-    int64_t* tri_off = nullptr;
-    double* pbuf = nullptr;                      // back-solve rectangle partial sums
+    double* pbuf = nullptr;                      // rectangle partial sums of the solves
     int32_t* level_nodes = nullptr;              // small nodes of every level, concatenated
     std::vector<int64_t> small_begin;            // per level offset into level_nodes
     int32_t* all_nodes = nullptr;                // all nodes of every level (solves)
@@ -170,15 +165,14 @@ struct Engine::Dev {
     double* sn_faild = nullptr;
     double* sn_faila = nullptr;
     Stats* st = nullptr;
-    double* vbuf = nullptr;                      // solve front vectors
-    double* vbuf2 = nullptr;                     // solved diagonal blocks (same layout)
-    int64_t vbuf_rhs = 0;
-    double* bbuf = nullptr;                      // contiguous copy of B (ldb = NEQ)
-    int64_t bbuf_rhs = 0;
+    double* vbuf = nullptr;                      // update vectors of the forward sweep
+    double* ybuf = nullptr;                      // solved rows of the large fronts
+    int64_t vbuf_rhs = 0;                        // right-hand sides that vbuf, ybuf and pbuf hold
+    int64_t pass_rhs = kPassRHS;                 // right-hand sides per pass (kMaxRHS once kPassRHS did not fit)
     uint8_t* skip = nullptr;                     // node mask of a split run
     bool skip_on = false;
     int32_t* tri_tasks = nullptr;                // the solves' triangle tasks (node, block)
-    int32_t* tri_sync = nullptr;                 // block-ready flags, then one task counter per level
+    int32_t* tri_sync = nullptr;                 // per level a task counter and an abort word
     std::vector<void*> owned;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     // page-locked, device-mapped mailbox for the few words the host reads
@@ -1539,13 +1533,16 @@ inline size_t small_solve_smem(int maxF, int nrhs) {
 }
 
 __global__ void __launch_bounds__(kSolveThreads)
-k_forward(const int32_t* nodes, PV P, double* vbuf, double* b, int64_t ldb, int nrhs) {
+k_forward(const int32_t* nodes, PV P, double* vbuf, double* b, int64_t ldb, int nrhs_all) {
     extern __shared__ double wsm[];           // w[i * nrhs + r], then Ls[(i - j0) * (kSmallBlk + 1) + c]
     const int js = nodes[blockIdx.x];
     if (node_off(P, js)) return;
     const int F = P.F[js], S = P.S[js], fst = P.fst[js];
+    // this CTA's right-hand sides: kMaxRHS from rg on
+    const int rg = blockIdx.y * kMaxRHS, nrhs = min(kMaxRHS, nrhs_all - rg);
+    b += (int64_t)rg * ldb;
     double* Ls = wsm + (size_t)F * nrhs;
-    double* wg = vbuf + P.rbase[js] * nrhs;   // update rows for the parent (r*F + i)
+    double* wg = vbuf + P.rbase[js] * nrhs_all + (int64_t)rg * F;   // update rows for the parent (r*F + i)
     const double* Lb = P.lnz + P.lnz_off[js];
     const int tid = threadIdx.x, lane = tid & 31;
     for (int e = tid; e < F * nrhs; e += blockDim.x) {
@@ -1554,7 +1551,7 @@ k_forward(const int32_t* nodes, PV P, double* vbuf, double* b, int64_t ldb, int 
         const int64_t e0 = P.cptr[P.rbase[js] + i], e1 = P.cptr[P.rbase[js] + i + 1];
         for (int64_t q = e0; q < e1; ++q) {
             const int c = P.cchild[q], t = P.ct[q];
-            v += vbuf[P.rbase[c] * nrhs + (int64_t)r * P.F[c] + P.S[c] + t];
+            v += vbuf[P.rbase[c] * nrhs_all + (int64_t)(rg + r) * P.F[c] + P.S[c] + t];
         }
         wsm[i * nrhs + r] = v;
     }
@@ -1594,16 +1591,18 @@ k_forward(const int32_t* nodes, PV P, double* vbuf, double* b, int64_t ldb, int 
 }
 
 __global__ void __launch_bounds__(kSolveThreads)
-k_backward(const int32_t* nodes, PV P, double* vbuf, double* b, int64_t ldb, int nrhs) {
+k_backward(const int32_t* nodes, PV P, double* b, int64_t ldb, int nrhs_all) {
     extern __shared__ double wsm[];
     const int js = nodes[blockIdx.x];
     if (node_off(P, js)) return;
     if (is_retained(P, js)) return;
     const int F = P.F[js], S = P.S[js], fst = P.fst[js];
+    // this CTA's right-hand sides: kMaxRHS from rg on
+    const int rg = blockIdx.y * kMaxRHS, nrhs = min(kMaxRHS, nrhs_all - rg);
+    b += (int64_t)rg * ldb;
     double* Ls = wsm + (size_t)F * nrhs;
     const double* Lb = P.lnz + P.lnz_off[js];
     const int tid = threadIdx.x, lane = tid & 31;
-    (void)vbuf;
     // own rows (forward result) and the ancestors' solved rows; the row list
     // of front js starts at rbase[js] (LINDX concatenates the row lists)
     for (int e = tid; e < F * nrhs; e += blockDim.x) {
@@ -1646,42 +1645,43 @@ k_backward(const int32_t* nodes, PV P, double* vbuf, double* b, int64_t ldb, int
 }
 
 // ---------------------------------------------------------------------------
-// Solves of the large fronts: batched like the factorisation, one launch per
-// panel step for all large fronts of a level.  L is read from LNZ (packed).
+// Solves of the large fronts, per tree level: forward k_fwd_tri (rows [0, S))
+// and k_fwd_rect (rows [S, F)), back k_bwd_rect and k_bwd_tri.  L is read
+// from LNZ (packed).  Right-hand sides go in groups of NG = 1, 2 or 4 (nrp in
+// all, with the last group's padding): a group's values of an equation lie
+// together, y[(group * NEQ + equation) * NG + r], so that the groups are
+// independent tasks which share L through L2.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ const double* lcol(const PV& P, int js, int F, int j) {
-    return P.lnz + P.lnz_off[js] + lnz_col(j, F) - j;      // index with the row
+// row i of front js in the forward sweep: own row of B (i < S) plus the
+// children's update vectors, in SPRF12's order
+__device__ __forceinline__ double gather_row(const PV& P, const double* vbuf, const double* b, int64_t ldb, int nrhs,
+                                             int js, int i, int r) {
+    double v = i < P.S[js] ? b[(int64_t)(P.fst[js] + i) + r * ldb] : 0.0;
+    const int64_t e0 = P.cptr[P.rbase[js] + i], e1 = P.cptr[P.rbase[js] + i + 1];
+    for (int64_t e = e0; e < e1; ++e) {
+        const int c = P.cchild[e], t = P.ct[e];
+        v += vbuf[P.rbase[c] * nrhs + (int64_t)r * P.F[c] + P.S[c] + t];
+    }
+    return v;
 }
 
-// gather of the forward sweep: own rows of B plus the children's update vectors
-__global__ void k_fwd_gather(const Job* jobs, int64_t njobs, const int32_t* tmap, int64_t ntasks, PV P, double* vbuf,
-                             const double* b, int64_t ldb, int nrhs) {
+// A retained front passes its gathered sums on: own rows to B, the rest to
+// its parent (thread per row).
+__global__ void k_fwd_retained(const Job* jobs, int64_t njobs, const int32_t* tmap, int64_t ntasks, PV P, double* vbuf,
+                               double* b, int64_t ldb, int nrhs) {
     const int64_t task = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (task >= ntasks) return;
     const Job& jb = job_of(jobs, njobs, tmap, task);
     const int js = jb.node;
-    if (node_off(P, js)) return;
+    if (node_off(P, js) || !is_retained(P, js)) return;
     const int i = (int)(task - jb.task0);
-    const int F = P.F[js], S = P.S[js], fst = P.fst[js];
-    double* w = vbuf + P.rbase[js] * nrhs;
-    const int64_t e0 = P.cptr[P.rbase[js] + i], e1 = P.cptr[P.rbase[js] + i + 1];
     for (int r = 0; r < nrhs; ++r) {
-        double v = (i < S) ? b[(int64_t)(fst + i) + r * ldb] : 0.0;
-        for (int64_t e = e0; e < e1; ++e) {
-            const int c = P.cchild[e], t = P.ct[e];
-            v += vbuf[P.rbase[c] * nrhs + (int64_t)r * P.F[c] + P.S[c] + t];
-        }
-        w[(int64_t)r * F + i] = v;
+        const double v = gather_row(P, vbuf, b, ldb, nrhs, js, i, r);
+        if (i < P.S[js]) b[(int64_t)(P.fst[js] + i) + r * ldb] = v;
+        else vbuf[P.rbase[js] * nrhs + (int64_t)r * P.F[js] + i] = v;
     }
 }
 
-// Solve steps of kSolveBlock (256) columns.  Forward: one CTA per front
-// solves the block's unit-lower triangle (4 diagonal blocks of 64, each a
-// product with its stored inverse X, then the rows below it inside the
-// block), stores the block in ysol; then k_fwd_blk_upd applies it to every
-// row below the block (thread per row, SPRFS6).  Backward mirrors it.
-
-// w[m] -= sum_{c < n} L[row0 + c, m] x[c][.] by one warp (column m of L contiguous)
 // Reduce-scatter of NR per-lane partial sums over a warp: halving exchanges
 // (NR/2 + NR/4 + ... shuffles) then full sums over the remaining lane bits.
 // Returns the total of partial index `rhs`; the lanes whose remaining bits
@@ -1707,555 +1707,352 @@ __device__ __forceinline__ double warp_reduce_scatter(double (&v)[NR], int lane,
     return v[0];
 }
 
-__device__ __forceinline__ void warp_col_dot_smem(const double* cm_row0, int n, const double (*x)[kSolveBlock],
-                                                  double* wm, int64_t F, int nrhs) {
-    const int lane = threadIdx.x & 31;
-    double acc[kMaxRHS];
-#pragma unroll
-    for (int r = 0; r < kMaxRHS; ++r) acc[r] = 0.0;
-    for (int c = lane; c < n; c += 32) {
-        const double l = cm_row0[c];
-#pragma unroll
-        for (int r = 0; r < kMaxRHS; ++r)
-            if (r < nrhs) acc[r] += l * x[r][c];
-    }
-    int r, om;
-    const double v = warp_reduce_scatter<kMaxRHS>(acc, lane, r, om);
-    if ((lane & om) == 0 && r < nrhs) wm[(int64_t)r * F] = __ldcg(wm + (int64_t)r * F) - v;
-}
-
-// In-block update of the back sweep: w[m] -= L[k0:k1, m]' x_block for the
-// columns m in [0, k0) of the block's front (kBwdCols columns per task).
-__device__ void bwd_blk_upd_task(const Job* jobs, int64_t njobs, const int32_t* tmap, int64_t task, const PV& P,
-                                 double* vbuf, const double* xsol, int nrhs, double* sh) {
-    double(*x)[kSolveBlock] = reinterpret_cast<double(*)[kSolveBlock]>(sh);     // RHS-major
-    const Job& jb = job_of(jobs, njobs, tmap, task);
-    const int js = jb.node, k0 = jb.k_lo, k1 = jb.k_hi;
-    const int F = P.F[js], nbk = k1 - k0;
-    const int64_t vb = P.rbase[js] * nrhs;
-    double* w = vbuf + vb;
-    const double* base = P.lnz + P.lnz_off[js];
-    for (int e = threadIdx.x; e < nbk * nrhs; e += blockDim.x) {
-        const int i = e % nbk, r = e / nbk;
-        x[r][i] = __ldcg(xsol + vb + (int64_t)r * F + k0 + i);
-    }
-    __syncthreads();
-    const int m = (int)(task - jb.task0) * kBwdCols + (threadIdx.x >> 5);
-    if (m >= jb.c_end) return;
-    warp_col_dot_smem(base + lnz_col(m, F) - m + k0, nbk, x, w + m, F, nrhs);
-}
-
-constexpr size_t kBwdSmem = sizeof(double) * (size_t)kMaxRHS * kSolveBlock;
-
-__global__ void __launch_bounds__(256) k_bwd_blk_upd(const Job* jobs, int64_t njobs, const int32_t* tmap, PV P, double* vbuf,
-                                                     const double* xsol, int nrhs) {
-    extern __shared__ double bsh[];
-    bwd_blk_upd_task(jobs, njobs, tmap, blockIdx.x, P, vbuf, xsol, nrhs, bsh);
-}
-
-// Inverse X = L_blk^-1 of one kSolveBlock-wide unit-lower diagonal block of a
-// large front, from the stored 64x64 inverses: X_jj = inv(L_jj),
-// X_ij = -X_ii sum_{k=j}^{i-1} L_ik X_kj (64x64 tiles, FP64 CUDA cores).
-// Written column-major (ld = nb) into xinv; used by the block solves.
-constexpr size_t kInvSmem = sizeof(double) * 3 * (size_t)kNB * (kNB + 1);
-
-__device__ void tile_mm(const double (*A)[kNB + 1], const double (*B)[kNB + 1], double acc[4][4], int tid) {
-    const int r0 = (tid & 15) * 4, c0 = (tid >> 4) * 4;
-    for (int k = 0; k < kNB; ++k) {
-        double a[4], b[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            a[u] = A[r0 + u][k];
-            b[u] = B[k][c0 + u];
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-#pragma unroll
-            for (int v = 0; v < 4; ++v) acc[u][v] += a[u] * b[v];
-    }
-}
-
-__global__ void __launch_bounds__(256) k_inv_block(const Job* jobs, PV P) {
-    extern __shared__ double ish[];
-    double(*As)[kNB + 1] = reinterpret_cast<double(*)[kNB + 1]>(ish);
-    double(*Bs)[kNB + 1] = As + kNB;
-    double(*Ts)[kNB + 1] = Bs + kNB;
-    const Job& jb = jobs[blockIdx.x];
-    const int js = jb.node, k0 = jb.k_lo, nb = jb.k_hi - jb.k_lo;
-    if ((P.sn_bad && P.sn_bad[js]) || node_off(P, js)) return;
-    const int F = P.F[js];
-    const double* base = P.lnz + P.lnz_off[js];
-    const double* lv0 = P.linv + P.linv_off[js] + (int64_t)(k0 / kNB) * kNB * kNB;
-    double* X = P.xinv + P.xinv_off[js] + (int64_t)(k0 / kSolveBlock) * kSolveBlock * kSolveBlock;
-    const int tid = threadIdx.x;
-    const int q = (nb + kNB - 1) / kNB;
-    const int r0 = (tid & 15) * 4, c0 = (tid >> 4) * 4;
-    auto xat = [&](int i, int j) -> double& { return X[(int64_t)i + (int64_t)j * nb]; };
-    for (int j = 0; j < q; ++j) {
-        const int sj = min(kNB, nb - kNB * j);
-        // diagonal block and the zero blocks above it
-        for (int e = tid; e < kNB * kNB; e += blockDim.x) {
-            const int a = e % kNB, b = e / kNB;
-            if (a < sj && b < sj) xat(kNB * j + a, kNB * j + b) = lv0[(int64_t)j * kNB * kNB + e];
-        }
-        for (int i = 0; i < j; ++i)
-            for (int e = tid; e < kNB * kNB; e += blockDim.x) {
-                const int a = e % kNB, b = e / kNB;
-                if (kNB * i + a < nb && b < sj) xat(kNB * i + a, kNB * j + b) = 0.0;
-            }
-        __syncthreads();
-        for (int i = j + 1; i < q; ++i) {
-            const int si = min(kNB, nb - kNB * i);
-            double acc[4][4] = {};
-            for (int k = j; k < i; ++k) {
-                const int sk = min(kNB, nb - kNB * k);
-                for (int e = tid; e < kNB * kNB; e += blockDim.x) {
-                    const int a = e % kNB, b = e / kNB;
-                    const int row = k0 + kNB * i + a, col = k0 + kNB * k + b;
-                    As[a][b] = (a < si && b < sk) ? base[lnz_col(col, F) - col + row] : 0.0;
-                    Bs[a][b] = (a < sk && b < sj) ? xat(kNB * k + a, kNB * j + b) : 0.0;
-                }
-                __syncthreads();
-                tile_mm(As, Bs, acc, tid);
-                __syncthreads();
-            }
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-#pragma unroll
-                for (int v = 0; v < 4; ++v) Ts[r0 + u][c0 + v] = acc[u][v];
-            for (int e = tid; e < kNB * kNB; e += blockDim.x) {
-                const int a = e % kNB, b = e / kNB;
-                As[a][b] = (a < si && b < si) ? lv0[(int64_t)i * kNB * kNB + e] : 0.0;
-            }
-            __syncthreads();
-            double acc2[4][4] = {};
-            tile_mm(As, Ts, acc2, tid);
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-#pragma unroll
-                for (int v = 0; v < 4; ++v)
-                    if (r0 + u < si && c0 + v < sj) xat(kNB * i + r0 + u, kNB * j + c0 + v) = -acc2[u][v];
-            __syncthreads();
-        }
-    }
-}
-
-// y_block = X w_block: 32 rows per CTA, 8 warps split the columns
-constexpr size_t kMvSmem = sizeof(double) * ((size_t)kSolveBlock * kMaxRHS + 8 * 32 * (kMaxRHS + 1));
-constexpr size_t kUpdSmem = sizeof(double) * ((size_t)kSolveBlock * kMaxRHS + (size_t)128 * (kMaxRHS + 1));
-
-__device__ void fwd_blk_mv_task(const Job* jobs, int64_t njobs, const int32_t* tmap, int64_t task, const PV& P,
-                                const double* vbuf, double* ysol, int nrhs, double* msh) {
-    double(*wb)[kMaxRHS] = reinterpret_cast<double(*)[kMaxRHS]>(msh);
-    double(*part)[32][kMaxRHS + 1] = reinterpret_cast<double(*)[32][kMaxRHS + 1]>(msh + kSolveBlock * kMaxRHS);
-    const Job& jb = job_of(jobs, njobs, tmap, task);
-    const int js = jb.node, k0 = jb.k_lo, nb = jb.k_hi - jb.k_lo;
-    const int F = P.F[js];
-    const int64_t vb = P.rbase[js] * nrhs;
-    const double* w = vbuf + vb;
-    const double* X = P.xinv + P.xinv_off[js] + (int64_t)(k0 / kSolveBlock) * kSolveBlock * kSolveBlock;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    for (int e = tid; e < nb * nrhs; e += blockDim.x) {
-        const int i = e % nb, r = e / nb;
-        wb[i][r] = __ldcg(w + (int64_t)r * F + k0 + i);
-    }
-    __syncthreads();
-    const int i = (int)(task - jb.task0) * 32 + lane;
-    double acc[kMaxRHS];
-#pragma unroll
-    for (int r = 0; r < kMaxRHS; ++r) acc[r] = 0.0;
-    if (i < nb) {
-        const int m1 = min(32 * warp + 32, i + 1);
-        for (int m = 32 * warp; m < m1; ++m) {
-            const double x = X[(int64_t)i + (int64_t)m * nb];
-#pragma unroll
-            for (int r = 0; r < kMaxRHS; ++r)
-                if (r < nrhs) acc[r] += x * wb[m][r];
-        }
-    }
-#pragma unroll
-    for (int r = 0; r < kMaxRHS; ++r)
-        if (r < nrhs) part[warp][lane][r] = acc[r];
-    __syncthreads();
-    if (warp == 0 && i < nb)
-        for (int r = 0; r < nrhs; ++r) {
-            double v = 0.0;
-            for (int g = 0; g < 8; ++g) v += part[g][lane][r];
-            ysol[vb + (int64_t)r * F + k0 + i] = v;
-        }
-}
-
-__global__ void __launch_bounds__(256) k_fwd_blk_mv(const Job* jobs, int64_t njobs, const int32_t* tmap, PV P, const double* vbuf,
-                                                    double* ysol, int nrhs) {
-    extern __shared__ double msh[];
-    fwd_blk_mv_task(jobs, njobs, tmap, blockIdx.x, P, vbuf, ysol, nrhs, msh);
-}
-
-// x_block = X' w_block: 32 columns per CTA, 4 per warp, lanes over rows
-__device__ void bwd_blk_mv_task(const Job* jobs, int64_t njobs, const int32_t* tmap, int64_t task, const PV& P,
-                                const double* vbuf, double* xsol, int nrhs, double* sh) {
-    double(*wb)[kSolveBlock] = reinterpret_cast<double(*)[kSolveBlock]>(sh);     // RHS-major
-    const Job& jb = job_of(jobs, njobs, tmap, task);
-    const int js = jb.node, k0 = jb.k_lo, nb = jb.k_hi - jb.k_lo;
-    const int F = P.F[js];
-    const int64_t vb = P.rbase[js] * nrhs;
-    const double* w = vbuf + vb;
-    const double* X = P.xinv + P.xinv_off[js] + (int64_t)(k0 / kSolveBlock) * kSolveBlock * kSolveBlock;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    for (int e = tid; e < nb * nrhs; e += blockDim.x) {
-        const int i = e % nb, r = e / nb;
-        wb[r][i] = __ldcg(w + (int64_t)r * F + k0 + i);
-    }
-    __syncthreads();
-    for (int cc = 0; cc < 4; ++cc) {
-        const int c = (int)(task - jb.task0) * 32 + warp * 4 + cc;
-        if (c >= nb) break;
-        double acc[kMaxRHS];
-#pragma unroll
-        for (int r = 0; r < kMaxRHS; ++r) acc[r] = 0.0;
-        for (int m = c + lane; m < nb; m += 32) {
-            const double x = X[(int64_t)m + (int64_t)c * nb];
-#pragma unroll
-            for (int r = 0; r < kMaxRHS; ++r)
-                if (r < nrhs) acc[r] += x * wb[r][m];
-        }
-        int r, om;
-        const double v = warp_reduce_scatter<kMaxRHS>(acc, lane, r, om);
-        if ((lane & om) == 0 && r < nrhs) xsol[vb + (int64_t)r * F + k0 + c] = v;
-    }
-}
-
-__global__ void __launch_bounds__(256) k_bwd_blk_mv(const Job* jobs, int64_t njobs, const int32_t* tmap, PV P, const double* vbuf,
-                                                    double* xsol, int nrhs) {
-    extern __shared__ double bsh[];
-    bwd_blk_mv_task(jobs, njobs, tmap, blockIdx.x, P, vbuf, xsol, nrhs, bsh);
-}
-
-// rows below a solve block: w[i] -= L[i, k0:k1] y; 128 rows per CTA, the two
-// halves of the 256 columns summed through shared memory
-__device__ void fwd_blk_upd2_task(const Job* jobs, int64_t njobs, const int32_t* tmap, int64_t task, const PV& P,
-                                  double* vbuf, const double* ysol, int nrhs, double* ush) {
-    double(*y)[kMaxRHS] = reinterpret_cast<double(*)[kMaxRHS]>(ush);
-    double(*part)[kMaxRHS + 1] = reinterpret_cast<double(*)[kMaxRHS + 1]>(ush + kSolveBlock * kMaxRHS);
-    const Job& jb = job_of(jobs, njobs, tmap, task);
-    const int js = jb.node, k0 = jb.k_lo, k1 = jb.k_hi;
-    const int F = P.F[js], nbk = k1 - k0;
-    const int64_t vb = P.rbase[js] * nrhs;
-    double* w = vbuf + vb;
-    const double* base = P.lnz + P.lnz_off[js];
-    const int tid = threadIdx.x;
-    for (int e = tid; e < nbk * nrhs; e += blockDim.x) {
-        const int i = e % nbk, r = e / nbk;
-        y[i][r] = __ldcg(ysol + vb + (int64_t)r * F + k0 + i);
-    }
-    __syncthreads();
-    const int row = tid & (kSolveRows - 1), half = tid / kSolveRows;
-    const int i = jb.c0 + (int)(task - jb.task0) * kSolveRows + row;
-    double acc[kMaxRHS];
-#pragma unroll
-    for (int r = 0; r < kMaxRHS; ++r) acc[r] = 0.0;
-    const int hc = (nbk + 1) / 2;
-    const int r_end = jb.r_end;
-    if (i < r_end) {
-        const int c0 = half * hc, c1 = min(nbk, c0 + hc);
-#pragma unroll 8
-        for (int c = c0; c < c1; ++c) {
-            const int col = k0 + c;
-            const double l = base[lnz_col(col, F) - col + i];
-#pragma unroll
-            for (int r = 0; r < kMaxRHS; ++r)
-                if (r < nrhs) acc[r] += l * y[c][r];
-        }
-    }
-    if (half == 1)
-#pragma unroll
-        for (int r = 0; r < kMaxRHS; ++r)
-            if (r < nrhs) part[row][r] = acc[r];
-    __syncthreads();
-    if (half == 0 && i < r_end)
-#pragma unroll
-        for (int r = 0; r < kMaxRHS; ++r)
-            if (r < nrhs) w[(int64_t)r * F + i] = __ldcg(w + (int64_t)r * F + i) - (acc[r] + part[row][r]);
-}
-
-__global__ void __launch_bounds__(256) k_fwd_blk_upd2(const Job* jobs, int64_t njobs, const int32_t* tmap, PV P,
-                                                      double* vbuf, const double* ysol, int nrhs) {
-    extern __shared__ double ush[];
-    fwd_blk_upd2_task(jobs, njobs, tmap, blockIdx.x, P, vbuf, ysol, nrhs, ush);
-}
-
-
-// forward sweep, rows [S, F): w[i] -= sum_{c < S} L[i][c] y[c].  Phase 1: one
-// CTA per (kRectRows rows, kRectCols columns) tile, a thread per row, writes
-// the tile's partial sums; phase 2 (k_fwd_rect_sum) adds the column tiles'
-// partials of each row in a fixed order (deterministic).
-template <int NR>
-__global__ void __launch_bounds__(256) k_fwd_rect_part(const Job* jobs, int64_t njobs, const int32_t* tmap, PV P,
-                                                       const double* ysol, double* pbuf, int nrhs) {
-    __shared__ double ys[kRectCols][kMaxRHS];
+// Forward sweep, rows [S, F): w[i] = gathered[i] - sum_{c < S} L[i][c] y[c].
+// One CTA per tile and M groups of right-hand sides.  Fronts of at most
+// kFwdNarrow columns (most of them): 256 rows, a thread per row, all columns.
+// Wider ones: kFwdRows rows x kFwdCols columns, a thread per row and quarter of the
+// columns, the quarters added in shared memory; a front of one column tile is
+// finished here, with several each tile writes its partial sums and
+// k_fwd_rect_sum adds them in a fixed order.  Latency bounds it in all but the
+// largest levels (loads of L go in unpredicated batches: 48^3, 4 right-hand
+// sides 2.0 ms, 3.4 ms with a test per load).  Every front with 64-column tiles and
+// partials, a launch to add them and launches to gather before and to finish
+// after took 3.5 ms there, and on 512 boxes of 3^3 to 12^3 with 16 right-hand
+// sides 4.5 ms (now 1.9 ms).
+template <int NG, int M>
+__global__ void __launch_bounds__(256, M > 1 ? 3 : 4) k_fwd_rect(const Job* jobs, int64_t njobs, const int32_t* tmap, PV P,
+                                                  const double* y, double* vbuf, double* pbuf, int nrhs, int nrp,
+                                                  int64_t neq) {
+    constexpr int NR = NG * M;
+    constexpr int LB = NR >= 4 ? 8 : 16;                       // loads of L in flight per thread
+    __shared__ __align__(16) double ys[kFwdCols * NR];
+    __shared__ double part[M == 1 ? 4 : 3][NR][kFwdRows];
     const int64_t task = blockIdx.x;
     const Job& jb = job_of(jobs, njobs, tmap, task);
     const int js = jb.node;
     if (node_off(P, js)) return;
-    const int F = P.F[js], S = P.S[js];
-    const int ncc = jb.k_hi;
+    const int F = P.F[js], S = P.S[js], fst = P.fst[js];
+    const int ncc = jb.k_hi, g0 = blockIdx.y * M;                 // first group
     const int64_t u = task - jb.task0;
     const int cc = (int)(u % ncc), rc = (int)(u / ncc);
-    const int64_t vb = P.rbase[js] * nrhs;
     const int tid = threadIdx.x;
-    const int rbeg = S + rc * kRectRows, nr = min(kRectRows, F - rbeg);
-    const int cbeg = cc * kRectCols, ncol = min(kRectCols, S - cbeg);
-    for (int e = tid; e < ncol * nrhs; e += blockDim.x) {
-        const int c = e % ncol, r = e / ncol;
-        ys[c][r] = ysol[vb + (int64_t)r * F + cbeg + c];
+    const bool narrow = S <= kFwdNarrow;
+    const int row = narrow ? tid : tid & (kFwdRows - 1), q = narrow ? 0 : tid >> 6;
+    const int i = S + rc * (narrow ? 256 : kFwdRows) + row;
+    const int cbeg = cc * kFwdCols, ncol = min(kFwdCols, S - cbeg);
+    const int r0 = g0 * NG, nr = min(NR, nrhs - r0);             // this CTA's right-hand sides
+#pragma unroll
+    for (int m = 0; m < M; ++m) {
+        const double* yg = y + ((int64_t)(g0 + m) * neq + fst + cbeg) * NG;
+        for (int e = tid; e < ncol * NG; e += 256)
+            ys[(e / NG) * NR + m * NG + e % NG] = (g0 + m) * NG < nrhs ? yg[e] : 0.0;
+    }
+    // the gathered entries (a chain of dependent loads): a narrow tile's thread
+    // takes all of its row's, a wide one's r = q, q + 4, ..; ahead of L with few
+    // right-hand sides, after it where the registers would cost occupancy
+    double w[NR];
+    if constexpr (M == 1) {
+#pragma unroll
+    for (int r = 0; r < NR; ++r) w[r] = 0.0;
+    if (i < F && ncc == 1) {
+        const int64_t e0 = P.cptr[P.rbase[js] + i], e1 = P.cptr[P.rbase[js] + i + 1];
+        for (int64_t e = e0; e < e1; ++e) {
+            const int c = P.cchild[e], fc = P.F[c];
+            const double* v = vbuf + P.rbase[c] * nrhs + (int64_t)r0 * fc + P.S[c] + P.ct[e];
+            if (narrow) {
+#pragma unroll
+                for (int r = 0; r < NR; ++r)
+                    if (r < nr) w[r] += v[(int64_t)r * fc];
+            } else {
+#pragma unroll
+                for (int k = 0; k < (NR + 3) / 4; ++k)
+                    if (q + 4 * k < nr) w[k] += v[(int64_t)(q + 4 * k) * fc];
+            }
+        }
+    }
     }
     __syncthreads();
-    if (tid >= nr) return;
-    const int i = rbeg + tid;
-    const double* base = P.lnz + P.lnz_off[js];
     double acc[NR];
 #pragma unroll
     for (int r = 0; r < NR; ++r) acc[r] = 0.0;
-#pragma unroll 16
-    for (int c = 0; c < ncol; ++c) {
-        const int col = cbeg + c;
-        const double l = __ldcs(base + lnz_col(col, F) - col + i);
+    if (i < F) {
+        const int c0 = 64 * q, c1 = min(c0 + 64, ncol);
+        const double* p = P.lnz + P.lnz_off[js] + lnz_col(cbeg + c0, F) - (cbeg + c0) + i;
+        int64_t step = F - (cbeg + c0) - 1;                     // to the next column, same row
+        int c = c0;
+        for (; c + LB <= c1; c += LB) {
+            double l[LB];
+#pragma unroll
+            for (int k = 0; k < LB; ++k) {
+                l[k] = __ldg(p);
+                p += step--;
+            }
+#pragma unroll
+            for (int k = 0; k < LB; ++k)
+#pragma unroll
+                for (int r = 0; r < NR; ++r) acc[r] += l[k] * ys[(c + k) * NR + r];
+        }
+        if (c < c1) {
+            double l[LB];
+#pragma unroll
+            for (int k = 0; k < LB; ++k) {
+                l[k] = c + k < c1 ? __ldg(p) : 0.0;
+                p += step--;
+            }
+#pragma unroll
+            for (int k = 0; k < LB; ++k)
+                if (c + k < c1)
+#pragma unroll
+                    for (int r = 0; r < NR; ++r) acc[r] += l[k] * ys[(c + k) * NR + r];
+        }
+    }
+    if constexpr (M > 1) {
+#pragma unroll
+    for (int r = 0; r < NR; ++r) w[r] = 0.0;
+    if (i < F && ncc == 1) {
+        const int64_t e0 = P.cptr[P.rbase[js] + i], e1 = P.cptr[P.rbase[js] + i + 1];
+        for (int64_t e = e0; e < e1; ++e) {
+            const int c = P.cchild[e], fc = P.F[c];
+            const double* v = vbuf + P.rbase[c] * nrhs + (int64_t)r0 * fc + P.S[c] + P.ct[e];
+            if (narrow) {
+#pragma unroll
+                for (int r = 0; r < NR; ++r)
+                    if (r < nr) w[r] += v[(int64_t)r * fc];
+            } else {
+#pragma unroll
+                for (int k = 0; k < (NR + 3) / 4; ++k)
+                    if (q + 4 * k < nr) w[k] += v[(int64_t)(q + 4 * k) * fc];
+            }
+        }
+    }
+    }
+    if (narrow) {
+        if (i >= F) return;
+        double* out = vbuf + P.rbase[js] * nrhs + (int64_t)r0 * F + i;
 #pragma unroll
         for (int r = 0; r < NR; ++r)
-            if (r < nrhs) acc[r] += l * ys[c][r];
+            if (r < nr) out[(int64_t)r * F] = w[r] - acc[r];
+        return;
     }
-    double* part = pbuf + (P.fwd_off[js] + (int64_t)cc * (F - S) + (i - S)) * kMaxRHS;
+    // quarters 1 .. 3 through shared memory (all four when a thread finishes
+    // one right-hand side), then thread (row, q) takes r = q, q + 4, ..
+    if constexpr (M == 1) {
 #pragma unroll
-    for (int r = 0; r < NR; ++r)
-        if (r < nrhs) part[r] = acc[r];
+        for (int r = 0; r < NR; ++r) part[q][r][row] = acc[r];
+        __syncthreads();
+        if (i >= F || q >= nr) return;
+        const double s = (part[0][q][row] + part[1][q][row]) + (part[2][q][row] + part[3][q][row]);
+        if (ncc == 1)
+            vbuf[P.rbase[js] * nrhs + (int64_t)(r0 + q) * F + i] = w[0] - s;
+        else
+            pbuf[(P.fwd_off[js] + (int64_t)cc * (F - S) + (i - S)) * nrp + r0 + q] = s;
+    } else {
+        if (q)
+#pragma unroll
+            for (int r = 0; r < NR; ++r) part[q - 1][r][row] = acc[r];
+        __syncthreads();
+        if (q == 0)
+#pragma unroll
+            for (int r = 0; r < NR; ++r)
+                part[0][r][row] = (acc[r] + part[0][r][row]) + (part[1][r][row] + part[2][r][row]);
+        __syncthreads();
+        if (i >= F) return;
+#pragma unroll
+        for (int k = 0; k < NR / 4; ++k) {
+            const int r = q + 4 * k;
+            if (r >= nr) break;
+            const double s = part[0][r][row];
+            if (ncc == 1)
+                vbuf[P.rbase[js] * nrhs + (int64_t)(r0 + r) * F + i] = w[k] - s;
+            else
+                pbuf[(P.fwd_off[js] + (int64_t)cc * (F - S) + (i - S)) * nrp + r0 + r] = s;
+        }
+    }
 }
 
+// thread per (row, right-hand side) of the fronts with several column tiles
 __global__ void k_fwd_rect_sum(const Job* jobs, int64_t njobs, const int32_t* tmap, int64_t ntasks, PV P, double* vbuf,
-                               const double* pbuf, int nrhs) {
-    const int64_t task = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+                               const double* pbuf, const double* b, int64_t ldb, int nrhs, int nrp) {
+    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int64_t task = t / nrhs;
+    const int r = (int)(t % nrhs);
     if (task >= ntasks) return;
     const Job& jb = job_of(jobs, njobs, tmap, task);
     const int js = jb.node;
     if (node_off(P, js)) return;
     const int F = P.F[js], S = P.S[js];
     const int row = S + (int)(task - jb.task0);
-    const int ncc = (S + kRectCols - 1) / kRectCols;
-    double* w = vbuf + P.rbase[js] * nrhs;
-    const double* part = pbuf + (P.fwd_off[js] + (row - S)) * kMaxRHS;
-    // column tiles in ascending order for every right-hand side; the loads
-    // of several tiles are in flight together
-    double v[kMaxRHS];
-#pragma unroll
-    for (int r = 0; r < kMaxRHS; ++r) v[r] = 0.0;
-#pragma unroll 4
-    for (int k = 0; k < ncc; ++k) {
-        const double* pk = part + (int64_t)k * (F - S) * kMaxRHS;
-#pragma unroll
-        for (int r = 0; r < kMaxRHS; ++r)
-            if (r < nrhs) v[r] += __ldcg(pk + r);
-    }
-#pragma unroll
-    for (int r = 0; r < kMaxRHS; ++r)
-        if (r < nrhs) w[(int64_t)r * F + row] -= v[r];
+    const int ncc = (S + kFwdCols - 1) / kFwdCols;
+    const double* part = pbuf + (P.fwd_off[js] + (row - S)) * nrp + r;
+    const double w = gather_row(P, vbuf, b, ldb, nrhs, js, row, r);
+    double v = 0.0;
+#pragma unroll 8
+    for (int k = 0; k < ncc; ++k) v += __ldcg(part + (int64_t)k * (F - S) * nrp);
+    vbuf[P.rbase[js] * nrhs + (int64_t)r * F + row] = w - v;
 }
 
-// back sweep, update rows [S, F): w[c] -= L[S:F, c]' w[S:F].  Phase 1: one
-// CTA per (kRectCols columns, kRectRows rows) stages its rows of the vector in
-// shared memory once and writes one partial dot product per column (a warp
-// per column at a time, 32 columns per warp); phase 2 (k_bwd_rect_sum) adds
-// the partials of each column in a fixed order, so the result is
-// deterministic.
-template <int NR>
-__global__ void __launch_bounds__(256, NR <= 4 ? 3 : 2) k_bwd_rect_part(const Job* jobs, int64_t njobs, const int32_t* tmap, PV P,
-                                                       const double* vbuf, double* pbuf, int nrhs) {
-    __shared__ double ws[kMaxRHS][kRectRows];
+// Back sweep, update rows [S, F): partial sums of L[S:F, c]' x[S:F].  One CTA
+// per (kRectCols columns, kRectRows rows) and group stages the ancestors'
+// solution rows in shared memory once and writes one partial dot product per
+// column (a warp per CG columns at a time, lanes along the rows); k_bwd_tri adds
+// a column's partials in a fixed order.
+// kOnce: one group, so L is read once
+template <int NG, bool kOnce>
+__global__ void __launch_bounds__(256) k_bwd_rect(const Job* jobs, int64_t njobs, const int32_t* tmap, PV P,
+                                                  double* pbuf, const double* b, int64_t ldb, int nrhs, int nrp) {
+    __shared__ double ws[NG][kRectRows];
+    __shared__ double segs[8][4][NG];
     const int64_t task = blockIdx.x;
     const Job& jb = job_of(jobs, njobs, tmap, task);
     const int js = jb.node;
     if (node_off(P, js)) return;
     const int F = P.F[js], S = P.S[js];
-    const int ncc = jb.k_hi;
+    const int ncc = jb.k_hi, g = blockIdx.y;
     const int64_t u = task - jb.task0;
     const int cc = (int)(u % ncc), rc = (int)(u / ncc);
-    const int64_t vb = P.rbase[js] * nrhs;
-    const double* w = vbuf + vb;
     const double* base = P.lnz + P.lnz_off[js];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int rbeg = S + rc * kRectRows, nr = min(kRectRows, F - rbeg);
-    for (int e = tid; e < nr * nrhs; e += blockDim.x) {
-        const int i = e % nr, r = e / nr;
-        ws[r][i] = w[(int64_t)r * F + rbeg + i];
+    if (tid < nr) {
+        const int64_t row = P.rows[P.rbase[js] + rbeg + tid];
+#pragma unroll
+        for (int r = 0; r < NG; ++r) ws[r][tid] = g * NG + r < nrhs ? b[row + (g * NG + r) * ldb] : 0.0;
     }
     __syncthreads();
-    double* part = pbuf + (P.rect_off[js] + (int64_t)rc * S) * kMaxRHS;
-    const int cw = kRectCols / 8;
-    // CG columns at a time per warp (CG x UR loads in flight per lane)
-    constexpr int CG = NR <= 4 ? 4 : 2;
-    constexpr int UR = NR <= 4 ? 4 : 2;                // row steps in flight
-    for (int a = 0; a < cw; a += CG) {
-        const int c0 = cc * kRectCols + warp * cw + a;
-        if (c0 >= S) break;
+    double* part = pbuf + (P.rect_off[js] + (int64_t)rc * S) * nrp + g * NG;
+    constexpr int cw = kRectCols / 8;
+    constexpr int CG = 4, UR = 4;                      // columns and row steps with loads in flight
+    // a front of few columns has fewer column groups than warps: the warps then
+    // split the rows as well and the segments are added in shared memory
+    const int ncg = (min(S, kRectCols) + CG - 1) / CG, nseg = ncg <= 1 ? 8 : ncg <= 2 ? 4 : ncg <= 4 ? 2 : 1;
+    const int seg = nseg > 1 ? warp % nseg : 0, rows = kRectRows / nseg;
+    const int a1 = nseg > 1 ? CG : cw;
+    for (int a = 0; a < a1; a += CG) {
+        const int c0 = cc * kRectCols + (nseg > 1 ? warp / nseg * CG : warp * cw + a);
+        const bool any = c0 < S;
+        if (!any && nseg == 1) break;
         const double* col[CG];
         bool cv[CG];
 #pragma unroll
         for (int q = 0; q < CG; ++q) {
             cv[q] = c0 + q < S;
-            const int c = cv[q] ? c0 + q : c0;
+            const int c = cv[q] ? c0 + q : min(c0, S - 1);
             col[q] = base + lnz_col(c, F) - c + rbeg;
         }
-        double acc[CG][NR];
+        double acc[CG][NG];
 #pragma unroll
         for (int q = 0; q < CG; ++q)
 #pragma unroll
-            for (int r = 0; r < NR; ++r) acc[q][r] = 0.0;
+            for (int r = 0; r < NG; ++r) acc[q][r] = 0.0;
+        const int i1 = any ? min(nr, (seg + 1) * rows) : 0;
 #pragma unroll(UR)
-        for (int i = lane; i < nr; i += 32) {
+        for (int i = seg * rows + lane; i < i1; i += 32) {
             double l[CG];
 #pragma unroll
-            for (int q = 0; q < CG; ++q) l[q] = __ldcs(col[q] + i);
+            for (int q = 0; q < CG; ++q) l[q] = kOnce ? __ldcs(col[q] + i) : __ldg(col[q] + i);
 #pragma unroll
-            for (int r = 0; r < NR; ++r)
-                if (r < nrhs) {
-                    const double x = ws[r][i];
+            for (int r = 0; r < NG; ++r) {
+                const double x = ws[r][i];
 #pragma unroll
-                    for (int q = 0; q < CG; ++q) acc[q][r] += l[q] * x;
-                }
+                for (int q = 0; q < CG; ++q) acc[q][r] += l[q] * x;
+            }
         }
 #pragma unroll
         for (int q = 0; q < CG; ++q) {
             int r, om;
-            const double v = warp_reduce_scatter<NR>(acc[q], lane, r, om);
-            if ((lane & om) == 0 && cv[q] && r < nrhs) part[(int64_t)(c0 + q) * kMaxRHS + r] = v;
+            const double v = warp_reduce_scatter<NG>(acc[q], lane, r, om);
+            if ((lane & om) == 0) {
+                if (nseg > 1) segs[warp][q][r] = v;
+                else if (cv[q]) part[(int64_t)(c0 + q) * nrp + r] = v;
+            }
         }
     }
-}
-
-// Each column is summed by a group of kSumLanes lanes: lane g of the group
-// adds the row tiles g, g + kSumLanes, ... in ascending order, and the
-// group's partial sums are added by a fixed butterfly (deterministic), so
-// the few row tiles of a column are loaded together instead of one after
-// another.
-constexpr int kSumLanes = 8;
-__device__ __forceinline__ double group_sum(double v) {
-    const unsigned gmask = 0xffu << (threadIdx.x & 31 & ~(kSumLanes - 1));
-#pragma unroll
-    for (int o = kSumLanes / 2; o > 0; o >>= 1) v += __shfl_xor_sync(gmask, v, o, kSumLanes);
-    return v;
-}
-
-__global__ void k_bwd_rect_sum(const Job* jobs, int64_t njobs, const int32_t* tmap, int64_t ntasks, PV P, double* vbuf,
-                               const double* pbuf, int nrhs) {
-    const int64_t gt = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    const int64_t task = gt / kSumLanes;              // the group's lanes share the task
-    const int g = (int)(gt % kSumLanes);
-    if (task >= ntasks) return;
-    const Job& jb = job_of(jobs, njobs, tmap, task);
-    const int js = jb.node;
-    if (node_off(P, js)) return;
-    const int F = P.F[js], S = P.S[js];
-    if (F <= S || is_retained(P, js)) return;
-    const int c = (int)(task - jb.task0);
-    const int nrc = (F - S + kRectRows - 1) / kRectRows;
-    double* w = vbuf + P.rbase[js] * nrhs;
-    const double* part = pbuf + (P.rect_off[js] + c) * kMaxRHS;
-    double v[kMaxRHS];
-#pragma unroll
-    for (int r = 0; r < kMaxRHS; ++r) v[r] = 0.0;
-#pragma unroll 2
-    for (int k = g; k < nrc; k += kSumLanes) {
-        const double* pk = part + (int64_t)k * S * kMaxRHS;
-#pragma unroll
-        for (int r = 0; r < kMaxRHS; ++r)
-            if (r < nrhs) v[r] += __ldcg(pk + r);
-    }
-#pragma unroll
-    for (int r = 0; r < kMaxRHS; ++r)
-        if (r < nrhs) {
-            const double t = group_sum(v[r]);
-            if (g == 0) w[(int64_t)r * F + c] -= t;
+    if (nseg > 1) {
+        __syncthreads();
+        const int e = tid;                                        // (column, right-hand side)
+        if (e < ncg * CG * NG) {
+            const int c = e / NG, r = e % NG;
+            double v = 0.0;
+            for (int k = 0; k < nseg; ++k) v += segs[c / CG * nseg + k][c % CG][r];
+            if (c < S) part[(int64_t)c * nrp + r] = v;
         }
-}
-
-// y_j /= d_j and scatter of the own rows (thread per column)
-// (a retained front passes its gathered sums through: the rows keep them)
-__global__ void k_fwd_finish(const Job* jobs, int64_t njobs, const int32_t* tmap, int64_t ntasks, PV P, const double* ysol,
-                             const double* gathered, double* b, int64_t ldb, int nrhs) {
-    const int64_t task = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (task >= ntasks) return;
-    const Job& jb = job_of(jobs, njobs, tmap, task);
-    const int js = jb.node;
-    if (node_off(P, js)) return;
-    const int j = (int)(task - jb.task0);
-    const int F = P.F[js], fst = P.fst[js];
-    if (is_retained(P, js)) {
-        const double* g = gathered + P.rbase[js] * nrhs;
-        for (int r = 0; r < nrhs; ++r) b[(int64_t)(fst + j) + r * ldb] = g[(int64_t)r * F + j];
-        return;
     }
-    const double* y = ysol + P.rbase[js] * nrhs;
-    const double d = lcol(P, js, F, j)[j];
-    for (int r = 0; r < nrhs; ++r) b[(int64_t)(fst + j) + r * ldb] = y[(int64_t)r * F + j] / d;
 }
 
 // ---------------------------------------------------------------------------
-// Triangles of the solves as one dataflow launch per level.  Task (js, rb) is
-// the 64-row block rb of front js (rows [64 rb, 64 rb + 64) of [0, S)).
-// Forward: y_rb = X_rb (w_rb - sum_{b < rb} L[rb, b] y_b), X_rb = L_rb,rb^-1
-// (the stored 64x64 inverse); backward: x_cb = X_cb' (w_cb - sum_{r > cb}
-// L[r, cb]' x_r).  Persistent CTAs take tasks in order from a counter (forward
-// block-major ascending, backward descending), so a task only waits for
-// tasks taken before it, by CTAs that are running: the waits always end.
+// Triangles of the solves as one dataflow launch per level.  Task (js, rb,
+// group) is the 64-row block rb of front js (rows [64 rb, 64 rb + 64) of [0, S))
+// for one group of right-hand sides.  Forward: y_rb = X_rb (w_rb - sum_{b < rb}
+// L[rb, b] y_b), X_rb = L_rb,rb^-1 (the stored 64x64 inverse), w_rb gathered
+// here, B = D^-1 y; backward: x_cb = X_cb' (w_cb - sum_{r > cb} L[r, cb]' x_r).
+// Persistent CTAs take tasks in order from a counter (forward block-major
+// ascending, backward descending), so a task only waits for tasks taken before
+// it, by CTAs that are running: the waits always end.
+// The chain of a front's blocks bounds it, one hand-over per block, so the
+// values themselves say that they are there: the y array is filled with
+// kNoValue (a NaN no computation produces; a NaN result is stored as
+// another), a consumer thread takes its value with one load, prefetched a block
+// ahead, and repeats it while it is missing.  48^3, 4 right-hand sides: 2.0 and
+// 2.45 ms a sweep; with a flag per block (store, fence, flag; poll, barrier, load)
+// 2.7 and 3.1 ms.  The groups keep one task at 4 right-hand sides: 24^3, 40 of
+// them, both sweeps 1.6 ms in one pass, 10.7 ms in three passes of 16.
 // Each wait is bounded (PV::wait_ns); one that gives up sets
-// Stats::solve_timeout and an abort word every CTA checks, and the host
-// turns it into an error.  Per tile, a thread owns one row (forward) or one
-// column (backward) and a quarter of the 64 columns (rows).
+// Stats::solve_timeout and an abort word every waiting thread checks, and the
+// host turns it into an error.  Per tile, a thread owns one row (forward) or
+// one column (backward) and a quarter of the 64 columns (rows).
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ int ld_acquire(const int* p) {
-    int v;
-    asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+constexpr unsigned long long kNoValue = 0xffffffffffffffffull;
+
+__device__ __forceinline__ double ld_value(const double* p) {
+    double v;
+    asm volatile("ld.relaxed.gpu.global.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
     return v;
 }
-__device__ __forceinline__ void st_release(int* p, int v) {
-    asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+__device__ __forceinline__ void st_value(double* p, double v) {
+    if (v != v) v = __longlong_as_double(0x7ff8000000000000ll);
+    asm volatile("st.relaxed.gpu.global.f64 [%0], %1;" ::"l"(p), "d"(v) : "memory");
 }
+__device__ __forceinline__ bool no_value(double v) { return (unsigned long long)__double_as_longlong(v) == kNoValue; }
 __device__ __forceinline__ unsigned long long tri_now() {
     unsigned long long t;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
     return t;
 }
 
-// thread 0 waits (bounded) for flag; returns false when the launch aborts
-__device__ __forceinline__ bool tri_wait(const int* flag, int* abort_word, const PV& P) {
-    if (ld_acquire(flag)) return true;
+// waits (bounded) for the value at p; ok = false when the launch aborts
+__device__ __forceinline__ double tri_wait(const double* p, int* abort_word, const PV& P, bool& ok) {
     const unsigned long long t0 = tri_now();
-    for (int spin = 0;; ++spin) {
-        if (ld_acquire(flag)) return true;
-        if (ld_acquire(abort_word)) return false;
-        if ((spin & 63) == 63 && tri_now() - t0 > P.wait_ns) {
-            atomicExch(&P.st->solve_timeout, 1);
-            st_release(abort_word, 1);
-            return false;
+    for (int spin = 1;; ++spin) {
+        const double v = ld_value(p);
+        if (!no_value(v)) return v;
+        if ((spin & 15) == 0) {
+            if (*(volatile int*)abort_word) break;
+            if (tri_now() - t0 > P.wait_ns) {
+                atomicExch(&P.st->solve_timeout, 1);
+                atomicExch(abort_word, 1);
+                break;
+            }
         }
-        __nanosleep(64);
     }
+    ok = false;
+    return 0.0;
 }
 
-constexpr int kTriLd = kMaxRHS + 1;
-
-template <int NR>
-__global__ void __launch_bounds__(256) k_fwd_tri(const int32_t* tasks, int ntasks, int32_t* flags, int32_t* counter,
-                                                 PV P, const double* vbuf, double* ysol, int nrhs) {
-    __shared__ double ys[kNB][kTriLd];
-    __shared__ double part[4][kNB][kTriLd];
-    __shared__ int task_sh, ok_sh;
+template <int NG>
+__global__ void __launch_bounds__(256) k_fwd_tri(const int32_t* tasks, int ntasks, int ng, int32_t* counter, PV P,
+                                                 const double* vbuf, double* y, double* b, int64_t ldb, int nrhs,
+                                                 int64_t neq) {
+    __shared__ __align__(16) double ys[2][kNB * NG];
+    __shared__ double part[4][NG][kNB];
+    __shared__ int task_sh;
     int* abort_word = counter + 1;
     const int tid = threadIdx.x, row = tid & (kNB - 1), q = tid >> 6;
     for (;;) {
         if (tid == 0) task_sh = atomicAdd(counter, 1);
         __syncthreads();
         const int t = task_sh;
-        if (t >= ntasks) break;
-        const int js = tasks[2 * t], rb = tasks[2 * t + 1];
+        if (t >= ntasks * ng) break;
+        const int js = tasks[2 * (t / ng)], rb = tasks[2 * (t / ng) + 1], g = t % ng;
         if (node_off(P, js)) {
             __syncthreads();                                          // all have read task_sh
             continue;
@@ -2263,117 +2060,97 @@ __global__ void __launch_bounds__(256) k_fwd_tri(const int32_t* tasks, int ntask
         const int F = P.F[js], S = P.S[js];
         const int r0 = rb * kNB, nrow = min(kNB, S - r0);
         const double* base = P.lnz + P.lnz_off[js];
-        const int64_t vb = P.rbase[js] * nrhs;
-        int32_t* fl = flags + P.tri_off[js];
-        // loads that need no other task: this row's X entries (the product
-        // with the block inverse at the end) and the right-hand side
+        double* yf = y + ((int64_t)g * neq + P.fst[js]) * NG;              // the front's y
+        // what needs no other task: this row's X entries (the product with the
+        // block inverse at the end), the gathered right-hand side and the pivot
         const double* lv = P.linv + P.linv_off[js] + (int64_t)rb * kNB * kNB;
-        constexpr bool kPreX = NR <= 4;                                      // registers allow it
-        double xr[kPreX ? 16 : 1];
-        if constexpr (kPreX) {
+        double xr[16];
 #pragma unroll
-            for (int k = 0; k < 16; ++k) {
-                const int m = 16 * q + k;
-                xr[k] = (m <= row) ? __ldg(lv + row + m * kNB) : 0.0;       // X[row][m], unit lower
-            }
+        for (int k = 0; k < 16; ++k) {
+            const int m = 16 * q + k;
+            xr[k] = (m <= row) ? __ldg(lv + row + m * kNB) : 0.0;         // X[row][m], unit lower
         }
-        double wv[NR];
+        const int rr = g * NG + q;                                        // thread (row, q < NG) finishes entry (row, q)
+        const bool fin = q < NG && row < nrow;
+        double w = 0.0, d = 1.0;
+        if (fin && rr < nrhs) {
+            w = gather_row(P, vbuf, b, ldb, nrhs, js, r0 + row, rr);
+            d = base[lnz_col(r0 + row, F)];
+        }
+        double acc[NG];
 #pragma unroll
-        for (int r = 0; r < NR; ++r)
-            wv[r] = (tid < kNB && row < nrow && r < nrhs) ? __ldcg(vbuf + vb + (int64_t)r * F + r0 + row) : 0.0;
-        double acc[NR];
-#pragma unroll
-        for (int r = 0; r < NR; ++r) acc[r] = 0.0;
+        for (int r = 0; r < NG; ++r) acc[r] = 0.0;
         bool ok = true;
-        for (int b = 0; b < rb; ++b) {
-            // this thread's 16 entries of the tile L[rb, b] first: they do not
-            // depend on block b, so their latency overlaps the wait for it
+        double next = (tid < kNB * NG && rb > 0) ? ld_value(yf + tid) : 0.0;
+        for (int blk = 0; blk < rb; ++blk) {
+            // this thread's 16 entries of the tile L[rb, blk], ahead of the wait
             double lr[16];
             {
-                const int c0 = kNB * b + 16 * q;
-                int64_t p = lnz_col(c0, F) - c0 + r0 + row;           // L[r0 + row][c0]
+                const int c0 = kNB * blk + 16 * q;
+                int64_t p = lnz_col(c0, F) - c0 + r0 + row;               // L[r0 + row][c0]
 #pragma unroll
                 for (int k = 0; k < 16; ++k) {
                     lr[k] = (row < nrow) ? __ldg(base + p) : 0.0;
-                    p += F - (c0 + k) - 1;                            // next column, same row
+                    p += F - (c0 + k) - 1;                                // next column, same row
                 }
             }
-            if (tid == 0) ok_sh = tri_wait(fl + b, abort_word, P);
-            __syncthreads();
-            if (!ok_sh) {
+            double* yb = ys[blk & 1];
+            if (tid < kNB * NG) {
+                const double* at = yf + (int64_t)kNB * NG * blk + tid;
+                double v = next;
+                if (no_value(v)) v = tri_wait(at, abort_word, P, ok);
+                yb[tid] = v;
+                if (blk + 1 < rb) next = ld_value(at + kNB * NG);
+            }
+            if (!__syncthreads_and(ok)) {
                 ok = false;
                 break;
             }
-            for (int e = tid; e < kNB * nrhs; e += blockDim.x) {
-                const int i = e & (kNB - 1), r = e >> 6;
-                ys[i][r] = __ldcg(ysol + vb + (int64_t)r * F + kNB * b + i);
-            }
-            __syncthreads();
 #pragma unroll
             for (int k = 0; k < 16; ++k)
 #pragma unroll
-                for (int r = 0; r < NR; ++r)
-                    if (r < nrhs) acc[r] += lr[k] * ys[16 * q + k][r];
-            __syncthreads();
+                for (int r = 0; r < NG; ++r) acc[r] += lr[k] * yb[(16 * q + k) * NG + r];
         }
         if (!ok) break;
         // v = w - sum of the four quarters, then y = X v
 #pragma unroll
-        for (int r = 0; r < NR; ++r)
-            if (r < nrhs) part[q][row][r] = acc[r];
+        for (int r = 0; r < NG; ++r) part[q][r][row] = acc[r];
         __syncthreads();
-        if (tid < kNB)
-#pragma unroll
-            for (int r = 0; r < NR; ++r)
-                if (r < nrhs)
-                    ys[row][r] = (row < nrow) ? wv[r] - ((part[0][row][r] + part[1][row][r]) +
-                                                         (part[2][row][r] + part[3][row][r]))
-                                              : 0.0;
+        if (q < NG) ys[0][row * NG + q] = w - ((part[0][q][row] + part[1][q][row]) + (part[2][q][row] + part[3][q][row]));
         __syncthreads();
 #pragma unroll
-        for (int r = 0; r < NR; ++r) acc[r] = 0.0;
+        for (int r = 0; r < NG; ++r) acc[r] = 0.0;
 #pragma unroll
-        for (int k = 0; k < 16; ++k) {
-            double x;
-            if constexpr (kPreX) {
-                x = xr[k];
-            } else {
-                const int m = 16 * q + k;
-                x = (m <= row) ? __ldg(lv + row + m * kNB) : 0.0;
-            }
+        for (int k = 0; k < 16; ++k)
 #pragma unroll
-            for (int r = 0; r < NR; ++r)
-                if (r < nrhs) acc[r] += x * ys[16 * q + k][r];
+            for (int r = 0; r < NG; ++r) acc[r] += xr[k] * ys[0][(16 * q + k) * NG + r];
+#pragma unroll
+        for (int r = 0; r < NG; ++r) part[q][r][row] = acc[r];
+        __syncthreads();
+        if (fin) {
+            const double v = (part[0][q][row] + part[1][q][row]) + (part[2][q][row] + part[3][q][row]);
+            // (watchdog test switch: the first task of the launch never reports)
+            if (!(P.tc_drop && t == 0)) st_value(yf + (int64_t)(r0 + row) * NG + q, v);
+            if (rr < nrhs) b[(int64_t)(P.fst[js] + r0 + row) + rr * ldb] = v / d;
         }
-#pragma unroll
-        for (int r = 0; r < NR; ++r)
-            if (r < nrhs) part[q][row][r] = acc[r];
-        __syncthreads();
-        if (tid < kNB && row < nrow)
-            for (int r = 0; r < nrhs; ++r)
-                ysol[vb + (int64_t)r * F + r0 + row] =
-                    (part[0][row][r] + part[1][row][r]) + (part[2][row][r] + part[3][row][r]);
-        __threadfence();
-        __syncthreads();
-        // (watchdog test switch: the first task of the launch never reports)
-        if (tid == 0 && !(P.tc_drop && t == 0)) st_release(fl + rb, 1);
     }
 }
 
-template <int NR>
-__global__ void __launch_bounds__(256) k_bwd_tri(const int32_t* tasks, int ntasks, int32_t* flags, int32_t* counter,
-                                                 PV P, const double* vbuf, double* xsol, int nrhs) {
-    __shared__ double xs[kNB][kTriLd];
-    __shared__ double part[4][kNB][kTriLd];
-    __shared__ int task_sh, ok_sh;
+template <int NG>
+__global__ void __launch_bounds__(256) k_bwd_tri(const int32_t* tasks, int ntasks, int ng, int32_t* counter, PV P,
+                                                 const double* pbuf, double* x, double* b, int64_t ldb, int nrhs,
+                                                 int nrp, int64_t neq) {
+    __shared__ __align__(16) double xs[2][kNB * NG];
+    __shared__ double part[4][NG][kNB];
+    __shared__ int task_sh;
     int* abort_word = counter + 1;
     const int tid = threadIdx.x, col = tid & (kNB - 1), q = tid >> 6;
     for (;;) {
         if (tid == 0) task_sh = atomicAdd(counter, 1);
         __syncthreads();
-        if (task_sh >= ntasks) break;
-        const int t = ntasks - 1 - task_sh;                          // descending blocks
-        const int js = tasks[2 * t], cb = tasks[2 * t + 1];
+        if (task_sh >= ntasks * ng) break;
+        const int t = ntasks * ng - 1 - task_sh;                         // descending blocks
+        const int js = tasks[2 * (t / ng)], cb = tasks[2 * (t / ng) + 1], g = t % ng;
         if (node_off(P, js)) {
             __syncthreads();
             continue;
@@ -2382,126 +2159,84 @@ __global__ void __launch_bounds__(256) k_bwd_tri(const int32_t* tasks, int ntask
         const int c0 = cb * kNB, ncol = min(kNB, S - c0);
         const int nblk = (S + kNB - 1) / kNB;
         const double* base = P.lnz + P.lnz_off[js];
-        const int64_t vb = P.rbase[js] * nrhs;
-        int32_t* fl = flags + P.tri_off[js];
-        double acc[NR];
-#pragma unroll
-        for (int r = 0; r < NR; ++r) acc[r] = 0.0;
-        bool ok = true;
+        double* xf = x + ((int64_t)g * neq + P.fst[js]) * NG;
         const int64_t pc = (col < ncol) ? lnz_col(c0 + col, F) - (c0 + col) : 0;   // column c0 + col, row 0
         const double* lv = P.linv + P.linv_off[js] + (int64_t)cb * kNB * kNB;
-        constexpr bool kPreX = NR <= 4;
-        double xr[kPreX ? 16 : 1];
-        if constexpr (kPreX) {
+        double xr[16];
 #pragma unroll
-            for (int k = 0; k < 16; ++k) {
-                const int m = 16 * q + k;
-                xr[k] = (m >= col) ? __ldg(lv + m + col * kNB) : 0.0;       // X[m][col]
-            }
+        for (int k = 0; k < 16; ++k) {
+            const int m = 16 * q + k;
+            xr[k] = (m >= col) ? __ldg(lv + m + col * kNB) : 0.0;         // X[m][col]
         }
-        double wv[NR];
+        // own row less the partial sums of the rows below the triangle
+        const int rr = g * NG + q;
+        const bool fin = q < NG && col < ncol;
+        double w = 0.0;
+        if (fin && rr < nrhs) {
+            const int nrc = (F - S + kRectRows - 1) / kRectRows;
+            const double* pp = pbuf + (P.rect_off[js] + c0 + col) * nrp + rr;
+            double s = 0.0;
+#pragma unroll 8
+            for (int k = 0; k < nrc; ++k) s += __ldcg(pp + (int64_t)k * S * nrp);
+            w = b[(int64_t)(P.fst[js] + c0 + col) + rr * ldb] - s;
+        }
+        double acc[NG];
 #pragma unroll
-        for (int r = 0; r < NR; ++r)
-            wv[r] = (tid < kNB && col < ncol && r < nrhs) ? __ldcg(vbuf + vb + (int64_t)r * F + c0 + col) : 0.0;
-        // the blocks below finish from the bottom up: take them in that order,
-        // so that only the nearest one (cb + 1, the last to finish) is waited for
+        for (int r = 0; r < NG; ++r) acc[r] = 0.0;
+        bool ok = true;
+        // the blocks below finish from the bottom up: taken in that order, so
+        // that only the nearest one (cb + 1, the last to finish) is waited for;
+        // the last block may be short: its missing rows count as zero
+        const int nlast = S - (nblk - 1) * kNB;
+        double next = 0.0;
+        if (tid < kNB * NG && cb + 1 < nblk && tid < nlast * NG) next = ld_value(xf + (int64_t)kNB * NG * (nblk - 1) + tid);
         for (int rb = nblk - 1; rb > cb; --rb) {
-            const int nr = min(kNB, S - rb * kNB);
+            const int nr = rb == nblk - 1 ? nlast : kNB;
             double lr[16];                                   // L[64 rb + 16 q + k][c0 + col], ahead of the wait
             {
                 const int i0 = kNB * rb + 16 * q;
 #pragma unroll
                 for (int k = 0; k < 16; ++k) lr[k] = (col < ncol && 16 * q + k < nr) ? __ldg(base + pc + i0 + k) : 0.0;
             }
-            if (tid == 0) ok_sh = tri_wait(fl + rb, abort_word, P);
-            __syncthreads();
-            if (!ok_sh) {
+            double* xb = xs[rb & 1];
+            if (tid < kNB * NG) {
+                const double* at = xf + (int64_t)kNB * NG * rb + tid;
+                double v = next;
+                if (tid < nr * NG && no_value(v)) v = tri_wait(at, abort_word, P, ok);
+                xb[tid] = v;
+                if (rb - 1 > cb) next = ld_value(at - kNB * NG);
+            }
+            if (!__syncthreads_and(ok)) {
                 ok = false;
                 break;
             }
-            for (int e = tid; e < kNB * nrhs; e += blockDim.x) {
-                const int i = e & (kNB - 1), r = e >> 6;
-                xs[i][r] = (i < nr) ? __ldcg(xsol + vb + (int64_t)r * F + kNB * rb + i) : 0.0;
-            }
-            __syncthreads();
 #pragma unroll
             for (int k = 0; k < 16; ++k)
 #pragma unroll
-                for (int r = 0; r < NR; ++r)
-                    if (r < nrhs) acc[r] += lr[k] * xs[16 * q + k][r];
-            __syncthreads();
+                for (int r = 0; r < NG; ++r) acc[r] += lr[k] * xb[(16 * q + k) * NG + r];
         }
         if (!ok) break;
 #pragma unroll
-        for (int r = 0; r < NR; ++r)
-            if (r < nrhs) part[q][col][r] = acc[r];
+        for (int r = 0; r < NG; ++r) part[q][r][col] = acc[r];
         __syncthreads();
-        if (tid < kNB)
-#pragma unroll
-            for (int r = 0; r < NR; ++r)
-                if (r < nrhs)
-                    xs[col][r] = (col < ncol) ? wv[r] - ((part[0][col][r] + part[1][col][r]) +
-                                                         (part[2][col][r] + part[3][col][r]))
-                                              : 0.0;
+        if (q < NG) xs[0][col * NG + q] = w - ((part[0][q][col] + part[1][q][col]) + (part[2][q][col] + part[3][q][col]));
         __syncthreads();
         // x = X' v: x[col] = sum_{m >= col} X[m][col] v[m]
 #pragma unroll
-        for (int r = 0; r < NR; ++r) acc[r] = 0.0;
+        for (int r = 0; r < NG; ++r) acc[r] = 0.0;
 #pragma unroll
-        for (int k = 0; k < 16; ++k) {
-            const int m = 16 * q + k;
-            double x;
-            if constexpr (kPreX) {
-                x = xr[k];
-            } else {
-                x = (m >= col) ? __ldg(lv + m + col * kNB) : 0.0;
-            }
+        for (int k = 0; k < 16; ++k)
 #pragma unroll
-            for (int r = 0; r < NR; ++r)
-                if (r < nrhs) acc[r] += x * xs[m][r];
+            for (int r = 0; r < NG; ++r) acc[r] += xr[k] * xs[0][(16 * q + k) * NG + r];
+#pragma unroll
+        for (int r = 0; r < NG; ++r) part[q][r][col] = acc[r];
+        __syncthreads();
+        if (fin) {
+            const double v = (part[0][q][col] + part[1][q][col]) + (part[2][q][col] + part[3][q][col]);
+            if (!(P.tc_drop && t == ntasks * ng - 1)) st_value(xf + (int64_t)(c0 + col) * NG + q, v);
+            if (rr < nrhs) b[(int64_t)(P.fst[js] + c0 + col) + rr * ldb] = v;
         }
-#pragma unroll
-        for (int r = 0; r < NR; ++r)
-            if (r < nrhs) part[q][col][r] = acc[r];
-        __syncthreads();
-        if (tid < kNB && col < ncol)
-            for (int r = 0; r < nrhs; ++r)
-                xsol[vb + (int64_t)r * F + c0 + col] =
-                    (part[0][col][r] + part[1][col][r]) + (part[2][col][r] + part[3][col][r]);
-        __threadfence();
-        __syncthreads();
-        if (tid == 0 && !(P.tc_drop && t == ntasks - 1)) st_release(fl + cb, 1);
     }
-}
-
-// gather of the back sweep: own rows (forward result) and ancestors' solution
-__global__ void k_bwd_gather(const Job* jobs, int64_t njobs, const int32_t* tmap, int64_t ntasks, PV P, double* vbuf,
-                             const double* b, int64_t ldb, int nrhs) {
-    const int64_t task = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (task >= ntasks) return;
-    const Job& jb = job_of(jobs, njobs, tmap, task);
-    const int js = jb.node;
-    if (node_off(P, js)) return;
-    const int i = (int)(task - jb.task0);
-    const int F = P.F[js], S = P.S[js], fst = P.fst[js];
-    double* w = vbuf + P.rbase[js] * nrhs;
-    const int row = (i < S) ? (fst + i) : P.rows[P.rbase[js] + i];
-    for (int r = 0; r < nrhs; ++r) w[(int64_t)r * F + i] = b[(int64_t)row + r * ldb];
-}
-
-
-__global__ void k_bwd_finish(const Job* jobs, int64_t njobs, const int32_t* tmap, int64_t ntasks, PV P, const double* xsol, double* b,
-                             int64_t ldb, int nrhs) {
-    const int64_t task = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (task >= ntasks) return;
-    const Job& jb = job_of(jobs, njobs, tmap, task);
-    const int js = jb.node;
-    if (node_off(P, js)) return;
-    if (is_retained(P, js)) return;
-    const int j = (int)(task - jb.task0);
-    const int F = P.F[js], fst = P.fst[js];
-    const double* w = xsol + P.rbase[js] * nrhs;
-    for (int r = 0; r < nrhs; ++r) b[(int64_t)(fst + j) + r * ldb] = w[(int64_t)r * F + j];
 }
 
 // ---------------------------------------------------------------------------
@@ -2852,8 +2587,8 @@ Engine::~Engine() {
     for (void* p : d_->owned) cudaFree(p);
     if (d_->arena) cudaFree(d_->arena);
     if (d_->vbuf) cudaFree(d_->vbuf);
-    if (d_->vbuf2) cudaFree(d_->vbuf2);
-    if (d_->bbuf) cudaFree(d_->bbuf);
+    if (d_->ybuf) cudaFree(d_->ybuf);
+    if (d_->pbuf) cudaFree(d_->pbuf);
     if (d_->ev0) cudaEventDestroy(d_->ev0);
     if (d_->ev1) cudaEventDestroy(d_->ev1);
 }
@@ -2896,15 +2631,10 @@ int Engine::open(const int64_t* mspar, const int64_t* mtrees, const int64_t* msi
         dev_upload(o, &D.rel_off, P_.rel_off) || dev_upload(o, &D.rbase, P_.rbase) ||
         dev_upload(o, &D.cptr, P_.cptr) || dev_upload(o, &D.buf_off, P_.buf_off) ||
         dev_upload(o, &D.upd_off, P_.upd_off) || dev_upload(o, &D.jobs, P_.jobs) ||
-        dev_upload(o, &D.linv_off, P_.linv_off) || dev_upload(o, &D.xinv_off, P_.xinv_off) ||
+        dev_upload(o, &D.linv_off, P_.linv_off) ||
         dev_upload(o, &D.rect_off, P_.rect_off) || dev_upload(o, &D.fwd_off, P_.fwd_off) ||
         dev_upload(o, &D.task_map, P_.task_map))
         return -4;
-    CK(cudaMalloc((void**)&D.pbuf,
-                  std::max<int64_t>(std::max(P_.rect_entries, P_.fwd_entries), 1) * kMaxRHS * sizeof(double)));
-    o.push_back(D.pbuf);
-    CK(cudaMalloc((void**)&D.xinv, std::max<int64_t>(P_.xinv_doubles, 1) * sizeof(double)));
-    o.push_back(D.xinv);
     CK(cudaMalloc((void**)&D.linv, std::max<int64_t>(P_.linv_doubles, 1) * sizeof(double)));
     o.push_back(D.linv);
     std::vector<int32_t> small, all;
@@ -2940,13 +2670,8 @@ int Engine::open(const int64_t* mspar, const int64_t* mtrees, const int64_t* msi
     CK(cudaMalloc((void**)&D.hbuf, sizeof(unsigned long long)));
     o.push_back(D.hbuf);
     if (dev_upload(o, &D.tri_tasks, P_.tri_tasks)) return -4;
-    if (dev_upload(o, &D.tri_off, P_.tri_off)) return -4;
-    CK(cudaMalloc((void**)&D.tri_sync, sizeof(int32_t) * (size_t)(P_.tri_flags + 2 * (int64_t)P_.levels.size() + 2)));
+    CK(cudaMalloc((void**)&D.tri_sync, sizeof(int32_t) * (size_t)(2 * P_.levels.size() + 2)));
     o.push_back(D.tri_sync);
-    {
-        const char* v = std::getenv("SPR_B200_SOLVE_BLOCKS");
-        tri_solve_ = !(v && v[0] == '1');
-    }
     CK(cudaHostAlloc((void**)&D.mbox, 32 * sizeof(unsigned long long), cudaHostAllocMapped));
     CK(cudaHostGetDevicePointer((void**)&D.mbox_dev, D.mbox, 0));
     CK(cudaEventCreate(&D.ev0));
@@ -2960,11 +2685,8 @@ int Engine::open(const int64_t* mspar, const int64_t* mtrees, const int64_t* msi
     CK(cudaFuncSetAttribute(k_small_front<kPivotChol>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need));
     CK(cudaFuncSetAttribute(k_small_front<kPivotChol4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need));
     CK(cudaFuncSetAttribute(k_trsm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTrsmSmem));
-    CK(cudaFuncSetAttribute(k_fwd_blk_mv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMvSmem));
-    CK(cudaFuncSetAttribute(k_fwd_blk_upd2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kUpdSmem));
     CK(cudaFuncSetAttribute(k_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmallSolveSmem));
     CK(cudaFuncSetAttribute(k_backward, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmallSolveSmem));
-    CK(cudaFuncSetAttribute(k_inv_block, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kInvSmem));
     CK(cudaFuncSetAttribute(K_GEMM_BIG, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GemmBig::smem));
     CK(cudaFuncSetAttribute(K_GEMM_SMALL, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GemmSmall::smem));
     CK(cudaFuncSetAttribute(K_GEMM_TINY, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GemmTiny::smem));
@@ -3100,11 +2822,8 @@ static PV make_view(Engine::Dev& D, const Plan& P, double* d_sm, double tol1) {
     v.st = D.st;
     v.linv_off = D.linv_off;
     v.linv = D.linv;
-    v.xinv_off = D.xinv_off;
-    v.xinv = D.xinv;
     v.rect_off = D.rect_off;
     v.fwd_off = D.fwd_off;
-    v.tri_off = D.tri_off;
     v.tol1 = tol1;
     v.fc3 = 0;
     v.tol4 = 0.0;
@@ -3471,10 +3190,6 @@ void Engine::enqueue_factor(const PV& pv, cudaStream_t s, std::vector<cudaEvent_
         }
     }
     mark(8);
-    if (!tri_solve_ && P_.inv_blocks.job_count > 0) {
-        k_inv_block<<<(int)P_.inv_blocks.job_count, 256, kInvSmem, s>>>(D.jobs + P_.inv_blocks.job_begin, pv);
-        ++timing.launches;
-    }
     k_reduce<true><<<1, 1024, 0, s>>>(pv.dvec, P_.neq, &D.st->mindpos);
     ++timing.launches;
 }
@@ -4028,34 +3743,53 @@ int Engine::sn_stats(int32_t* neg, int32_t* fail) {
     return 0;
 }
 
-void Engine::ensure_vectors(int64_t nrhs) {
+// Buffers for up to nrhs right-hand sides in a pass; returns how many a pass
+// may take (0: not even kMaxRHS fit).
+int64_t Engine::ensure_vectors(int64_t nrhs) {
     Dev& D = *d_;
-    if (D.vbuf_rhs < nrhs) {
-        if (D.vbuf) cudaFree(D.vbuf);
-        if (D.vbuf2) cudaFree(D.vbuf2);
-        D.vbuf = D.vbuf2 = nullptr;
-        const size_t bytes = std::max<int64_t>(P_.rbase.back(), 1) * nrhs * sizeof(double);
-        if (cudaMalloc((void**)&D.vbuf, bytes) != cudaSuccess || cudaMalloc((void**)&D.vbuf2, bytes) != cudaSuccess)
-            return;
-        D.vbuf_rhs = nrhs;
+    if (nrhs <= 0) return D.vbuf ? 1 : 0;                // nothing to solve
+    for (;;) {
+        const int64_t want = std::min(nrhs, D.pass_rhs);
+        if (D.vbuf && D.vbuf_rhs >= want) return want;
+        for (double** p : {&D.vbuf, &D.ybuf, &D.pbuf}) {
+            if (*p) cudaFree(*p);
+            *p = nullptr;
+        }
+        D.vbuf_rhs = 0;
+        const int64_t nrp = (want + 3) / 4 * 4;
+        const size_t d = sizeof(double);
+        if (cudaMalloc((void**)&D.vbuf, std::max<int64_t>(P_.rbase.back(), 1) * want * d) == cudaSuccess &&
+            cudaMalloc((void**)&D.ybuf, P_.neq * nrp * d) == cudaSuccess &&
+            cudaMalloc((void**)&D.pbuf, std::max<int64_t>(std::max(P_.rect_entries, P_.fwd_entries), 1) * nrp * d) ==
+                cudaSuccess) {
+            D.vbuf_rhs = want;
+            return want;
+        }
+        cudaGetLastError();
+        if (want <= kMaxRHS) return 0;
+        D.pass_rhs = kMaxRHS;
     }
 }
 
-void Engine::enqueue_solve(const PV& pv, cudaStream_t s, double* d_b, int64_t ldb, int64_t nrhs, int which,
-                           int64_t& nl) {
+void Engine::enqueue_solve(const PV& pv, cudaStream_t s, double* d_b, int64_t ldb, int64_t nrhs, int64_t chunk,
+                           int which, int64_t& nl) {
     Dev& D = *d_;
     auto mark = [&](int phase) {
         if (profile_) marks_.emplace_back(9 + phase, record_event(s));
     };
-    const int64_t chunk = std::min<int64_t>(nrhs, kMaxRHS);
+    const Job* jobs = D.jobs;
+    const int64_t neq = P_.neq;
+    auto blocks = [](int64_t threads) { return (int)((threads + 255) / 256); };
+    const size_t ctr_bytes = sizeof(int32_t) * 2 * P_.levels.size();
     for (int64_t r0 = 0; r0 < nrhs; r0 += chunk) {
         const int nr = (int)std::min<int64_t>(chunk, nrhs - r0);
+        // ng groups of gw right-hand sides; y and the partials are padded to whole groups
+        const int gw = nr == 1 ? 1 : nr == 2 ? 2 : 4, ng = (nr + gw - 1) / gw, nrp = gw * ng;
+        const int sg = (nr + kMaxRHS - 1) / kMaxRHS, sr = std::min(nr, kMaxRHS);
         double* b = d_b + r0 * ldb;
-        const Job* jobs = D.jobs;
-        auto blocks = [](int64_t threads) { return (int)((threads + 255) / 256); };
-        const size_t tri_bytes = sizeof(int32_t) * (size_t)(P_.tri_flags + 2 * (int64_t)P_.levels.size());
         if (which & 1) {
-            if (tri_solve_) cudaMemsetAsync(D.tri_sync, 0, tri_bytes, s);
+            cudaMemsetAsync(D.tri_sync, 0, ctr_bytes, s);
+            if (P_.any_large) cudaMemsetAsync(D.ybuf, 0xff, neq * nrp * sizeof(double), s);
             // split run: the other ranks' subtree roots' update vectors come in
             // before their parent's level, this rank's go out after their level
             ExchangeHooks vx;
@@ -4078,127 +3812,104 @@ void Engine::enqueue_solve(const PV& pv, cudaStream_t s, double* d_b, int64_t ld
                 if (!lp.small_nodes.empty()) {
                     mark(0);
                     for (const LevelPlan::SmallClass& c : lp.small_classes) {
-                        k_forward<<<c.count, small_threads(c.maxF), small_solve_smem(c.maxF, nr), s>>>(
+                        k_forward<<<dim3(c.count, sg), small_threads(c.maxF), small_solve_smem(c.maxF, sr), s>>>(
                             D.level_nodes + D.small_begin[L] + c.begin, pv, D.vbuf, b, ldb, nr);
                         ++nl;
                     }
                 }
                 if (lp.large_nodes.empty()) continue;
-                const Launch& ga = lp.assemble;
-                mark(1);
-                k_fwd_gather<<<blocks(ga.ntasks), 256, 0, s>>>(jobs + ga.job_begin, ga.job_count, TMAP(ga), ga.ntasks, pv,
-                                                               D.vbuf, b, ldb, nr);
-                ++nl;
-                mark(2);
-                if (tri_solve_ && lp.tri_count > 0) {
-                    const int nt = (int)lp.tri_count;
-                    const int grid = std::min(nt, 4 * std::max(sm_count_, 1));
-                    int32_t* ctr = D.tri_sync + P_.tri_flags + 2 * L;
-                    if (nr <= 4)
-                        k_fwd_tri<4><<<grid, 256, 0, s>>>(D.tri_tasks + 2 * lp.tri_begin, nt, D.tri_sync, ctr, pv,
-                                                          D.vbuf, D.vbuf2, nr);
-                    else
-                        k_fwd_tri<kMaxRHS><<<grid, 256, 0, s>>>(D.tri_tasks + 2 * lp.tri_begin, nt, D.tri_sync, ctr, pv,
-                                                                D.vbuf, D.vbuf2, nr);
+                if (lp.retained_large) {
+                    mark(1);
+                    const Launch& ga = lp.assemble;
+                    k_fwd_retained<<<blocks(ga.ntasks), 256, 0, s>>>(jobs + ga.job_begin, ga.job_count, TMAP(ga),
+                                                                     ga.ntasks, pv, D.vbuf, b, ldb, nr);
                     ++nl;
-                } else {
-                    for (size_t sb = 0; sb < lp.fs_upd.size(); ++sb) {
-                        const Launch& ml = lp.blk_mv[sb];
-                        k_fwd_blk_mv<<<(int)ml.ntasks, 256, kMvSmem, s>>>(jobs + ml.job_begin, ml.job_count, TMAP(ml), pv,
-                                                                     D.vbuf, D.vbuf2, nr);
-                        ++nl;
-                        const Launch& fl = lp.fs_upd[sb];
-                        if (fl.ntasks > 0) {
-                            k_fwd_blk_upd2<<<(int)fl.ntasks, 256, kUpdSmem, s>>>(jobs + fl.job_begin, fl.job_count,
-                                                                           TMAP(fl), pv, D.vbuf, D.vbuf2, nr);
-                            ++nl;
-                        }
-                    }
+                }
+                if (lp.tri_count > 0) {
+                    mark(2);
+                    const int nt = (int)lp.tri_count;
+                    const int grid = (int)std::min<int64_t>((int64_t)nt * ng, 4 * (int64_t)std::max(sm_count_, 1));
+                    const int32_t* tasks = D.tri_tasks + 2 * lp.tri_begin;
+                    int32_t* ctr = D.tri_sync + 2 * L;
+                    if (gw == 1)
+                        k_fwd_tri<1><<<grid, 256, 0, s>>>(tasks, nt, ng, ctr, pv, D.vbuf, D.ybuf, b, ldb, nr, neq);
+                    else if (gw == 2)
+                        k_fwd_tri<2><<<grid, 256, 0, s>>>(tasks, nt, ng, ctr, pv, D.vbuf, D.ybuf, b, ldb, nr, neq);
+                    else
+                        k_fwd_tri<4><<<grid, 256, 0, s>>>(tasks, nt, ng, ctr, pv, D.vbuf, D.ybuf, b, ldb, nr, neq);
+                    ++nl;
                 }
                 const Launch& rl = lp.rect;
                 if (rl.ntasks > 0) {
                     mark(3);
-                    if (nr <= 4)
-                        k_fwd_rect_part<4><<<(int)rl.ntasks, 256, 0, s>>>(jobs + rl.job_begin, rl.job_count, TMAP(rl),
-                                                                          pv, D.vbuf2, D.pbuf, nr);
+                    const Job* j = jobs + rl.job_begin;
+                    const unsigned nt = (unsigned)rl.ntasks;
+                    // from two groups on a CTA takes two: L is read half as often from L2
+                    if (gw == 1)
+                        k_fwd_rect<1, 1><<<dim3(nt, ng), 256, 0, s>>>(j, rl.job_count, TMAP(rl), pv, D.ybuf, D.vbuf, D.pbuf,
+                                                                      nr, nrp, neq);
+                    else if (gw == 2)
+                        k_fwd_rect<2, 1><<<dim3(nt, ng), 256, 0, s>>>(j, rl.job_count, TMAP(rl), pv, D.ybuf, D.vbuf, D.pbuf,
+                                                                      nr, nrp, neq);
+                    else if (ng == 1)
+                        k_fwd_rect<4, 1><<<dim3(nt, ng), 256, 0, s>>>(j, rl.job_count, TMAP(rl), pv, D.ybuf, D.vbuf, D.pbuf,
+                                                                      nr, nrp, neq);
                     else
-                        k_fwd_rect_part<kMaxRHS><<<(int)rl.ntasks, 256, 0, s>>>(jobs + rl.job_begin, rl.job_count,
-                                                                                TMAP(rl), pv, D.vbuf2, D.pbuf, nr);
+                        k_fwd_rect<4, 2><<<dim3(nt, (ng + 1) / 2), 256, 0, s>>>(j, rl.job_count, TMAP(rl), pv, D.ybuf, D.vbuf,
+                                                                                D.pbuf, nr, nrp, neq);
+                    ++nl;
                     const Launch& rr = lp.rect_rows;
-                    k_fwd_rect_sum<<<blocks(rr.ntasks), 256, 0, s>>>(jobs + rr.job_begin, rr.job_count, TMAP(rr),
-                                                                      rr.ntasks, pv, D.vbuf, D.pbuf, nr);
-                    nl += 2;
+                    if (rr.ntasks > 0) {
+                        k_fwd_rect_sum<<<blocks(rr.ntasks * nr), 256, 0, s>>>(jobs + rr.job_begin, rr.job_count, TMAP(rr),
+                                                                              rr.ntasks, pv, D.vbuf, D.pbuf, b, ldb, nr,
+                                                                              nrp);
+                        ++nl;
+                    }
                 }
-                const Launch& wb = lp.writeback;
-                mark(4);
-                k_fwd_finish<<<blocks(wb.ntasks), 256, 0, s>>>(jobs + wb.job_begin, wb.job_count, TMAP(wb), wb.ntasks, pv,
-                                                               D.vbuf2, D.vbuf, b, ldb, nr);
-                ++nl;
             }
         }
         if (which & 2) {
-            if (tri_solve_) cudaMemsetAsync(D.tri_sync, 0, tri_bytes, s);
+            cudaMemsetAsync(D.tri_sync, 0, ctr_bytes, s);
+            if (P_.any_large) cudaMemsetAsync(D.ybuf, 0xff, neq * nrp * sizeof(double), s);
             for (size_t L = P_.levels.size(); L-- > 0;) {
                 const LevelPlan& lp = P_.levels[L];
                 if (!lp.small_nodes.empty()) {
                     mark(5);
                     for (const LevelPlan::SmallClass& c : lp.small_classes) {
-                        k_backward<<<c.count, small_threads(c.maxF), small_solve_smem(c.maxF, nr), s>>>(
-                            D.level_nodes + D.small_begin[L] + c.begin, pv, D.vbuf, b, ldb, nr);
+                        k_backward<<<dim3(c.count, sg), small_threads(c.maxF), small_solve_smem(c.maxF, sr), s>>>(
+                            D.level_nodes + D.small_begin[L] + c.begin, pv, b, ldb, nr);
                         ++nl;
                     }
                 }
-                if (lp.large_nodes.empty()) continue;
-                const Launch& ga = lp.assemble;
-                mark(6);
-                k_bwd_gather<<<blocks(ga.ntasks), 256, 0, s>>>(jobs + ga.job_begin, ga.job_count, TMAP(ga), ga.ntasks, pv,
-                                                               D.vbuf, b, ldb, nr);
-                ++nl;
-                const Launch& wb = lp.writeback;
-                const Launch& rl = lp.rect;
+                const Launch& rl = lp.rect_back;
                 if (rl.ntasks > 0) {
                     mark(7);
-                    if (nr <= 4)
-                        k_bwd_rect_part<4><<<(int)rl.ntasks, 256, 0, s>>>(jobs + rl.job_begin, rl.job_count, TMAP(rl),
-                                                                          pv, D.vbuf, D.pbuf, nr);
+                    const dim3 grid((unsigned)rl.ntasks, ng);
+                    const Job* j = jobs + rl.job_begin;
+                    if (gw == 1)
+                        k_bwd_rect<1, true><<<grid, 256, 0, s>>>(j, rl.job_count, TMAP(rl), pv, D.pbuf, b, ldb, nr, nrp);
+                    else if (gw == 2)
+                        k_bwd_rect<2, true><<<grid, 256, 0, s>>>(j, rl.job_count, TMAP(rl), pv, D.pbuf, b, ldb, nr, nrp);
+                    else if (ng == 1)
+                        k_bwd_rect<4, true><<<grid, 256, 0, s>>>(j, rl.job_count, TMAP(rl), pv, D.pbuf, b, ldb, nr, nrp);
                     else
-                        k_bwd_rect_part<kMaxRHS><<<(int)rl.ntasks, 256, 0, s>>>(jobs + rl.job_begin, rl.job_count,
-                                                                                TMAP(rl), pv, D.vbuf, D.pbuf, nr);
-                    ++nl;
-                    k_bwd_rect_sum<<<blocks(wb.ntasks * kSumLanes), 256, 0, s>>>(jobs + wb.job_begin, wb.job_count, TMAP(wb), wb.ntasks, pv,
-                                                                      D.vbuf, D.pbuf, nr);
+                        k_bwd_rect<4, false><<<grid, 256, 0, s>>>(j, rl.job_count, TMAP(rl), pv, D.pbuf, b, ldb, nr, nrp);
                     ++nl;
                 }
-                mark(8);
-                if (tri_solve_ && lp.tri_count > 0) {
+                if (lp.tri_count > 0) {
+                    mark(8);
                     const int nt = (int)lp.tri_count;
-                    const int grid = std::min(nt, 4 * std::max(sm_count_, 1));
-                    int32_t* ctr = D.tri_sync + P_.tri_flags + 2 * L;
-                    if (nr <= 4)
-                        k_bwd_tri<4><<<grid, 256, 0, s>>>(D.tri_tasks + 2 * lp.tri_begin, nt, D.tri_sync, ctr, pv,
-                                                          D.vbuf, D.vbuf2, nr);
+                    const int grid = (int)std::min<int64_t>((int64_t)nt * ng, 4 * (int64_t)std::max(sm_count_, 1));
+                    const int32_t* tasks = D.tri_tasks + 2 * lp.tri_begin;
+                    int32_t* ctr = D.tri_sync + 2 * L;
+                    if (gw == 1)
+                        k_bwd_tri<1><<<grid, 256, 0, s>>>(tasks, nt, ng, ctr, pv, D.pbuf, D.ybuf, b, ldb, nr, nrp, neq);
+                    else if (gw == 2)
+                        k_bwd_tri<2><<<grid, 256, 0, s>>>(tasks, nt, ng, ctr, pv, D.pbuf, D.ybuf, b, ldb, nr, nrp, neq);
                     else
-                        k_bwd_tri<kMaxRHS><<<grid, 256, 0, s>>>(D.tri_tasks + 2 * lp.tri_begin, nt, D.tri_sync, ctr, pv,
-                                                                D.vbuf, D.vbuf2, nr);
+                        k_bwd_tri<4><<<grid, 256, 0, s>>>(tasks, nt, ng, ctr, pv, D.pbuf, D.ybuf, b, ldb, nr, nrp, neq);
                     ++nl;
-                } else {
-                    for (size_t sb = lp.bs_upd.size(); sb-- > 0;) {
-                        const Launch& ml = lp.blk_mv[sb];
-                        k_bwd_blk_mv<<<(int)ml.ntasks, 256, kBwdSmem, s>>>(jobs + ml.job_begin, ml.job_count, TMAP(ml), pv,
-                                                                     D.vbuf, D.vbuf2, nr);
-                        ++nl;
-                        const Launch& bl = lp.bs_upd[sb];
-                        if (bl.ntasks > 0) {
-                            k_bwd_blk_upd<<<(int)bl.ntasks, 256, kBwdSmem, s>>>(jobs + bl.job_begin, bl.job_count,
-                                                                         TMAP(bl), pv, D.vbuf, D.vbuf2, nr);
-                            ++nl;
-                        }
-                    }
                 }
-                mark(10);
-                k_bwd_finish<<<blocks(wb.ntasks), 256, 0, s>>>(jobs + wb.job_begin, wb.job_count, TMAP(wb), wb.ntasks, pv,
-                                                               D.vbuf2, b, ldb, nr);
-                ++nl;
             }
         }
     }
@@ -4211,9 +3922,8 @@ int Engine::solve(const double* d_sm, double* d_b, int64_t ldb, int64_t nrhs, in
     PV pv = make_view(D, P_, const_cast<double*>(d_sm), 0.0);
     pv.wait_ns = wait_ns_;
     pv.tc_drop = tc_drop_ ? 1 : 0;
-    const int64_t chunk = std::min<int64_t>(nrhs, kMaxRHS);
-    ensure_vectors(chunk);
-    if (!D.vbuf || !D.vbuf2) return -4;
+    const int64_t chunk = ensure_vectors(nrhs);
+    if (chunk <= 0) return -4;
     CK(cudaEventRecord(D.ev0, s));
     int64_t nl = 0;
     CK(cudaMemsetAsync(&D.st->solve_timeout, 0, sizeof(int), s));
@@ -4224,12 +3934,6 @@ int Engine::solve(const double* d_sm, double* d_b, int64_t ldb, int64_t nrhs, in
                     k_linv<<<(int)pl.job_count, 64, 0, s>>>(D.jobs + pl.job_begin, pv);
                     ++nl;
                 }
-        if (!tri_solve_ && P_.inv_blocks.job_count > 0) {
-            PV pvi = pv;
-            pvi.sn_bad = nullptr;
-            k_inv_block<<<(int)P_.inv_blocks.job_count, 256, kInvSmem, s>>>(D.jobs + P_.inv_blocks.job_begin, pvi);
-            ++nl;
-        }
         linv_valid_ = true;
     }
     if (use_graphs_ && !profile_ && s != nullptr && !tc_drop_ && wait_ns_ == 2000000000ull && !split_) {
@@ -4237,7 +3941,7 @@ int Engine::solve(const double* d_sm, double* d_b, int64_t ldb, int64_t nrhs, in
         cudaGraphExec_t exec = find_graph(key);
         if (!exec) {
             CK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-            enqueue_solve(pv, s, d_b, ldb, nrhs, which, nl);
+            enqueue_solve(pv, s, d_b, ldb, nrhs, chunk, which, nl);
             cudaGraph_t g = nullptr;
             CK(cudaStreamEndCapture(s, &g));
             CK(cudaGraphInstantiate(&exec, g, 0));
@@ -4248,7 +3952,7 @@ int Engine::solve(const double* d_sm, double* d_b, int64_t ldb, int64_t nrhs, in
         }
         CK(cudaGraphLaunch(exec, s));
     } else {
-        enqueue_solve(pv, s, d_b, ldb, nrhs, which, nl);
+        enqueue_solve(pv, s, d_b, ldb, nrhs, chunk, which, nl);
     }
     CK(cudaEventRecord(D.ev1, s));
     CK(cudaGetLastError());

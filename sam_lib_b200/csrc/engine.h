@@ -206,11 +206,10 @@ private:
     int64_t graph_launches(const GraphKey& k);
     void store_graph(const GraphKey& k, cudaGraphExec_t exec, int64_t launches);
     void enqueue_factor(const struct PV& pv, cudaStream_t s, std::vector<cudaEvent_t>& gev);
-    void enqueue_solve(const struct PV& pv, cudaStream_t s, double* d_b, int64_t ldb, int64_t nrhs, int which,
-                       int64_t& nl);
+    void enqueue_solve(const struct PV& pv, cudaStream_t s, double* d_b, int64_t ldb, int64_t nrhs, int64_t chunk,
+                       int which, int64_t& nl);
     std::vector<GraphEntry> graphs_;
     bool use_graphs_ = true;
-    bool tri_solve_ = true;                  // solve triangles as one dataflow launch per level
     std::vector<Xfer> fout_, fin_, vout_, vin_;   // exchange lists of a split run
     bool split_ = false;                     // a mask or exchange lists are set (no graphs)
     void block_copy(int32_t js, double* buf, bool out, cudaStream_t s);
@@ -268,7 +267,7 @@ private:
     void launch_gemm(const Launch& l, cudaStream_t s, const struct PV& pv, std::vector<cudaEvent_t>& gev);
     void launch_diag(const Launch& pl, cudaStream_t s, const struct PV& pv);
     void upload_plan();
-    void ensure_vectors(int64_t nrhs);
+    int64_t ensure_vectors(int64_t nrhs);
     Plan P_;
     cudaStream_t stream_ = nullptr;
     bool profile_ = false;

@@ -245,15 +245,6 @@ int build_plan(const int64_t* mspar, const int64_t* mtrees, const int64_t* msifa
             }
     }
     P.arena_doubles = arena.peak();
-    P.xinv_off.assign(ns, -1);
-    P.xinv_doubles = 0;
-    for (int64_t js = 0; js < ns; ++js)
-        if (P.F[js] > kSmallMaxF) {
-            const int64_t nsb = (P.S[js] + kSolveBlock - 1) / kSolveBlock;
-            const int64_t last = P.S[js] - (nsb - 1) * kSolveBlock;
-            P.xinv_off[js] = P.xinv_doubles;
-            P.xinv_doubles += ((nsb - 1) * kSolveBlock * kSolveBlock + last * last + 31) / 32 * 32;
-        }
     P.linv_off.assign(ns, -1);
     P.linv_doubles = 0;
     for (int64_t js = 0; js < ns; ++js)
@@ -317,8 +308,6 @@ int build_plan(const int64_t* mspar, const int64_t* mtrees, const int64_t* msifa
         const int32_t nsteps = (smax + kNB - 1) / kNB;
         lp.panel.assign(nsteps, Launch());
         lp.update.assign(nsteps, std::vector<Launch>());
-        lp.fsolve.assign(nsteps, Launch());
-        lp.bsolve.assign(nsteps, Launch());
         // Schur-update jobs of one step, split into a big-tile and a small-tile launch
         auto emit_updates = [&](std::vector<Job>& jl, std::vector<Launch>& out) {
             for (int pass = 0; pass < 2; ++pass) {
@@ -486,78 +475,37 @@ int build_plan(const int64_t* mspar, const int64_t* mtrees, const int64_t* msifa
             emit_updates(jahead, lp.ahead[st]);
             emit_updates(jfar, lp.far[st]);
             emit_tc(jfar, lp.far_tc[st], P.slab_rows_far);
-            open_launch(lp.fsolve[st]);
-            for (int32_t js : elim) {
-                const int32_t s = P.S[js], f = P.F[js];
-                if (k0 >= s) continue;
-                const int32_t nb = std::min(kNB, s - k0);
-                const int64_t nrb = (f - (k0 + nb) + kTRSMRows - 1) / kTRSMRows;
-                add_job(lp.fsolve[st], Job{js, k0 + nb, k0 + nb, f, k0, k0 + nb, 0}, 1 + nrb);
-            }
-            close_launch(lp.fsolve[st]);
-            open_launch(lp.bsolve[st]);
-            for (int32_t js : elim) {
-                const int32_t s = P.S[js], f = P.F[js];
-                if (k0 >= s) continue;
-                const int32_t nb = std::min(kNB, s - k0);
-                add_job(lp.bsolve[st], Job{js, 0, k0, f, k0, k0 + nb, 0}, 1 + (k0 + kBwdCols - 1) / kBwdCols);
-            }
-            close_launch(lp.bsolve[st]);
-        }
-        const int32_t nsb = (smax + kSolveBlock - 1) / kSolveBlock;
-        lp.fs_upd.assign(nsb, Launch());
-        lp.bs_upd.assign(nsb, Launch());
-        lp.blk_mv.assign(nsb, Launch());
-        for (int32_t sb = 0; sb < nsb; ++sb) {
-            const int32_t k0 = sb * kSolveBlock;
-            open_launch(lp.blk_mv[sb]);
-            for (int32_t js : elim) {
-                const int32_t s = P.S[js], f = P.F[js];
-                if (k0 >= s) continue;
-                const int32_t k1 = std::min(k0 + kSolveBlock, s);
-                add_job(lp.blk_mv[sb], Job{js, k0, k1, f, k0, k1, 0}, (k1 - k0 + 31) / 32);
-            }
-            close_launch(lp.blk_mv[sb]);
-            open_launch(lp.fs_upd[sb]);
-            for (int32_t js : elim) {
-                const int32_t s = P.S[js], f = P.F[js];
-                if (k0 >= s) continue;
-                const int32_t k1 = std::min(k0 + kSolveBlock, s);
-                // rows [k1, S) of the diagonal part; rows [S, F) go to the rectangle launch
-                add_job(lp.fs_upd[sb], Job{js, k1, k1, s, k0, k1, 0}, (s - k1 + kSolveRows - 1) / kSolveRows, true);
-            }
-            close_launch(lp.fs_upd[sb]);
-            open_launch(lp.bs_upd[sb]);
-            for (int32_t js : elim) {
-                const int32_t s = P.S[js], f = P.F[js];
-                if (k0 >= s) continue;
-                const int32_t k1 = std::min(k0 + kSolveBlock, s);
-                add_job(lp.bs_upd[sb], Job{js, 0, k0, f, k0, k1, 0}, (k0 + kBwdCols - 1) / kBwdCols, true);
-            }
-            close_launch(lp.bs_upd[sb]);
         }
         open_launch(lp.rect);
         int64_t roff = 0, foff = 0;
         for (int32_t js : elim) {
             const int32_t s = P.S[js], f = P.F[js];
             if (f <= s) continue;
-            const int64_t nrc = (f - s + kRectRows - 1) / kRectRows;
-            const int64_t ncc = (s + kRectCols - 1) / kRectCols;
-            P.rect_off[js] = roff;
-            roff += nrc * s;
+            const int64_t nrc = (f - s + fwd_rows(s) - 1) / fwd_rows(s), ncc = (s + kFwdCols - 1) / kFwdCols;
             P.fwd_off[js] = foff;
             foff += ncc * (f - s);
             add_job(lp.rect, Job{js, 0, s, f, (int32_t)nrc, (int32_t)ncc, 0}, nrc * ncc);
         }
+        close_launch(lp.rect);
+        open_launch(lp.rect_back);
+        for (int32_t js : elim) {
+            const int32_t s = P.S[js], f = P.F[js];
+            if (f <= s) continue;
+            const int64_t nrc = (f - s + kRectRows - 1) / kRectRows, ncc = (s + kRectCols - 1) / kRectCols;
+            P.rect_off[js] = roff;
+            roff += nrc * s;
+            add_job(lp.rect_back, Job{js, 0, s, f, (int32_t)nrc, (int32_t)ncc, 0}, nrc * ncc);
+        }
+        close_launch(lp.rect_back);
         P.rect_entries = std::max(P.rect_entries, roff);
         P.fwd_entries = std::max(P.fwd_entries, foff);
-        close_launch(lp.rect);
         open_launch(lp.rect_rows);
         for (int32_t js : elim) {
             const int32_t s = P.S[js], f = P.F[js];
-            if (f > s) add_job(lp.rect_rows, Job{js, s, f, f, 0, 0, 0}, f - s);
+            if (f > s && s > kFwdCols) add_job(lp.rect_rows, Job{js, s, f, f, 0, 0, 0}, f - s);
         }
         close_launch(lp.rect_rows);
+        lp.retained_large = elim.size() != lp.large_nodes.size();
         {
             std::vector<Job> jl;
             for (int32_t js : elim) {
@@ -623,6 +571,7 @@ int build_plan(const int64_t* mspar, const int64_t* mtrees, const int64_t* msifa
         build_map(lp.writeback);
         for (Launch& l : lp.wb_sp) build_map(l);
         build_map(lp.rect);
+        build_map(lp.rect_back);
         build_map(lp.rect_rows);
         for (Launch& l : lp.panel) build_map(l);
         for (auto& v : lp.update)
@@ -654,14 +603,9 @@ int build_plan(const int64_t* mspar, const int64_t* mtrees, const int64_t* msifa
                 for (Launch& l : t.rest) build_map(l);
                 for (Launch& l : t.far_rest) build_map(l);
             }
-        for (Launch& l : lp.fs_upd) build_map(l);
-        for (Launch& l : lp.bs_upd) build_map(l);
-        for (Launch& l : lp.blk_mv) build_map(l);
     }
     // triangle tasks of the solves: per level, block-major (every task's
     // dependencies, the lower blocks of its own front, come earlier)
-    P.tri_off.assign(ns, -1);
-    P.tri_flags = 0;
     P.tri_tasks.clear();
     for (LevelPlan& lp : P.levels) {
         std::vector<int32_t> fr;
@@ -669,10 +613,7 @@ int build_plan(const int64_t* mspar, const int64_t* mtrees, const int64_t* msifa
         for (int32_t js : lp.elim_nodes) {
             if (P.F[js] <= kSmallMaxF) continue;
             fr.push_back(js);
-            P.tri_off[js] = P.tri_flags;
-            const int32_t nb = (P.S[js] + kNB - 1) / kNB;
-            P.tri_flags += nb;
-            nbmax = std::max(nbmax, nb);
+            nbmax = std::max(nbmax, (P.S[js] + kNB - 1) / kNB);
         }
         lp.tri_begin = (int64_t)P.tri_tasks.size() / 2;
         for (int32_t b = 0; b < nbmax; ++b)
@@ -683,14 +624,6 @@ int build_plan(const int64_t* mspar, const int64_t* mtrees, const int64_t* msifa
                 }
         lp.tri_count = (int64_t)P.tri_tasks.size() / 2 - lp.tri_begin;
     }
-    open_launch(P.inv_blocks);
-    for (int64_t js = 0; js < ns; ++js) {
-        if (P.F[js] <= kSmallMaxF || P.retained[js]) continue;
-        for (int32_t k0 = 0; k0 < P.S[js]; k0 += kSolveBlock)
-            add_job(P.inv_blocks, Job{(int32_t)js, k0, std::min(k0 + kSolveBlock, P.S[js]), P.F[js], k0,
-                                      std::min(k0 + kSolveBlock, P.S[js]), 0}, 1);
-    }
-    close_launch(P.inv_blocks);
     return 0;
 }
 
@@ -925,21 +858,12 @@ int64_t check_solve_plan(const Plan& P, int plant, int64_t* tasks) {
         return -1;
     }
     int64_t bad = 0, nt = 0;
-    // ready flags: one per block of each eliminated large front, disjoint
+    // solved rows: the equations of each eliminated large front, disjoint
     {
         std::vector<std::pair<int64_t, int64_t>> iv;
-        std::vector<uint8_t> elim(ns, 0);
         for (const LevelPlan& lp : P.levels)
-            for (int32_t js : lp.elim_nodes) elim[js] = 1;
-        for (int64_t js = 0; js < ns; ++js) {
-            if (!elim[js]) continue;
-            if (P.tri_off[js] < 0) {
-                ++bad;
-                continue;
-            }
-            iv.emplace_back(P.tri_off[js], P.tri_off[js] + (P.S[js] + kNB - 1) / kNB);
-        }
-        bad += range_faults(iv, P.tri_flags);
+            for (int32_t js : lp.elim_nodes) iv.emplace_back(P.fst[js], (int64_t)P.fst[js] + P.S[js]);
+        bad += range_faults(iv, P.neq);
     }
     for (const LevelPlan& lp : P.levels) {
         // triangle tasks: each block once, after the block above it
@@ -967,24 +891,28 @@ int64_t check_solve_plan(const Plan& P, int plant, int64_t* tasks) {
         }
         for (int64_t v : pos)
             if (v < 0) ++bad;                                            // a block never listed
-        // rectangles: one job per front with F > S, of the right sizes, with
-        // disjoint partial-sum ranges
-        std::vector<int64_t> nrect(ns, 0), nrows(ns, 0);
+        // rectangles: one job per sweep and front with F > S, of the right sizes,
+        // with disjoint partial-sum ranges
+        std::vector<int64_t> nrect(ns, 0), nback(ns, 0), nrows(ns, 0);
         std::vector<std::pair<int64_t, int64_t>> riv, fiv;
-        for (int64_t j = 0; j < lp.rect.job_count; ++j) {
-            const Job& jb = P.jobs[lp.rect.job_begin + j];
-            const int32_t js = jb.node;
-            if (js < 0 || js >= ns || first[js] < 0) {
-                ++bad;
-                continue;
+        auto check_rect = [&](const Launch& l, std::vector<int64_t>& count, int64_t tc, bool fwd) {
+            for (int64_t j = 0; j < l.job_count; ++j) {
+                const Job& jb = P.jobs[l.job_begin + j];
+                const int32_t js = jb.node;
+                if (js < 0 || js >= ns || first[js] < 0) {
+                    ++bad;
+                    continue;
+                }
+                const int64_t f = P.F[js], s = P.S[js], tr = fwd ? fwd_rows((int)s) : kRectRows;
+                const int64_t nrc = (f - s + tr - 1) / tr, ncc = (s + tc - 1) / tc;
+                if (f <= s || jb.k_lo != nrc || jb.k_hi != ncc || job_tasks(P, l, j) != nrc * ncc) ++bad;
+                ++count[js];
+                if (fwd) fiv.emplace_back(fo[js], fo[js] + ncc * (f - s));
+                else riv.emplace_back(P.rect_off[js], P.rect_off[js] + nrc * s);
             }
-            const int64_t f = P.F[js], s = P.S[js];
-            const int64_t nrc = (f - s + kRectRows - 1) / kRectRows, ncc = (s + kRectCols - 1) / kRectCols;
-            if (f <= s || jb.k_lo != nrc || jb.k_hi != ncc || job_tasks(P, lp.rect, j) != nrc * ncc) ++bad;
-            ++nrect[js];
-            riv.emplace_back(P.rect_off[js], P.rect_off[js] + nrc * s);
-            fiv.emplace_back(fo[js], fo[js] + ncc * (f - s));
-        }
+        };
+        check_rect(lp.rect, nrect, kFwdCols, true);
+        check_rect(lp.rect_back, nback, kRectCols, false);
         for (int64_t j = 0; j < lp.rect_rows.job_count; ++j) {
             const Job& jb = P.jobs[lp.rect_rows.job_begin + j];
             const int32_t js = jb.node;
@@ -997,7 +925,7 @@ int64_t check_solve_plan(const Plan& P, int plant, int64_t* tasks) {
         }
         for (int32_t js : lp.elim_nodes) {
             const int64_t want = P.F[js] > P.S[js] ? 1 : 0;
-            if (nrect[js] != want || nrows[js] != want) ++bad;
+            if (nrect[js] != want || nback[js] != want || nrows[js] != (P.S[js] > kFwdCols ? want : 0)) ++bad;
         }
         bad += range_faults(riv, P.rect_entries);
         bad += range_faults(fiv, P.fwd_entries);

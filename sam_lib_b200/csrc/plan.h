@@ -122,15 +122,11 @@ struct LevelPlan {
     // per panel step: the columns of the super-panels that end at that step
     // (their last panel's TRSM is done), for writing LNZ early
     std::vector<Launch> wb_sp;
-    std::vector<Launch> fsolve;               // forward step: 1 diagonal CTA + row blocks below
-    std::vector<Launch> bsolve;               // back step: 1 diagonal CTA + column groups [0, k0)
-    // solves in kSolveBlock-wide steps: per step, the diagonal-block launch uses
-    // the job list (one CTA per job), the update launch its tasks
-    std::vector<Launch> fs_upd;               // rows [k1, F) below the block, kSolveRows per task
-    std::vector<Launch> bs_upd;               // columns [0, k0) before the block, kBwdCols per task
-    std::vector<Launch> blk_mv;               // product with the block inverse, 32 rows/columns per task
-    Launch rect;                              // rectangle rows [S, F): one task per 256 x 256 tile
-    Launch rect_rows;                         // forward solve, rows [S, F): one task per row
+    // solves, rows [S, F) of the eliminated large fronts: forward one task per
+    // kFwdRows x kFwdCols tile, back one per kRectRows x kRectCols tile
+    Launch rect, rect_back;
+    Launch rect_rows;                         // forward, fronts of several column tiles: one task per row
+    bool retained_large = false;              // the level has a retained large front
     // triangle of the solves as one dataflow launch: tasks (node, 64-row
     // block) of the level's eliminated large fronts, block-major, in
     // Plan::tri_tasks[tri_begin .. tri_begin + tri_count)
@@ -146,11 +142,10 @@ struct LevelPlan {
     std::vector<TcLaunch> outer_tc;                 // mixed precision: the K = S update
 };
 
-constexpr int kBwdCols = 8;                   // columns per CTA in the back-solve update
-constexpr int kSolveBlock = 256;              // width of a solve step (4 diagonal blocks of kNB)
-constexpr int kSolveRows = 128;               // rows per CTA in the forward update (x 2 column halves)
-constexpr int kRectCols = 64;                 // columns per CTA of the solves' rectangle launches
-constexpr int kRectRows = 256;                // rows per CTA of the solves' rectangle launches
+constexpr int kFwdRows = 64, kFwdCols = 256;   // tile of the forward rectangle launches
+constexpr int kFwdNarrow = 64;                 // up to this S a tile has 256 rows and all S columns
+constexpr int fwd_rows(int s) { return s <= kFwdNarrow ? 256 : kFwdRows; }
+constexpr int kRectCols = 64, kRectRows = 256; // tile of the back rectangle launches
 
 struct Plan {
     // sizes
@@ -181,23 +176,15 @@ struct Plan {
     // of node js is the column-major kNB x kNB matrix at linv_off[js] + st*kNB*kNB
     std::vector<int64_t> linv_off;
     int64_t linv_doubles = 0;
-    // inverses of the kSolveBlock-wide unit-lower diagonal blocks (the solves):
-    // block b of node js is column-major nb x nb (nb = min(kSolveBlock, S - b*kSolveBlock))
-    // at xinv_off[js] + b*kSolveBlock*kSolveBlock
-    std::vector<int64_t> xinv_off;
-    int64_t xinv_doubles = 0;
-    Launch inv_blocks;                        // one task per (large front, solve block)
-    // back-solve rectangle partial sums: node js uses rect_off[js] .. + nchunk*S entries
-    // (each kMaxRHS doubles) of a scratch of rect_entries entries (max over levels)
+    // rectangle partial sums (one per right-hand side and entry): back, node js
+    // uses rect_off[js] .. + nrc*S, forward fwd_off[js] .. + ncc*(F-S) entries of a
+    // scratch of rect_entries / fwd_entries (max over levels)
     std::vector<int64_t> rect_off;
     int64_t rect_entries = 0;
-    std::vector<int64_t> fwd_off;            // forward-sweep rectangle partials, per level
+    std::vector<int64_t> fwd_off;
     int64_t fwd_entries = 0;
     // the solves' triangle tasks (pairs node, 64-row block) of every level
-    // and, per large front, the first of its blocks' ready flags
     std::vector<int32_t> tri_tasks;
-    std::vector<int64_t> tri_off;
-    int64_t tri_flags = 0;
     bool any_large = false;
     // levels and tasks
     std::vector<LevelPlan> levels;
@@ -245,10 +232,10 @@ int64_t check_schedule(const Plan& P, bool tc, int skip_join);
 // Self-check of the solves' plan: every eliminated large front of a level has
 // each of its 64-row triangle blocks as one task of that level's dataflow
 // launch, after the task of the block above it (the forward sweep takes them
-// in list order, the back sweep in reverse), with its own ready flag (the
-// fronts' flag ranges disjoint and inside Plan::tri_flags); each front with
-// F > S has one rectangle job and one forward-rows job of the right sizes,
-// and the partial-sum ranges of a level's fronts (rect_off, fwd_off) are
+// in list order, the back sweep in reverse), with its own equations (the
+// fronts' solved rows disjoint and inside NEQ); each front with F > S has one
+// rectangle job per sweep and, with several column tiles, one forward-rows
+// job, of the right sizes, and the partial-sum ranges of a level's fronts (rect_off, fwd_off) are
 // disjoint and inside their scratch.  Returns the number of violations.
 // plant: 0 checks P as built; 1 swaps the first two blocks of a front in a
 // copy, 2 moves one front's forward partials onto another's in a copy (a
