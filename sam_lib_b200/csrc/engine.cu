@@ -385,9 +385,6 @@ __global__ void k_reduce(const double* v, int64_t n, double* out) {
 // TOL(1) max(1, |TOL(4) a_jj|) and recorded in DCOR(1:2, j).
 enum PivotRule { kPivotLDL = 0, kPivotReplace = 1, kPivotChol = 2, kPivotChol4 = 3 };
 
-// A NaN or infinite pivot (a NaN or Inf anywhere in SM reaches some pivot
-// through the Schur updates) fails the test as well, so that the call reports
-// an error instead of a factor full of NaN.
 // 1/c for the pivots: the hardware reciprocal approximation (rcp.approx.ftz.f64)
 // refined by two Newton-Raphson steps x <- x + x (1 - c x), each with fused
 // multiply-adds; within one ulp of 1/c for normal c (tests compare it with
@@ -395,12 +392,24 @@ enum PivotRule { kPivotLDL = 0, kPivotReplace = 1, kPivotChol = 2, kPivotChol4 =
 // non-finite c take the quotient itself.  It replaces a division on the
 // pivot chain of every elimination step.
 __device__ __forceinline__ double recip_nr(double c) {
-    const double ac = fabs(c);
-    if (!(ac >= 2.2250738585072014e-308 && ac <= 8.98846567431158e307)) return 1.0 / c;
+    // (the approximation first, so that it does not wait for the test)
     double r;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(c));
+    asm volatile("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(c));
     r = fma(r, fma(-c, r, 1.0), r);
     r = fma(r, fma(-c, r, 1.0), r);
+    const unsigned e = ((unsigned)__double2hiint(c) >> 20) & 0x7ffu;
+    if (e - 1u > 2044u) r = 1.0 / c;                 // biased exponents 1 .. 2045: 2^-1022 <= |c| < 2^1023
+    return r;
+}
+
+// the same where c is the same in all lanes of the warp: a uniform branch
+__device__ __forceinline__ double recip_nr_uniform(double c) {
+    double r;
+    asm volatile("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(c));
+    r = fma(r, fma(-c, r, 1.0), r);
+    r = fma(r, fma(-c, r, 1.0), r);
+    const unsigned e = ((unsigned)__double2hiint(c) >> 20) & 0x7ffu;
+    if (__any_sync(0xffffffffu, e - 1u > 2044u)) r = 1.0 / c;
     return r;
 }
 
@@ -412,6 +421,9 @@ __global__ void k_recip_check(const double* x, int64_t n, double* out) {
     }
 }
 
+// A NaN or infinite pivot (a NaN or Inf anywhere in SM reaches some pivot
+// through the Schur updates) fails the test as well, so that the call reports
+// an error instead of a factor full of NaN.
 __device__ __forceinline__ bool pivot_fails(int rule, double d, double ad, double tol1) {
     if (!isfinite(d)) return true;
     if (rule == kPivotChol4) return d < -tol1 * fabs(ad);
@@ -444,178 +456,359 @@ __device__ __forceinline__ bool near_zero_pivot(const PV& P, double d, double ad
     return P.near_tol > 0.0 && fabs(d) < P.near_tol * fabs(ad);
 }
 
+namespace gemm {
+__device__ __forceinline__ void dmma(double& c0, double& c1, double a, double b) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+                 : "+d"(c0), "+d"(c1)
+                 : "d"(a), "d"(b));
+}
+}  // namespace gemm
+
+constexpr int kDG = 16;                              // columns of an elimination group
+template <int V>
+struct IntC {
+    static constexpr int value = V;
+};
+
+// barrier of the first n warps of the CTA (barrier 1)
+__device__ __forceinline__ void sync_warps(int n) { asm volatile("bar.sync 1, %0;" ::"r"(32 * n) : "memory"); }
+
+// One 16x16 tile of a packed front: A(i, j) -= sum_{k < K} w_ik (w_jk / d_k) for
+// i0 <= i < F, j0 <= j < jend, i >= j, by one warp with DMMA (2x2 tiles of 8x8,
+// k ascending: DMMA chains its products in order, like a loop of multiply-adds).
+// A holds the unscaled columns w, rd the reciprocal pivots.
+__device__ __forceinline__ void small_tile(double* A, const double* rd, int F, int K, int i0, int j0, int jend,
+                                           int lane) {
+    const int fr = lane >> 2, fk = lane & 3;
+    double c[2][2][2];
+#pragma unroll
+    for (int a = 0; a < 2; ++a)
+#pragma unroll
+        for (int b = 0; b < 2; ++b)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int i = i0 + 8 * a + fr, j = j0 + 8 * b + 2 * fk + h;
+                c[a][b][h] = (i < F && j < jend && i >= j) ? A[pk(i, j, F)] : 0.0;
+            }
+    const bool vi0 = i0 + fr < F, vi1 = i0 + 8 + fr < F, vj0 = j0 + fr < F, vj1 = j0 + 8 + fr < F;
+    int base = pk(0, fk, F), k = fk;                 // A[base + i] = w_ik
+    for (int k4 = 0; k4 < K; k4 += 4) {
+        const bool vk = k < K;
+        const double r = vk ? rd[k] : 0.0;
+        const double a0 = vk && vi0 ? -A[base + i0 + fr] : 0.0, a1 = vk && vi1 ? -A[base + i0 + 8 + fr] : 0.0;
+        const double b0 = vk && vj0 ? A[base + j0 + fr] * r : 0.0, b1 = vk && vj1 ? A[base + j0 + 8 + fr] * r : 0.0;
+        gemm::dmma(c[0][0][0], c[0][0][1], a0, b0);
+        gemm::dmma(c[0][1][0], c[0][1][1], a0, b1);
+        gemm::dmma(c[1][0][0], c[1][0][1], a1, b0);
+        gemm::dmma(c[1][1][0], c[1][1][1], a1, b1);
+        base += 4 * F - 4 * k - 10;                  // pk(0, k + 4) - pk(0, k)
+        k += 4;
+    }
+#pragma unroll
+    for (int a = 0; a < 2; ++a)
+#pragma unroll
+        for (int b = 0; b < 2; ++b)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int i = i0 + 8 * a + fr, j = j0 + 8 * b + 2 * fk + h;
+                if (i < F && j < jend && i >= j) A[pk(i, j, F)] = c[a][b][h];
+            }
+}
+
+// The published column of an elimination step: entry j of the columns after
+// the current one, for every lane of the warp.
+template <int W>
+__device__ __forceinline__ void read_column(const double* cb, double (&c)[kDG]) {
+#pragma unroll
+    for (int j = 0; j < (W + 1) / 2; ++j) {
+        const double2 v = *reinterpret_cast<const double2*>(cb + 2 * j);
+        c[2 * j] = v.x;
+        c[2 * j + 1] = v.y;
+    }
+}
+
+// Elimination of the columns c0 .. c0 + kmax - 1 of a packed front by one warp,
+// without a CTA barrier: lanes 0-15 hold the group's own rows (every warp
+// repeats them), and every lane one row below, 32 of them from c0 + 16 + 32 w on,
+// 16 entries each in registers; the pivot goes round by a shuffle, the column
+// through the warp's own shared memory cb (2 x 32).  The columns stay unscaled
+// (w).  The registers move down by one each step (a[0] is always the current
+// column), so that the loop over the columns is a loop and not 16 copies, which a
+// kernel of one pass pays for in instruction fetches, and a step has no branch
+// but the loop's (the reciprocal's is uniform): 610 clocks a step with one, about 150
+// without.
+// Returns the failing column or -1.
+template <int PR>
+__device__ __forceinline__ int small_group(const PV& P, int js, double* A, double* rd, double* dd, double* cb, int F,
+                                           int c0, int kmax, int w, int sets, int lane) {
+    const int fst = P.fst[js];
+    const bool own = lane < kDG && c0 + lane < F;
+    const int row = c0 + kDG + 32 * w + lane;
+    const bool below = row < F;
+    const double adr = lane < kmax ? P.adiag[fst + c0 + lane] : 0.0;
+    double a[kDG], x[kDG];
+#pragma unroll
+    for (int j = 0; j < kDG; ++j) {
+        a[j] = (own && j < kmax && j <= lane) ? A[pk(c0 + lane, c0 + j, F)] : 0.0;
+        x[j] = (below && j < kmax) ? A[pk(row, c0 + j, F)] : 0.0;
+    }
+    if (sets > 1) sync_warps(sets);                    // all have read the own rows, which set 0 writes back
+    double dmine = 1.0, rmine = 1.0;                   // lane k keeps pivot k
+    double* ap = A + pk(0, c0, F);                     // the current column, row 0
+    const int own_row = w == 0 && own ? c0 + lane : -1;
+    auto step = [&](int k, auto width) -> bool {
+        constexpr int W = decltype(width)::value;
+        double* cbk = cb + (k & 1) * 32;
+        const double a0 = a[0], x0 = x[0];
+        double d = __shfl_sync(0xffffffffu, a0, k);
+        if (PR == kPivotReplace || PR == kPivotChol4) {
+            const double ad = __shfl_sync(0xffffffffu, adr, k);
+            const int col = c0 + k;
+            if (PR == kPivotReplace) {
+                const double d0 = d;
+                d = fc3_pivot(P, d0, ad);
+                if (w == 0 && lane == 0) fc3_record(P, fst + col, d0, d);
+            } else {
+                if (pivot_fails(PR, d, ad, P.tol1)) {            // sprfc4.f:980
+                    if (w == 0 && lane == 0) {
+                        record_fail(P, js, col, d, ad);
+                        chol4_fail_record(P, fst + col, d);
+                    }
+                    return false;
+                }
+                d = chol4_pivot(P, fst + col, d, ad, w == 0 && lane == 0);
+            }
+        }
+        cbk[(lane - k - 1) & 31] = a0;                           // lane k + 1 + j to entry j
+        const double r = recip_nr_uniform(d);
+        dmine = lane == k ? d : dmine;
+        rmine = lane == k ? r : rmine;
+        if (own_row >= c0 + k) ap[own_row] = lane == k ? d : a0;
+        if (below) ap[row] = x0;
+        ap += F - (c0 + k) - 1;
+        __syncwarp();
+        double c[kDG];
+        read_column<W>(cbk, c);
+#pragma unroll
+        for (int j = 0; j < W; ++j) {
+            const double l = c[j] * r;
+            a[j] = fma(-a0, l, a[j + 1]);
+            x[j] = fma(-x0, l, x[j + 1]);
+        }
+        return true;
+    };
+    int k = 0;
+    bool go = true;
+#pragma unroll 1
+    for (; k < min(kmax, kDG / 2) && go; ++k) go = step(k, IntC<kDG - 1>());
+#pragma unroll 1
+    for (; k < kmax && go; ++k) go = step(k, IntC<kDG / 2 - 1>());
+    if (w == 0 && lane < kmax) {
+        dd[c0 + lane] = dmine;
+        rd[c0 + lane] = rmine;
+    }
+    if (PR == kPivotChol4) return go ? -1 : c0 + k - 1;
+    if (PR == kPivotReplace || w != 0) return -1;
+    // the first failing pivot (sprfc1.f:1274, sprfc2.f:1004); the steps after it
+    // only computed values that are thrown away
+    const unsigned m = __ballot_sync(0xffffffffu, lane < kmax && pivot_fails(PR, dmine, adr, P.tol1));
+    if (!m) return -1;
+    const int f = __ffs(m) - 1;
+    if (lane == f) record_fail(P, js, c0 + f, dmine, adr);
+    return c0 + f;
+}
+
+// The chain of S pivots and the latency of the children's loads bound a small
+// front, so the columns are eliminated in groups of 16 by warps (small_group)
+// after one DMMA update by everything before them, the trailing block takes
+// one DMMA update at the end, and the children's data are loaded ahead.  Every
+// entry takes its multiply-adds in ascending k.  One rank-1 step of all
+// threads and two barriers per column before: all small fronts of 12^3 0.80
+// ms, now 0.65 ms; of 512 boxes of 3^3 to 12^3 6.8 and 6.0 ms; 4^3 alone 0.42
+// and 0.28 ms.
 template <int PR>
 __global__ void __launch_bounds__(256) k_small_front(const int32_t* nodes, PV P) {
     extern __shared__ double sh[];
+    __shared__ __align__(16) double cbuf[8][64];
+    __shared__ int16_t srel[2][kSmallMaxF];
+    __shared__ int64_t s_rel[32], s_upd[32];
+    __shared__ int s_q[32], s_ld[32];
+    __shared__ int s_fail;
     if (P.st->any_fail) return;
     const int js = nodes[blockIdx.x];
     if (node_off(P, js)) return;
-    if (children_bad(P, js)) {
-        if (threadIdx.x == 0) P.sn_bad[js] = 1;
-        return;
-    }
     const int F = P.F[js], S = P.S[js], fst = P.fst[js];
+    const int kid0 = P.child_ptr[js], nkid = P.child_ptr[js + 1] - kid0;
     const int npk = F * (F + 1) / 2;
     double* A = sh;
-    double* wcol = sh + npk;
-    double* rdk = wcol + F;                   // 1 / d_k of the S pivots
+    double* rd = sh + npk;                    // 1 / d_k of the S pivots
+    double* dd = rd + F;                      // the pivots
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarp = blockDim.x >> 5;
+    if (tid == 0) s_fail = F;
+    // the first 32 children, last sibling first (sprfc1.f:534-584), one thread each
+    auto load_kids = [&](int m0) {
+        if (tid < 32 && m0 + tid < nkid) {
+            const int c = P.child[kid0 + nkid - 1 - (m0 + tid)];
+            s_q[tid] = P.F[c] - P.S[c];
+            s_rel[tid] = P.rel_off[c];
+            s_upd[tid] = P.upd_off[c];
+            s_ld[tid] = P.buf_ld[c];
+        }
+    };
+    load_kids(0);
+    int bad = 0;
+    for (int k = tid; k < nkid; k += blockDim.x) bad |= P.sn_bad[P.child[kid0 + k]];
     // fully-summed columns: the packed trapezoid of LNZ is the front's first SUPSZE entries
     const int supsze = F * S - (S * (S - 1)) / 2;
     const double* lnz = P.lnz + P.lnz_off[js];
-    for (int i = tid; i < npk; i += blockDim.x) A[i] = (i < supsze) ? lnz[i] : 0.0;
-    __syncthreads();
-    // extend-add, children last sibling first (sprfc1.f:534-584)
-    for (int k = P.child_ptr[js + 1] - 1; k >= P.child_ptr[js]; --k) {
-        const int c = P.child[k];
-        const int q = P.F[c] - P.S[c];
-        if (q <= 0) continue;
-        const int32_t* rel = P.rel + P.rel_off[c];
-        const double* U = P.arena + P.upd_off[c];
-        const int ld = P.buf_ld[c];
-        for (int t = warp; t < q; t += nwarp) {
-            const int pj = rel[t];
-            const double* Ut = U + (int64_t)t * ld;
-            int r = t + lane;
-            for (; r + 32 < q; r += 64) {
-                const int p0 = pk(rel[r], pj, F), p1 = pk(rel[r + 32], pj, F);
-                const double u0 = __ldcg(Ut + r), u1 = __ldcg(Ut + r + 32);
-                const double a0 = A[p0], a1 = A[p1];
-                A[p0] = a0 + u0;
-                A[p1] = a1 + u1;
-            }
-            if (r < q) A[pk(rel[r], pj, F)] += Ut[r];
+    for (int i0 = tid; i0 < npk; i0 += 8 * (int)blockDim.x) {
+        double v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const int i = i0 + u * (int)blockDim.x;
+            v[u] = i < supsze ? lnz[i] : 0.0;
         }
-        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const int i = i0 + u * (int)blockDim.x;
+            if (i < npk) A[i] = v[u];
+        }
     }
-    // LDL' of the S fully-summed columns with the trailing (Schur) update;
-    // a retained front is only assembled
-    int neg = 0;
-    double tmax = 0.0;
-    bool failed = false;
-    const bool ret = is_retained(P, js);
-    for (int k = 0; k < (ret ? 0 : S); ++k) {
-        double d = A[pk(k, k, F)];
-        const double ad = P.adiag[fst + k];
-        if (PR == kPivotReplace) {
-            const double d0 = d;
-            d = fc3_pivot(P, d0, ad);
-            if (tid == 0) fc3_record(P, fst + k, d0, d);
-        } else if (pivot_fails(PR, d, ad, P.tol1)) {   // sprfc1.f:1274, sprfc2.f:1004, sprfc4.f:980
-            if (tid == 0) {
-                record_fail(P, js, k, d, ad);
-                if (PR == kPivotChol4) chol4_fail_record(P, fst + k, d);
-            }
-            failed = true;
-            break;
-        } else if (PR == kPivotChol4) {
-            d = chol4_pivot(P, fst + k, d, ad, tid == 0);
-        }
-        if (d < 0.0) ++neg;
-        if (tid == 0 && near_zero_pivot(P, d, ad)) atomicAdd(&P.st->near_piv, 1ull);
-        tmax = fmax(tmax, ad / d);
-        const double rd = recip_nr(d);
-        if (tid == 0) rdk[k] = rd;
-        // rows below the S columns stay unscaled until the trailing update
-        for (int i = k + 1 + tid; i < F; i += blockDim.x) {
-            const double a = A[pk(i, k, F)];
-            wcol[i] = a;
-            if (i < S) A[pk(i, k, F)] = a * rd;
-        }
-        __syncthreads();
-        if ((PR == kPivotReplace || PR == kPivotChol4) && tid == 0) A[pk(k, k, F)] = d;   // every thread has read the old pivot
-        // rank-1 update of the remaining fully-summed columns (all their rows)
-        for (int j = k + 1 + warp; j < S; j += nwarp) {
-            const double ljk = A[pk(j, k, F)];
-            double* cj = A + pk(j, j, F) - j;
-            // loads of four rows ahead of their stores (shared-memory latency overlaps)
-            int i = j + lane;
-            for (; i + 96 < F; i += 128) {
-                const double a0 = cj[i], a1 = cj[i + 32], a2 = cj[i + 64], a3 = cj[i + 96];
-                const double w0 = wcol[i], w1 = wcol[i + 32], w2 = wcol[i + 64], w3 = wcol[i + 96];
-                cj[i] = a0 - w0 * ljk;
-                cj[i + 32] = a1 - w1 * ljk;
-                cj[i + 64] = a2 - w2 * ljk;
-                cj[i + 96] = a3 - w3 * ljk;
-            }
-            for (; i < F; i += 32) cj[i] -= wcol[i] * ljk;
-        }
-        __syncthreads();
-    }
-    if (failed) {
-        if (tid == 0) {
-            P.sn_neg[js] = neg;
-            atomicAdd(&P.st->numneg, (unsigned long long)neg);
-        }
+    if (__syncthreads_or(bad)) {              // a child failed, or depends on a failure
+        if (tid == 0) P.sn_bad[js] = 1;
         return;
     }
-    if (!ret && S > 0 && S < F) {
-        // The trailing (F-S)^2 block: each thread keeps 4x4 tiles in registers
-        // and applies c -= w_ik (w_jk / d_k) for k = 0 .. S-1 in order, the
-        // same operations in the same order as S rank-1 steps, with one
-        // shared-memory read-modify-write per entry instead of S.
-        const int q = F - S, nt = (q + 3) >> 2;
-        const int ntiles = nt * (nt + 1) / 2;
-        for (int t = tid; t < ntiles; t += blockDim.x) {
-            int bi = (int)((sqrtf(8.0f * (float)t + 1.0f) - 1.0f) * 0.5f);
-            while (bi * (bi + 1) / 2 > t) --bi;
-            while ((bi + 1) * (bi + 2) / 2 <= t) ++bi;
-            const int bj = t - bi * (bi + 1) / 2;
-            const int i0 = S + 4 * bi, j0 = S + 4 * bj;
-            double c[4][4];
+    // extend-add: a warp takes every nwarp-th column of a child, in 32-row
+    // pieces, kExt pieces at a time; the next pieces (of this child or the
+    // next one) and the next child's rows are loaded while these are added
+    constexpr int kExt = 8;
+    struct Piece {
+        int t, r0;
+    };
+    auto first = [&]() { return Piece{warp, warp & ~31}; };
+    auto advance = [&](Piece& p, int q) {
+        p.r0 += 32;
+        if (p.r0 >= q) {
+            p.t += nwarp;
+            p.r0 = p.t & ~31;
+        }
+    };
+    auto load = [&](int m, Piece& p, double (&u)[kExt]) {
+        const int q = s_q[m], ld = s_ld[m];
+        const double* U = P.arena + s_upd[m];
 #pragma unroll
-            for (int a = 0; a < 4; ++a)
-#pragma unroll
-                for (int b = 0; b < 4; ++b) {
-                    const int i = i0 + a, j = j0 + b;
-                    c[a][b] = (i < F && j <= i) ? A[pk(i, j, F)] : 0.0;
+        for (int e = 0; e < kExt; ++e) {
+            const int r = p.r0 + lane;
+            u[e] = (p.t < q && r >= p.t && r < q) ? __ldcg(U + r + (int64_t)p.t * ld) : 0.0;
+            advance(p, q);
+        }
+    };
+    for (int m0 = 0; m0 < nkid; m0 += 32) {
+        const int n = min(32, nkid - m0);
+        if (m0) {
+            __syncthreads();                   // the last child's adds are done
+            load_kids(m0);
+            __syncthreads();
+        }
+        double u[kExt];
+        Piece pl = first();
+        load(0, pl, u);
+        if (tid < s_q[0]) srel[0][tid] = (int16_t)P.rel[s_rel[0] + tid];
+        for (int m = 0; m < n; ++m) {
+            const int q = s_q[m];
+            const int16_t* rel = srel[m & 1];
+            int next_rel = 0;
+            if (m + 1 < n && tid < s_q[m + 1]) next_rel = P.rel[s_rel[m + 1] + tid];
+            __syncthreads();                   // rel is there, the child before is added
+            Piece pa = first();
+            for (;;) {
+                double un[kExt];
+                const bool more = pl.t < q;
+                if (more) {
+                    load(m, pl, un);
+                } else if (m + 1 < n) {
+                    pl = first();
+                    load(m + 1, pl, un);
                 }
-            for (int k = 0; k < S; ++k) {
-                const double r = rdk[k];
-                const int base = pk(0, k, F);            // A[base + i] = entry (i, k), i >= k
-                double w[4], l[4];
 #pragma unroll
-                for (int a = 0; a < 4; ++a) w[a] = (i0 + a < F) ? A[base + i0 + a] : 0.0;
+                for (int e = 0; e < kExt; ++e) {
+                    const int r = pa.r0 + lane;
+                    if (pa.t < q && r >= pa.t && r < q) A[pk(rel[r], rel[pa.t], F)] += u[e];
+                    advance(pa, q);
+                }
 #pragma unroll
-                for (int b = 0; b < 4; ++b) l[b] = ((j0 + b < F) ? A[base + j0 + b] : 0.0) * r;
-#pragma unroll
-                for (int a = 0; a < 4; ++a)
-#pragma unroll
-                    for (int b = 0; b < 4; ++b) c[a][b] -= w[a] * l[b];
+                for (int e = 0; e < kExt; ++e) u[e] = un[e];
+                if (!more) break;
             }
-#pragma unroll
-            for (int a = 0; a < 4; ++a)
-#pragma unroll
-                for (int b = 0; b < 4; ++b) {
-                    const int i = i0 + a, j = j0 + b;
-                    if (i < F && j <= i) A[pk(i, j, F)] = c[a][b];
-                }
+            if (m + 1 < n && tid < s_q[m + 1]) srel[(m + 1) & 1][tid] = (int16_t)next_rel;
         }
-        __syncthreads();
-        // and now the rows below the S columns to L
-        for (int e = tid; e < S * q; e += blockDim.x) {
-            const int k = e / q, i = S + e % q;
-            A[pk(i, k, F)] *= rdk[k];
-        }
-        __syncthreads();
     }
-    // write back the S columns (LNZ layout == packed layout) and the pivots
+    __syncthreads();
+    const bool ret = is_retained(P, js);       // a retained front is only assembled
+    for (int c0 = 0; c0 < (ret ? 0 : S); c0 += kDG) {
+        const int kmax = min(kDG, S - c0);
+        if (c0 > 0) {
+            for (int i0 = c0 + kDG * warp; i0 < F; i0 += kDG * nwarp) small_tile(A, rd, F, c0, i0, c0, c0 + kmax, lane);
+            __syncthreads();
+        }
+        const int rest = F - c0 - kDG, sets = rest > 0 ? (rest + 31) / 32 : 1;
+        if (warp < sets) {                        // at most 5 sets (of 8 warps), 2 (of 4) up to F = 64
+            const int f = small_group<PR>(P, js, A, rd, dd, cbuf[warp], F, c0, kmax, warp, sets, lane);
+            if (f >= 0 && lane == 0) s_fail = f;      // (set 0's, or every warp's the same)
+        }
+        __syncthreads();
+        if (s_fail < F) break;
+    }
+    const int kend = ret ? 0 : min(S, s_fail);
+    if (warp == 0) {
+        // inertia and TOL(2) of the processed columns (sprfc1.f:1280-1290)
+        int neg = 0, near = 0;
+        double tmax = 0.0;
+        for (int k = lane; k < kend; k += 32) {
+            const double d = dd[k], ad = P.adiag[fst + k];
+            neg += d < 0.0;
+            near += near_zero_pivot(P, d, ad);
+            tmax = fmax(tmax, ad / d);
+        }
+        for (int o = 16; o > 0; o >>= 1) {
+            neg += __shfl_xor_sync(0xffffffffu, neg, o);
+            near += __shfl_xor_sync(0xffffffffu, near, o);
+            tmax = fmax(tmax, __shfl_xor_sync(0xffffffffu, tmax, o));
+        }
+        if (lane == 0) {
+            P.sn_neg[js] = neg;
+            if (neg) atomicAdd(&P.st->numneg, (unsigned long long)neg);
+            if (near) atomicAdd(&P.st->near_piv, (unsigned long long)near);
+            if (s_fail >= F) atomic_max_double(&P.st->tol2, tmax);
+        }
+    }
+    if (s_fail < F) return;
+    // write back the S columns (LNZ layout == packed layout) as L, and the pivots
     double* lnzw = P.lnz + P.lnz_off[js];
-    for (int i = tid; i < supsze; i += blockDim.x) lnzw[i] = A[i];
+    for (int k = warp; k < S; k += nwarp) {
+        const int base = pk(0, k, F);
+        const double r = ret ? 1.0 : rd[k];
+        for (int i = k + lane; i < F; i += 32) lnzw[base + i] = (i == k || ret) ? A[base + i] : A[base + i] * r;
+    }
     if (!ret)
-        for (int j = tid; j < S; j += blockDim.x) P.dvec[fst + j] = A[pk(j, j, F)];
+        for (int j = tid; j < S; j += blockDim.x) P.dvec[fst + j] = dd[j];
     const int q = F - S;
-    if (q > 0) {
-        double* U = P.arena + P.upd_off[js];
-        const int ld = P.buf_ld[js];
-        for (int t = warp; t < q; t += nwarp)
-            for (int r = t + lane; r < q; r += 32) U[r + (int64_t)t * ld] = A[pk(S + r, S + t, F)];
+    if (q <= 0) return;
+    if (!ret) {
+        // the trailing (F-S)^2 block in 16x16 tiles
+        const int nt = (q + kDG - 1) / kDG;
+        int ti = 0, tj = warp;
+        for (int t = warp; t < nt * (nt + 1) / 2; t += nwarp) {
+            while (tj > ti) tj -= ++ti;
+            small_tile(A, rd, F, S, S + kDG * ti, S + kDG * tj, F, lane);
+            tj += nwarp;
+        }
+        __syncthreads();
     }
-    if (tid == 0) {
-        P.sn_neg[js] = neg;
-        atomicAdd(&P.st->numneg, (unsigned long long)neg);
-        atomic_max_double(&P.st->tol2, tmax);
-    }
+    double* U = P.arena + P.upd_off[js];
+    const int ld = P.buf_ld[js];
+    for (int t = warp; t < q; t += nwarp)
+        for (int r = t + lane; r < q; r += 32) U[r + (int64_t)t * ld] = A[pk(S + r, S + t, F)];
 }
 
 // ---------------------------------------------------------------------------
@@ -740,124 +933,194 @@ __global__ void __launch_bounds__(256) k_assemble(const Job* jobs, int64_t njobs
     }
 }
 
-namespace gemm {
-__device__ __forceinline__ void dmma(double& c0, double& c1, double a, double b) {
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-                 : "+d"(c0), "+d"(c1)
-                 : "d"(a), "d"(b));
-}
-}  // namespace gemm
-
 // LDL' of one nb x nb diagonal block, pivot test / inertia / TOL(2) as
 // SPRF17 (sprfc1.f:1272-1294), and X = L11^-1 (unit lower) for the panel TRSM
 // and the solves.  One CTA per block, so a chain of kNB dependent pivots
-// bounds it: reciprocal, scaling, update, next pivot.  The block goes in four
-// groups of 16 columns.  A group's columns are eliminated by up to three
-// warps without a CTA barrier: a lane holds one row's 16 entries in registers,
-// lanes 0-15 the group's own rows (every warp repeats them) and lanes 16-31 a
-// set of 16 rows below; the pivot goes round by a shuffle, the unscaled column
-// (a_ij -= a_ik * a_jk / d_k) through the warp's own shared memory.  The
-// columns after the group are updated with DMMA tiles (K = 16) by all warps.
-// The inverse of each group's 16x16 triangle is formed beside the next group's
-// elimination, and the 32- and 64-wide inverses by doubling (X21 = -X22 (L21 X11))
-// with DMMA.  Every entry takes its multiply-adds in ascending k (DMMA chains
-// them in that order), so the factors do not depend on the grouping.  32^3, one block: 39 us with 256 threads in lockstep, one barrier
-// per column.
-constexpr int kDG = 16;                              // columns of a group
-constexpr int kDPanLd = kDG + 4;                     // bank-conflict-free DMMA fragments
+// bounds it: reciprocal, scaling, update, next pivot.  The block goes in eight
+// groups of 8 columns.  A group's columns are eliminated by up to three
+// warps without a CTA barrier: a lane holds one row's 8 entries in registers,
+// lanes 0-7 the group's own rows (every warp repeats them) and lanes 8-31 24
+// rows below; the pivot and the unscaled column (a_ij -= a_ik * a_jk / d_k) go
+// round by shuffles, the column's ahead of the reciprocal.  The columns after the
+// group are updated with DMMA tiles (K = 8), up to four at a time per warp: a
+// DMMA takes some 130 clocks to its result, a multiply-add of one warp 8.
+// The inverse of each group's 8x8 triangle is formed beside the next group's
+// elimination, the wider ones by doubling (X21 = -X22 (L21 X11)) with DMMA.
+// Every entry takes its multiply-adds in ascending k (DMMA chains them in that
+// order), so the factors do not depend on the grouping.  20 us a full block
+// alone; all blocks of a 32^3 box 9.8 ms (groups of 16 with the column through
+// shared memory 10.5 ms, one barrier a column 15.0 ms).
+constexpr int kD8 = 8;                               // columns of a group
+constexpr int kDPanLd = kD8 + 1;
 
 // one group's elimination by one warp: rows below in set w (rows
-// c0 + 16 + 16 w ..), kmax columns; returns the failing column for the rule that
+// c0 + 8 + 24 w ..), kmax columns; returns the failing column for the rule that
 // stops at once (kPivotChol4), or -1
 template <int PR>
-__device__ __forceinline__ int diag_group(const PV& P, int js, int k0, int c0, int kmax, int w, int lane, int nb,
-                                          double (*A)[kNB + 1], double (*Wp)[kDPanLd], double* colbuf,
-                                          double* dd, double* rdv, const double* adv) {
+__device__ __forceinline__ int diag_group(const PV& P, int js, int k0, int c0, int kmax, int w, int sets, int lane, int nb,
+                                          double (*A)[kNB + 1], double (*Wp)[kDPanLd], double* dd, double* rdv,
+                                          const double* adv) {
     const int fst = P.fst[js];
-    const bool own = lane < kDG;
-    const int row = own ? c0 + lane : c0 + kDG * w + lane;       // 16 + 16 w + (lane - 16)
-    double a[kDG];
+    const bool own = lane < kD8;
+    const int row = own ? c0 + lane : c0 + 24 * w + lane;        // c0 + 8 + 24 w + (lane - 8)
+    double a[kD8];
 #pragma unroll
-    for (int j = 0; j < kDG; ++j) a[j] = (row < nb && row >= c0 + j) ? A[row][c0 + j] : 0.0;
+    for (int j = 0; j < kD8; ++j) a[j] = (row < nb && row >= c0 + j) ? A[row][c0 + j] : 0.0;
+    if (sets > 1) sync_warps(sets);                    // all have read the own rows, which set 0 writes
+    double dmine = 1.0, rmine = 1.0;                   // lane k keeps pivot k
+    const bool keep = row < nb && (!own || w == 0);
+    double* ap = &A[keep ? row : 0][c0];
+    const bool below = !own && row < nb;
+    double* wp = &Wp[below ? row : kD8][0];
+    const int k_row = !keep ? -1 : own ? lane : kD8;   // columns k < k_row of this lane's row are L
+    int k = 0;
+    bool go = true;
+    // the registers move down by one each step (a[0] is always the current
+    // column): one copy of the step in the instruction stream
+#pragma unroll 1
+    for (; k < kmax && go; ++k) {
+        const double a0 = a[0];
+        double d = __shfl_sync(0xffffffffu, a0, k);
+        double c[kD8 - 1];                             // the column below the pivot
 #pragma unroll
-    for (int k = 0; k < kDG; ++k) {
-        if (k >= kmax) break;
-        double* cb = colbuf + (k & 1) * kDG;
-        double d = __shfl_sync(0xffffffffu, a[k], k);
-        const int col = c0 + k;
+        for (int j = 0; j < kD8 - 1; ++j) c[j] = __shfl_sync(0xffffffffu, a0, k + 1 + j);
         if (PR == kPivotReplace) {
             const double d0 = d;
-            d = fc3_pivot(P, d0, adv[col]);
-            if (w == 0 && lane == 0) fc3_record(P, fst + k0 + col, d0, d);
+            d = fc3_pivot(P, d0, adv[c0 + k]);
+            if (w == 0 && lane == 0) fc3_record(P, fst + k0 + c0 + k, d0, d);
         }
         if (PR == kPivotChol4) {
             // records replacements while it goes, so it stops at a failing pivot
+            const int col = c0 + k;
             if (pivot_fails(PR, d, adv[col], P.tol1)) {
                 if (w == 0 && lane == 0) {
                     record_fail(P, js, k0 + col, d, adv[col]);
                     chol4_fail_record(P, fst + k0 + col, d);
                 }
-                return col;
+                go = false;
+                continue;
             }
             d = chol4_pivot(P, fst + k0 + col, d, adv[col], w == 0 && lane == 0);
         }
-        if (own && lane > k) cb[lane] = a[k];                    // the unscaled column
-        const double rd = recip_nr(d);
-        if (w == 0 && lane == k) {
-            dd[col] = d;
-            rdv[col] = rd;
-        }
-        const double l = a[k] * rd;
-        __syncwarp();
+        const double rd = recip_nr_uniform(d);
+        const double l = a0 * rd;
 #pragma unroll
-        for (int j = k + 1; j < kDG; ++j) a[j] -= l * cb[j];
-        if (own) {
-            if (w == 0 && lane > k && row < nb) A[row][col] = l;
-        } else if (row < nb) {
-            A[row][col] = l;
-            Wp[row][k] = a[k];
-        }
+        for (int j = 0; j < kD8 - 1; ++j) a[j] = fma(-l, c[j], a[j + 1]);
+        dmine = lane == k ? d : dmine;
+        rmine = lane == k ? rd : rmine;
+        if (k < k_row) ap[k] = l;
+        if (below) wp[k] = a0;
     }
-    return -1;
+    if (w == 0 && lane < kmax) {
+        dd[c0 + lane] = dmine;
+        rdv[c0 + lane] = rmine;
+    }
+    return go ? -1 : c0 + k - 1;
 }
 
-// inverse of the unit-lower kDG x kDG block at c0 by one warp: doubling from
-// order b = 1 (X21 = -X22 (L21 X11)); X[i][j] goes to A[c0 + j][c0 + i] (the free
-// upper triangle), T = L21 X11 through t
-__device__ __forceinline__ void diag_group_inverse(double (*A)[kNB + 1], double* t, int c0, int nb, int lane) {
+// one doubling pass of the inverse inside a group, by one warp: the pairs of
+// blocks of order B; T = L21 X11 through t
+template <int B>
+__device__ __forceinline__ void diag_invert_pass(double (*A)[kNB + 1], double* t, int c0, int nb, int lane) {
+    constexpr int BB = B * B, TOT = kD8 / 2 * B;
+    static_assert(TOT <= 32, "one element a lane");
+    const int bs = c0 + lane / BB * 2 * B, i = lane % BB / B, j = lane % B;
+    if (lane < TOT) {
+        double v = 0.0;
+        if (bs + B + i < nb) {
+            v = A[bs + B + i][bs + j];                                     // X11[j][j] = 1
 #pragma unroll
-    for (int b = 1; b < kDG; b <<= 1) {
-        const int bb = b * b, tot = kDG / 2 * b;
-        for (int e = lane; e < tot; e += 32) {
-            const int bs = c0 + e / bb * 2 * b, i = e % bb / b, j = e % b;
-            double v = 0.0;
-            if (bs + b + i < nb) {
-                v = A[bs + b + i][bs + j];                                 // X11[j][j] = 1
-#pragma unroll
-                for (int m = 1; m < b; ++m)
-                    if (m > j) v = fma(A[bs + b + i][bs + m], A[bs + j][bs + m], v);
+            for (int m = 1; m < B; ++m) {
+                const double f = fma(A[bs + B + i][bs + m], A[bs + j][bs + m], v);
+                v = m > j ? f : v;
             }
-            t[e] = v;
         }
-        __syncwarp();
-        for (int e = lane; e < tot; e += 32) {
-            const int bs = c0 + e / bb * 2 * b, i = e % bb / b, j = e % b;
-            double v = t[e];                                               // X22[i][i] = 1
-#pragma unroll
-            for (int m = 0; m + 1 < b; ++m)
-                if (m < i) v = fma(A[bs + b + m][bs + b + i], t[e / bb * bb + m * b + j], v);
-            A[bs + j][bs + b + i] = -v;
-        }
-        __syncwarp();
+        t[lane] = v;
     }
+    __syncwarp();
+    if (lane < TOT) {
+        double v = t[lane];                                                // X22[i][i] = 1
+#pragma unroll
+        for (int m = 0; m + 1 < B; ++m) {
+            const double f = fma(A[bs + B + m][bs + B + i], t[lane / BB * BB + m * B + j], v);
+            v = m < i ? f : v;
+        }
+        A[bs + j][bs + B + i] = -v;
+    }
+    __syncwarp();
+}
+
+// inverse of the unit-lower kD8 x kD8 block at c0 by one warp: doubling from
+// order 1 (X21 = -X22 (L21 X11)); X[i][j] goes to A[c0 + j][c0 + i] (the free
+// upper triangle)
+__device__ __forceinline__ void diag_group_inverse(double (*A)[kNB + 1], double* t, int c0, int nb, int lane) {
+    diag_invert_pass<1>(A, t, c0, nb, lane);
+    diag_invert_pass<2>(A, t, c0, nb, lane);
+    diag_invert_pass<4>(A, t, c0, nb, lane);
+}
+
+// one doubling pass by the CTA, B = 8, 16 or 32, with DMMA: X21 = -X22 (L21 X11)
+// of the pairs of aligned blocks of order B; T holds L21 X11.  A warp's tiles
+// run side by side.
+template <int B>
+__device__ __forceinline__ void diag_invert_pairs(double (*A)[kNB + 1], double* T, int nb, int warp, int lane) {
+    constexpr int TB = B / 8, LDT = B + 4, NT = kNB / (2 * B) * TB * TB, NW = (NT + 7) / 8;
+    const int fr = lane >> 2, fk = lane & 3;
+    double c[NW][2];
+    if (warp < NT) {
+#pragma unroll
+        for (int q = 0; q < NW; ++q) c[q][0] = c[q][1] = 0.0;
+#pragma unroll
+        for (int m0 = 0; m0 < B; m0 += 4)                  // X11[m][j] = 0 for m < j, 1 for m = j
+#pragma unroll
+            for (int q = 0; q < NW; ++q) {
+                const int t = 8 * q + warp, bs = t / (TB * TB) * 2 * B, i0 = t / TB % TB * 8, j0 = t % TB * 8;
+                const int gi = bs + B + i0 + fr, j = j0 + fr, m = m0 + fk;
+                const double xv = A[bs + j][bs + m], lv = A[gi][bs + m];
+                gemm::dmma(c[q][0], c[q][1], gi < nb ? lv : 0.0, m > j ? xv : m == j ? 1.0 : 0.0);
+            }
+#pragma unroll
+        for (int q = 0; q < NW; ++q) {
+            const int t = 8 * q + warp, bs = t / (TB * TB) * 2 * B, i0 = t / TB % TB * 8, j0 = t % TB * 8;
+            double* to = T + bs / (2 * B) * B * LDT + (i0 + fr) * LDT + j0 + 2 * fk;
+            to[0] = c[q][0];
+            to[1] = c[q][1];
+        }
+    }
+    __syncthreads();
+    if (warp < NT) {
+#pragma unroll
+        for (int q = 0; q < NW; ++q) {                     // X22[i][i] = 1
+            const int t = 8 * q + warp, bs = t / (TB * TB) * 2 * B, i0 = t / TB % TB * 8, j0 = t % TB * 8;
+            const double* to = T + bs / (2 * B) * B * LDT + (i0 + fr) * LDT + j0 + 2 * fk;
+            c[q][0] = to[0];
+            c[q][1] = to[1];
+        }
+#pragma unroll
+        for (int m0 = 0; m0 < B; m0 += 4)                  // X22[i][m] = 0 for m > i
+#pragma unroll
+            for (int q = 0; q < NW; ++q) {
+                const int t = 8 * q + warp, bs = t / (TB * TB) * 2 * B, i0 = t / TB % TB * 8, j0 = t % TB * 8;
+                const int i = i0 + fr, gb = bs + B, m = m0 + fk;
+                const double xv = A[gb + m][gb + i];
+                gemm::dmma(c[q][0], c[q][1], m < i ? xv : 0.0, T[bs / (2 * B) * B * LDT + m * LDT + j0 + fr]);
+            }
+#pragma unroll
+        for (int q = 0; q < NW; ++q) {
+            const int t = 8 * q + warp, bs = t / (TB * TB) * 2 * B, i0 = t / TB % TB * 8, j0 = t % TB * 8;
+            const int jc = bs + j0 + 2 * fk, gi = bs + B + i0 + fr;
+            A[jc][gi] = -c[q][0];
+            A[jc + 1][gi] = -c[q][1];
+        }
+    }
+    __syncthreads();
 }
 
 template <int PR>
 __global__ void __launch_bounds__(256) k_diag(const Job* jobs, PV P) {
     __shared__ double A[kNB][kNB + 1];      // L (lower, d on the diagonal), X transposed above
-    __shared__ double pan[kNB / 2 * (kNB / 2 + 4)];   // W of a group's rows below (16 .. 63); later T
-    __shared__ double colbuf[3][2 * kDG];
-    __shared__ double tinv[kDG * kDG / 4];
+    __shared__ double pan[kNB / 2 * (kNB / 2 + 4)];   // W of a group's rows below (8 .. 63); later T
+    __shared__ double tinv[kD8 * kD8 / 4];
     __shared__ double rdv[kNB];
     __shared__ double dd[kNB];
     __shared__ double adv[kNB];
@@ -869,8 +1132,8 @@ __global__ void __launch_bounds__(256) k_diag(const Job* jobs, PV P) {
     const int ld = P.buf_ld[js], fst = P.fst[js];
     double* front = P.arena + P.buf_off[js];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    // W's rows are 16 .. 63: a group's own rows are not among them
-    double(*Wp)[kDPanLd] = reinterpret_cast<double(*)[kDPanLd]>(pan) - kDG;
+    // W's rows are 8 .. 63: a group's own rows are not among them
+    double(*Wp)[kDPanLd] = reinterpret_cast<double(*)[kDPanLd]>(pan) - kD8;
     {
         double v[kNB * kNB / 256];
 #pragma unroll
@@ -885,14 +1148,15 @@ __global__ void __launch_bounds__(256) k_diag(const Job* jobs, PV P) {
     }
     __syncthreads();
     int failed = -1;
-    for (int c0 = 0; c0 < nb; c0 += kDG) {
-        const int kmax = min(kDG, nb - c0), rest = nb - c0 - kDG;         // rest: rows below the group
-        const int sets = rest > 0 ? (rest + kDG - 1) / kDG : 1;
+#pragma unroll 1
+    for (int c0 = 0; c0 < nb; c0 += kD8) {
+        const int kmax = min(kD8, nb - c0), rest = nb - c0 - kD8;         // rest: rows below the group
+        const int sets = rest > 0 ? (rest + 23) / 24 : 1;
         if (warp < sets) {
-            const int f = diag_group<PR>(P, js, k0, c0, kmax, warp, lane, nb, A, Wp, colbuf[warp], dd, rdv, adv);
+            const int f = diag_group<PR>(P, js, k0, c0, kmax, warp, sets, lane, nb, A, Wp, dd, rdv, adv);
             if (PR == kPivotChol4 && f >= 0 && lane == 0) s_fail = f;     // every warp finds the same column
         } else if (warp == 4 && c0 > 0) {
-            diag_group_inverse(A, tinv, c0 - kDG, nb, lane);
+            diag_group_inverse(A, tinv, c0 - kD8, nb, lane);
         }
         __syncthreads();
         if (PR == kPivotChol4 && s_fail < kNB) {
@@ -900,22 +1164,39 @@ __global__ void __launch_bounds__(256) k_diag(const Job* jobs, PV P) {
             break;
         }
         if (rest <= 0) continue;
-        // A[i][j] -= sum_k L[i][k] W[j][k] on the lower 8x8 tiles of what follows
-        const int nt = (rest + 7) >> 3, r0 = c0 + kDG;
-        for (int t = warp; t < nt * (nt + 1) / 2; t += 8) {
-            int ti = 0, u = t;
-            while (u > ti) u -= ++ti;
-            const int i = r0 + 8 * ti + (lane >> 2), j = r0 + 8 * u + (lane >> 2);
-            const int jc = r0 + 8 * u + 2 * (lane & 3);
-            double c[2] = {i < nb && i >= jc ? A[i][jc] : 0.0, i < nb && i > jc ? A[i][jc + 1] : 0.0};
+        // A[i][j] -= sum_k L[i][k] W[j][k] on the lower 8x8 tiles of what follows:
+        // up to 28, tiles warp, warp + 8, .. side by side
+        const int nt = (rest + 7) >> 3, ntile = nt * (nt + 1) / 2, r0 = c0 + kD8;
+        const int fr = lane >> 2, fk = lane & 3;
+        double c[4][2], fa[4][2], fb[4][2];
+        int ci[4], cj[4];
 #pragma unroll
-            for (int kk = 0; kk < kDG; kk += 4)
-                gemm::dmma(c[0], c[1], i < nb ? -A[i][c0 + kk + (lane & 3)] : 0.0, j < nb ? Wp[j][kk + (lane & 3)] : 0.0);
-            if (i < nb) {
-                if (i >= jc) A[i][jc] = c[0];
-                if (i > jc) A[i][jc + 1] = c[1];
+        for (int q = 0; q < 4; ++q) {
+            const int t = warp + 8 * q;
+            const int ti = (t >= 1) + (t >= 3) + (t >= 6) + (t >= 10) + (t >= 15) + (t >= 21) + (t >= 28);
+            const int tj = t - ti * (ti + 1) / 2;
+            const int i = r0 + 8 * ti + fr, j = r0 + 8 * tj + fr;
+            const bool on = t < ntile;
+            ci[q] = on && i < nb ? i : -1;
+            cj[q] = r0 + 8 * tj + 2 * fk;
+            const bool vj = on && j < nb;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                c[q][h] = ci[q] >= cj[q] + h ? A[ci[q]][cj[q] + h] : 0.0;
+                fa[q][h] = ci[q] >= 0 ? -A[ci[q]][c0 + 4 * h + fk] : 0.0;
+                fb[q][h] = vj ? Wp[j][4 * h + fk] : 0.0;
             }
         }
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                if (warp + 8 * q < ntile) gemm::dmma(c[q][0], c[q][1], fa[q][h], fb[q][h]);
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+                if (ci[q] >= cj[q] + h) A[ci[q]][cj[q] + h] = c[q][h];
         __syncthreads();
     }
     // the first failing pivot (sprfc1.f:1274-1279), for the rules tested here (the
@@ -934,79 +1215,58 @@ __global__ void __launch_bounds__(256) k_diag(const Job* jobs, PV P) {
         __syncthreads();
         failed = s_fail < nb ? s_fail : -1;
     }
-    // inertia and TOL(2) of the processed columns (sprfc1.f:1280-1290)
-    if (tid < 32) {
+    if (warp == 0) {
+        // inertia and TOL(2) of the processed columns (sprfc1.f:1280-1290)
         const int kend = failed < 0 ? nb : failed;
         int neg = 0, near = 0;
         double tmax = 0.0;
-        for (int k = tid; k < kend; k += 32) {
-            if (dd[k] < 0.0) ++neg;
-            if (near_zero_pivot(P, dd[k], adv[k])) ++near;
-            tmax = fmax(tmax, adv[k] / dd[k]);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int k = lane + 32 * h;
+            const double d = k < kend ? dd[k] : 1.0, ad = k < kend ? adv[k] : 0.0;
+            neg += __popc(__ballot_sync(0xffffffffu, d < 0.0));
+            near += __popc(__ballot_sync(0xffffffffu, k < kend && near_zero_pivot(P, d, ad)));
+            tmax = fmax(tmax, ad / d);
         }
-        for (int o = 16; o > 0; o >>= 1) {
-            neg += __shfl_xor_sync(0xffffffffu, neg, o);
-            near += __shfl_xor_sync(0xffffffffu, near, o);
-            tmax = fmax(tmax, __shfl_xor_sync(0xffffffffu, tmax, o));
-        }
-        if (tid == 0) {
+        for (int o = 16; o > 0; o >>= 1) tmax = fmax(tmax, __shfl_xor_sync(0xffffffffu, tmax, o));
+        if (lane == 0) {
             P.sn_neg[js] += neg;
-            atomicAdd(&P.st->numneg, (unsigned long long)neg);
+            if (neg) atomicAdd(&P.st->numneg, (unsigned long long)neg);
             if (near) atomicAdd(&P.st->near_piv, (unsigned long long)near);
             if (failed < 0) atomic_max_double(&P.st->tol2, tmax);
         }
     }
     if (failed >= 0) return;
-    // L and D back to the front (final since the last group)
-    if (warp >= 1)
-        for (int e = tid - 32; e < kNB * kNB; e += 224) {
-            const int i = e & (kNB - 1), j = e >> 6;
-            if (i >= j && i < nb) front[(int64_t)(k0 + i) + (int64_t)(k0 + j) * ld] = i == j ? dd[i] : A[i][j];
+    // the last group's inverse, the pivots, and L and D back to the front (final
+    // since the last group) by different warps
+    if (warp == 4) {
+        diag_group_inverse(A, tinv, (nb - 1) / kD8 * kD8, nb, lane);
+    } else if (warp == 5) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int e = lane + 32 * h;
+            if (e < nb) {
+                const double d = dd[e];
+                P.dvec[fst + k0 + e] = d;
+                if (P.sqd) {
+                    const double s = sqrt(fabs(d)), er = s > 0.0 ? fma(-s, s, fabs(d)) / (2.0 * s) : 0.0;
+                    P.sqd[2 * (int64_t)(fst + k0 + e)] = copysign(s, d);
+                    P.sqd[2 * (int64_t)(fst + k0 + e) + 1] = copysign(1.0, d) * er;
+                }
+            }
         }
-    if (tid < nb) {
-        const double d = dd[tid];
-        P.dvec[fst + k0 + tid] = d;
-        if (P.sqd) {
-            const double s = sqrt(fabs(d)), e = s > 0.0 ? fma(-s, s, fabs(d)) / (2.0 * s) : 0.0;
-            P.sqd[2 * (int64_t)(fst + k0 + tid)] = copysign(s, d);
-            P.sqd[2 * (int64_t)(fst + k0 + tid) + 1] = copysign(1.0, d) * e;
+    } else if (warp > 0) {
+        const int w5 = warp < 4 ? warp - 1 : warp - 3;         // five warps, a column at a time
+        double* out = front + k0 + (int64_t)k0 * ld;
+        for (int j = w5; j < nb; j += 5) {
+            if (j + lane < nb) out[j + lane + (int64_t)j * ld] = lane == 0 ? dd[j] : A[j + lane][j];
+            if (j + lane + 32 < nb) out[j + lane + 32 + (int64_t)j * ld] = A[j + lane + 32][j];
         }
     }
-    if (warp == 4) diag_group_inverse(A, tinv, (nb - 1) / kDG * kDG, nb, lane);
     __syncthreads();
-    // inverses of the aligned diagonal blocks of order 2b from those of order b
-    double* T = pan;                                          // T = L21 X11, (b x b) per pair
-    for (int b = kDG; b < kNB && b < nb; b <<= 1) {
-        const int tb = b >> 3, ldt = b + 4, npair = kNB / (2 * b);
-        for (int t = warp; t < npair * tb * tb; t += 8) {
-            const int bs = t / (tb * tb) * 2 * b, i0 = t / tb % tb * 8, j0 = t % tb * 8;
-            const int gi = bs + b + i0 + (lane >> 2), j = j0 + (lane >> 2);
-            double c[2] = {0.0, 0.0};
-            for (int m0 = j0; m0 < b; m0 += 4) {               // X11[m][j] = 0 for m < j
-                const int m = m0 + (lane & 3);
-                const double x = m > j ? A[bs + j][bs + m] : m == j ? 1.0 : 0.0;
-                gemm::dmma(c[0], c[1], gi < nb ? A[gi][bs + m] : 0.0, x);
-            }
-            double* to = T + (bs / (2 * b)) * b * ldt + (i0 + (lane >> 2)) * ldt + j0 + 2 * (lane & 3);
-            to[0] = c[0];
-            to[1] = c[1];
-        }
-        __syncthreads();
-        for (int t = warp; t < npair * tb * tb; t += 8) {
-            const int bs = t / (tb * tb) * 2 * b, i0 = t / tb % tb * 8, j0 = t % tb * 8;
-            const int i = i0 + (lane >> 2), gb = bs + b;
-            const double* tp = T + (bs / (2 * b)) * b * ldt;
-            double c[2] = {tp[i * ldt + j0 + 2 * (lane & 3)], tp[i * ldt + j0 + 2 * (lane & 3) + 1]};   // X22[i][i] = 1
-            for (int m0 = 0; m0 < i0 + 8; m0 += 4) {           // X22[i][m] = 0 for m > i
-                const int m = m0 + (lane & 3);
-                gemm::dmma(c[0], c[1], m < i ? A[gb + m][gb + i] : 0.0, tp[m * ldt + j0 + (lane >> 2)]);
-            }
-            const int jc = bs + j0 + 2 * (lane & 3);
-            A[jc][gb + i] = -c[0];
-            A[jc + 1][gb + i] = -c[1];
-        }
-        __syncthreads();
-    }
+    if (nb > kD8) diag_invert_pairs<kD8>(A, pan, nb, warp, lane);
+    if (nb > 2 * kD8) diag_invert_pairs<2 * kD8>(A, pan, nb, warp, lane);
+    if (nb > 4 * kD8) diag_invert_pairs<4 * kD8>(A, pan, nb, warp, lane);
     double* lv = P.linv + P.linv_off[js] + (int64_t)(k0 / kNB) * kNB * kNB;
     for (int e = tid; e < kNB * kNB; e += blockDim.x) {
         const int i = e % kNB, j = e / kNB;
