@@ -3405,7 +3405,6 @@ void Engine::enqueue_factor(const PV& pv, cudaStream_t s, std::vector<cudaEvent_
                 if (trail_i8) {
                     launch_i8_gemm(lp.trail_i8[st].far, u, pv, gev, true);
                     for (const Launch& fl : lp.trail_i8[st].far_rest) launch_gemm(fl, u, pv, gev);
-                    for (const Launch& fl : lp.trail_i8[st].far_rest) launch_gemm(fl, u, pv, gev);
                 } else if (far_tc) {
                     for (const TcLaunch& t : lp.far_tc[st]) launch_tc(t, u, pv, gev, true);
                     timing.tc_flops += lp.far_flops[st];

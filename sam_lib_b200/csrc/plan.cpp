@@ -411,7 +411,6 @@ int build_plan(const int64_t* mspar, const int64_t* mtrees, const int64_t* msifa
                         j.aux_job = b.aux_job;
                         j.aux = b.aux + (f.c0 - b.c0);
                         out.flops += update_flops(j.c0, j.c_end, j.r_end, j.k_hi - j.k_lo);
-                        out.flops += update_flops(j.c0, j.c_end, j.r_end, j.k_hi - j.k_lo);
                         add_job(out.far, j, tiles(j));
                     }
             close_launch(out.far);

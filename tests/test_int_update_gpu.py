@@ -18,6 +18,7 @@ import numpy as np
 import pytest
 
 from dense_structure import dense_chain, pack_dense
+from test_pivot_blocks_gpu import forest
 
 pytestmark = pytest.mark.gpu
 
@@ -93,6 +94,47 @@ def test_levels_with_large_and_small_fronts():
     rg, fg = _factor(ds, sm, math.inf)
     assert r['lierr'] == rg['lierr'] == 0 and launches > ds.info()['launches']
     assert np.abs(f - fg).max() <= 1e-10 * np.abs(fg).max()
+    ds.close()
+
+
+def test_far_columns_of_a_small_front_beside_a_large_one():
+    """Two fronts of one level in the same panel steps, both with columns beyond
+    the next super-panel: after 512 columns one has 1238 rows left (digit
+    form), the other 618 (FP64 kernel)."""
+    import sam_lib_b200 as spr
+    widths, root = [1700, 1080], 50
+    own = np.cumsum([0] + widths)
+    neq = sum(widths) + root
+    structure = forest(widths, root)
+    rows, xlnz = structure[3], structure[5]
+    structure = structure[:3]
+    a, s, nneg = _matrix(neq, 7, True)
+    a[own[0]:own[1], own[1]:own[2]] = a[own[1]:own[2], own[0]:own[1]] = 0.0
+    starts = np.concatenate([own, [neq]])
+    sm = np.zeros(neq + int(structure[0][15]))
+
+    def columns():
+        for j, r in enumerate(rows):
+            p = neq + int(xlnz[j]) - 1
+            for c in range(starts[j], starts[j + 1]):
+                i = r[r > c] - 1
+                yield c, i, slice(p, p + len(i))
+                p += len(i)
+    for c, i, at in columns():
+        sm[at] = a[i, c]
+    ds = spr.DeviceSolver(*structure)
+    r, f = _factor(ds, sm, 0.0)
+    launches = ds.info()['launches']
+    rg, _ = _factor(ds, sm, math.inf)
+    assert r['lierr'] == rg['lierr'] == 0 and r['numneg'] == rg['numneg'] == nneg
+    assert launches > ds.info()['launches']
+    low = np.zeros((neq, neq))
+    for c, i, at in columns():
+        low[i, c] = f[at]
+    d = low.diagonal().copy()
+    np.fill_diagonal(low, 1.0)
+    err = np.abs(a - (low * d) @ low.T) / (s[:, None] * s[None, :])
+    assert err.max() <= 8 * neq * 2.0 ** -53
     ds.close()
 
 

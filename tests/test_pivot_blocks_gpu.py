@@ -15,15 +15,16 @@ from dense_structure import dense_chain, pack_dense
 pytestmark = pytest.mark.gpu
 
 
-def _star(leaves, width, root):
-    """`leaves` supernodes of `width` columns over one root of `root` columns."""
-    mspar, _, _ = dense_chain([width] * leaves + [root])
-    m, neq = leaves + 1, leaves * width + root
-    xsuper = np.concatenate([1 + width * np.arange(leaves + 1), [neq + 1]])
+def forest(widths, root):
+    """Leaf supernodes of the given widths, each dense, over one root of `root` columns."""
+    mspar, _, _ = dense_chain(list(widths) + [root])
+    leaves, neq = len(widths), sum(widths) + root
+    m = leaves + 1
+    xsuper = np.cumsum([1] + list(widths) + [root])
     xsibl = np.concatenate([np.ones(m), [m]])
     sibl = np.concatenate([np.arange(1, m), [1, 1]])[:m + 1]
-    rows = [np.concatenate([np.arange(xsuper[j], xsuper[j] + width), np.arange(xsuper[leaves], neq + 1)])
-            for j in range(leaves)] + [np.arange(xsuper[leaves], neq + 1)]
+    top = np.arange(xsuper[leaves], neq + 1)
+    rows = [np.concatenate([np.arange(xsuper[j], xsuper[j + 1]), top]) for j in range(leaves)] + [top]
     f, s = np.array([len(r) for r in rows]), np.diff(xsuper)
     xlindx = np.concatenate([[1], 1 + np.cumsum(f)])
     xlnz = np.concatenate([[1], 1 + np.cumsum(f * s - s * (s - 1) // 2)])
@@ -92,7 +93,7 @@ def test_orders_at_the_edges_of_the_groups(widths):
 @pytest.mark.parametrize('leaves,width,root', [(2, 1, 1), (3, 17, 20), (31, 2, 9), (32, 2, 40), (33, 3, 50), (70, 1, 159),
                                                (65, 2, 65)])
 def test_many_children(leaves, width, root):
-    mspar, mtrees, msifa, rows, xsuper, xlnz = _star(leaves, width, root)
+    mspar, mtrees, msifa, rows, xsuper, xlnz = forest([width] * leaves, root)
     neq = leaves * width + root
     a = _dense(neq, neq)
     own = np.arange(neq) // width
