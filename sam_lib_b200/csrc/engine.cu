@@ -193,7 +193,7 @@ struct Engine::Dev {
     alignas(64) CUtensorMap i8_map_a, i8_map_b;
     double* sqd = nullptr;                       // (sqrt|d| with d's sign, its rounding error) per equation
     cudaStream_t side = nullptr;                 // side stream: trailing updates beyond the next super-panel
-    cudaStream_t ahead = nullptr;                // look-ahead stream: in-super-panel columns after the next panel
+    cudaStream_t ahead = nullptr;                // look-ahead stream: in-super-panel columns after the next two panels
     cudaStream_t wbs = nullptr;                  // early writes of final super-panels to LNZ (streamed copies)
     std::vector<cudaEvent_t> evpool;             // fork/join events of one factorisation
 };
@@ -556,11 +556,13 @@ __device__ __forceinline__ int small_group(const PV& P, int js, double* A, doubl
     double dmine = 1.0, rmine = 1.0;                   // lane k keeps pivot k
     double* ap = A + pk(0, c0, F);                     // the current column, row 0
     const int own_row = w == 0 && own ? c0 + lane : -1;
+    double d_next = __shfl_sync(0xffffffffu, a[0], 0);
     auto step = [&](int k, auto width) -> bool {
         constexpr int W = decltype(width)::value;
         double* cbk = cb + (k & 1) * 32;
         const double a0 = a[0], x0 = x[0];
-        double d = __shfl_sync(0xffffffffu, a0, k);
+        double d = d_next;
+        const double ann = __shfl_sync(0xffffffffu, a[1], (k + 1) & 31);     // the next pivot before this step
         if (PR == kPivotReplace || PR == kPivotChol4) {
             const double ad = __shfl_sync(0xffffffffu, adr, k);
             const int col = c0 + k;
@@ -589,6 +591,7 @@ __device__ __forceinline__ int small_group(const PV& P, int js, double* A, doubl
         __syncwarp();
         double c[kDG];
         read_column<W>(cbk, c);
+        d_next = fma(-c[0], c[0] * r, ann);                      // as lane k + 1 does below, without its shuffle
 #pragma unroll
         for (int j = 0; j < W; ++j) {
             const double l = c[j] * r;
@@ -944,12 +947,15 @@ __global__ void __launch_bounds__(256) k_assemble(const Job* jobs, int64_t njobs
 // round by shuffles, the column's ahead of the reciprocal.  The columns after the
 // group are updated with DMMA tiles (K = 8), up to four at a time per warp: a
 // DMMA takes some 130 clocks to its result, a multiply-add of one warp 8.
-// The inverse of each group's 8x8 triangle is formed beside the next group's
-// elimination, the wider ones by doubling (X21 = -X22 (L21 X11)) with DMMA.
+// The next pivot comes from the values before the step, in every lane, so that
+// no shuffle is on the pivots' chain.
+// The inverse goes by doubling (X21 = -X22 (L21 X11)) with DMMA; the idle warps
+// form what is final of it, and write finished columns of L, beside the next
+// groups' eliminations: after the last group 3 us are left of 5.
 // Every entry takes its multiply-adds in ascending k (DMMA chains them in that
-// order), so the factors do not depend on the grouping.  20 us a full block
-// alone; all blocks of a 32^3 box 9.8 ms (groups of 16 with the column through
-// shared memory 10.5 ms, one barrier a column 15.0 ms).
+// order), so the factors do not depend on the grouping.  All blocks of a 32^3
+// box by themselves: one barrier a column 15.0 ms, groups of 16 with the column
+// through shared memory 10.5 ms, this 8.
 constexpr int kD8 = 8;                               // columns of a group
 constexpr int kDPanLd = kD8 + 1;
 
@@ -975,15 +981,17 @@ __device__ __forceinline__ int diag_group(const PV& P, int js, int k0, int c0, i
     const int k_row = !keep ? -1 : own ? lane : kD8;   // columns k < k_row of this lane's row are L
     int k = 0;
     bool go = true;
+    double d_next = __shfl_sync(0xffffffffu, a[0], 0);
     // the registers move down by one each step (a[0] is always the current
     // column): one copy of the step in the instruction stream
 #pragma unroll 1
     for (; k < kmax && go; ++k) {
         const double a0 = a[0];
-        double d = __shfl_sync(0xffffffffu, a0, k);
+        double d = d_next;
         double c[kD8 - 1];                             // the column below the pivot
 #pragma unroll
         for (int j = 0; j < kD8 - 1; ++j) c[j] = __shfl_sync(0xffffffffu, a0, k + 1 + j);
+        const double ann = __shfl_sync(0xffffffffu, a[1], k + 1);      // the next pivot before this step
         if (PR == kPivotReplace) {
             const double d0 = d;
             d = fc3_pivot(P, d0, adv[c0 + k]);
@@ -1004,6 +1012,7 @@ __device__ __forceinline__ int diag_group(const PV& P, int js, int k0, int c0, i
         }
         const double rd = recip_nr_uniform(d);
         const double l = a0 * rd;
+        d_next = fma(-(c[0] * rd), c[0], ann);         // as lane k + 1 does below, without its shuffle
 #pragma unroll
         for (int j = 0; j < kD8 - 1; ++j) a[j] = fma(-l, c[j], a[j + 1]);
         dmine = lane == k ? d : dmine;
@@ -1059,108 +1068,169 @@ __device__ __forceinline__ void diag_group_inverse(double (*A)[kNB + 1], double*
     diag_invert_pass<4>(A, t, c0, nb, lane);
 }
 
-// one doubling pass by the CTA, B = 8, 16 or 32, with DMMA: X21 = -X22 (L21 X11)
-// of the pairs of aligned blocks of order B; T holds L21 X11.  A warp's tiles
-// run side by side.
-template <int B>
-__device__ __forceinline__ void diag_invert_pairs(double (*A)[kNB + 1], double* T, int nb, int warp, int lane) {
-    constexpr int TB = B / 8, LDT = B + 4, NT = kNB / (2 * B) * TB * TB, NW = (NT + 7) / 8;
+// A doubling step of the inverse with DMMA, X21 = -X22 (L21 X11) for the pair of
+// blocks of order B at bs, in its two products: T = L21 X11, then X21.  A warp
+// takes the 8 x 8 tiles w, w + NW, .., up to NQ of them side by side.
+template <int B, int NW, int NQ>
+__device__ __forceinline__ void diag_pair_t(double (*A)[kNB + 1], double* T, int bs, int nb, int w, int lane) {
+    constexpr int TB = B / 8, LDT = B + 4;
+    static_assert(NW * NQ == TB * TB, "every tile once");
     const int fr = lane >> 2, fk = lane & 3;
-    double c[NW][2];
-    if (warp < NT) {
+    double c[NQ][2];
 #pragma unroll
-        for (int q = 0; q < NW; ++q) c[q][0] = c[q][1] = 0.0;
+    for (int q = 0; q < NQ; ++q) c[q][0] = c[q][1] = 0.0;
 #pragma unroll
-        for (int m0 = 0; m0 < B; m0 += 4)                  // X11[m][j] = 0 for m < j, 1 for m = j
+    for (int m0 = 0; m0 < B; m0 += 4)                      // X11[m][j] = 0 for m < j, 1 for m = j
 #pragma unroll
-            for (int q = 0; q < NW; ++q) {
-                const int t = 8 * q + warp, bs = t / (TB * TB) * 2 * B, i0 = t / TB % TB * 8, j0 = t % TB * 8;
-                const int gi = bs + B + i0 + fr, j = j0 + fr, m = m0 + fk;
-                const double xv = A[bs + j][bs + m], lv = A[gi][bs + m];
-                gemm::dmma(c[q][0], c[q][1], gi < nb ? lv : 0.0, m > j ? xv : m == j ? 1.0 : 0.0);
-            }
-#pragma unroll
-        for (int q = 0; q < NW; ++q) {
-            const int t = 8 * q + warp, bs = t / (TB * TB) * 2 * B, i0 = t / TB % TB * 8, j0 = t % TB * 8;
-            double* to = T + bs / (2 * B) * B * LDT + (i0 + fr) * LDT + j0 + 2 * fk;
-            to[0] = c[q][0];
-            to[1] = c[q][1];
+        for (int q = 0; q < NQ; ++q) {
+            const int t = w + NW * q, i0 = t / TB * 8, j0 = t % TB * 8;
+            const int gi = bs + B + i0 + fr, j = j0 + fr, m = m0 + fk;
+            const double xv = A[bs + j][bs + m], lv = A[gi][bs + m];
+            gemm::dmma(c[q][0], c[q][1], gi < nb ? lv : 0.0, m > j ? xv : m == j ? 1.0 : 0.0);
         }
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+        const int t = w + NW * q, i0 = t / TB * 8, j0 = t % TB * 8;
+        double* to = T + (i0 + fr) * LDT + j0 + 2 * fk;
+        to[0] = c[q][0];
+        to[1] = c[q][1];
     }
-    __syncthreads();
-    if (warp < NT) {
-#pragma unroll
-        for (int q = 0; q < NW; ++q) {                     // X22[i][i] = 1
-            const int t = 8 * q + warp, bs = t / (TB * TB) * 2 * B, i0 = t / TB % TB * 8, j0 = t % TB * 8;
-            const double* to = T + bs / (2 * B) * B * LDT + (i0 + fr) * LDT + j0 + 2 * fk;
-            c[q][0] = to[0];
-            c[q][1] = to[1];
-        }
-#pragma unroll
-        for (int m0 = 0; m0 < B; m0 += 4)                  // X22[i][m] = 0 for m > i
-#pragma unroll
-            for (int q = 0; q < NW; ++q) {
-                const int t = 8 * q + warp, bs = t / (TB * TB) * 2 * B, i0 = t / TB % TB * 8, j0 = t % TB * 8;
-                const int i = i0 + fr, gb = bs + B, m = m0 + fk;
-                const double xv = A[gb + m][gb + i];
-                gemm::dmma(c[q][0], c[q][1], m < i ? xv : 0.0, T[bs / (2 * B) * B * LDT + m * LDT + j0 + fr]);
-            }
-#pragma unroll
-        for (int q = 0; q < NW; ++q) {
-            const int t = 8 * q + warp, bs = t / (TB * TB) * 2 * B, i0 = t / TB % TB * 8, j0 = t % TB * 8;
-            const int jc = bs + j0 + 2 * fk, gi = bs + B + i0 + fr;
-            A[jc][gi] = -c[q][0];
-            A[jc + 1][gi] = -c[q][1];
-        }
-    }
-    __syncthreads();
 }
 
-template <int PR>
-__global__ void __launch_bounds__(256) k_diag(const Job* jobs, PV P) {
-    __shared__ double A[kNB][kNB + 1];      // L (lower, d on the diagonal), X transposed above
-    __shared__ double pan[kNB / 2 * (kNB / 2 + 4)];   // W of a group's rows below (8 .. 63); later T
-    __shared__ double tinv[kD8 * kD8 / 4];
-    __shared__ double rdv[kNB];
-    __shared__ double dd[kNB];
-    __shared__ double adv[kNB];
-    __shared__ int s_fail;
-    if (P.st->any_fail) return;
-    const Job& jb = jobs[blockIdx.x];
-    const int js = jb.node, k0 = jb.k_lo, nb = jb.k_hi - jb.k_lo;
-    if (P.sn_bad[js] || node_off(P, js)) return;
-    const int ld = P.buf_ld[js], fst = P.fst[js];
-    double* front = P.arena + P.buf_off[js];
+template <int B, int NW, int NQ>
+__device__ __forceinline__ void diag_pair_x(double (*A)[kNB + 1], const double* T, int bs, int w, int lane) {
+    constexpr int TB = B / 8, LDT = B + 4;
+    const int fr = lane >> 2, fk = lane & 3;
+    double c[NQ][2];
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {                         // X22[i][i] = 1
+        const int t = w + NW * q, i0 = t / TB * 8, j0 = t % TB * 8;
+        const double* to = T + (i0 + fr) * LDT + j0 + 2 * fk;
+        c[q][0] = to[0];
+        c[q][1] = to[1];
+    }
+#pragma unroll
+    for (int m0 = 0; m0 < B; m0 += 4)                      // X22[i][m] = 0 for m > i
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+            const int t = w + NW * q, i0 = t / TB * 8, j0 = t % TB * 8;
+            const int i = i0 + fr, gb = bs + B, m = m0 + fk;
+            const double xv = A[gb + m][gb + i];
+            gemm::dmma(c[q][0], c[q][1], m < i ? xv : 0.0, T[m * LDT + j0 + fr]);
+        }
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+        const int t = w + NW * q, i0 = t / TB * 8, j0 = t % TB * 8;
+        const int jc = bs + j0 + 2 * fk, gi = bs + B + i0 + fr;
+        A[jc][gi] = -c[q][0];
+        A[jc + 1][gi] = -c[q][1];
+    }
+}
+
+// both products by one warp
+template <int B>
+__device__ __forceinline__ void diag_pair(double (*A)[kNB + 1], double* T, int bs, int nb, int lane) {
+    diag_pair_t<B, 1, B * B / 64>(A, T, bs, nb, 0, lane);
+    __syncwarp();
+    diag_pair_x<B, 1, B * B / 64>(A, T, bs, 0, lane);
+    __syncwarp();
+}
+
+// what a diagonal block's elimination keeps in shared memory beside A and pan
+struct DiagShared {
+    double w[(kNB - kD8) * kDPanLd];        // W of a group's rows below
+    double t8[2][8 * 12], t16[16 * 20], t32[32 * 36], tinv[kD8 * kD8 / 4];
+    double rdv[kNB], dd[kNB], adv[kNB];
+    int fail;
+};
+
+// columns c0 .. c0 + n - 1 of L and D to the front, by nw warps; block: where the block starts
+__device__ __forceinline__ void diag_store(double* block, int ld, int c0, int n, int nb, double (*A)[kNB + 1],
+                                           const double* dd, int w, int nw, int lane) {
+    for (int j = c0 + w; j < c0 + n; j += nw) {
+        if (j + lane < nb) block[j + lane + (int64_t)j * ld] = lane == 0 ? dd[j] : A[j + lane][j];
+        if (j + lane + 32 < nb) block[j + lane + 32 + (int64_t)j * ld] = A[j + lane + 32][j];
+    }
+}
+
+// 32 x 32 of the inverse to lv at (i0, j0), by nw warps
+__device__ __forceinline__ void diag_store_x(double* lv, int i0, int j0, int nb, double (*A)[kNB + 1], int w, int nw,
+                                             int lane) {
+    const int i = i0 + lane;
+#pragma unroll 8
+    for (int j = j0 + w; j < j0 + 32; j += nw)
+        lv[i + j * kNB] = (i < nb && j < nb) ? (i > j ? A[j][i] : (i == j ? 1.0 : 0.0)) : 0.0;
+}
+
+// The rows [k0 + 64, next_end) of panel k0 transposed into the front's free upper
+// triangle, for k_chain; by 96 threads
+__device__ __forceinline__ void diag_copy_next(double* front, int ld, int k0, int nb, int next_end, int t) {
+    const int n = next_end - (k0 + kNB);
+    const double* from = front + k0 + kNB + (int64_t)k0 * ld;
+    double* to = front + k0 + (int64_t)(k0 + kNB) * ld;
+    for (int e0 = t; e0 < kNB * kNB && n > 0; e0 += 8 * 96) {
+        double v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const int e = e0 + 96 * u, j = e & (kNB - 1), m = e >> 6;
+            v[u] = j < n && m < nb ? __ldcg(from + j + (int64_t)m * ld) : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const int e = e0 + 96 * u, j = e & (kNB - 1), m = e >> 6;
+            if (j < n && m < nb) to[m + (int64_t)j * ld] = v[u];
+        }
+    }
+}
+
+// The block in A (lower, zero elsewhere), its a_jj in S.adv, S.fail = kNB; all
+// synchronised.  next_end: with Copy, the end of the next panel's rows.
+template <int PR, bool Copy>
+__device__ __forceinline__ void diag_block(const PV& P, int js, int k0, int nb, double* front, int ld, int next_end,
+                                           double (*A)[kNB + 1], DiagShared& S) {
+    const int fst = P.fst[js];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     // W's rows are 8 .. 63: a group's own rows are not among them
-    double(*Wp)[kDPanLd] = reinterpret_cast<double(*)[kDPanLd]>(pan) - kD8;
-    {
-        double v[kNB * kNB / 256];
-#pragma unroll
-        for (int q = 0; q < kNB * kNB / 256; ++q) {
-            const int i = tid & (kNB - 1), j = (tid >> 6) + 4 * q;
-            v[q] = (i >= j && i < nb) ? __ldcg(front + (int64_t)(k0 + i) + (int64_t)(k0 + j) * ld) : 0.0;
-        }
-        if (tid < nb) adv[tid] = __ldcg(P.adiag + fst + k0 + tid);
-        if (tid == 0) s_fail = kNB;
-#pragma unroll
-        for (int q = 0; q < kNB * kNB / 256; ++q) A[tid & (kNB - 1)][(tid >> 6) + 4 * q] = v[q];
-    }
-    __syncthreads();
+    double(*Wp)[kDPanLd] = reinterpret_cast<double(*)[kDPanLd]>(S.w) - kD8;
+    double* block = front + k0 + (int64_t)k0 * ld;
+    double* lv = P.linv + P.linv_off[js] + (int64_t)(k0 / kNB) * kNB * kNB;
+    const bool full = nb == kNB;
     int failed = -1;
 #pragma unroll 1
     for (int c0 = 0; c0 < nb; c0 += kD8) {
         const int kmax = min(kD8, nb - c0), rest = nb - c0 - kD8;         // rest: rows below the group
         const int sets = rest > 0 ? (rest + 23) / 24 : 1;
         if (warp < sets) {
-            const int f = diag_group<PR>(P, js, k0, c0, kmax, warp, sets, lane, nb, A, Wp, dd, rdv, adv);
-            if (PR == kPivotChol4 && f >= 0 && lane == 0) s_fail = f;     // every warp finds the same column
-        } else if (warp == 4 && c0 > 0) {
-            diag_group_inverse(A, tinv, c0 - kD8, nb, lane);
+            const int f = diag_group<PR>(P, js, k0, c0, kmax, warp, sets, lane, nb, A, Wp, S.dd, S.rdv, S.adv);
+            if (PR == kPivotChol4 && f >= 0 && lane == 0) S.fail = f;     // every warp finds the same column
+        } else if (c0 > 0) {
+            // beside the group, what is final of the ones before: their inverses (of a
+            // full block as far as they go, as the schedule below), L to the front
+            const int g = c0 / kD8;
+            if (warp == 4) {
+                diag_group_inverse(A, S.tinv, c0 - kD8, nb, lane);
+                if (full && g == 7) diag_pair_t<8, 1, 1>(A, S.t8[0], 48, nb, 0, lane);
+            } else if (warp == 5) {
+                if (full && g == 3) diag_pair<8>(A, S.t8[1], 0, nb, lane);
+                if (full && g == 5) diag_pair<8>(A, S.t8[1], 16, nb, lane);
+                if (full && g == 6) diag_pair<16>(A, S.t16, 0, nb, lane);
+                if (full && g == 7) {
+                    diag_pair<8>(A, S.t8[1], 32, nb, lane);
+                    diag_pair_t<16, 1, 4>(A, S.t16, 32, nb, 0, lane);
+                }
+            } else if (warp >= 6) {
+                diag_store(block, ld, c0 - kD8, kD8, nb, A, S.dd, warp - 6, 2, lane);
+            } else if (full && g == 7) {
+                if (warp == 3) diag_store_x(lv, 0, 0, nb, A, 0, 1, lane);
+            } else if (full && g == 4 && warp == 3) {
+                for (int j = 32; j < kNB; ++j) lv[lane + j * kNB] = 0.0;
+            }
+            if (full && g == 7 && (warp & 2)) diag_pair_t<32, 4, 4>(A, S.t32, 0, nb, (warp >> 2) * 2 + (warp & 1), lane);
         }
+        if (Copy && c0 == 0 && warp >= 5) diag_copy_next(front, ld, k0, nb, next_end, tid - 160);
         __syncthreads();
-        if (PR == kPivotChol4 && s_fail < kNB) {
-            failed = s_fail;
+        if (PR == kPivotChol4 && S.fail < kNB) {
+            failed = S.fail;
             break;
         }
         if (rest <= 0) continue;
@@ -1205,15 +1275,15 @@ __global__ void __launch_bounds__(256) k_diag(const Job* jobs, PV P) {
         if (tid < 32) {
             int f = nb;
             for (int k = tid; k < nb; k += 32)
-                if (pivot_fails(PR, dd[k], adv[k], P.tol1)) f = min(f, k);
+                if (pivot_fails(PR, S.dd[k], S.adv[k], P.tol1)) f = min(f, k);
             for (int o = 16; o > 0; o >>= 1) f = min(f, __shfl_xor_sync(0xffffffffu, f, o));
             if (tid == 0) {
-                if (f < nb) record_fail(P, js, k0 + f, dd[f], adv[f]);
-                s_fail = f;
+                if (f < nb) record_fail(P, js, k0 + f, S.dd[f], S.adv[f]);
+                S.fail = f;
             }
         }
         __syncthreads();
-        failed = s_fail < nb ? s_fail : -1;
+        failed = S.fail < nb ? S.fail : -1;
     }
     if (warp == 0) {
         // inertia and TOL(2) of the processed columns (sprfc1.f:1280-1290)
@@ -1223,7 +1293,7 @@ __global__ void __launch_bounds__(256) k_diag(const Job* jobs, PV P) {
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const int k = lane + 32 * h;
-            const double d = k < kend ? dd[k] : 1.0, ad = k < kend ? adv[k] : 0.0;
+            const double d = k < kend ? S.dd[k] : 1.0, ad = k < kend ? S.adv[k] : 0.0;
             neg += __popc(__ballot_sync(0xffffffffu, d < 0.0));
             near += __popc(__ballot_sync(0xffffffffu, k < kend && near_zero_pivot(P, d, ad)));
             tmax = fmax(tmax, ad / d);
@@ -1237,16 +1307,25 @@ __global__ void __launch_bounds__(256) k_diag(const Job* jobs, PV P) {
         }
     }
     if (failed >= 0) return;
-    // the last group's inverse, the pivots, and L and D back to the front (final
-    // since the last group) by different warps
+    // the last group's inverse and the pairs that wait for it, the pivots, and the
+    // last group of L and D, by different warps
+    const int cl = (nb - 1) / kD8 * kD8;
     if (warp == 4) {
-        diag_group_inverse(A, tinv, (nb - 1) / kD8 * kD8, nb, lane);
+        diag_group_inverse(A, S.tinv, cl, nb, lane);
+        if (full) {
+            diag_pair_x<8, 1, 1>(A, S.t8[0], 48, 0, lane);
+            __syncwarp();
+            diag_pair_x<16, 1, 4>(A, S.t16, 32, 0, lane);
+        } else {
+            for (int bs = 0; bs + 8 < nb; bs += 16) diag_pair<8>(A, S.t8[0], bs, nb, lane);
+            for (int bs = 0; bs + 16 < nb; bs += 32) diag_pair<16>(A, S.t16, bs, nb, lane);
+        }
     } else if (warp == 5) {
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const int e = lane + 32 * h;
             if (e < nb) {
-                const double d = dd[e];
+                const double d = S.dd[e];
                 P.dvec[fst + k0 + e] = d;
                 if (P.sqd) {
                     const double s = sqrt(fabs(d)), er = s > 0.0 ? fma(-s, s, fabs(d)) / (2.0 * s) : 0.0;
@@ -1255,23 +1334,57 @@ __global__ void __launch_bounds__(256) k_diag(const Job* jobs, PV P) {
                 }
             }
         }
-    } else if (warp > 0) {
-        const int w5 = warp < 4 ? warp - 1 : warp - 3;         // five warps, a column at a time
-        double* out = front + k0 + (int64_t)k0 * ld;
-        for (int j = w5; j < nb; j += 5) {
-            if (j + lane < nb) out[j + lane + (int64_t)j * ld] = lane == 0 ? dd[j] : A[j + lane][j];
-            if (j + lane + 32 < nb) out[j + lane + 32 + (int64_t)j * ld] = A[j + lane + 32][j];
-        }
+    } else if (warp >= 6) {
+        diag_store(block, ld, cl, nb - cl, nb, A, S.dd, warp - 6, 2, lane);
     }
     __syncthreads();
-    if (nb > kD8) diag_invert_pairs<kD8>(A, pan, nb, warp, lane);
-    if (nb > 2 * kD8) diag_invert_pairs<2 * kD8>(A, pan, nb, warp, lane);
-    if (nb > 4 * kD8) diag_invert_pairs<4 * kD8>(A, pan, nb, warp, lane);
-    double* lv = P.linv + P.linv_off[js] + (int64_t)(k0 / kNB) * kNB * kNB;
-    for (int e = tid; e < kNB * kNB; e += blockDim.x) {
-        const int i = e % kNB, j = e / kNB;
-        lv[e] = (i < nb && j < nb) ? (i > j ? A[j][i] : (i == j ? 1.0 : 0.0)) : 0.0;
+    if (nb > 32) {
+        if (!full) {
+            diag_pair_t<32, 8, 2>(A, S.t32, 0, nb, warp, lane);
+            __syncthreads();
+        }
+        diag_pair_x<32, 8, 2>(A, S.t32, 0, warp, lane);
+        __syncthreads();
     }
+    if (!full) {
+        diag_store_x(lv, 0, 0, nb, A, warp, 8, lane);
+        diag_store_x(lv, 0, 32, nb, A, warp, 8, lane);
+    }
+    diag_store_x(lv, 32, 0, nb, A, warp, 8, lane);
+    diag_store_x(lv, 32, 32, nb, A, warp, 8, lane);
+}
+
+constexpr size_t kDiagSmem = sizeof(double) * kNB * (kNB + 1) + sizeof(DiagShared);
+
+// next: with it, k_chain follows, and takes the next panel's rows of this one
+// from the upper triangle
+template <int PR>
+__global__ void __launch_bounds__(256) k_diag(const Job* jobs, PV P, int next) {
+    extern __shared__ __align__(16) double dsh[];
+    double(*A)[kNB + 1] = reinterpret_cast<double(*)[kNB + 1]>(dsh);    // L (lower, d on the diagonal), X transposed above
+    DiagShared& S = *reinterpret_cast<DiagShared*>(dsh + kNB * (kNB + 1));
+    if (P.st->any_fail) return;
+    const Job& jb = jobs[blockIdx.x];
+    const int js = jb.node, k0 = jb.k_lo, nb = jb.k_hi - jb.k_lo;
+    if (P.sn_bad[js] || node_off(P, js)) return;
+    const int ld = P.buf_ld[js], fst = P.fst[js];
+    double* front = P.arena + P.buf_off[js];
+    const int tid = threadIdx.x;
+    {
+        double v[kNB * kNB / 256];
+#pragma unroll
+        for (int q = 0; q < kNB * kNB / 256; ++q) {
+            const int i = tid & (kNB - 1), j = (tid >> 6) + 4 * q;
+            v[q] = (i >= j && i < nb) ? __ldcg(front + (int64_t)(k0 + i) + (int64_t)(k0 + j) * ld) : 0.0;
+        }
+        if (tid < nb) S.adv[tid] = __ldcg(P.adiag + fst + k0 + tid);
+        if (tid == 0) S.fail = kNB;
+#pragma unroll
+        for (int q = 0; q < kNB * kNB / 256; ++q) A[tid & (kNB - 1)][(tid >> 6) + 4 * q] = v[q];
+    }
+    __syncthreads();
+    const int next_end = next ? min(k0 + 2 * kNB, P.S[js]) : 0;
+    diag_block<PR, true>(P, js, k0, nb, front, ld, next_end, A, S);
 }
 
 // Panel TRSM as a product with the stored inverse: for a 64-row block of the
@@ -1349,6 +1462,290 @@ __global__ void __launch_bounds__(128) k_trsm(const Job* jobs, int64_t njobs, co
     }
 }
 
+// A step of the panel chain inside a super-panel, panel p = [k0, k0 + 64) whose
+// diagonal block is done: the panel's TRSM, the update of the next panel's
+// columns by panels p - 1 and p (the columns after them get panel p beside the
+// next step, k_gemm), and the next diagonal block.  Separate launches of the
+// three before put two launches and two reads of the next panel on the chain, which
+// bounds fronts of a few thousand rows.
+// A CTA has 64 rows (the first CTA the next diagonal block's), and each
+// forms the next panel's rows of L itself, from the copy of them that the step
+// before left in the front's upper triangle (in place they are being replaced by
+// the first CTA): one product of 64 x 64 x 64 more instead of a grid-wide wait.
+// Products of 64 columns at a time and in the separate kernels' order: the same
+// bits.  Fronts that end with panel p only take the TRSM.  The diagonal block's CTA
+// takes its products' lower tiles and X's lower triangle alone; the block's own
+// elimination is two thirds of its time.  Separate launches before: 20^3 factor 10.6
+// -> 9.7 ms, 32^3 33.6 -> 30.8 ms, 48^3 250 -> 245 ms.
+constexpr size_t kChainSmem = sizeof(double) * (3 * (size_t)kNB * kTrsmLds + 4 * kNB);
+static_assert(sizeof(DiagShared) <= sizeof(double) * kNB * kTrsmLds, "in the inverse's buffer");
+
+namespace gemm {
+__device__ __forceinline__ void cp_async16(double* dst, const double* src, int bytes) {
+    const unsigned saddr = (unsigned)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(saddr), "l"(src), "r"(bytes));
+}
+__device__ __forceinline__ void cp_async8(double* dst, const double* src, bool valid) {
+    const unsigned saddr = (unsigned)__cvta_generic_to_shared(dst);
+    const int sz = valid ? 8 : 0;
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(saddr), "l"(src), "r"(sz));
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
+}  // namespace gemm
+
+// 64 x 64 doubles, rows contiguous in memory, to buf[col][row]; rows x cols of them
+// are there.  even: src is 16-byte aligned (ld is a multiple of four)
+__device__ __forceinline__ void chain_load(double (*buf)[kTrsmLds], const double* src, int ld, int rows, int cols, bool even) {
+    if (even) {
+#pragma unroll
+        for (int u = 0; u < kNB * kNB / 512; ++u) {
+            const int e = threadIdx.x + 256 * u, i = 2 * (e & 31), m = e >> 5;
+            const int n = m < cols ? max(0, min(2, rows - i)) : 0;
+            gemm::cp_async16(&buf[m][i], n > 0 ? src + i + (int64_t)m * ld : src, 8 * n);
+        }
+    } else {
+#pragma unroll 4
+        for (int u = 0; u < kNB * kNB / 256; ++u) {
+            const int e = threadIdx.x + 256 * u, i = e & 63, m = e >> 6;
+            const bool in = m < cols && i < rows;
+            gemm::cp_async8(&buf[m][i], in ? src + i + (int64_t)m * ld : src, in);
+        }
+    }
+}
+
+// the same from the transpose: element (i, m) at src[m + i * ld]
+__device__ __forceinline__ void chain_load_t(double (*buf)[kTrsmLds], const double* src, int ld, int rows) {
+#pragma unroll
+    for (int u = 0; u < kNB * kNB / 256; ++u) {
+        const int e = threadIdx.x + 256 * u;
+        const int m = (e & 3) + 4 * (e >> 5 & 15), i = (e >> 2 & 7) + 8 * (e >> 9);
+        gemm::cp_async8(&buf[m][i], i < rows ? src + m + (int64_t)i * ld : src, i < rows);
+    }
+}
+
+// acc = sum_k (a[k][i] d[k]) b[k][j] (without D: a[k][i] b[k][j]) by DMMA, a warp 32 x 16
+template <bool D>
+__device__ __forceinline__ void chain_product(double (&acc)[4][2][2], const double (*a)[kTrsmLds], const double (*b)[kTrsmLds],
+                                              const double* d, int wm, int wn, int lane, int kend) {
+#pragma unroll
+    for (int mi = 0; mi < 4; ++mi)
+#pragma unroll
+        for (int ni = 0; ni < 2; ++ni) acc[mi][ni][0] = acc[mi][ni][1] = 0.0;
+#pragma unroll 4
+    for (int k4 = 0; k4 < kend; k4 += 4) {
+        const int kk = k4 + (lane & 3);
+        double av[4], bv[2];
+#pragma unroll
+        for (int mi = 0; mi < 4; ++mi) av[mi] = D ? a[kk][wm + mi * 8 + (lane >> 2)] * d[kk] : a[kk][wm + mi * 8 + (lane >> 2)];
+#pragma unroll
+        for (int ni = 0; ni < 2; ++ni) bv[ni] = b[kk][wn + ni * 8 + (lane >> 2)];
+#pragma unroll
+        for (int mi = 0; mi < 4; ++mi)
+#pragma unroll
+            for (int ni = 0; ni < 2; ++ni) gemm::dmma(acc[mi][ni][0], acc[mi][ni][1], av[mi], bv[ni]);
+    }
+}
+
+// The 36 lower 8 x 8 tiles of 64 x 64: row tiles p and 7 - p have nine, and go to
+// warps p and p + 4, five and four of them (one scheduler's two warps: nine)
+struct ChainTiles {
+    int i[5], j[5], n;
+    __device__ __forceinline__ explicit ChainTiles(int warp) {
+        const int p = warp & 3, h = warp >> 2;
+        n = 5 - h;
+#pragma unroll
+        for (int q = 0; q < 5; ++q) {
+            const int t = min(2 * q + h, 8);
+            i[q] = t <= p ? p : 7 - p;
+            j[q] = t <= p ? t : t - p - 1;
+        }
+    }
+    __device__ __forceinline__ bool on(int q) const { return q < n; }
+};
+
+// c -= sum_k (a[k][i] d[k]) a[k][j] on them
+__device__ __forceinline__ void chain_lower(double (&c)[5][2], const double (*a)[kTrsmLds], const double* d,
+                                            const ChainTiles& tl, int lane) {
+    double acc[5][2];
+#pragma unroll
+    for (int q = 0; q < 5; ++q) acc[q][0] = acc[q][1] = 0.0;
+#pragma unroll 4
+    for (int k4 = 0; k4 < kNB; k4 += 4) {
+        const int kk = k4 + (lane & 3);
+        const double dv = d[kk];
+        double av[5], bv[5];
+#pragma unroll
+        for (int q = 0; q < 5; ++q) {
+            av[q] = a[kk][8 * tl.i[q] + (lane >> 2)] * dv;
+            bv[q] = a[kk][8 * tl.j[q] + (lane >> 2)];
+        }
+#pragma unroll
+        for (int q = 0; q < 5; ++q)
+            if (q < 4 || tl.on(q)) gemm::dmma(acc[q][0], acc[q][1], av[q], bv[q]);
+    }
+#pragma unroll
+    for (int q = 0; q < 5; ++q)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) c[q][h] -= acc[q][h];
+}
+
+template <int PR>
+__global__ void __launch_bounds__(256, 2) k_chain(const Job* jobs, int64_t njobs, const int32_t* tmap, PV P) {
+    extern __shared__ __align__(16) double csh[];
+    using Buf = double(*)[kTrsmLds];
+    const Buf B0 = reinterpret_cast<Buf>(csh), B1 = B0 + kNB, B2 = B1 + kNB;
+    double* dp = csh + 3 * kNB * kTrsmLds;                  // D of panel p - 1
+    double* dk = dp + kNB;                                  // and of p
+    double* rd = dk + kNB;                                  // 1 / D of p
+    double* adv = rd + kNB;
+    DiagShared& S = *reinterpret_cast<DiagShared*>(&B2[0][0]);             // once X is read
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int any_fail = P.st->any_fail;
+    const int64_t task = blockIdx.x;
+    const Job& jb = job_of(jobs, njobs, tmap, task);
+    const int js = jb.node, k0 = jb.k_lo, nb = jb.k_hi - jb.k_lo, c0 = jb.c0;
+    const int F = P.F[js], ld = P.buf_ld[js], sn_s = P.S[js];
+    const int64_t buf = P.buf_off[js], linv = P.linv_off[js];
+    // the first CTA may mark the front as failed while others start: one thread asks
+    if (__syncthreads_or(tid == 0 && (any_fail || P.sn_bad[js] || node_off(P, js)))) return;
+    const int sp1 = min((k0 / kSuperPanel + 1) * kSuperPanel, sn_s);
+    const bool chain = c0 < sp1, prev = chain && k0 % kSuperPanel != 0;
+    const int c1 = min(c0 + kNB, sp1);                      // the next panel's columns end
+    const int blk = (int)(task - jb.task0), r0 = c0 + blk * kNB;
+    double* front = P.arena + buf;
+    const double* pcol = front + (int64_t)k0 * ld;
+    const bool first = blk == 0;
+    const Buf own = first ? B1 : B0;                        // A, later L, of the CTA's rows
+    // a warp's 32 x 16 of the products; X is lower triangular, so columns wn .. of
+    // L21 take wn + 16 terms: the two warps of a scheduler have 80 together
+    const int wm = (warp & 1) * 32, wn = (warp & 2 ? 16 : 0) ^ (warp & 4 ? 48 : 0);
+    double cv[4][2][2], acc[4][2][2];
+    if (prev) {
+        const double* q = front + (int64_t)(k0 - kNB) * ld;
+        chain_load(B0, q + r0, ld, F - r0, kNB, true);
+        if (!first) chain_load(B1, q + c0, ld, c1 - c0, kNB, true);
+        gemm::cp_async_commit();
+    }
+    chain_load(B2, P.linv + linv + (int64_t)(k0 / kNB) * kNB * kNB, kNB, kNB, kNB, true);
+    if (first || !prev) {
+        chain_load(own, pcol + r0, ld, F - r0, nb, (c0 & 1) == 0);      // (odd: S is, chain is off)
+        if (!first && chain) chain_load_t(B1, front + k0 + (int64_t)c0 * ld, ld, c1 - c0);
+    }
+    gemm::cp_async_commit();
+    if (tid < kNB) {
+        const double d = tid < nb ? __ldcg(pcol + k0 + tid + (int64_t)tid * ld) : 0.0;
+        dk[tid] = d;
+        rd[tid] = tid < nb ? 1.0 / d : 0.0;
+        if (prev) dp[tid] = __ldcg(front + (int64_t)(k0 - kNB + tid) * (ld + 1));
+        if (first && chain && c0 + tid < c1) adv[tid] = __ldcg(P.adiag + P.fst[js] + c0 + tid);
+    }
+    const ChainTiles tl(warp);
+    double (&ct)[5][2] = *reinterpret_cast<double (*)[5][2]>(&cv[0][0][0]);
+    if (chain && first) {
+#pragma unroll
+        for (int q = 0; q < 5; ++q)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int r = c0 + 8 * tl.i[q] + (lane >> 2), c = c0 + 8 * tl.j[q] + 2 * (lane & 3) + h;
+                ct[q][h] = (r < F && c < c1 && r >= c) ? __ldcg(front + r + (int64_t)c * ld) : 0.0;
+            }
+    } else if (chain) {
+#pragma unroll
+        for (int mi = 0; mi < 4; ++mi)
+#pragma unroll
+            for (int ni = 0; ni < 2; ++ni)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int r = r0 + wm + mi * 8 + (lane >> 2), c = c0 + wn + ni * 8 + 2 * (lane & 3) + h;
+                    cv[mi][ni][h] = (r < F && c < c1 && r >= c) ? __ldcg(front + r + (int64_t)c * ld) : 0.0;
+                }
+    }
+    if (prev) {
+        gemm::cp_async_wait<1>();
+        __syncthreads();
+        if (first) chain_lower(ct, B0, dp, tl, lane);
+        else chain_product<true>(acc, B0, B1, dp, wm, wn, lane, kNB);
+        if (!first) {
+#pragma unroll
+            for (int mi = 0; mi < 4; ++mi)
+#pragma unroll
+                for (int ni = 0; ni < 2; ++ni)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) cv[mi][ni][h] -= acc[mi][ni][h];
+            __syncthreads();
+            chain_load(own, pcol + r0, ld, F - r0, nb, true);
+            chain_load_t(B1, front + k0 + (int64_t)c0 * ld, ld, c1 - c0);
+            gemm::cp_async_commit();
+        }
+    }
+    gemm::cp_async_wait<0>();
+    __syncthreads();
+    // L21 = (A21 X') D^-1
+    chain_product<false>(acc, own, B2, nullptr, wm, wn, lane, wn + 16);
+    __syncthreads();
+#pragma unroll
+    for (int mi = 0; mi < 4; ++mi)
+#pragma unroll
+        for (int ni = 0; ni < 2; ++ni)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int i = wm + mi * 8 + (lane >> 2), c = wn + ni * 8 + 2 * (lane & 3) + h;
+                const double l = acc[mi][ni][h] * rd[c];
+                own[c][i] = l;
+                if (r0 + i < F && c < nb) front[r0 + i + (int64_t)(k0 + c) * ld] = l;
+            }
+    if (!chain) return;
+    if (first) {
+        __syncthreads();
+        chain_lower(ct, own, dk, tl, lane);
+        double(*A)[kNB + 1] = reinterpret_cast<double(*)[kNB + 1]>(csh);     // in B0
+        for (int e = tid; e < kNB * kNB; e += 256)
+            if ((e & 63) < (e >> 6)) A[e & 63][e >> 6] = 0.0;
+#pragma unroll
+        for (int q = 0; q < 5; ++q)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int i = 8 * tl.i[q] + (lane >> 2), j = 8 * tl.j[q] + 2 * (lane & 3) + h, r = c0 + i, c = c0 + j;
+                if (!tl.on(q) || i < j) continue;
+                A[i][j] = r < c1 ? ct[q][h] : 0.0;                             // (c <= r)
+                if (r >= c1 && r < F && c < c1) front[r + (int64_t)c * ld] = ct[q][h];
+            }
+        if (c0 + tid < c1) S.adv[tid & (kNB - 1)] = adv[tid & (kNB - 1)];
+        if (tid == 0) S.fail = kNB;
+        __syncthreads();
+        diag_block<PR, false>(P, js, c0, c1 - c0, front, ld, 0, A, S);
+        return;
+    }
+    chain_product<false>(acc, B1, B2, nullptr, wm, wn, lane, wn + 16);
+    __syncthreads();
+#pragma unroll
+    for (int mi = 0; mi < 4; ++mi)
+#pragma unroll
+        for (int ni = 0; ni < 2; ++ni)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int i = wm + mi * 8 + (lane >> 2), c = wn + ni * 8 + 2 * (lane & 3) + h;
+                B1[c][i] = acc[mi][ni][h] * rd[c];
+            }
+    __syncthreads();
+    chain_product<true>(acc, own, B1, dk, wm, wn, lane, kNB);
+    const bool copy = blk == 1 && c1 < sp1;                 // these are the panel after the next's rows
+#pragma unroll
+    for (int mi = 0; mi < 4; ++mi)
+#pragma unroll
+        for (int ni = 0; ni < 2; ++ni)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int r = r0 + wm + mi * 8 + (lane >> 2), c = c0 + wn + ni * 8 + 2 * (lane & 3) + h;
+                if (r >= F || c >= c1) continue;
+                const double v = cv[mi][ni][h] - acc[mi][ni][h];
+                front[r + (int64_t)c * ld] = v;
+                if (copy && r < sp1) front[c + (int64_t)r * ld] = v;
+            }
+}
+
 // Inverse of the unit-lower diagonal blocks straight from LNZ (used when the
 // factor in SM was not produced by this engine, e.g. a solve-only call).
 __global__ void __launch_bounds__(64) k_linv(const Job* jobs, PV P) {
@@ -1386,19 +1783,6 @@ __global__ void __launch_bounds__(64) k_linv(const Job* jobs, PV P) {
 // a STAGES-deep cp.async pipeline (16-byte copies of row pairs).
 namespace gemm {
 constexpr int BK = 16;
-
-__device__ __forceinline__ void cp_async16(double* dst, const double* src, int bytes) {
-    const unsigned saddr = (unsigned)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(saddr), "l"(src), "r"(bytes));
-}
-__device__ __forceinline__ void cp_async8(double* dst, const double* src, bool valid) {
-    const unsigned saddr = (unsigned)__cvta_generic_to_shared(dst);
-    const int sz = valid ? 8 : 0;
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(saddr), "l"(src), "r"(sz));
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
 
 template <int T, int WM, int WN, int STAGES>
 struct Cfg {
@@ -2945,6 +3329,12 @@ int Engine::open(const int64_t* mspar, const int64_t* mtrees, const int64_t* msi
     CK(cudaFuncSetAttribute(k_small_front<kPivotChol>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need));
     CK(cudaFuncSetAttribute(k_small_front<kPivotChol4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need));
     CK(cudaFuncSetAttribute(k_trsm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTrsmSmem));
+    for (const void* f : {(const void*)k_diag<kPivotLDL>, (const void*)k_diag<kPivotReplace>, (const void*)k_diag<kPivotChol>,
+                          (const void*)k_diag<kPivotChol4>})
+        CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDiagSmem));
+    for (const void* f : {(const void*)k_chain<kPivotLDL>, (const void*)k_chain<kPivotReplace>, (const void*)k_chain<kPivotChol>,
+                          (const void*)k_chain<kPivotChol4>})
+        CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kChainSmem));
     CK(cudaFuncSetAttribute(k_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmallSolveSmem));
     CK(cudaFuncSetAttribute(k_backward, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmallSolveSmem));
     CK(cudaFuncSetAttribute(K_GEMM_BIG, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GemmBig::smem));
@@ -3101,10 +3491,21 @@ static PV make_view(Engine::Dev& D, const Plan& P, double* d_sm, double tol1) {
 void Engine::launch_diag(const Launch& pl, cudaStream_t s, const PV& pv) {
     const Job* jobs = d_->jobs + pl.job_begin;
     const int n = (int)pl.job_count;
-    if (pv.fc3 == 2) k_diag<kPivotChol4><<<n, 256, 0, s>>>(jobs, pv);
-    else if (pv.fc3) k_diag<kPivotReplace><<<n, 256, 0, s>>>(jobs, pv);
-    else if (chol_) k_diag<kPivotChol><<<n, 256, 0, s>>>(jobs, pv);
-    else k_diag<kPivotLDL><<<n, 256, 0, s>>>(jobs, pv);
+    if (pv.fc3 == 2) k_diag<kPivotChol4><<<n, 256, kDiagSmem, s>>>(jobs, pv, 1);
+    else if (pv.fc3) k_diag<kPivotReplace><<<n, 256, kDiagSmem, s>>>(jobs, pv, 1);
+    else if (chol_) k_diag<kPivotChol><<<n, 256, kDiagSmem, s>>>(jobs, pv, 1);
+    else k_diag<kPivotLDL><<<n, 256, kDiagSmem, s>>>(jobs, pv, 1);
+    ++timing.launches;
+}
+
+void Engine::launch_chain(const Launch& pl, cudaStream_t s, const PV& pv) {
+    const Job* jobs = d_->jobs + pl.job_begin;
+    const int n = (int)pl.ntasks;
+    if (pv.fc3 == 2) k_chain<kPivotChol4><<<n, 256, kChainSmem, s>>>(jobs, pl.job_count, TMAP(pl), pv);
+    else if (pv.fc3) k_chain<kPivotReplace><<<n, 256, kChainSmem, s>>>(jobs, pl.job_count, TMAP(pl), pv);
+    else if (chol_) k_chain<kPivotChol><<<n, 256, kChainSmem, s>>>(jobs, pl.job_count, TMAP(pl), pv);
+    else k_chain<kPivotLDL><<<n, 256, kChainSmem, s>>>(jobs, pl.job_count, TMAP(pl), pv);
+    ++timing.launches;
 }
 
 void Engine::launch_gemm(const Launch& l, cudaStream_t s, const PV& pv, std::vector<cudaEvent_t>& gev) {
@@ -3257,23 +3658,24 @@ void Engine::enqueue_factor(const PV& pv, cudaStream_t s, std::vector<cudaEvent_
     auto mark = [&](int phase) {
         if (profile_) marks_.emplace_back(phase, record_event(s));
     };
+    constexpr size_t kSteps = kSuperPanel / kNB;
     // side stream for the trailing-update columns beyond the next super-panel,
-    // look-ahead stream for the in-super-panel columns after the next panel
+    // look-ahead stream for the in-super-panel columns after the next two panels
     // (profile mode keeps everything on one stream so the events time it)
     cudaStream_t u = (profile_ || !D.side) ? s : D.side;
     cudaStream_t la = (profile_ || !D.ahead) ? s : D.ahead;
     size_t evi = 0;
-    cudaEvent_t far_done = nullptr, ahead_done = nullptr;
+    cudaEvent_t far_done = nullptr, ahead_done[2] = {nullptr, nullptr};      // ahead: of even and odd steps
     auto join_far = [&]() {
         if (far_done) {
             cudaStreamWaitEvent(s, far_done, 0);
             far_done = nullptr;
         }
     };
-    auto join_ahead = [&]() {
-        if (ahead_done) {
-            cudaStreamWaitEvent(s, ahead_done, 0);
-            ahead_done = nullptr;
+    auto join_ahead = [&](size_t st) {
+        if (ahead_done[st & 1]) {
+            cudaStreamWaitEvent(s, ahead_done[st & 1], 0);
+            ahead_done[st & 1] = nullptr;
         }
     };
     mark(0);
@@ -3327,13 +3729,24 @@ void Engine::enqueue_factor(const PV& pv, cudaStream_t s, std::vector<cudaEvent_
         }
         for (size_t st = 0; st < lp.panel.size(); ++st) {
             const Launch& pl = lp.panel[st];
-            mark(3);
-            launch_diag(pl, s, pv);
-            ++timing.launches;
+            // a super-panel's first diagonal block has a launch of its own, the others
+            // come with the step before
+            if (st % kSteps == 0) {
+                mark(3);
+                launch_diag(pl, s, pv);
+            }
+            const bool chain = (st + 1) % kSteps != 0;
+            // the look-ahead update of two steps before wrote the columns that
+            // this step is about to update (and the event's slot is free again)
+            join_ahead(st);
             if (pl.ntasks > 0) {
-                mark(4);
-                k_trsm<<<(int)pl.ntasks, 128, kTrsmSmem, s>>>(jobs + pl.job_begin, pl.job_count, TMAP(pl), pv);
-                ++timing.launches;
+                mark(chain ? 3 : 4);
+                if (chain) {
+                    launch_chain(pl, s, pv);
+                } else {
+                    k_trsm<<<(int)pl.ntasks, 128, kTrsmSmem, s>>>(jobs + pl.job_begin, pl.job_count, TMAP(pl), pv);
+                    ++timing.launches;
+                }
             }
             const bool has_far = !lp.far[st].empty() || !lp.far_tc[st].empty();
             const bool far_tc = mixed_ == 1 && lp.far_flops[st] >= tc_min_flops_;
@@ -3360,22 +3773,15 @@ void Engine::enqueue_factor(const PV& pv, cudaStream_t s, std::vector<cudaEvent_
             mark(5);
             // a trailing update's next-super-panel columns were also updated by
             // the previous super-panel's far launch: wait for it first
-            if ((st + 1) % (kSuperPanel / kNB) == 0) join_far();
-            // the previous step's look-ahead update also wrote the columns
-            // that this step's chain update is about to update
-            join_ahead();
+            if (!chain) join_far();
             cudaEvent_t fork_ahead = nullptr;
             if (!lp.ahead[st].empty() && la != s) {
                 fork_ahead = D.evpool[evi++];
                 cudaEventRecord(fork_ahead, s);
             }
-            // the updates inside the panel chain (K = 64: the next panel's
-            // columns; K = kSuperPanel: the next super-panel's columns) are on the
-            // critical path.  The K = 64 ones are small: the FP64 kernel's
-            // 64x64 tiles start sooner than a split + tensor-core pair, so they
-            // stay FP64 in both modes; in mixed mode the K = kSuperPanel one takes the
-            // tensor cores when large enough.  They are issued first, the
-            // look-ahead columns after them.
+            // the K = kSuperPanel update of the next super-panel's columns is on
+            // the critical path; in mixed mode it takes the tensor cores when large
+            // enough (the next panel's K = 64 updates stay FP64 in every mode)
             if (trail_i8) {
                 // one split serves both column ranges; the slabs are free again
                 // because the previous far update was joined above
@@ -3397,8 +3803,8 @@ void Engine::enqueue_factor(const PV& pv, cudaStream_t s, std::vector<cudaEvent_
                 if (fork_ahead) cudaStreamWaitEvent(la, fork_ahead, 0);
                 for (const Launch& al : lp.ahead[st]) launch_gemm(al, la, pv, gev);
                 if (la != s) {
-                    ahead_done = D.evpool[evi++];
-                    cudaEventRecord(ahead_done, la);
+                    ahead_done[st & 1] = D.evpool[evi++];
+                    cudaEventRecord(ahead_done[st & 1], la);
                 }
             }
             if (has_far) {
@@ -3418,7 +3824,8 @@ void Engine::enqueue_factor(const PV& pv, cudaStream_t s, std::vector<cudaEvent_
                 }
             }
         }
-        join_ahead();
+        join_ahead(0);
+        join_ahead(1);
         join_far();
         mark(6);
         if (mixed_ == 1 && lp.outer_flops >= tc_min_flops_) {
@@ -4264,6 +4671,7 @@ size_t dense_scratch_bytes(int64_t n) {
 int dense_factor_setup() {
     // k_trsm and the small-tile update use more than the default 48 KB of
     // dynamic shared memory; the opt-in is per function and per device.
+    CK(cudaFuncSetAttribute(k_diag<kPivotLDL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDiagSmem));
     CK(cudaFuncSetAttribute(k_trsm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTrsmSmem));
     CK(cudaFuncSetAttribute(K_GEMM_SMALL, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GemmSmall::smem));
     return 0;
@@ -4360,7 +4768,7 @@ int dense_factor_with_scratch(double* a, int64_t n, int64_t lda, double tol1, do
     pv.tol1 = tol1;
     for (int64_t stp = 0; stp < nblk; ++stp) {
         const StepJobs& sj = steps[stp];
-        k_diag<kPivotLDL><<<1, 256, 0, s>>>(jobs + sj.panel_begin, pv);
+        k_diag<kPivotLDL><<<1, 256, kDiagSmem, s>>>(jobs + sj.panel_begin, pv, 0);
         if (sj.panel_tasks > 0) k_trsm<<<(int)sj.panel_tasks, 128, kTrsmSmem, s>>>(jobs + sj.panel_begin, 1, nullptr, pv);
         if (sj.upd_tasks > 0)
             K_GEMM_SMALL<<<(int)sj.upd_tasks, GemmSmall::NT, GemmSmall::smem, s>>>(jobs + sj.upd_begin, sj.upd_jobs, nullptr,

@@ -266,6 +266,7 @@ private:
     int64_t nbuf_cap_ = 0;
     void launch_gemm(const Launch& l, cudaStream_t s, const struct PV& pv, std::vector<cudaEvent_t>& gev);
     void launch_diag(const Launch& pl, cudaStream_t s, const struct PV& pv);
+    void launch_chain(const Launch& pl, cudaStream_t s, const struct PV& pv);
     void upload_plan();
     int64_t ensure_vectors(int64_t nrhs);
     Plan P_;

@@ -444,12 +444,14 @@ int build_plan(const int64_t* mspar, const int64_t* mtrees, const int64_t* msifa
                 const int32_t sp0 = (k0 / kSuperPanel) * kSuperPanel;
                 const int32_t sp1 = std::min(sp0 + kSuperPanel, s);
                 if (c0 < sp1) {                                     // inside the super-panel
-                    // the next panel's columns on the panel chain; the ones
-                    // after it beside the next diagonal block and TRSM
-                    const int32_t c1 = std::min(c0 + kNB, sp1);
-                    jl.push_back(Job{js, c0, c1, f, k0, c0, 0});
-                    if (c1 < sp1) jahead.push_back(Job{js, c1, sp1, f, k0, c0, 0});
-                    P.gemm_flops += update_flops(c0, sp1, f, nb);
+                    // the next panel's columns with the panel's own launch (by
+                    // this panel and the one before), the ones after the next
+                    // two panels beside the next step
+                    const int32_t c2 = c0 + 2 * kNB;
+                    if (c2 < sp1) {
+                        jahead.push_back(Job{js, c2, sp1, f, k0, c0, 0});
+                        P.gemm_flops += update_flops(c2, sp1, f, nb);
+                    }
                 }
                 if (c0 == sp1 && sp1 < s) {                          // trailing, K = kSuperPanel
                     // the next super-panel's columns now; the columns beyond
@@ -688,6 +690,18 @@ void check_plan(const Plan& P, int64_t& oob, int64_t& overlaps) {
     }
 }
 
+// the update that a panel step's launch makes of the next panel's columns, by
+// its own panel and the one before it in the super-panel (empty past the last)
+static Job chain_update(const Plan& P, const Job& panel) {
+    Job j = panel;
+    const int32_t sp0 = panel.k_lo / kSuperPanel * kSuperPanel;
+    j.c0 = panel.k_hi;
+    j.c_end = std::max(j.c0, std::min({j.c0 + kNB, sp0 + kSuperPanel, P.S[j.node]}));
+    j.r_end = P.F[j.node];
+    j.k_lo = std::max(sp0, panel.k_lo - kNB);
+    return j;
+}
+
 void check_coverage(const Plan& P, int64_t& fp64, int64_t& tc) {
     fp64 = tc = 0;
     const int64_t ns = P.nsuper;
@@ -713,6 +727,13 @@ void check_coverage(const Plan& P, int64_t& fp64, int64_t& tc) {
                 }
                 for (const Launch& l : lp.update[st]) add(l);
             }
+            for (const Launch& l : lp.panel)
+                for (int64_t j = 0; j < l.job_count; ++j) {
+                    const Job c = chain_update(P, P.jobs[l.job_begin + j]);
+                    auto& v = cov[c.node];
+                    if (v.empty()) v.resize(P.F[c.node]);
+                    for (int32_t col = c.c0; col < c.c_end; ++col) v[col].emplace_back(c.k_lo, c.k_hi);
+                }
             for (const auto& v : lp.ahead)
                 for (const Launch& l : v) add(l);
             if (which == 0) {
@@ -767,10 +788,11 @@ void check_coverage(const Plan& P, int64_t& fp64, int64_t& tc) {
 // Stream-schedule check of the factorisation (a race detector on the host).
 //
 // Replays the launch order of the factorisation of every level: per panel
-// step the diagonal block + TRSM and the panel-chain updates on the main
-// stream; inside a super-panel the update of the columns after the next
-// panel on the look-ahead stream, forked by an event after the step's TRSM
-// and joined before the next step's chain update; at the end of a
+// step the TRSM, the update of the next panel's columns by this panel and the
+// one before and the next diagonal block on the main stream; inside a
+// super-panel the update of the columns after the next two panels on the
+// look-ahead stream, forked by an event after the step and joined before the
+// step after the next; at the end of a
 // super-panel the far columns' update on the side stream, forked by an event
 // after the step's TRSM and joined before the next trailing update (every
 // kSuperPanel / kNB steps) and before the K = S update.  Vector clocks give
@@ -939,8 +961,8 @@ int64_t check_schedule(const Plan& P, bool tc, int skip_join) {
         if (lp.elim_nodes.empty()) continue;
         std::map<int32_t, std::vector<SchedOp>> ops;     // per front, in issue order
         int64_t vc[kStreams][kStreams] = {};            // per stream: its vector clock
-        int64_t far_done[kStreams], ahead_done[kStreams];
-        bool far_open = false, ahead_open = false;
+        int64_t far_done[kStreams], ahead_done[2][kStreams];
+        bool far_open = false, ahead_open[2] = {false, false};
         auto issue = [&](int stream, const Job& j, int kind) {
             ++vc[stream][stream];
             SchedOp o;
@@ -980,24 +1002,39 @@ int64_t check_schedule(const Plan& P, bool tc, int skip_join) {
             if (far_open && !(skip_join & 1)) wait(0, far_done);
             far_open = false;
         };
-        auto join_ahead = [&]() {
-            if (ahead_open && !(skip_join & 2)) wait(0, ahead_done);
-            ahead_open = false;
+        auto join_ahead = [&](size_t st) {
+            if (ahead_open[st & 1] && !(skip_join & 2)) wait(0, ahead_done[st & 1]);
+            ahead_open[st & 1] = false;
         };
         for (size_t st = 0; st < lp.panel.size(); ++st) {
-            issue_launch(0, lp.panel[st], 0);
+            // a super-panel's first diagonal block, then the TRSM, the next panel's columns
+            // and its diagonal block
+            const Launch& pl = lp.panel[st];
+            constexpr size_t kSteps = kSuperPanel / kNB;
+            if (st % kSteps == 0) issue_launch(0, pl, 0);
+            join_ahead(st);
+            issue_launch(0, pl, 0);
+            if ((st + 1) % kSteps != 0)
+                for (int64_t k = 0; k < pl.job_count; ++k) {
+                    const Job c = chain_update(P, P.jobs[pl.job_begin + k]);
+                    if (c.c0 >= c.c_end) continue;
+                    issue(0, c, 1);
+                    Job d = c;
+                    d.k_lo = c.c0;
+                    d.k_hi = c.c_end;
+                    issue(0, d, 0);
+                }
             const bool has_far = tc ? !lp.far_tc[st].empty() : !lp.far[st].empty();
             if (has_far) wait(1, vc[0]);                 // fork after the step's TRSM
-            if ((st + 1) % (kSuperPanel / kNB) == 0) join();
-            join_ahead();
+            if ((st + 1) % kSteps == 0) join();
             int64_t fork[kStreams];
             record(0, fork);
             for (const Launch& ul : lp.update[st]) issue_launch(0, ul, 1);
             if (!lp.ahead[st].empty()) {
                 wait(2, fork);
                 for (const Launch& al : lp.ahead[st]) issue_launch(2, al, 1);
-                record(2, ahead_done);
-                ahead_open = true;
+                record(2, ahead_done[st & 1]);
+                ahead_open[st & 1] = true;
             }
             if (has_far) {
                 if (tc)
@@ -1008,7 +1045,8 @@ int64_t check_schedule(const Plan& P, bool tc, int skip_join) {
                 far_open = true;
             }
         }
-        join_ahead();
+        join_ahead(0);
+        join_ahead(1);
         join();
         if (tc)
             for (const TcLaunch& t : lp.outer_tc) issue_launch(0, t.gemm, 1);

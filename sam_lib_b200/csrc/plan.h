@@ -107,10 +107,14 @@ struct LevelPlan {
     };
     std::vector<SmallClass> small_classes;
     Launch assemble;                          // large fronts: extend-add into dense fronts
-    std::vector<Launch> panel;                // per panel step: diagonal block + TRSM
-    std::vector<std::vector<Launch>> update;  // per panel step: Schur updates (one launch per tile size)
+    // per panel step: the panel's diagonal block and TRSM; inside a super-panel
+    // the launch of the TRSM also updates the next panel's columns (by this panel
+    // and the one before) and does the next diagonal block
+    std::vector<Launch> panel;
+    // per step that ends a super-panel: the next super-panel's columns (one launch per tile size)
+    std::vector<std::vector<Launch>> update;
     // per panel step inside a super-panel: the update of the columns after the
-    // next panel (look-ahead stream, beside the next diagonal block and TRSM)
+    // next two panels (look-ahead stream, beside the next step)
     std::vector<std::vector<Launch>> ahead;
     // mixed precision: a super-panel's K = kSuperPanel update of the next super-panel's
     // columns (the update[st] jobs of a step that ends a super-panel) as a

@@ -80,8 +80,10 @@ def _chain(widths):
                                     [80], [81], [112], [113], [144], [145], [175], [176],
                                     [1, 1], [1, 175], [16, 32], [16, 33], [17, 31], [3, 45, 16], [100, 76], [5, 20, 151],
                                     [177], [183], [184], [185], [193], [200], [201], [223], [225], [239], [255], [256],
-                                    [9, 168], [65, 200]])
-def test_orders_at_the_edges_of_the_groups(widths):
+                                    [9, 168], [65, 200], [129, 1], [192, 1], [193, 60], [257, 127], [320, 128], [449, 77],
+                                    [511, 130], [512, 64], [513, 1], [577, 63], [640, 129], [641, 65], [1025, 100],
+                                    [100, 449, 200]])
+def test_orders_at_the_edges_of_the_groups_and_panels(widths):
     structure, rows, xsuper, xlnz = _chain(widths)
     neq = sum(widths)
     a = _dense(neq, neq)
