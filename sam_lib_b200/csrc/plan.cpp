@@ -233,7 +233,12 @@ int build_plan(const int64_t* mspar, const int64_t* mtrees, const int64_t* msifa
                 const int32_t c = cls(P.F[lp.small_nodes[k]]);
                 int32_t e = k;
                 while (e < (int32_t)lp.small_nodes.size() && cls(P.F[lp.small_nodes[e]]) == c) ++e;
-                lp.small_classes.push_back(LevelPlan::SmallClass{k, e - k, P.F[lp.small_nodes[k]]});
+                int32_t nl = 0;
+                for (int32_t q = k; q < e; ++q) {
+                    const int32_t f = P.F[lp.small_nodes[q]], w = P.S[lp.small_nodes[q]];
+                    nl = std::max(nl, f * w - w * (w - 1) / 2);
+                }
+                lp.small_classes.push_back(LevelPlan::SmallClass{k, e - k, P.F[lp.small_nodes[k]], nl});
                 k = e;
             }
         }

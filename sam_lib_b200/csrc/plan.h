@@ -101,9 +101,9 @@ struct LevelPlan {
     int32_t small_maxF = 0;
     // small fronts in size classes (F <= 64, 96, 128, 176), one launch each so
     // that the smaller fronts get the shared memory (and occupancy) they need:
-    // {first index into small_nodes, count, largest F}
+    // {first index into small_nodes, count, largest F, largest trapezoid of L}
     struct SmallClass {
-        int32_t begin, count, maxF;
+        int32_t begin, count, maxF, maxL;
     };
     std::vector<SmallClass> small_classes;
     Launch assemble;                          // large fronts: extend-add into dense fronts
