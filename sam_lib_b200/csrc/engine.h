@@ -265,6 +265,9 @@ private:
     double* nbuf_ = nullptr;      // the residual's max norms (3 per right-hand side)
     int64_t nbuf_cap_ = 0;
     void launch_gemm(const Launch& l, cudaStream_t s, const struct PV& pv, std::vector<cudaEvent_t>& gev);
+    struct SmallStreams;
+    SmallStreams small_streams(const struct LevelPlan& lp, cudaStream_t s, size_t& evi);
+    void join_small(const SmallStreams& r, cudaStream_t s, size_t& evi);
     void launch_diag(const Launch& pl, cudaStream_t s, const struct PV& pv);
     void launch_chain(const Launch& pl, cudaStream_t s, const struct PV& pv);
     void upload_plan();
