@@ -3307,6 +3307,13 @@ void Engine::store_graph(const GraphKey& k, cudaGraphExec_t exec, int64_t launch
     }
     graphs_.push_back(GraphEntry{k, exec, launches});
 }
+// The solves' graphs (the factorisation's have no B in their key).
+void Engine::drop_solve_graphs() {
+    for (auto& g : graphs_)
+        if (g.key.b) cudaGraphExecDestroy(g.exec);
+    graphs_.erase(std::remove_if(graphs_.begin(), graphs_.end(), [](const GraphEntry& g) { return g.key.b != nullptr; }),
+                  graphs_.end());
+}
 
 Engine::~Engine() {
     for (auto& g : graphs_) cudaGraphExecDestroy(g.exec);
@@ -4579,13 +4586,15 @@ int Engine::sn_stats(int32_t* neg, int32_t* fail) {
 }
 
 // Buffers for up to nrhs right-hand sides in a pass; returns how many a pass
-// may take (0: not even kMaxRHS fit).
+// may take (0: not even kMaxRHS fit).  Graphs captured on the old buffers go
+// with them: the three move independently, and a new one may lie where another was.
 int64_t Engine::ensure_vectors(int64_t nrhs) {
     Dev& D = *d_;
     if (nrhs <= 0) return D.vbuf ? 1 : 0;                // nothing to solve
     for (;;) {
         const int64_t want = std::min(nrhs, D.pass_rhs);
         if (D.vbuf && D.vbuf_rhs >= want) return want;
+        drop_solve_graphs();
         for (double** p : {&D.vbuf, &D.ybuf, &D.pbuf}) {
             if (*p) cudaFree(*p);
             *p = nullptr;
@@ -4790,7 +4799,7 @@ int Engine::solve(const double* d_sm, double* d_b, int64_t ldb, int64_t nrhs, in
         linv_valid_ = true;
     }
     if (use_graphs_ && !profile_ && s != nullptr && !tc_drop_ && wait_ns_ == 2000000000ull && !split_) {
-        const GraphKey key{(const void*)d_sm, (const void*)d_b, (double)ldb, nrhs, which, (int64_t)(uintptr_t)D.vbuf};
+        const GraphKey key{(const void*)d_sm, (const void*)d_b, (double)ldb, nrhs, which, chunk};
         cudaGraphExec_t exec = find_graph(key);
         if (!exec) {
             CK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));

@@ -205,6 +205,7 @@ private:
     cudaGraphExec_t find_graph(const GraphKey& k);
     int64_t graph_launches(const GraphKey& k);
     void store_graph(const GraphKey& k, cudaGraphExec_t exec, int64_t launches);
+    void drop_solve_graphs();
     void enqueue_factor(const struct PV& pv, cudaStream_t s, std::vector<cudaEvent_t>& gev);
     void enqueue_solve(const struct PV& pv, cudaStream_t s, double* d_b, int64_t ldb, int64_t nrhs, int64_t chunk,
                        int which, int64_t& nl);
