@@ -94,6 +94,15 @@ __device__ __forceinline__ void tile_of_i8(int64_t u, int nct, int nr, int& it, 
 
 __device__ __forceinline__ int k_blocks_i8(const Job& jb) { return (jb.k_hi - jb.k_lo + kK - 1) / kK; }
 
+// What the split leaves in a job's flag: 0, 1 with a negative pivot, or that the
+// front's update is left out.  k_gemm_i8 goes by this alone: PV::sn_bad may change
+// while the columns beyond the next super-panel run beside the same front's panel
+// chain, and the roles of a CTA, each on its own way through the tiles, have to
+// agree on the ones that are skipped.  A front that fails after its split
+// gets the rest of that update, which nobody reads.
+constexpr double kOffI8 = -1.0;
+__device__ __forceinline__ bool off_i8(const Job& jb, const double* scales) { return scales[jb.aux_job] < 0.0; }
+
 // 2^e for -1022 <= e <= 1023
 __device__ __forceinline__ double pow2(int e) { return __longlong_as_double((long long)(e + 1023) << 52); }
 
@@ -114,9 +123,12 @@ __global__ void __launch_bounds__(256) k_split_i8(const Job* jobs, int64_t njobs
     const int64_t task = blockIdx.x;
     const Job& jb = job_of(jobs, njobs, tmap, task);
     const int js = jb.node;
-    if (P.sn_bad[js] || node_off(P, js)) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int rb = (int)(task - jb.task0);
+    if (P.sn_bad[js] || node_off(P, js)) {
+        if (rb == 0 && tid == 0) scales[jb.aux_job] = kOffI8;
+        return;
+    }
     const int K = jb.k_hi - jb.k_lo, nkb = k_blocks_i8(jb);
     const int64_t np = jb.np, ld = P.buf_ld[js];
     const int r = jb.c0 + rb * 32 + lane;
@@ -251,7 +263,7 @@ __global__ void __launch_bounds__(i8::kThreadsI8, 1)
         bool stop = false;
         for (int64_t task = blockIdx.x; task < ntasks && !stop && !*(volatile int*)&failed; task += gridDim.x) {
             const Job& jb = job_of(jobs, njobs, tmap, task);
-            if (P.sn_bad[jb.node] || node_off(P, jb.node)) continue;
+            if (off_i8(jb, scales)) continue;
             int it, jt;
             tile_of_i8(task - jb.task0, (jb.c_end - jb.c0 + kN - 1) / kN, (jb.r_end - jb.c0 + kM - 1) / kM, it, jt);
             const int nkb = k_blocks_i8(jb), np = jb.np;
@@ -302,7 +314,7 @@ __global__ void __launch_bounds__(i8::kThreadsI8, 1)
         const uint64_t ad0 = sw128_desc(sa), bd0 = sw128_desc(sb);
         for (int64_t task = blockIdx.x; task < ntasks && !stop; task += gridDim.x) {
             const Job& jb = job_of(jobs, njobs, tmap, task);
-            if (P.sn_bad[jb.node] || node_off(P, jb.node)) continue;
+            if (off_i8(jb, scales)) continue;
             const int nkb = k_blocks_i8(jb);
             if (tile >= 1 && !mbar_wait(acce, (tile - 1) & 1u, P.wait_ns)) {
                 stop = true;
@@ -365,7 +377,7 @@ __global__ void __launch_bounds__(i8::kThreadsI8, 1)
         for (int64_t task = blockIdx.x; task < ntasks; task += gridDim.x) {
             const Job& jb = job_of(jobs, njobs, tmap, task);
             const int js = jb.node;
-            if (P.sn_bad[js] || node_off(P, js)) continue;
+            if (off_i8(jb, scales)) continue;
             int it, jt;
             tile_of_i8(task - jb.task0, (jb.c_end - jb.c0 + kN - 1) / kN, (jb.r_end - jb.c0 + kM - 1) / kM, it, jt);
             const int row = it * kM + 32 * q + lane, col0 = jt * kN + kEpiCols * h;

@@ -50,7 +50,7 @@ struct Job {
     int64_t task0;                   // first task of this job within its launch
     int64_t slab = 0;                // tensor-core updates: first row of the job's operand slabs
     // integer-digit updates: where the job's row scales and the job's flag
-    // (negative pivots) are, and the slabs' padded rows
+    // (negative pivots, or left out) are, and the slabs' padded rows
     int64_t aux = 0, aux_job = 0;
     int32_t np = 0;
 };
