@@ -186,6 +186,7 @@ struct Engine::Dev {
     float* slab = nullptr;
     alignas(64) CUtensorMap slab_map;
     float* slab_far = nullptr;                   // slabs of the side-stream launches
+    int32_t* tc_off = nullptr;                   // fronts left out, per supernode: launches on the stream, side-stream ones
     alignas(64) CUtensorMap slab_map_far;
     // integer-digit updates: digit slabs, row scales, the TMA maps over the slabs
     uint8_t* i8_slab = nullptr;
@@ -3324,6 +3325,7 @@ Engine::~Engine() {
     if (d_->mbox) cudaFreeHost(d_->mbox);
     if (d_->slab) cudaFree(d_->slab);
     if (d_->slab_far) cudaFree(d_->slab_far);
+    if (d_->tc_off) cudaFree(d_->tc_off);
     if (d_->i8_slab) cudaFree(d_->i8_slab);
     if (d_->i8_scales) cudaFree(d_->i8_scales);
     if (d_->sqd) cudaFree(d_->sqd);
@@ -3498,7 +3500,8 @@ static int make_slab(int64_t rows_needed, float** slab, CUtensorMap* map) {
 
 int Engine::ensure_slabs() {
     Dev& D = *d_;
-    if (D.slab && D.slab_far) return 0;
+    if (D.slab && D.slab_far && D.tc_off) return 0;
+    if (!D.tc_off) CK(cudaMalloc((void**)&D.tc_off, 2 * P_.nsuper * sizeof(int32_t)));
     if (!D.slab) {
         const int rc = make_slab(P_.slab_rows, &D.slab, &D.slab_map);
         if (rc != 0) return rc;
@@ -3678,14 +3681,16 @@ void Engine::launch_tc(const TcLaunch& t, cudaStream_t s, const PV& pv, std::vec
         tc_pairs_.push_back(gev.size());
         gev.push_back(record_event(s));
     }
+    int32_t* off = D.tc_off + (far ? P_.nsuper : 0);
     k_split_tc<<<(int)t.split.ntasks, 256, 0, s>>>(D.jobs + t.split.job_begin, t.split.job_count, TMAP(t.split), pv,
-                                                   far ? D.slab_far : D.slab);
+                                                   far ? D.slab_far : D.slab, off);
     // a side-stream launch leaves a quarter of the SMs to the panel chain
     // (a persistent tensor-core CTA holds most of an SM's shared memory)
     const int cap = (far && !profile_) ? std::max(1, sm_count_ * far_cap_q_ / 4) : sm_count_;
     const int grid = (int)std::min<int64_t>(t.gemm.ntasks, cap);
     k_gemm_tc<<<grid, tc::kThreads, tc::kSmem, s>>>(D.jobs + t.gemm.job_begin, t.gemm.job_count, TMAP(t.gemm),
-                                                    t.gemm.ntasks, pv, far ? D.slab_map_far : D.slab_map);
+                                                    t.gemm.ntasks, pv, off,
+                                                    far ? D.slab_map_far : D.slab_map);
     if (profile_) gev.push_back(record_event(s));
     timing.launches += 2;
     ++timing.gemm_launches;

@@ -197,18 +197,24 @@ __device__ __forceinline__ void tile_of(int64_t u, int nct, int nr, int& it, int
 // Split kernel: one CTA (256 threads) per 32-row x 32-column block of a job's
 // panel; the transpose goes through shared memory so that both the FP64
 // reads (column-major front) and the FP32 slab writes (row-major) coalesce.
+// off: per supernode, whether the launch leaves its front out.  k_gemm_tc goes by
+// this alone: PV::sn_bad may change while a far update runs beside the same
+// front's panel chain, and the roles of a CTA, each on its own way through the
+// tiles, have to agree on the ones that are skipped.
 __global__ void __launch_bounds__(256) k_split_tc(const Job* jobs, int64_t njobs, const int32_t* tmap, PV P,
-                                                   float* slab) {
+                                                   float* slab, int32_t* off) {
     __shared__ float sw[2][32][33];
     __shared__ float sl[2][32][33];
     if (P.st->any_fail) return;
     const int64_t task = blockIdx.x;
     const Job& jb = job_of(jobs, njobs, tmap, task);
     const int js = jb.node;
-    if (P.sn_bad[js] || node_off(P, js)) return;
+    const int64_t u = task - jb.task0;
+    const bool skip = P.sn_bad[js] || node_off(P, js);
+    if (u == 0 && threadIdx.x == 0) off[js] = skip;
+    if (__syncthreads_or(skip)) return;
     const int64_t np = tc::padded_rows(jb);
     const int nkb = tc::k_blocks(jb);
-    const int64_t u = task - jb.task0;
     const int kb = (int)(u % nkb);
     const int rb = (int)(u / nkb);
     const int ld = P.buf_ld[js];
@@ -253,7 +259,7 @@ __global__ void __launch_bounds__(256) k_split_tc(const Job* jobs, int64_t njobs
 // kChunk K blocks; between chunks the epilogue warps add the chunk into FP64
 // partial sums kept in tensor memory, and the last chunk goes to the front.
 __global__ void __launch_bounds__(tc::kThreads, 1)
-    k_gemm_tc(const Job* jobs, int64_t njobs, const int32_t* tmap, int64_t ntasks, PV P,
+    k_gemm_tc(const Job* jobs, int64_t njobs, const int32_t* tmap, int64_t ntasks, PV P, const int32_t* off,
               const __grid_constant__ CUtensorMap tm) {
     using namespace tc;
     extern __shared__ uint8_t tc_raw[];
@@ -294,7 +300,7 @@ __global__ void __launch_bounds__(tc::kThreads, 1)
         int64_t g = 0;
         for (int64_t task = blockIdx.x; task < ntasks && !*(volatile int*)&failed; task += gridDim.x) {
             const Job& jb = job_of(jobs, njobs, tmap, task);
-            if (P.sn_bad[jb.node] || node_off(P, jb.node)) continue;
+            if (off[jb.node]) continue;
             int it, jt;
             tile_of(task - jb.task0, (jb.c_end - jb.c0 + kTM - 1) / kTM, (jb.r_end - jb.c0 + kTM - 1) / kTM, it, jt);
             const int64_t np = padded_rows(jb);
@@ -326,7 +332,7 @@ __global__ void __launch_bounds__(tc::kThreads, 1)
         int64_t g = 0, h = 0;
         for (int64_t task = blockIdx.x; task < ntasks; task += gridDim.x) {
             const Job& jb = job_of(jobs, njobs, tmap, task);
-            if (P.sn_bad[jb.node] || node_off(P, jb.node)) continue;
+            if (off[jb.node]) continue;
             const int nkb = k_blocks(jb);
             bool stop = false;
             for (int c0 = 0; c0 < nkb && !stop; c0 += kChunk, ++h) {
@@ -377,7 +383,7 @@ __global__ void __launch_bounds__(tc::kThreads, 1)
         for (int64_t task = blockIdx.x; task < ntasks; task += gridDim.x) {
             const Job& jb = job_of(jobs, njobs, tmap, task);
             const int js = jb.node;
-            if (P.sn_bad[js] || node_off(P, js)) continue;
+            if (off[jb.node]) continue;
             int it, jt;
             tile_of(task - jb.task0, (jb.c_end - jb.c0 + kTM - 1) / kTM, (jb.r_end - jb.c0 + kTM - 1) / kTM, it, jt);
             const int i0 = jb.c0 + it * kTM, j0 = jb.c0 + jt * kTM;
