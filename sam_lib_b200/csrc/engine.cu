@@ -56,10 +56,12 @@ void trace_point(const char* what) {
 }
 
 
+// (the error is taken off the thread: after a failed allocation the next call starts clean)
 #define CK(x)                                                                    \
     do {                                                                         \
         cudaError_t e_ = (x);                                                    \
         if (e_ != cudaSuccess) {                                                 \
+            cudaGetLastError();                                                  \
             fprintf(stderr, "spr_b200: CUDA error %s at %s:%d\n",                \
                     cudaGetErrorString(e_), __FILE__, __LINE__);                 \
             return -4;                                                           \
@@ -5103,13 +5105,12 @@ int Engine::build_residual(const double* d_sm_assembled) {
     cudaStream_t s = stream_;
     PV pv = make_view(D, P_, const_cast<double*>(d_sm_assembled), 0.0);
     const int64_t neq = P_.neq;
-    // the row arrays and the scratch stay with the handle; the entry arrays grow
-    if (!csr_.rowptr) {
-        CK(cudaMalloc((void**)&csr_.rowptr, (neq + 1) * sizeof(int64_t)));
-        CK(cudaMalloc((void**)&csr_.fill, (neq + 1) * sizeof(int64_t)));
-        CK(cudaMalloc((void**)&csr_.cnt, neq * sizeof(int)));
-    }
+    // the row arrays and the scratch stay with the handle (each asked for by itself: an
+    // earlier call may have got some of them only); the entry arrays grow
     csr_.nnz = -1;                                       // no matrix until this one is complete
+    if (!csr_.rowptr) CK(cudaMalloc((void**)&csr_.rowptr, (neq + 1) * sizeof(int64_t)));
+    if (!csr_.fill) CK(cudaMalloc((void**)&csr_.fill, (neq + 1) * sizeof(int64_t)));
+    if (!csr_.cnt) CK(cudaMalloc((void**)&csr_.cnt, neq * sizeof(int)));
     CK(cudaMemsetAsync(csr_.cnt, 0, neq * sizeof(int), s));
     CK(cudaMemsetAsync(D.hbuf, 0, sizeof(unsigned long long), s));
     const int grid = (int)std::min<int64_t>((neq * 32 + 255) / 256, 16 * (int64_t)std::max(sm_count_, 1));
