@@ -3160,8 +3160,9 @@ __global__ void k_csr_rank(const int64_t* rowptr, int64_t neq, const int32_t* ci
             for (int64_t q = p0; q < p1; ++q) at += ci[q] < c;
             co[at] = c;
             vo[at] = cv[p];
-            sabs += fabs(cv[p]);
         }
+        __syncwarp();                                        // the sum in the columns' order
+        for (int64_t p = p0 + lane; p < p1; p += 32) sabs += fabs(vo[p]);
         for (int o = 16; o > 0; o >>= 1) sabs += __shfl_xor_sync(0xffffffffu, sabs, o);
         if (lane == 0 && sabs == sabs) atomicMax(norm, (unsigned long long)__double_as_longlong(sabs));
     }
