@@ -12,10 +12,22 @@
 // 0..7, i.e. 34 of the 49 digit products (the splitting of Ozaki, Ogita, Oishi
 // and Rump, "Error-free transformations of matrix multiplication by using fast
 // routines of matrix multiplication", 2012, with integer digits).
-// What is dropped is about 2^-61 2^(E_i+E_j) per term (E_i: the row's largest
-// entry), where the FP64 multiply-adds of k_gemm round every partial sum; with
-// levels 0..6 alone (28 products) it was 2^-56, and the factor's error against
-// an 80-bit factorisation came out up to 13 % larger than k_gemm's.
+// What is lost, per term of the sum unless said otherwise:
+//   operands  each rounded by up to 2^-56 2^E: 2^-56 (2^E_i |M_jk| + 2^E_j |M_ik|), at most
+//             2^-55 2^(E_i+E_j); the leading part
+//   levels    8 .. 12, left out: at most 2^-61.6 2^(E_i+E_j), typically 2^-64 (with levels 0 .. 6
+//             alone, 28 products, at most 2^-53.4, typically 2^-56, and the factor's error against
+//             an 80-bit factorisation came out up to 13 % larger than k_gemm's)
+//   sum       rounded once to FP64; before that its levels 6 and 7 to 2^-59 2^(E_i+E_j)
+// where the FP64 multiply-adds of k_gemm round every partial sum, by up to 2^-53 of its size.
+// The measure is the rows' scales and not a term's own size: an entry 2^-20 of its row's
+// largest keeps 35 bits, and two rows whose large entries lie in different columns have
+// a sum that is less accurate than k_gemm's relative to itself, though not to
+// |M_i| |M_j|, by which the update of the diagonal is rounded.  Measured: one update's
+// errors (root mean square) are 1/7, 1/15 and 1/26 of k_gemm's at K = 128, 512 and 1600, for
+// rows whose entries span six decades 1/3, 1/5 and 1/9; solutions against ones refined with
+// 80-bit residuals (16^3 to 48^3, shifted and not, 60 right-hand sides) 0.93 of those with
+// k_gemm alone (geometric mean).
 //
 // Two kernels per update:
 //   k_split_i8  forms the digits of a panel: slabs of 128-column blocks,
