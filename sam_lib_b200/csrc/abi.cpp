@@ -282,7 +282,7 @@ int ensure_b(Ctx* c, int64_t n) {
     if (c->d_b) cudaFree(c->d_b);
     c->d_b = nullptr;
     c->b_cap = 0;
-    if (cudaMalloc((void**)&c->d_b, n * sizeof(double)) != cudaSuccess) return -4;
+    if (c->eng.alloc((void**)&c->d_b, n * sizeof(double)) != cudaSuccess) return -4;
     c->b_cap = n;
     return 0;
 }
@@ -356,7 +356,8 @@ I do_factor(Ctx* c, I* mspar, double* sm, double* tol, I lpu, double* dcor = nul
         return -4;
     Engine::Singular fc3{0.0, nullptr};
     if (dcor) {
-        if (!c->d_dcor && cudaMalloc((void**)&c->d_dcor, 2 * std::max<int64_t>(neq, 1) * sizeof(double)) != cudaSuccess)
+        if (!c->d_dcor &&
+            c->eng.alloc((void**)&c->d_dcor, 2 * std::max<int64_t>(neq, 1) * sizeof(double)) != cudaSuccess)
             return -4;
         fc3.tol4 = tol[3];
         fc3.d_dcor = c->d_dcor;

@@ -3478,14 +3478,14 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
-static int make_slab(int64_t rows_needed, float** slab, CUtensorMap* map) {
+static int make_slab(Engine& eng, int64_t rows_needed, float** slab, CUtensorMap* map) {
     const int64_t rows = std::max<int64_t>(rows_needed, tc::kTM);
     if (rows >= (int64_t(1) << 31)) return -3;                 // TMA row coordinates are 32-bit
     void* fn = nullptr;
     cudaDriverEntryPointQueryResult q;
     if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q) != cudaSuccess || !fn)
         return -4;
-    CK(cudaMalloc((void**)slab, rows * tc::kBK * sizeof(float)));
+    CK(eng.alloc((void**)slab, rows * tc::kBK * sizeof(float)));
     const cuuint64_t dims[2] = {(cuuint64_t)tc::kBK, (cuuint64_t)rows};
     const cuuint64_t strides[1] = {(cuuint64_t)tc::kBK * sizeof(float)};
     const cuuint32_t box[2] = {(cuuint32_t)tc::kBK, (cuuint32_t)tc::kTM};
@@ -3504,12 +3504,12 @@ static int make_slab(int64_t rows_needed, float** slab, CUtensorMap* map) {
 int Engine::ensure_slabs() {
     Dev& D = *d_;
     if (D.slab && D.slab_far && D.tc_off) return 0;
-    if (!D.tc_off) CK(cudaMalloc((void**)&D.tc_off, 2 * P_.nsuper * sizeof(int32_t)));
+    if (!D.tc_off) CK(alloc((void**)&D.tc_off, 2 * P_.nsuper * sizeof(int32_t)));
     if (!D.slab) {
-        const int rc = make_slab(P_.slab_rows, &D.slab, &D.slab_map);
+        const int rc = make_slab(*this, P_.slab_rows, &D.slab, &D.slab_map);
         if (rc != 0) return rc;
     }
-    if (!D.slab_far) return make_slab(P_.slab_rows_far, &D.slab_far, &D.slab_map_far);
+    if (!D.slab_far) return make_slab(*this, P_.slab_rows_far, &D.slab_far, &D.slab_map_far);
     return 0;
 }
 
@@ -3550,6 +3550,27 @@ int Engine::ensure_i8() {
     }
     D.i8_slab = slab;
     return 0;
+}
+
+void Engine::release_i8() {
+    Dev& D = *d_;
+    for (auto& g : graphs_)
+        if (!g.key.b) cudaGraphExecDestroy(g.exec);              // factorisations captured on the slab
+    graphs_.erase(std::remove_if(graphs_.begin(), graphs_.end(), [](const GraphEntry& g) { return g.key.b == nullptr; }),
+                  graphs_.end());
+    cudaFree(D.i8_slab);
+    D.i8_slab = nullptr;
+}
+
+cudaError_t Engine::alloc(void** p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e != cudaSuccess && d_->i8_slab) {
+        cudaGetLastError();
+        release_i8();
+        e = cudaMalloc(p, bytes);
+    }
+    if (e != cudaSuccess) *p = nullptr;
+    return e;
 }
 
 static cudaEvent_t record_event(cudaStream_t s) {
@@ -4076,7 +4097,7 @@ int Engine::factor(double* d_sm, double tol1, FactorResult& res, const Singular*
             if (guard_copy_) cudaFree(guard_copy_);
             guard_copy_ = nullptr;
             guard_cap_ = 0;
-            CK(cudaMalloc((void**)&guard_copy_, nsm * sizeof(double)));
+            CK(alloc((void**)&guard_copy_, nsm * sizeof(double)));
             guard_cap_ = nsm;
         }
         CK(cudaMemcpyAsync(guard_copy_, d_sm, nsm * sizeof(double), cudaMemcpyDeviceToDevice, s));
@@ -4411,7 +4432,7 @@ int Engine::factor_streamed(double* h_sm, double* d_sm, double tol1, FactorResul
                 append(t->dranges[g], off, len);
             }
         }
-        if (nbackup > 0) CK(cudaMalloc((void**)&t->d_backup, nbackup * sizeof(double)));
+        if (nbackup > 0) CK(alloc((void**)&t->d_backup, nbackup * sizeof(double)));
         t->up.resize(ng);
         t->done.resize(ng);
         for (int g = 0; g < ng; ++g) {
@@ -4430,7 +4451,7 @@ int Engine::factor_streamed(double* h_sm, double* d_sm, double tol1, FactorResul
         for (int64_t js = 0; js < P_.nsuper; ++js)
             for (int64_t j = 0; j < P_.S[js]; ++j) t->diag_pos[P_.fst[js] + j] = P_.lnz_off[js] + lnz_col(j, P_.F[js]);
         CK(cudaMallocHost((void**)&t->h_diag, std::max<int64_t>(neq, 1) * sizeof(double)));
-        CK(cudaMalloc((void**)&t->d_diag, std::max<int64_t>(neq, 1) * sizeof(double)));
+        CK(alloc((void**)&t->d_diag, std::max<int64_t>(neq, 1) * sizeof(double)));
         xfer_ = std::move(t);
     }
     Transfer& t = *xfer_;
@@ -4610,10 +4631,12 @@ int64_t Engine::ensure_vectors(int64_t nrhs) {
         D.vbuf_rhs = 0;
         const int64_t nrp = (want + 3) / 4 * 4;
         const size_t d = sizeof(double);
-        if (cudaMalloc((void**)&D.vbuf, std::max<int64_t>(P_.rbase.back(), 1) * want * d) == cudaSuccess &&
-            cudaMalloc((void**)&D.ybuf, P_.neq * nrp * d) == cudaSuccess &&
-            cudaMalloc((void**)&D.pbuf, std::max<int64_t>(std::max(P_.rect_entries, P_.fwd_entries), 1) * nrp * d) ==
-                cudaSuccess) {
+        // (a narrower pass comes before the integer updates' slabs are given up)
+        auto get = [&](double** p, int64_t n) {
+            return (want > kMaxRHS ? cudaMalloc((void**)p, n * d) : alloc((void**)p, n * d)) == cudaSuccess;
+        };
+        if (get(&D.vbuf, std::max<int64_t>(P_.rbase.back(), 1) * want) && get(&D.ybuf, P_.neq * nrp) &&
+            get(&D.pbuf, std::max<int64_t>(std::max(P_.rect_entries, P_.fwd_entries), 1) * nrp)) {
             D.vbuf_rhs = want;
             return want;
         }
@@ -5109,9 +5132,9 @@ int Engine::build_residual(const double* d_sm_assembled) {
     // the row arrays and the scratch stay with the handle (each asked for by itself: an
     // earlier call may have got some of them only); the entry arrays grow
     csr_.nnz = -1;                                       // no matrix until this one is complete
-    if (!csr_.rowptr) CK(cudaMalloc((void**)&csr_.rowptr, (neq + 1) * sizeof(int64_t)));
-    if (!csr_.fill) CK(cudaMalloc((void**)&csr_.fill, (neq + 1) * sizeof(int64_t)));
-    if (!csr_.cnt) CK(cudaMalloc((void**)&csr_.cnt, neq * sizeof(int)));
+    if (!csr_.rowptr) CK(alloc((void**)&csr_.rowptr, (neq + 1) * sizeof(int64_t)));
+    if (!csr_.fill) CK(alloc((void**)&csr_.fill, (neq + 1) * sizeof(int64_t)));
+    if (!csr_.cnt) CK(alloc((void**)&csr_.cnt, neq * sizeof(int)));
     CK(cudaMemsetAsync(csr_.cnt, 0, neq * sizeof(int), s));
     CK(cudaMemsetAsync(D.hbuf, 0, sizeof(unsigned long long), s));
     const int grid = (int)std::min<int64_t>((neq * 32 + 255) / 256, 16 * (int64_t)std::max(sm_count_, 1));
@@ -5127,10 +5150,10 @@ int Engine::build_residual(const double* d_sm_assembled) {
         csr_.cv = csr_.cv2 = nullptr;
         csr_.cap = 0;
         const int64_t n = std::max<int64_t>(nnz, 1);
-        CK(cudaMalloc((void**)&csr_.ci, n * sizeof(int32_t)));
-        CK(cudaMalloc((void**)&csr_.cv, n * sizeof(double)));
-        CK(cudaMalloc((void**)&csr_.ci2, n * sizeof(int32_t)));
-        CK(cudaMalloc((void**)&csr_.cv2, n * sizeof(double)));
+        CK(alloc((void**)&csr_.ci, n * sizeof(int32_t)));
+        CK(alloc((void**)&csr_.cv, n * sizeof(double)));
+        CK(alloc((void**)&csr_.ci2, n * sizeof(int32_t)));
+        CK(alloc((void**)&csr_.cv2, n * sizeof(double)));
         csr_.cap = nnz;
     }
     k_csr_fill<<<grid, 256, 0, s>>>(pv, P_.nsuper, neq, csr_.fill, csr_.ci2, csr_.cv2);
@@ -5150,7 +5173,7 @@ int Engine::residual(const double* d_b, const double* d_x, double* d_r, int64_t 
         if (nbuf_) cudaFree(nbuf_);
         nbuf_ = nullptr;
         nbuf_cap_ = 0;
-        CK(cudaMalloc((void**)&nbuf_, 3 * nrhs * sizeof(double)));
+        CK(alloc((void**)&nbuf_, 3 * nrhs * sizeof(double)));
         nbuf_cap_ = 3 * nrhs;
     }
     double* norms = nbuf_;
@@ -5191,7 +5214,7 @@ int Engine::refine(const double* d_sm, const double* d_b, double* d_x, int64_t l
         if (rbuf_) cudaFree(rbuf_);
         rbuf_ = nullptr;
         rbuf_cap_ = 0;
-        CK(cudaMalloc((void**)&rbuf_, n * sizeof(double)));
+        CK(alloc((void**)&rbuf_, n * sizeof(double)));
         rbuf_cap_ = n;
     }
     (void)D;

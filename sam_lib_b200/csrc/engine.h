@@ -68,6 +68,9 @@ public:
     int open(const int64_t* mspar, const int64_t* mtrees, const int64_t* msifa);
     const Plan& plan() const { return P_; }
     void set_stream(cudaStream_t s) { stream_ = s; }
+    // device memory; where there is none left, the digit slabs of the integer
+    // updates, which the factorisation can do without, are given up for it
+    cudaError_t alloc(void** p, size_t bytes);
     // least flops of a launch whose FP64 update runs on the integer tensor cores
     void set_int_min(double flops);
     cudaStream_t stream() const { return stream_; }
@@ -247,6 +250,7 @@ private:
     bool any_i8_ = false;         // the plan has such an update
     bool use_i8_ = false;         // and this factorisation runs them so
     int ensure_i8();
+    void release_i8();
     void launch_i8_split(const I8Launch& t, cudaStream_t s, const struct PV& pv, std::vector<cudaEvent_t>& gev);
     void launch_i8_gemm(const Launch& l, cudaStream_t s, const struct PV& pv, std::vector<cudaEvent_t>& gev, bool far);
     struct Csr {

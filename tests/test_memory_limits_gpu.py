@@ -88,3 +88,51 @@ def test_residual_after_an_allocation_that_failed(pages):
     assert np.allclose(d_x.cpu().numpy()[0], 1.0 / sm[neq:], rtol=1e-14)
     ds.close()
     warm.close()
+
+
+@pytest.mark.parametrize('own_stream', [False, True])
+def test_solves_take_the_place_of_the_digit_slabs(own_stream):
+    """20^3: the factorisation has its digit slabs and nothing is left.  Solves and
+    refinement go on, in their place; the factorisation that follows
+    does without them, and has them again when there is memory."""
+    import contextlib
+    import torch
+    import sam_lib_b200 as spr
+    from sam_lib_b200.system import HexSystem
+    hs = HexSystem(20)
+    sm = torch.from_numpy(hs.assemble()).cuda()
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stream) if own_stream else contextlib.nullcontext():
+        b0 = torch.from_numpy(np.random.default_rng(1).uniform(-1.0, 1.0, size=(2, hs.neq))).cuda()
+        d, x, y, first = sm.clone(), b0.clone(), torch.empty_like(b0), b0.clone()
+        warm = spr.DeviceSolver(hs.mspar, hs.mtrees, hs.msifa)   # the kernels are loaded
+        ds = spr.DeviceSolver(hs.mspar, hs.mtrees, hs.msifa)
+        if own_stream:
+            ds.set_stream(stream.cuda_stream)
+            warm.set_stream(stream.cuda_stream)
+        warm.build_residual(sm)
+        warm.factor(d)
+        launches = warm.info()['launches']
+        warm.solve(d, first, 2)
+        warm.close()
+        d.copy_(sm)
+        assert ds.factor(d)['lierr'] == 0 and ds.info()['launches'] == launches
+        ds.build_residual(sm)
+        filler = Filler()
+        try:
+            ds.solve(d, x, 2)                                # the slabs go
+            assert torch.equal(x, first)
+            d.copy_(sm)
+            assert ds.factor(d)['lierr'] == 0
+            assert ds.refine(d, b0, y, 2, tol=1e-30, maxit=0)[1] <= 1e-13
+            for r in ds.factor(d.copy_(sm)), ds.factor(d.copy_(sm)):
+                assert r['lierr'] == 0
+        finally:
+            filler.close()
+        d.copy_(sm)
+        assert ds.factor(d)['lierr'] == 0 and ds.info()['launches'] == launches
+        x.copy_(b0)
+        ds.solve(d, x, 2)
+        assert torch.equal(x, first)
+        ds.close()
