@@ -226,15 +226,26 @@ int spr_b200_set_profile(void* handle, int on);
  * the mixed mode's launch lists. */
 int spr_b200_plan_check(const SPR_INT* mspar, const SPR_INT* mtrees, const SPR_INT* msifa,
                         double* out);
-/* Host-only race check of the factorisation's three-stream launch schedule (no
- * GPU needed): happens-before of panels, panel-chain, look-ahead, far and K = S
- * updates and the write-back.  out (6 doubles): [0] ordering violations of the
+/* Host-only race check of the factorisation's launch schedule on its four streams
+ * (no GPU needed): happens-before of small fronts, panels, panel-chain, look-ahead, far and
+ * K = S updates and the write-back, and of the fronts' memory over the levels, without
+ * integer updates.  out (6 doubles): [0] ordering violations of the
  * FP64 schedule [1] of the schedule with tensor-core far and K = S updates
  * [2] of the FP64 schedule without its side-stream joins (a self-test; > 0
  * when [3] > 0) [3] far launches [4] of the FP64 schedule without its
  * look-ahead joins (> 0 when [5] > 0) [5] look-ahead launches. */
 int spr_b200_schedule_check(const SPR_INT* mspar, const SPR_INT* mtrees, const SPR_INT* msifa,
                             double* out);
+/* The same for one form of the factorisation: mixed = 0 or 1; FP64 launches of at
+ * least int_min flops on the integer tensor cores (see spr_b200_set_int_min);
+ * skip = joins left out, a sum of 1 (far updates), 2 (look-ahead updates), 8
+ * (write-back) and 16 (small fronts), and 4 for a digit split put before the join
+ * of the far launch that still reads its slab.  out (4 doubles): [0] ordering
+ * violations [1] splits that take the digit slab of a far launch on the side stream
+ * [2] fronts whose memory a later front takes [3] levels with small fronts on other
+ * streams. */
+int spr_b200_schedule_replay(const SPR_INT* mspar, const SPR_INT* mtrees, const SPR_INT* msifa,
+                             int mixed, double int_min, int skip, double* out);
 /* No reference counterpart.  Host-only self-check of the solves' plan (no GPU
  * needed): each eliminated large front's 64-row triangle blocks are tasks of
  * its level's dataflow launch, once each and after the block above, with

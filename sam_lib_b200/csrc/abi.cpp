@@ -21,6 +21,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <limits>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -1178,10 +1179,11 @@ int SPR_API(spr_b200_schedule_check)(const I* mspar, const I* mtrees, const I* m
     const int rc = sprb::build_plan(ms.data(), mt.data(), mf.data(), p);
     for (int i = 0; i < 6; ++i) out[i] = 0.0;
     if (rc != 0) return rc;
-    out[0] = (double)sprb::check_schedule(p, false, 0);
-    out[1] = (double)sprb::check_schedule(p, true, 0);
-    out[2] = (double)sprb::check_schedule(p, false, 1);
-    out[4] = (double)sprb::check_schedule(p, false, 2);
+    const double none = std::numeric_limits<double>::infinity();
+    out[0] = (double)sprb::check_schedule(p, false, none, 0);
+    out[1] = (double)sprb::check_schedule(p, true, none, 0);
+    out[2] = (double)sprb::check_schedule(p, false, none, sprb::kSkipFar);
+    out[4] = (double)sprb::check_schedule(p, false, none, sprb::kSkipAhead);
     int64_t nfar = 0, nahead = 0;
     for (const auto& lp : p.levels) {
         for (const auto& v : lp.far) nfar += (int64_t)v.size();
@@ -1189,6 +1191,28 @@ int SPR_API(spr_b200_schedule_check)(const I* mspar, const I* mtrees, const I* m
     }
     out[3] = (double)nfar;
     out[5] = (double)nahead;
+    return 0;
+}
+
+// Host-only race check of one form of the factorisation (no GPU needed): mixed = 0 or
+// 1, int_min as in spr_b200_set_int_min, skip = the joins left out (plan.h, SchedSkip).
+// out[0] = ordering violations, out[1] = splits that take the digit slab of a far launch
+// on the side stream, out[2] = fronts whose memory a later front takes, out[3] = levels
+// with small fronts on other streams.
+int SPR_API(spr_b200_schedule_replay)(const I* mspar, const I* mtrees, const I* msifa, int mixed, double int_min, int skip,
+                                      double* out) {
+    std::vector<int64_t> ms(60, 0);
+    for (int i = 0; i < 58; ++i) ms[i] = (int64_t)mspar[i];
+    std::vector<int64_t> mt = widen(mtrees, mspar[3]), mf = widen(msifa, mspar[2]);
+    sprb::Plan p;
+    const int rc = sprb::build_plan(ms.data(), mt.data(), mf.data(), p);
+    for (int i = 0; i < 4; ++i) out[i] = 0.0;
+    if (rc != 0) return rc;
+    sprb::SchedCounts n;
+    out[0] = (double)sprb::check_schedule(p, mixed != 0, int_min, skip, &n);
+    out[1] = (double)n.slab_shared;
+    out[2] = (double)n.reused;
+    out[3] = (double)n.small_beside;
     return 0;
 }
 

@@ -792,37 +792,167 @@ void check_coverage(const Plan& P, int64_t& fp64, int64_t& tc) {
 // ---------------------------------------------------------------------------
 // Stream-schedule check of the factorisation (a race detector on the host).
 //
-// Replays the launch order of the factorisation of every level: per panel
+// Replays the launch order of a factorisation without hooks, all levels in turn, on
+// four streams.  Per level: the small fronts by size classes on the side and
+// the look-ahead stream (the first on the main one where there is no large
+// front), joined at the level's end; the assembly of the large ones; per panel
 // step the TRSM, the update of the next panel's columns by this panel and the
 // one before and the next diagonal block on the main stream; inside a
 // super-panel the update of the columns after the next two panels on the
 // look-ahead stream, forked by an event after the step and joined before the
-// step after the next; at the end of a
-// super-panel the far columns' update on the side stream, forked by an event
-// after the step's TRSM and joined before the next trailing update (every
-// kSuperPanel / kNB steps) and before the K = S update.  Vector clocks give
-// the happens-before order of the three streams.  Per large front it counts
+// step after the next; at the end of a super-panel the far columns' update on
+// the side stream, forked by an event after the step's TRSM (as integer-digit
+// update: after the split, whose slab the far launch shares) and joined before the next
+// trailing update (every kSuperPanel / kNB steps) and before the K = S update; the
+// write-back on a stream of its own, joined two levels later.  Vector clocks give
+// the happens-before order.  Per large front it counts
 //   * a panel whose columns have not received exactly the K ranges [0, k0)
 //     from updates ordered before it, or that an unordered update writes;
 //   * an update whose K panel columns are not final (diagonal block + TRSM
 //     ordered before it);
 //   * two updates on different streams that write a common element unordered;
-//   * an update of the S columns not ordered before the write-back.
-// tc: the far and K = S updates take the tensor-core path (split + product on
-// the same stream as the FP64 launch they replace).  skip_join drops joins
-// (bit 0: the far updates', bit 1: the look-ahead updates'), which must make
-// the check fail wherever such launches exist.
+//   * an update of the S columns not ordered before the write-back;
+// and over all of the factorisation
+//   * a child's update block read before its last write;
+//   * a buffer written while a launch on the front that had the memory before is
+//     unordered with it, or such a launch issued later;
+//   * a digit slab written while a product that reads it is unordered with the
+//     split, or read by a product that its own split does not precede.
+// (The copy of the next panel's rows in the fronts' upper triangles is written and
+// read on the main stream alone.  With hooks the small fronts and the write-back are on
+// the main stream as well.)
 // ---------------------------------------------------------------------------
 namespace {
-constexpr int kStreams = 3;          // 0 main, 1 side (far columns), 2 look-ahead
+constexpr int kStreams = 4;          // 0 main, 1 side (far columns), 2 look-ahead, 3 write-back
+struct Clock {
+    int64_t t[kStreams] = {};
+};
 struct SchedOp {
     int stream;
-    int64_t vc[kStreams];            // vector clock after the op
+    Clock vc;                        // vector clock after the op
     int32_t c0, c_end, r0, r_end;    // written block (columns, rows)
     int32_t k_lo, k_hi;              // K range applied (updates)
     int kind;                        // 0 panel, 1 update, 2 write-back
 };
-bool hb(const SchedOp& a, const SchedOp& b) { return a.vc[a.stream] <= b.vc[a.stream]; }
+bool hb(const SchedOp& a, const SchedOp& b) { return a.vc.t[a.stream] <= b.vc.t[a.stream]; }
+
+struct Replay {
+    const Plan& P;
+    int64_t bad = 0, reused = 0;
+    Clock vc[kStreams];                                // per stream
+    std::vector<Clock> touched, written;             // per front: last launch of each stream that reads or writes its buffer / writes it
+    std::vector<uint8_t> gone;                       // its memory has another front's data
+    std::map<int64_t, std::pair<int64_t, int32_t>> room;   // arena: first double -> (end, front)
+    std::map<int32_t, std::vector<SchedOp>> ops;     // of the level's large fronts, in issue order
+
+    explicit Replay(const Plan& p) : P(p), touched(p.nsuper), written(p.nsuper), gone(p.nsuper, 0) {}
+    void wait(int dst, const Clock& ev) {
+        for (int q = 0; q < kStreams; ++q) vc[dst].t[q] = std::max(vc[dst].t[q], ev.t[q]);
+    }
+    bool after(int stream, const Clock& last) const {
+        for (int q = 0; q < kStreams; ++q)
+            if (last.t[q] > vc[stream].t[q]) return false;
+        return true;
+    }
+    void tick(int stream) { ++vc[stream].t[stream]; }
+    void touch(int32_t js, int stream, bool write) {
+        if (gone[js]) ++bad;
+        touched[js].t[stream] = vc[stream].t[stream];
+        if (write) written[js].t[stream] = vc[stream].t[stream];
+    }
+    // a front's first launch: its memory, and its children's update blocks
+    void begin(int32_t js, int stream) {
+        const int64_t lo = P.buf_off[js], hi = lo + buffer_doubles(P, js);
+        if (hi > lo) {
+            auto it = room.upper_bound(lo);
+            if (it != room.begin() && std::prev(it)->second.first > lo) --it;
+            while (it != room.end() && it->first < hi) {
+                const int64_t from = it->first, to = it->second.first;
+                const int32_t was = it->second.second;
+                if (!gone[was]) ++reused;
+                if (!after(stream, touched[was])) ++bad;
+                gone[was] = 1;
+                it = room.erase(it);
+                if (from < lo) room[from] = {lo, was};
+                if (to > hi) it = room.emplace(hi, std::make_pair(to, was)).first;
+            }
+            room[lo] = {hi, js};
+        }
+        for (int32_t k = P.child_ptr[js]; k < P.child_ptr[js + 1]; ++k) {
+            const int32_t c = P.child[k];
+            if (P.F[c] <= P.S[c]) continue;
+            if (!after(stream, written[c])) ++bad;
+            touch(c, stream, false);
+        }
+        touch(js, stream, true);
+    }
+    void issue(int stream, const Job& j, int kind) {
+        SchedOp o;
+        o.stream = stream;
+        o.vc = vc[stream];
+        o.kind = kind;
+        o.k_lo = j.k_lo;
+        o.k_hi = j.k_hi;
+        o.c0 = o.r0 = kind == 0 ? j.k_lo : kind == 1 ? j.c0 : 0;     // a panel: columns [k_lo, k_hi), rows to F
+        o.c_end = kind == 0 ? j.k_hi : j.c_end;
+        o.r_end = j.r_end;
+        ops[j.node].push_back(o);
+        touch(j.node, stream, kind != 2);
+    }
+    void launch(int stream, const Launch& l, int kind) {
+        tick(stream);
+        for (int64_t k = 0; k < l.job_count; ++k) issue(stream, P.jobs[l.job_begin + k], kind);
+    }
+    void fronts();
+};
+
+// the order of the launches on each of a level's large fronts
+void Replay::fronts() {
+    for (auto& kv : ops) {
+        const std::vector<SchedOp>& v = kv.second;
+        for (size_t a = 0; a < v.size(); ++a) {
+            const SchedOp& A = v[a];
+            if (A.kind == 0) {
+                // columns [k0, k0 + nb): K coverage [0, k0) from updates ordered before
+                for (int32_t c = A.c0; c < A.c_end; ++c) {
+                    std::vector<std::pair<int32_t, int32_t>> iv;
+                    for (const SchedOp& U : v) {
+                        if (U.kind != 1 || c < U.c0 || c >= U.c_end) continue;
+                        if (!hb(U, A)) {
+                            ++bad;
+                            continue;
+                        }
+                        iv.emplace_back(U.k_lo, U.k_hi);
+                    }
+                    std::sort(iv.begin(), iv.end());
+                    int32_t at = 0;
+                    bool ok = true;
+                    for (const auto& x : iv) {
+                        if (x.first != at) ok = false;
+                        at = x.second;
+                    }
+                    if (!ok || at != A.c0) ++bad;
+                }
+            } else if (A.kind == 1) {
+                // its K panel columns are final before it
+                for (const SchedOp& Q : v)
+                    if (Q.kind == 0 && Q.c0 < A.k_hi && A.k_lo < Q.c_end && !hb(Q, A)) ++bad;
+                // no unordered writer of a common element on another stream
+                for (size_t b = a + 1; b < v.size(); ++b) {
+                    const SchedOp& B = v[b];
+                    if (B.kind != 1 || B.stream == A.stream) continue;
+                    const bool cols = A.c0 < B.c_end && B.c0 < A.c_end;
+                    const bool rows = A.r0 < B.r_end && B.r0 < A.r_end;
+                    if (cols && rows && !hb(A, B) && !hb(B, A)) ++bad;
+                }
+            } else {
+                for (const SchedOp& U : v)
+                    if (U.kind == 1 && U.c0 < A.c_end && !hb(U, A)) ++bad;
+            }
+        }
+    }
+    ops.clear();
+}
 }  // namespace
 
 // number of tasks of job j of launch l
@@ -960,149 +1090,149 @@ int64_t check_solve_plan(const Plan& P, int plant, int64_t* tasks) {
     return bad;
 }
 
-int64_t check_schedule(const Plan& P, bool tc, int skip_join) {
-    int64_t bad = 0;
-    for (const LevelPlan& lp : P.levels) {
-        if (lp.elim_nodes.empty()) continue;
-        std::map<int32_t, std::vector<SchedOp>> ops;     // per front, in issue order
-        int64_t vc[kStreams][kStreams] = {};            // per stream: its vector clock
-        int64_t far_done[kStreams], ahead_done[2][kStreams];
-        bool far_open = false, ahead_open[2] = {false, false};
-        auto issue = [&](int stream, const Job& j, int kind) {
-            ++vc[stream][stream];
-            SchedOp o;
-            o.stream = stream;
-            for (int q = 0; q < kStreams; ++q) o.vc[q] = vc[stream][q];
-            o.kind = kind;
-            o.k_lo = j.k_lo;
-            o.k_hi = j.k_hi;
-            if (kind == 0) {                              // panel: columns [k_lo, k_hi), rows to F
-                o.c0 = j.k_lo;
-                o.c_end = j.k_hi;
-                o.r0 = j.k_lo;
-                o.r_end = j.r_end;
-            } else if (kind == 1) {
-                o.c0 = j.c0;
-                o.c_end = j.c_end;
-                o.r0 = j.c0;
-                o.r_end = j.r_end;
-            } else {
-                o.c0 = 0;
-                o.c_end = j.c_end;
-                o.r0 = 0;
-                o.r_end = j.r_end;
-            }
-            ops[j.node].push_back(o);
+int64_t check_schedule(const Plan& P, bool tc, double int_min, int skip, SchedCounts* counts) {
+    constexpr size_t kSteps = kSuperPanel / kNB;
+    Replay R(P);
+    SchedCounts n;
+    Clock far_done, ahead_done[2], wb_done[2];
+    bool far_open = false, ahead_open[2] = {false, false}, wb_open[2] = {false, false};
+    bool far_digits = false;                             // the open far launch reads the digit slab
+    auto join_far = [&]() {
+        if (far_open && !(skip & kSkipFar)) R.wait(0, far_done);
+        far_open = false;
+    };
+    auto join_ahead = [&](size_t st) {
+        if (ahead_open[st & 1] && !(skip & kSkipAhead)) R.wait(0, ahead_done[st & 1]);
+        ahead_open[st & 1] = false;
+    };
+    // the digit slab: its split, that split's place on the main stream, its readers
+    const I8Launch* slab_of = nullptr;
+    int64_t slab_at = 0;
+    Clock slab_read;
+    auto split = [&](const I8Launch& t) {
+        R.tick(0);
+        for (int64_t k = 0; k < t.split.job_count; ++k) R.touch(P.jobs[t.split.job_begin + k].node, 0, false);
+        if (!R.after(0, slab_read)) ++R.bad;
+        slab_of = &t;
+        slab_at = R.vc[0].t[0];
+    };
+    auto product = [&](int stream, const I8Launch& t, const Launch& l) {
+        R.launch(stream, l, 1);
+        if (slab_of != &t || slab_at > R.vc[stream].t[0]) ++R.bad;
+        slab_read.t[stream] = R.vc[stream].t[stream];
+    };
+    for (size_t L = 0; L < P.levels.size(); ++L) {
+        const LevelPlan& lp = P.levels[L];
+        if (wb_open[L & 1] && !(skip & kSkipWriteback)) R.wait(0, wb_done[L & 1]);
+        wb_open[L & 1] = false;
+        // small fronts
+        const int small[2] = {lp.large_nodes.empty() ? 0 : 1, lp.small_classes.size() > 1 ? 2 : 0};
+        const bool beside = !lp.small_classes.empty() && (small[0] || small[1]);
+        n.small_beside += beside;
+        if (!lp.small_classes.empty())
+            for (int t : small) R.wait(t, R.vc[0]);
+        for (size_t c = 0; c < lp.small_classes.size(); ++c) {
+            R.tick(small[c & 1]);
+            for (int32_t k = 0; k < lp.small_classes[c].count; ++k)
+                R.begin(lp.small_nodes[lp.small_classes[c].begin + k], small[c & 1]);
+        }
+        auto join_small = [&]() {
+            if (beside && !(skip & kSkipSmall))
+                for (int t : small) R.wait(0, R.vc[t]);
         };
-        auto issue_launch = [&](int stream, const Launch& l, int kind) {
-            for (int64_t k = 0; k < l.job_count; ++k) issue(stream, P.jobs[l.job_begin + k], kind);
-        };
-        auto wait = [&](int dst, const int64_t* ev) {       // dst waits for an event
-            for (int q = 0; q < kStreams; ++q) vc[dst][q] = std::max(vc[dst][q], ev[q]);
-        };
-        auto record = [&](int src, int64_t* ev) {
-            for (int q = 0; q < kStreams; ++q) ev[q] = vc[src][q];
-        };
-        auto join = [&]() {
-            if (far_open && !(skip_join & 1)) wait(0, far_done);
-            far_open = false;
-        };
-        auto join_ahead = [&](size_t st) {
-            if (ahead_open[st & 1] && !(skip_join & 2)) wait(0, ahead_done[st & 1]);
-            ahead_open[st & 1] = false;
-        };
+        if (lp.large_nodes.empty()) {
+            join_small();
+            continue;
+        }
+        // large fronts
+        R.tick(0);
+        for (int32_t js : lp.large_nodes) R.begin(js, 0);
         for (size_t st = 0; st < lp.panel.size(); ++st) {
             // a super-panel's first diagonal block, then the TRSM, the next panel's columns
             // and its diagonal block
             const Launch& pl = lp.panel[st];
-            constexpr size_t kSteps = kSuperPanel / kNB;
-            if (st % kSteps == 0) issue_launch(0, pl, 0);
+            const bool chain = (st + 1) % kSteps != 0;
+            if (st % kSteps == 0) R.launch(0, pl, 0);
             join_ahead(st);
-            issue_launch(0, pl, 0);
-            if ((st + 1) % kSteps != 0)
+            R.launch(0, pl, 0);
+            if (chain)
                 for (int64_t k = 0; k < pl.job_count; ++k) {
                     const Job c = chain_update(P, P.jobs[pl.job_begin + k]);
                     if (c.c0 >= c.c_end) continue;
-                    issue(0, c, 1);
+                    R.tick(0);
+                    R.issue(0, c, 1);
                     Job d = c;
                     d.k_lo = c.c0;
                     d.k_hi = c.c_end;
-                    issue(0, d, 0);
+                    R.tick(0);
+                    R.issue(0, d, 0);
                 }
-            const bool has_far = tc ? !lp.far_tc[st].empty() : !lp.far[st].empty();
-            if (has_far) wait(1, vc[0]);                 // fork after the step's TRSM
-            if ((st + 1) % kSteps == 0) join();
-            int64_t fork[kStreams];
-            record(0, fork);
-            for (const Launch& ul : lp.update[st]) issue_launch(0, ul, 1);
+            const bool has_far = !lp.far[st].empty() || !lp.far_tc[st].empty();
+            const I8Launch& t = lp.trail_i8[st];
+            const bool digits = !tc && t.gemm.ntasks > 0 && t.flops >= int_min;
+            if (has_far && !digits) R.wait(1, R.vc[0]);  // fork after the step's TRSM
+            n.slab_shared += digits && far_open && far_digits;
+            if (digits && (skip & kSkipSlab)) split(t);
+            if (!chain) join_far();
+            const Clock fork = R.vc[0];
+            if (digits) {
+                if (!(skip & kSkipSlab)) split(t);
+                if (has_far) R.wait(1, R.vc[0]);
+                product(0, t, t.gemm);
+                for (const Launch& ul : t.rest) R.launch(0, ul, 1);
+            } else {
+                for (const Launch& ul : lp.update[st]) R.launch(0, ul, 1);
+            }
             if (!lp.ahead[st].empty()) {
-                wait(2, fork);
-                for (const Launch& al : lp.ahead[st]) issue_launch(2, al, 1);
-                record(2, ahead_done[st & 1]);
+                R.wait(2, fork);
+                for (const Launch& al : lp.ahead[st]) R.launch(2, al, 1);
+                ahead_done[st & 1] = R.vc[2];
                 ahead_open[st & 1] = true;
             }
             if (has_far) {
-                if (tc)
-                    for (const TcLaunch& t : lp.far_tc[st]) issue_launch(1, t.gemm, 1);
-                else
-                    for (const Launch& fl : lp.far[st]) issue_launch(1, fl, 1);
-                record(1, far_done);
+                far_digits = digits && t.far.ntasks > 0;
+                if (digits) {
+                    if (far_digits) product(1, t, t.far);
+                    for (const Launch& fl : t.far_rest) R.launch(1, fl, 1);
+                } else if (tc) {
+                    for (const TcLaunch& f : lp.far_tc[st]) R.launch(1, f.gemm, 1);
+                } else {
+                    for (const Launch& fl : lp.far[st]) R.launch(1, fl, 1);
+                }
+                far_done = R.vc[1];
                 far_open = true;
             }
         }
         join_ahead(0);
         join_ahead(1);
-        join();
-        if (tc)
-            for (const TcLaunch& t : lp.outer_tc) issue_launch(0, t.gemm, 1);
-        else
-            for (const Launch& ol : lp.outer) issue_launch(0, ol, 1);
-        for (int32_t js : lp.elim_nodes) issue(0, Job{js, 0, P.S[js], P.F[js], 0, 0, 0}, 2);
-        for (auto& kv : ops) {
-            const std::vector<SchedOp>& v = kv.second;
-            for (size_t a = 0; a < v.size(); ++a) {
-                const SchedOp& A = v[a];
-                if (A.kind == 0) {
-                    // columns [k0, k0 + nb): K coverage [0, k0) from updates ordered before
-                    for (int32_t c = A.c0; c < A.c_end; ++c) {
-                        std::vector<std::pair<int32_t, int32_t>> iv;
-                        for (const SchedOp& U : v) {
-                            if (U.kind != 1 || c < U.c0 || c >= U.c_end) continue;
-                            if (!hb(U, A)) {
-                                ++bad;
-                                continue;
-                            }
-                            iv.emplace_back(U.k_lo, U.k_hi);
-                        }
-                        std::sort(iv.begin(), iv.end());
-                        int32_t at = 0;
-                        bool ok = true;
-                        for (const auto& x : iv) {
-                            if (x.first != at) ok = false;
-                            at = x.second;
-                        }
-                        if (!ok || at != A.c0) ++bad;
-                    }
-                } else if (A.kind == 1) {
-                    // its K panel columns are final before it
-                    for (const SchedOp& Q : v)
-                        if (Q.kind == 0 && Q.c0 < A.k_hi && A.k_lo < Q.c_end && !hb(Q, A)) ++bad;
-                    // no unordered writer of a common element on the other stream
-                    for (size_t b = a + 1; b < v.size(); ++b) {
-                        const SchedOp& B = v[b];
-                        if (B.kind != 1 || B.stream == A.stream) continue;
-                        const bool cols = A.c0 < B.c_end && B.c0 < A.c_end;
-                        const bool rows = A.r0 < B.r_end && B.r0 < A.r_end;
-                        if (cols && rows && !hb(A, B) && !hb(B, A)) ++bad;
-                    }
-                } else {
-                    for (const SchedOp& U : v)
-                        if (U.kind == 1 && U.c0 < A.c_end && !hb(U, A)) ++bad;
-                }
-            }
+        join_far();
+        R.wait(3, R.vc[0]);
+        R.tick(3);
+        for (int32_t js : lp.large_nodes) {
+            if (P.retained[js]) R.touch(js, 3, false);
+            else R.issue(3, Job{js, 0, P.S[js], P.F[js], 0, 0, 0}, 2);
         }
+        wb_done[L & 1] = R.vc[3];
+        wb_open[L & 1] = true;
+        if (tc) {
+            for (const TcLaunch& t : lp.outer_tc) R.launch(0, t.gemm, 1);
+        } else if (!lp.outer_i8.empty() && lp.outer_i8[0].flops >= int_min) {
+            for (const I8Launch& t : lp.outer_i8) {
+                if (t.gemm.ntasks > 0) {
+                    split(t);
+                    product(0, t, t.gemm);
+                }
+                for (const Launch& ol : t.rest) R.launch(0, ol, 1);
+            }
+        } else {
+            for (const Launch& ol : lp.outer) R.launch(0, ol, 1);
+        }
+        join_small();
+        R.fronts();
     }
-    return bad;
+    n.reused = R.reused;
+    if (counts) *counts = n;
+    return R.bad;
 }
 
 uint64_t sm_hash_host(const double* a, int64_t n, int threads) {

@@ -227,12 +227,21 @@ void check_plan(const Plan& P, int64_t& oob, int64_t& overlaps);
 // do not, for the FP64 launch lists (fp64) and the tensor-core lists in the
 // mixed mode's use (tc: FP64 panel-chain updates + tensor-core far and K = S).
 void check_coverage(const Plan& P, int64_t& fp64, int64_t& tc);
-// Happens-before check of the factorisation's two-stream launch schedule
-// (panels, panel-chain and far updates, K = S update, write-back): the number
-// of ordering violations, 0 for a race-free schedule.  tc: the far and K = S
-// updates on the tensor-core path; skip_join: the schedule without its
-// side-stream joins (a self-test: must report violations where far launches exist).
-int64_t check_schedule(const Plan& P, bool tc, int skip_join);
+// Happens-before check of the factorisation's launch schedule on its four streams
+// (small fronts, panels, look-ahead and far updates, K = S update, write-back), of
+// the fronts' memory over the levels and of the integer updates' digit slab: the number of
+// ordering violations, 0 for a race-free schedule.  tc: the far and K = S
+// updates on the tensor-core path; int_min: launches of at least this many flops as
+// integer-digit updates (infinity: none).  skip leaves out joins, or puts a split before
+// the join of the far launch that still reads the slab (self-tests: must report
+// violations where there is such a launch, see SchedCounts).
+enum SchedSkip { kSkipFar = 1, kSkipAhead = 2, kSkipSlab = 4, kSkipWriteback = 8, kSkipSmall = 16 };
+struct SchedCounts {
+    int64_t slab_shared = 0;         // splits that take the slab of a far launch on the side stream
+    int64_t reused = 0;              // fronts whose memory a later front takes
+    int64_t small_beside = 0;        // levels with small fronts on other streams
+};
+int64_t check_schedule(const Plan& P, bool tc, double int_min, int skip, SchedCounts* counts = nullptr);
 // Self-check of the solves' plan: every eliminated large front of a level has
 // each of its 64-row triangle blocks as one task of that level's dataflow
 // launch, after the task of the block above it (the forward sweep takes them
