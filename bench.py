@@ -70,6 +70,15 @@ def config(n=N_MESH):
 # ---------------------------------------------------------------------------
 # CPU: the reference SPR path on a bounded sample (oracle build; baseline only)
 # ---------------------------------------------------------------------------
+def reference_missing():
+    """Why the reference cannot run here (one line), or None."""
+    from oracle.refpipe import LIB_PATH
+    if os.path.exists(LIB_PATH):
+        return None
+    return ('%s is not built: it is translated from the reference\'s SPR sources, which are not here' %
+            os.path.relpath(LIB_PATH, ROOT))
+
+
 def _cpu_worker(args):
     n, reps = args
     from oracle.refpipe import RefSystem
@@ -609,6 +618,10 @@ def run_reference(args, rank, world):
     all-core aggregate of independent sample systems (one process per core)."""
     if rank != 0:
         return
+    missing = reference_missing()
+    if missing:
+        print(json.dumps({'impl': 'reference', 'unavailable': missing}), flush=True)
+        return
     ladder = []
     for n in (12, 16, 20, 24):
         nn, neq, r3, dt = _ladder_worker(n)
@@ -653,8 +666,10 @@ def _cpu_model():
 def run_ours(args, rank, world, local_rank):
     from sam_lib_b200.replicas import max_over_ranks, whole_job_rate
     # CPU baseline first (rank 0, N=1 only), before the GPU is touched
-    cpu = None
-    if rank == 0 and world == 1 and not args.no_cpu:
+    cpu, missing = None, reference_missing()
+    if missing:
+        cpu = {'unavailable': missing}
+    elif rank == 0 and world == 1 and not args.no_cpu:
         flops_s, times = cpu_sample(1, 1)
         t = times[0][0]
         cpu = {'value': flops_s / t / 1e9, 'unit': UNIT, 'cores': 1, 'kind': 'reference',
@@ -783,10 +798,11 @@ def run_ours(args, rank, world, local_rank):
         if rank == 0:
             forms = {'batched_sharded': bs}
     if rank == 0 and world == 1 and not args.no_forms and args.n == N_MESH:
-        forms = {'mixed_ir_vs_reference_cpu': form_mixed_vs_reference(torch, spr),
+        forms = {'mixed_ir_vs_reference_cpu': ({'unavailable': missing} if missing else
+                                               form_mixed_vs_reference(torch, spr)),
                  'mixed_ir_loguniform': form_mixed_ir(torch, spr, N_MESH, 'loguniform'),
                  'mixed_ir_uniform': form_mixed_ir(torch, spr, N_MESH, 'uniform'),
-                 'batched': form_batched(torch, cpu_procs=os.cpu_count() or 1), 'adjoint': form_adjoint(torch),
+                 'batched': form_batched(torch, cpu_procs=0 if missing else os.cpu_count() or 1), 'adjoint': form_adjoint(torch),
                  'assembly': form_assembly(torch)}
     if rank == 0:
         line = {'metric': METRIC, 'value': value, 'unit': UNIT, 'n_gpus': world, 'steps': args.steps,
