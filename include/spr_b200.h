@@ -141,8 +141,8 @@ int spr_b200_set_mode(void* handle, int mode);
  * Default tau = 1e-3; tau = 0 switches the guard and the copy off. */
 int spr_b200_set_inertia_guard(void* handle, double tau);
 /* No reference counterpart.  Watchdog of the kernels that wait on device
- * flags: the tensor-core update kernel's mbarrier waits and the solves'
- * block-ready flags each give up after wait_ns nanoseconds (default 2e9;
+ * flags: the tensor-core update kernels' mbarrier waits and the solves' waits
+ * for the blocks before each give up after wait_ns nanoseconds (default 2e9;
  * 1e6 .. 6e10 accepted); the kernel then returns (the tensor-core one after
  * freeing its tensor memory) and the factorisation or solve returns -4.
  * drop != 0 is a test switch: the first CTA of each tensor-core launch skips
@@ -178,10 +178,11 @@ int spr_b200_build_residual(void* handle, const double* d_sm_assembled);
 int spr_b200_refine(void* handle, const double* d_sm, const double* d_b, double* d_x, int64_t ld,
                     int64_t nrhs, double tol, int maxit, double* out);
 /* Profile mode only: last factorisation's time by phase, out[0..8] = pre-pass,
- * small fronts, extend-add, diagonal blocks, panel TRSM, in-panel/trailing
- * updates, K = S update, write-back, end; last solve's, out[9..19] =
- * forward: small fronts, gather, blocks, rectangles, finish;
- * back: small fronts, gather, rectangles, blocks, (unused), finish (ms).  out holds 20 doubles. */
+ * small fronts, extend-add, panel chain (diagonal blocks; TRSM, the next panel's
+ * columns and the next diagonal block), TRSM of a super-panel's last panel, other
+ * updates of the S columns, K = S update, write-back, end; last solve's, out[9..19] =
+ * forward: small fronts, retained fronts' gathers, triangles, rectangles, 0;
+ * back: small fronts, 0, rectangles, triangles, 0, 0 (ms).  out holds 20 doubles. */
 int spr_b200_phase_ms(void* handle, double* out);
 /* No reference counterpart.  Autotuner of the mixed-precision factorisation:
  * it times candidate choices (which Schur-update launches run on the tensor
@@ -209,9 +210,9 @@ int spr_b200_set_small_tile(void* handle, int tile);
  * sums of 8-bit digit products (1e9 by default; 0: all such trailing and K = S
  * updates, infinity: none). */
 int spr_b200_set_int_min(void* handle, double flops);
-/* Mixed mode: out[0] = algorithmic flops of the Schur updates that run on the
- * tensor cores (trailing columns beyond the next super-panel, K = S updates),
- * out[1] = their split + tensor-core time in the last profiled factor (ms). */
+/* out[0] = algorithmic flops of the Schur updates that run on tcgen05 (mixed mode:
+ * TF32 products; FP64 mode: integer-digit products), out[1] = their split and
+ * product time in the last profiled factor (ms). */
 int spr_b200_tc_stats(void* handle, double* out);
 /* Profile mode: CUDA events around every Schur-update launch. */
 int spr_b200_set_profile(void* handle, int on);
@@ -249,7 +250,7 @@ int spr_b200_schedule_replay(const SPR_INT* mspar, const SPR_INT* mtrees, const 
 /* No reference counterpart.  Host-only self-check of the solves' plan (no GPU
  * needed): each eliminated large front's 64-row triangle blocks are tasks of
  * its level's dataflow launch, once each and after the block above, with
- * disjoint ready flags; each front with F > S has one rectangle job and one
+ * disjoint solved rows; each front with F > S has one rectangle job and one
  * forward-rows job of the right sizes, with disjoint partial-sum ranges.
  * out (5 doubles): [0] rc [1] violations [2] triangle tasks checked [3] and
  * [4] violations with a planted mistake (two blocks of a front swapped; one

@@ -388,13 +388,16 @@ class DeviceSolver:
             raise ValueError('bad flops %r' % (flops,))
 
     def tc_stats(self):
-        """Mixed mode: (tensor-core update flops, their time in the last profiled factor, ms)."""
+        """(Schur-update flops on tcgen05, their time in the last profiled factor, ms):
+        integer-digit products in the FP64 mode, TF32 ones in the mixed mode."""
         out = np.zeros(2)
         self.lib.spr_b200_tc_stats(self.h, _ptr(out))
         return float(out[0]), float(out[1])
 
     def phase_ms(self):
-        """Profile mode: last factorisation's time by phase (ms)."""
+        """Profile mode: last factorisation's and solve's time by phase (ms).  'diag' is the
+        panel chain (diagonal blocks, TRSM, the next panel's columns), 'trsm' that of a
+        super-panel's last panel; 'fwd_finish', 'bwd_gather', 'unused' and 'bwd_finish' stay 0."""
         out = np.zeros(20)
         self.lib.spr_b200_phase_ms(self.h, _ptr(out))
         keys = ('prepass', 'small_fronts', 'extend_add', 'diag', 'trsm', 'updates', 'outer_update',

@@ -1113,10 +1113,10 @@ int SPR_API(spr_b200_set_int_min)(void* handle, double flops) {
     return 0;
 }
 
-// Mixed mode: out[0] = algorithmic flops of the updates that ran on tensor
-// cores in the last profiled factorisation (far trailing columns, the next
-// super-panels' columns and K = S updates above the tensor-core
-// threshold), out[1] = their split + tensor-core time (ms).
+// out[0] = algorithmic flops of the updates that ran on tcgen05 (mixed mode: TF32
+// products, FP64 mode: integer-digit products; far trailing columns, the next
+// super-panels' columns and K = S updates above the mode's threshold), out[1] =
+// their split and product time in the last profiled factorisation (ms).
 int SPR_API(spr_b200_tc_stats)(void* handle, double* out) {
     const Engine* e = static_cast<Engine*>(handle);
     out[0] = e->timing.tc_flops;

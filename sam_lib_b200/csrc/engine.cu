@@ -8,15 +8,19 @@
 //   LMMY18 Schur update ................. lmmy18.f:5-192
 //   SPRFS3/5/6 forward + diagonal ....... sprfs1.f:266-1141
 //   SPRBS4/6 back substitution .......... sprbs1.f:251-574
-// The arithmetic is FP64 throughout; the order of the floating-point updates
-// differs from the reference (blocked, FMA), so results agree to rounding.
+// The arithmetic is FP64, but for large Schur updates: sums of 8-bit digit
+// products whose errors are below those of FP64 multiply-adds (i8_gemm.cuh), or, in
+// the mixed modes, split TF32 products (tc_gemm.cuh, x3).  The order of the
+// floating-point updates differs from the reference (blocked, FMA), so results
+// agree to rounding.
 //
 // Execution: one pass per elimination-tree level (leaves first).  Fronts of
 // order <= kSmallMaxF are assembled, factored and written back by one CTA in
 // shared memory (fused extend-add + LDL' + Schur update).  Larger fronts are
 // assembled into dense column-major buffers in HBM and factored with a
-// blocked right-looking LDL' (diagonal block, panel TRSM, FP64 DMMA Schur
-// update), all fronts of the level batched into each launch.
+// blocked right-looking LDL' (a launch per panel step: TRSM, the next panel's
+// columns, the next diagonal block; DMMA or digit products for the other Schur
+// updates), all fronts of the level batched into each launch.
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <nvtx3/nvToolsExt.h>
@@ -69,7 +73,11 @@ void trace_point(const char* what) {
     } while (0)
 
 constexpr int kMaxRHS = 16;          // right-hand sides per CTA of the small fronts and per residual pass
-constexpr int kPassRHS = 48;         // right-hand sides per pass over the factor
+// Right-hand sides per pass over the factor.  A wider pass reads L less often and
+// fills the chain of a front's blocks better; the work buffers grow with it
+// (48: 3 times those of 16).  96 right-hand sides with 16, 32, 48, 64 and 96 a pass: 12^3 4.5,
+// 2.4, 1.7, 1.7, 1.0 ms; 24^3 13.0, 8.6, 7.2, 7.2, 5.9; 32^3 27.1, 21.4, 19.5, 19.5, 17.6.
+constexpr int kPassRHS = 48;
 
 // NVTX range for the host timeline of a profiler (no-op without one).
 struct NvtxRange {
@@ -155,8 +163,6 @@ struct Engine::Dev {
     double* pbuf = nullptr;                      // rectangle partial sums of the solves
     int32_t* level_nodes = nullptr;              // small nodes of every level, concatenated
     std::vector<int64_t> small_begin;            // per level offset into level_nodes
-    int32_t* all_nodes = nullptr;                // all nodes of every level (solves)
-    std::vector<int64_t> all_begin, all_count;
     // work
     double* arena = nullptr;
     double* adiag = nullptr;
@@ -3396,19 +3402,13 @@ int Engine::open(const int64_t* mspar, const int64_t* mtrees, const int64_t* msi
         return -4;
     CK(cudaMalloc((void**)&D.linv, std::max<int64_t>(P_.linv_doubles, 1) * sizeof(double)));
     o.push_back(D.linv);
-    std::vector<int32_t> small, all;
+    std::vector<int32_t> small;
     D.small_begin.clear();
-    D.all_begin.clear();
-    D.all_count.clear();
     for (const LevelPlan& lp : P_.levels) {
         D.small_begin.push_back((int64_t)small.size());
         small.insert(small.end(), lp.small_nodes.begin(), lp.small_nodes.end());
-        D.all_begin.push_back((int64_t)all.size());
-        all.insert(all.end(), lp.small_nodes.begin(), lp.small_nodes.end());
-        all.insert(all.end(), lp.large_nodes.begin(), lp.large_nodes.end());
-        D.all_count.push_back((int64_t)(lp.small_nodes.size() + lp.large_nodes.size()));
     }
-    if (dev_upload(o, &D.level_nodes, small) || dev_upload(o, &D.all_nodes, all)) return -4;
+    if (dev_upload(o, &D.level_nodes, small)) return -4;
     D.ret = nullptr;
     if (P_.any_retained && dev_upload(o, &D.ret, P_.retained)) return -4;
     CK(cudaMalloc((void**)&D.arena, std::max<int64_t>(P_.arena_doubles, 32) * sizeof(double)));
@@ -3722,7 +3722,10 @@ void Engine::launch_tc(const TcLaunch& t, cudaStream_t s, const PV& pv, std::vec
 
 // The integer-digit form of an update: the panel's digits, then the products.
 void Engine::launch_i8_split(const I8Launch& t, cudaStream_t s, const PV& pv, std::vector<cudaEvent_t>& gev) {
-    if (profile_) gev.push_back(record_event(s));
+    if (profile_) {
+        tc_pairs_.push_back(gev.size());
+        gev.push_back(record_event(s));
+    }
     k_split_i8<<<(int)t.split.ntasks, 256, 0, s>>>(d_->jobs + t.split.job_begin, t.split.job_count, TMAP(t.split), pv,
                                                    d_->i8_slab, d_->i8_scales);
     if (profile_) gev.push_back(record_event(s));
@@ -3732,7 +3735,10 @@ void Engine::launch_i8_split(const I8Launch& t, cudaStream_t s, const PV& pv, st
 void Engine::launch_i8_gemm(const Launch& l, cudaStream_t s, const PV& pv, std::vector<cudaEvent_t>& gev, bool far) {
     if (l.ntasks <= 0) return;
     Dev& D = *d_;
-    if (profile_) gev.push_back(record_event(s));
+    if (profile_) {
+        tc_pairs_.push_back(gev.size());
+        gev.push_back(record_event(s));
+    }
     // a side-stream launch leaves SMs to the panel chain (one CTA holds an SM's shared memory)
     const int cap = (far && !profile_) ? std::max(1, sm_count_ * i8_far_q_ / 8) : sm_count_;
     const int grid = (int)std::min<int64_t>(l.ntasks, cap);
@@ -3981,6 +3987,7 @@ void Engine::enqueue_factor(const PV& pv, cudaStream_t s, std::vector<cudaEvent_
                 // one split serves both column ranges; the slabs are free again
                 // because the previous far update was joined above
                 launch_i8_split(lp.trail_i8[st], s, pv, gev);
+                timing.tc_flops += lp.trail_i8[st].flops;
                 if (has_far && u != s) {
                     cudaEvent_t e = D.evpool[evi++];
                     cudaEventRecord(e, s);
@@ -4044,6 +4051,7 @@ void Engine::enqueue_factor(const PV& pv, cudaStream_t s, std::vector<cudaEvent_
                 if (t.gemm.ntasks > 0) {
                     launch_i8_split(t, s, pv, gev);
                     launch_i8_gemm(t.gemm, s, pv, gev, false);
+                    timing.tc_flops += t.flops;
                 }
                 for (const Launch& ol : t.rest) launch_gemm(ol, s, pv, gev);
             }

@@ -34,16 +34,17 @@ struct FactorResult {
 struct Timing {              // CUDA-event times of the last calls (ms)
     float factor_ms = 0.f, solve_ms = 0.f;
     float gemm_ms = 0.f;     // Schur-update kernels only (sum over launches)
-    float tc_ms = 0.f;       // of those, the split + tensor-core launch pairs
-    double tc_flops = 0.0;   // algorithmic flops of the tensor-core launches enqueued by the last factorisation
+    float tc_ms = 0.f;       // of those, the splits and products on tcgen05 (digits in FP64 mode, TF32 in mixed mode)
+    double tc_flops = 0.0;   // algorithmic flops of those, as enqueued by the last factorisation
     int64_t gemm_launches = 0, launches = 0, solve_launches = 0;
     // profile mode: factor time by phase (CUDA events between launch groups):
-    // 0 pre-pass, 1 small fronts, 2 extend-add, 3 diagonal blocks, 4 panel
-    // TRSM, 5 in-panel/trailing updates, 6 K = S update, 7 write-back, 8 end;
-    // solve: 9 small-front forward, 10 forward gather, 11 forward blocks
-    // (block products and in-block updates), 12 forward rectangles, 13 forward finish, 14 small-front
-    // back, 15 back gather, 16 back rectangles, 17 back blocks (block
-    // products and in-block updates), 18 unused, 19 back finish
+    // 0 pre-pass, 1 small fronts, 2 extend-add, 3 panel chain (diagonal blocks, and
+    // the steps that do TRSM, the next panel's columns and the next diagonal block
+    // in one launch), 4 TRSM of a super-panel's last panel, 5 other updates of the
+    // S columns, 6 K = S update, 7 write-back, 8 end;
+    // solve: 9 small-front forward, 10 retained fronts' gathers, 11 forward
+    // triangles, 12 forward rectangles, 14 small-front back, 16 back rectangles,
+    // 17 back triangles; 13, 15, 18 and 19 stay zero
     float phase_ms[20] = {};
 };
 
@@ -156,7 +157,7 @@ public:
     double last_trace() const { return last_trace_; }
     bool last_refactored() const { return last_refactor_; }
     // Watchdog of the kernels that wait on device flags (the tensor-core
-    // update's mbarriers, the solves' block-ready flags): time limit of each
+    // updates' mbarriers, the values that the solves' blocks hand on): time limit of each
     // wait (ns), and a test switch that makes some waits run out (one CTA's
     // operand load, one solve task's report is skipped); the factorisation or
     // solve then returns -4 and the engine stays usable.
