@@ -38,6 +38,7 @@ UNIT = 'GFLOP/s'
 N_MESH = 48
 NRHS = 4
 SAMPLE_N = 20          # bounded CPU sample: the 20^3 box of the same family
+I8_PRODUCTS = 34       # digit products of an entry of the FP64 update (i8_gemm.cuh)
 
 
 def parse():
@@ -222,9 +223,16 @@ def tf32_peak():
         return 1590.0 / 2.0, 'fallback bf16 1590 TFLOP/s / 2'
 
 
+def int8_peak():
+    """Dense int8 tensor peak: twice the measured bf16 burst rate (tcgen05 kind::i8
+    runs at twice the kind::f16 rate), else twice the fallback bf16 figure."""
+    half, src = tf32_peak()
+    return 4.0 * half, src.replace('/ 2', 'x 2')
+
+
 def read_traffic():
-    """dram bytes per Schur-update flop from the committed ncu summary, if any."""
-    p = os.path.join(ROOT, 'profiles', 'k_gemm_traffic.txt')
+    """dram bytes per Schur-update flop of the digit form from the committed ncu summary, if any."""
+    p = os.path.join(ROOT, 'profiles', 'k_gemm_i8_traffic.txt')
     if not os.path.exists(p):
         return None
     for line in open(p):
@@ -734,7 +742,7 @@ def run_ours(args, rank, world, local_rank):
     # Schur-update launch and between the launch groups of the factorisation
     ds.set_profile(True)
     prof_ms, inf = step(False)
-    gemm_ms = [inf['gemm_ms']]
+    tc_flops, tc_ms = ds.tc_stats()
     phases = ds.phase_ms()
     ds.set_profile(False)
     ms_step = max_over_ranks(float(np.mean(times)), dist, 'cuda')
@@ -775,19 +783,22 @@ def run_ours(args, rank, world, local_rank):
                'copies': {'upload_before_factor_ms': cs[0], 'factor_ms': cs[1], 'download_after_factor_ms': cs[2],
                           'note': 'last step: SM is pinned, so LNZ goes up and comes back level group by level '
                                   'group while the factorisation runs; these are the parts not overlapped'}}
-    peak = dgemm_peak(torch)
-    gemm_s = float(np.mean(gemm_ms)) / 1e3
-    achieved = info['gemm_flops'] / gemm_s / 1e12
+    dgemm = dgemm_peak(torch)
+    peak, peak_src = int8_peak()
     tpf = read_traffic()
-    launches_per_step = inf['gemm_launches']
-    roof = {'bound': 'tensor', 'achieved': achieved, 'peak': peak, 'unit': 'TFLOP/s',
-            'frac': achieved / peak,
-            'traffic': (tpf * info['gemm_flops'] / launches_per_step) if tpf else None,
-            'kernel': 'k_gemm: FP64 Schur update C -= L D L\' (mma.sync m8n8k4 f64)',
-            'flops_per_launch': info['gemm_flops'] / launches_per_step,
-            'peak_source': 'measured in-run: cuBLAS DGEMM 8192^3 via torch.matmul float64 '
-                           '(MEASURED_PEAKS.json has no FP64 figure)',
-            'time_share': gemm_s / (prof_ms / 1e3),
+    tc_s, other_s = tc_ms / 1e3, (inf['gemm_ms'] - tc_ms) / 1e3
+    other_flops = info['gemm_flops'] - tc_flops
+    roof = {'bound': 'tensor', 'achieved': I8_PRODUCTS * tc_flops / tc_s / 1e12 if tc_s else None, 'peak': peak,
+            'unit': 'TOP/s (int8)', 'frac': I8_PRODUCTS * tc_flops / tc_s / 1e12 / peak if tc_s else None,
+            'traffic': tpf * tc_flops if tpf else None,
+            'traffic_note': 'DRAM bytes of all these launches of one factorisation',
+            'kernel': 'k_gemm_i8 with its k_split_i8: FP64 Schur update C -= L D L\' as %d products of 8-bit digits '
+                      '(tcgen05.mma kind::i8)' % I8_PRODUCTS,
+            'flops': tc_flops, 'fp64_equivalent_tflops': tc_flops / tc_s / 1e12 if tc_s else None,
+            'peak_source': peak_src, 'time_share': tc_s / (prof_ms / 1e3),
+            'other_updates': {'kernel': 'k_gemm: the same in FP64 (mma.sync m8n8k4 f64), below the digit form\'s sizes',
+                              'tflops': other_flops / other_s / 1e12 if other_s else None,
+                              'cublas_dgemm_tflops': dgemm, 'time_share': other_s / (prof_ms / 1e3)},
             'timing': 'Schur-update launches timed with CUDA events in one extra profiled step (%.1f ms)' % prof_ms}
     del ds, d_sm0, d_sm, d_b0, d_b
     torch.cuda.empty_cache()
